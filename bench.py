@@ -182,10 +182,10 @@ def kernel_launches(steps, sorts, auto_period):
     """Kernels the tiled 3D/2D MLS step enqueues over `steps` steps with `sorts`
     re-binning sorts: four every step (fused transfer: grid update, the fused
     G2P + next P2G, the queued particles' return map and their P2G; split
-    transfer: P2G, grid update, G2P gather, return map), the four sort kernels
-    (count, scan, bucket, per-tile sort) per sort, and with the auto period the
-    velocity maximum that picks each period's length."""
-    return 4 * steps + (5 if auto_period else 4) * sorts
+    transfer: P2G, grid update, G2P gather, return map), the five sort kernels
+    (count, block sums, scan, bucket, per-tile sort) per sort, and with the auto
+    period the velocity maximum that picks each period's length."""
+    return 4 * steps + (6 if auto_period else 5) * sorts
 
 
 def active_nodes_initial(scene) -> int:

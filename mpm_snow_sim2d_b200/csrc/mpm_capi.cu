@@ -113,7 +113,8 @@ struct mpm_solver {
     // P2G-only prologue).
     bool fused = false;
     bool acc_pending = false;
-    int fused_grid = 0;
+    int fused_grid = 0, windows_grid = 0, direct_grid = 0;
+    bool direct = false;  // few windows: a warp per window, no staged boxes (k_g2p2g_direct)
     bool box_tma = false;  // fused step as the TMA box pipeline (MPM_BOX_LOAD=tma) instead of staged boxes
     CUtensorMap gv_map{};  // the node velocities (vf, wall flag) as a [nz][ny][nx][4] float tensor for TMA
 };
@@ -151,7 +152,8 @@ mpm_status cuda_fail(mpm_solver* s, cudaError_t e, const char* where) {
         if (e_ != cudaSuccess) return cuda_fail((s), e_, #call); \
     } while (0)
 
-int nacc(int dim, int form) { return form == kClassic ? 1 + 2 * dim : 1 + dim; }
+// int64 sums per node (MLS, QUAD: four, one 32-byte sector; see acc_channel)
+int nacc(int dim, int form) { return form == kClassic ? 1 + 2 * dim : 4; }
 
 template <typename T> cudaError_t dalloc(T** p, size_t count) {
     *p = nullptr;
@@ -193,6 +195,11 @@ void release(mpm_solver* s) {
     if (s->q.win) cudaFree(s->q.win);
     if (s->ti.tile_len) cudaFree(s->ti.tile_len);
     if (s->ti.fused_next) cudaFree(s->ti.fused_next);
+    int* more[] = {s->ti.n_items, s->ti.grid_done};
+    for (int* p : more)
+        if (p) cudaFree(p);
+    if (s->ti.items) cudaFree(s->ti.items);
+    if (s->ti.scan) cudaFree(s->ti.scan);
     if (s->own_stream) cudaStreamDestroy(s->own_stream);
 }
 
@@ -254,7 +261,9 @@ template <int D, int S> cudaError_t launch_sort(mpm_solver* s) {
     if (s->n == 0) { s->needs_sort = false; s->next_sort = s->step + s->cur_K; return cudaSuccess; }
     const int threads = 256, blocks = (s->n + threads - 1) / threads;
     k_sort_count<D, S><<<blocks, threads, 0, s->stream>>>(particle_view(s), s->C, s->ti);
-    k_sort_scan<<<1, 1024, 0, s->stream>>>(s->ti);
+    const int scan_blocks = (s->ti.n_tiles + kScanTiles - 1) / kScanTiles;
+    k_sort_block_sums<<<scan_blocks, kScanTiles, 0, s->stream>>>(s->ti);
+    k_sort_scan<<<scan_blocks, kScanTiles, 0, s->stream>>>(s->ti);
     k_sort_bucket<<<blocks, threads, 0, s->stream>>>(s->n, s->ti);
     SortBuffers dst = s->alt;
     if (s->fused) dst.A = nullptr;  // the fused path keeps A only within a step
@@ -416,17 +425,26 @@ template <int D, int S> cudaError_t launch_p2g_tiled(mpm_solver* s) {
 
 // ---- fused transfer ----
 
+// Dynamic shared memory of k_p2g_windows: one window of payloads per warp.
+size_t windows_smem(int dim) {
+    return dim == 3 ? sizeof(FusedSmem<3>::pay) : sizeof(FusedSmem<2>::pay);
+}
+
 // The fused kernel over the tiles of the last sort: G2P (this step) + P2G (next
 // step), or with G2P = false the P2G of the stored state (prologue).
 template <int D, int S, bool G2P> cudaError_t launch_fused(mpm_solver* s) {
-    cudaError_t e = cudaMemsetAsync(s->ti.fused_next, 0, sizeof(int), s->stream);
-    if (e == cudaSuccess && G2P) e = cudaMemsetAsync(s->q.count, 0, 2 * sizeof(int), s->stream);  // count, nwin
-    if (e != cudaSuccess) return e;
+    if (!G2P) {  // the step's grid update clears the counters (k_grid_marked)
+        cudaError_t e = cudaMemsetAsync(s->ti.fused_next, 0, sizeof(int), s->stream);
+        if (e != cudaSuccess) return e;
+    }
     if (s->n == 0) return cudaSuccess;
-    if (G2P && s->box_tma)
+    if (G2P && s->direct)
+        k_g2p2g_direct<D, S><<<s->direct_grid, FusedGeom<D>::THREADS, sizeof(FusedSmem<D>::pay), s->stream>>>(
+            particle_view(s), s->C, s->ti, s->gv, s->acc, s->q, s->status);
+    else if (G2P && s->box_tma)
         k_g2p2g_pipe<D, S><<<s->fused_grid, FusedGeom<D>::THREADS, sizeof(PipeSmem<D>), s->stream>>>(
             particle_view(s), s->C, s->ti, s->gv, s->acc, s->q, s->status, s->gv_map);
-    else
+    else if constexpr (D == 3 || !G2P)
         k_g2p2g<D, S, G2P><<<s->fused_grid, FusedGeom<D>::THREADS, sizeof(FusedSmem<D>), s->stream>>>(
             particle_view(s), s->C, s->ti, s->gv, s->acc, s->q, s->status);
     return cudaGetLastError();
@@ -439,8 +457,8 @@ template <int D, int S> cudaError_t launch_queued_fused(mpm_solver* s) {
     if (s->n == 0) return cudaSuccess;
     cudaError_t e = launch_return_map<D, S>(s);
     if (e != cudaSuccess) return e;
-    k_p2g_windows<D, S><<<s->fused_grid, FusedGeom<D>::THREADS, 0, s->stream>>>(particle_view(s), s->C, s->ti, s->q,
-                                                                                s->acc, s->status);
+    k_p2g_windows<D, S><<<s->windows_grid, FusedGeom<D>::THREADS, windows_smem(D), s->stream>>>(
+        particle_view(s), s->C, s->ti, s->q, s->acc, s->status);
     return cudaGetLastError();
 }
 
@@ -472,7 +490,6 @@ template <int D, int S> cudaError_t step_fused(mpm_solver* s) {
     if (e != cudaSuccess) return e;
     if (sort_due(s) && (e = launch_sort<D, S>(s)) != cudaSuccess) return e;
     if ((e = launch_grid_marked<D>(s)) != cudaSuccess) return e;
-    if ((e = cudaMemsetAsync(s->ti.n_marked, 0, sizeof(int), s->stream)) != cudaSuccess) return e;
     if ((e = launch_fused<D, S, true>(s)) != cudaSuccess) return e;
     return launch_queued_fused<D, S>(s);
 }
@@ -482,8 +499,6 @@ template <int D, int S> cudaError_t step_tiled(mpm_solver* s) {
     cudaError_t e = launch_p2g_tiled<D, S>(s);
     if (e != cudaSuccess) return e;
     e = launch_grid_marked<D>(s);
-    if (e != cudaSuccess) return e;
-    e = cudaMemsetAsync(s->ti.n_marked, 0, sizeof(int), s->stream);
     if (e != cudaSuccess) return e;
     return launch_g2p_split<D, S>(s);
 }
@@ -519,11 +534,7 @@ cudaError_t dispatch_p2g(mpm_solver* s) {
 // After a P2G-only pass: clear accumulators and node-block marks.
 cudaError_t clear_after_p2g(mpm_solver* s) {
     s->acc_pending = false;
-    if (s->tiled) {
-        cudaError_t e = s->dim == 2 ? launch_grid_marked<2>(s) : launch_grid_marked<3>(s);
-        if (e != cudaSuccess) return e;
-        return cudaMemsetAsync(s->ti.n_marked, 0, sizeof(int), s->stream);
-    }
+    if (s->tiled) return s->dim == 2 ? launch_grid_marked<2>(s) : launch_grid_marked<3>(s);
     return cudaMemsetAsync(s->acc, 0, sizeof(unsigned long long) * nacc(s->dim, s->form) * s->nodes, s->stream);
 }
 
@@ -613,8 +624,39 @@ mpm_status setup_tiled(mpm_solver* s) {
         s->p2g_warp_grid = s->sms * per;
     }
     s->q.capacity = n > 0 ? n : 1;
-    // windows of a sort: at most ceil(m / 32) per tile of m slots
-    s->q.win_capacity = s->q.capacity / 32 + ti.n_tiles + 1;
+    {
+        // MPM_TRANSFER=split selects the separate P2G / G2P kernels (for
+        // comparison), MPM_BOX_LOAD=tma node boxes by TMA tensor loads
+        const char* tr = std::getenv("MPM_TRANSFER");
+        s->fused = !(tr && std::strcmp(tr, "split") == 0);
+        const char* bl = std::getenv("MPM_BOX_LOAD");
+        s->box_tma = s->fused && bl && std::strcmp(bl, "tma") == 0;
+    }
+    // Window length of the fused transfer by how the scene's windows compare with
+    // the warps the GPU holds (5 CTAs of 4 per SM): a warp works through a window's
+    // stencils one after the other, so a scene of few windows takes shorter ones.
+    // 2D scenes, the quadratic stencil and 3D scenes of at most six windows per
+    // warp go without staged node boxes, an item per window (k_g2p2g_direct, which
+    // has the figures); else an item is a tile.
+    {
+        const long long warps = (long long)s->sms * (MPM_FUSED_MIN_BLOCKS) * FusedGeom<3>::WARPS;
+        const long long w32 = (n + 31) / 32;
+        ti.win = w32 <= warps / 4 ? 8 : (w32 <= warps / 2 ? 16 : 32);
+        const long long windows = (n + ti.win - 1) / ti.win;
+        s->direct = !s->box_tma && (D == 2 || s->stencil == 3 || windows <= 6 * warps);
+        s->direct_grid = (int)std::max(1ll, std::min((long long)s->sms * (MPM_FUSED_MIN_BLOCKS), windows + ti.n_tiles));
+        ti.item_win = s->direct ? 1 : 0;
+        const size_t most_items = (size_t)ti.n_tiles + (s->direct ? (size_t)n / (size_t)ti.win : 0);
+        if (dalloc(&ti.items, most_items) || dalloc(&ti.n_items, 1) || dalloc(&ti.grid_done, 1) ||
+            dalloc(&ti.scan, (size_t)(ti.n_tiles + kScanTiles - 1) / kScanTiles) ||
+            cudaMemset(ti.grid_done, 0, sizeof(int)) != cudaSuccess ||
+            cudaMemset(ti.n_items, 0, sizeof(int)) != cudaSuccess) {
+            cudaGetLastError();
+            return MPM_ERR_OUT_OF_MEMORY;
+        }
+    }
+    // windows of a sort: at most ceil(m / win) per tile of m slots
+    s->q.win_capacity = s->q.capacity / ti.win + ti.n_tiles + 1;
     if (dalloc(&s->q.list, (size_t)s->q.capacity) || dalloc(&s->q.count, 2) ||
         dalloc(&s->q.fh, (size_t)s->q.capacity * D * D) || dalloc(&s->q.win, (size_t)s->q.win_capacity) ||
         dalloc(&ti.tile_len, (size_t)ti.n_tiles) || dalloc(&ti.fused_next, 1)) {
@@ -622,15 +664,9 @@ mpm_status setup_tiled(mpm_solver* s) {
         return MPM_ERR_OUT_OF_MEMORY;
     }
     s->q.nwin = s->q.count + 1;
-    {
-        // MPM_TRANSFER=split selects the separate P2G / G2P kernels (for comparison)
-        const char* tr = std::getenv("MPM_TRANSFER");
-        s->fused = !(tr && std::strcmp(tr, "split") == 0);
-    }
+    ti.zero[0] = ti.fused_next;
+    ti.zero[1] = s->q.count;
     if (s->fused) {
-        // MPM_BOX_LOAD=tma: node boxes by TMA tensor loads (same results)
-        const char* bl = std::getenv("MPM_BOX_LOAD");
-        s->box_tma = bl && std::strcmp(bl, "tma") == 0;
         const void* kfn;
         size_t fsm, psm;
         const void* kpro;
@@ -646,7 +682,7 @@ mpm_status setup_tiled(mpm_solver* s) {
             if (s->box_tma)
                 kfn = s->stencil == 3 ? (const void*)k_g2p2g_pipe<2, 3> : (const void*)k_g2p2g_pipe<2, 4>;
             else
-                kfn = s->stencil == 3 ? (const void*)k_g2p2g<2, 3, true> : (const void*)k_g2p2g<2, 4, true>;
+                kfn = s->stencil == 3 ? (const void*)k_g2p2g<2, 3, false> : (const void*)k_g2p2g<2, 4, false>;
             kpro = s->stencil == 3 ? (const void*)k_g2p2g<2, 3, false> : (const void*)k_g2p2g<2, 4, false>;
             fsm = s->box_tma ? sizeof(PipeSmem<2>) : sizeof(FusedSmem<2>);
             psm = sizeof(FusedSmem<2>);
@@ -658,6 +694,12 @@ mpm_status setup_tiled(mpm_solver* s) {
             ef = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfn, FusedGeom<3>::THREADS, fsm);
         if (ef != cudaSuccess || per < 1) return MPM_ERR_CUDA;
         s->fused_grid = s->sms * per;
+        const void* kwin = D == 3 ? (s->stencil == 3 ? (const void*)k_p2g_windows<3, 3> : (const void*)k_p2g_windows<3, 4>)
+                                  : (s->stencil == 3 ? (const void*)k_p2g_windows<2, 3> : (const void*)k_p2g_windows<2, 4>);
+        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kwin, FusedGeom<3>::THREADS, windows_smem(D)) !=
+                cudaSuccess || per < 1)
+            return MPM_ERR_CUDA;
+        s->windows_grid = s->sms * per;
         if (s->box_tma) {
             mpm_status em = make_box_map(s);
             if (em != MPM_OK) return em;
@@ -760,22 +802,14 @@ template <int D, int S> cudaError_t stage_tiled(mpm_solver* s, int k) {
         return cudaSuccess;
     }
     if (k == 1) return launch_p2g_tiled_kernel<D, S>(s);
-    if (k == 2) {
-        cudaError_t e = launch_grid_marked<D>(s);
-        if (e != cudaSuccess) return e;
-        return cudaMemsetAsync(s->ti.n_marked, 0, sizeof(int), s->stream);
-    }
+    if (k == 2) return launch_grid_marked<D>(s);
     if (k == 3) return launch_g2p_gather<D, S>(s);
     return launch_return_map<D, S>(s);
 }
 template <int D, int S> cudaError_t stage_fused(mpm_solver* s, int k) {
     if (k == 0) return sort_due(s) ? launch_sort<D, S>(s) : cudaSuccess;
     if (k == 1) return fused_prologue<D, S>(s);
-    if (k == 2) {
-        cudaError_t e = launch_grid_marked<D>(s);
-        if (e != cudaSuccess) return e;
-        return cudaMemsetAsync(s->ti.n_marked, 0, sizeof(int), s->stream);
-    }
+    if (k == 2) return launch_grid_marked<D>(s);
     if (k == 3) return launch_fused<D, S, true>(s);
     return launch_queued_fused<D, S>(s);
 }
@@ -1131,15 +1165,17 @@ mpm_status mpm_rasterize(mpm_solver* s, double* node_mass, double* node_momentum
     const double ism = std::ldexp(1.0, -s->log2_sm), isp = std::ldexp(1.0, -s->log2_sp),
                  isf = std::ldexp(1.0, -s->log2_sf);
     const long long N = s->nodes;
+    const bool classic = s->form == kClassic;
+    auto sum = [&](int c, long long i) { return classic ? h[c * N + i] : h[i * 4 + acc_channel(c)]; };
     for (long long i = 0; i < N; ++i) {
-        if (node_mass) node_mass[i] = (double)h[i] * ism;
+        if (node_mass) node_mass[i] = (double)sum(0, i) * ism;
         for (int k = 0; k < D && node_momentum; ++k) {
-            double p = (double)h[(1 + k) * N + i] * isp;
-            if (s->form == kClassic) p -= (double)s->params.delta_time * ((double)h[(1 + D + k) * N + i] * isf);
+            double p = (double)sum(1 + k, i) * isp;
+            if (classic) p -= (double)s->params.delta_time * ((double)h[(1 + D + k) * N + i] * isf);
             node_momentum[i * D + k] = p;
         }
+        for (int c = 0; raw && c < 1 + D; ++c) raw[c * N + i] = sum(c, i);
     }
-    if (raw) std::memcpy(raw, h.data(), sizeof(long long) * (size_t)(1 + D) * N);
     return MPM_OK;
 }
 
@@ -1244,7 +1280,7 @@ mpm_status mpm_save_state(mpm_solver* s, const char* path) {
     }
     // the pending grid sums of the fused path, block by block
     uint32_t has_sums = 0;
-    int32_t sum_hdr[3] = {nacc(D, s->form), D == 3 ? TileGeom<3>::BN : TileGeom<2>::BN, 0};
+    int32_t sum_hdr[3] = {1 + D, D == 3 ? TileGeom<3>::BN : TileGeom<2>::BN, 0};
     std::vector<int> sum_blocks;
     std::vector<unsigned long long> sums;
     if (has_order && s->fused && s->acc_pending) {
@@ -1360,7 +1396,7 @@ mpm_status mpm_load_state(mpm_solver* s, const char* path) {
         ok = std::fread(&has_sums, 4, 1, f) == 1;
         if (ok && has_sums) {
             const int nb_max = s->ti.n_blocks;
-            ok = std::fread(sum_hdr, 4, 3, f) == 3 && sum_hdr[0] == nacc(s->dim, s->form) &&
+            ok = std::fread(sum_hdr, 4, 3, f) == 3 && sum_hdr[0] == 1 + s->dim &&
                  sum_hdr[1] == (s->dim == 3 ? TileGeom<3>::BN : TileGeom<2>::BN) && sum_hdr[2] >= 0 &&
                  sum_hdr[2] <= nb_max;
             if (ok) {
@@ -1405,7 +1441,16 @@ mpm_status mpm_load_state(mpm_solver* s, const char* path) {
         if (good) {
             const int ntl = (int)tiles.size();
             std::vector<int> tl(ntl), tlen(ntl), tstart(s->ti.n_tiles, 0);
-            for (int e = 0; e < ntl; ++e) { tl[e] = tiles[e].x; tlen[e] = tiles[e].z; tstart[tiles[e].x] = tiles[e].y; }
+            std::vector<int4> items;  // as k_sort_scan lists them
+            const int step = s->ti.item_win ? s->ti.win * s->ti.item_win : (int)n;
+            for (int e = 0; e < ntl; ++e) {
+                tl[e] = tiles[e].x;
+                tlen[e] = tiles[e].z;
+                tstart[tiles[e].x] = tiles[e].y;
+                for (int k = 0; k < tiles[e].z; k += step)
+                    items.push_back(make_int4(tiles[e].x, tiles[e].y + k, std::min(step, tiles[e].z - k), 0));
+            }
+            const int n_items = (int)items.size();
             // on the solver's stream, after the clear of the flags that mpm_set_state queued there
             cudaStream_t st = s->stream;
             MPM_CUDA(s, cudaMemcpyAsync(s->ti.tile_list, tl.data(), sizeof(int) * ntl, cudaMemcpyHostToDevice, st));
@@ -1413,6 +1458,8 @@ mpm_status mpm_load_state(mpm_solver* s, const char* path) {
             MPM_CUDA(s, cudaMemcpyAsync(s->ti.tile_start, tstart.data(), sizeof(int) * s->ti.n_tiles,
                                         cudaMemcpyHostToDevice, st));
             MPM_CUDA(s, cudaMemcpyAsync(s->ti.n_tile_list, &ntl, sizeof(int), cudaMemcpyHostToDevice, st));
+            MPM_CUDA(s, cudaMemcpyAsync(s->ti.items, items.data(), sizeof(int4) * n_items, cudaMemcpyHostToDevice, st));
+            MPM_CUDA(s, cudaMemcpyAsync(s->ti.n_items, &n_items, sizeof(int), cudaMemcpyHostToDevice, st));
             if (has_sums) {
                 // the next step's grid sums as the saved run held them: into the
                 // (cleared) accumulators, their blocks marked for the grid update

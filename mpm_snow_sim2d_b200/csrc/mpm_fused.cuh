@@ -2,38 +2,35 @@
 // one kernel per step (the G2P2G scheme of Wang et al., "A Massively Parallel
 // and Scalable Multi-GPU Material Point Method", ACM TOG 39(4), 2020).
 //
-// One CTA per non-empty cell tile of the last sort (tiles handed out from a
-// counter). The CTA stages the node velocities of a fixed box of BE^D nodes
-// around its tile in shared memory (the stencils of every particle sorted into
-// the tile that has since moved less than a cell): in k_g2p2g all threads load
-// it between two CTA barriers; k_g2p2g_pipe (MPM_BOX_LOAD=tma) instead runs a
-// two-stage pipeline of TMA tensor loads (cp.async.bulk.tensor, out-of-grid
-// nodes zero-filled) with mbarriers and no CTA barrier. Then each warp, on its own,
-// takes windows of 32 consecutive slots of the tile (handed out from a shared
-// counter) and for its window
-//   1. per particle (one lane each): gathers the grid from the box
+// Work is handed out as items. In k_g2p2g an item is a non-empty cell tile of
+// the last sort: a CTA stages the node velocities of a fixed box of BE^D nodes
+// around the tile in shared memory (the stencils of every particle sorted into
+// the tile that has since moved less than a cell), between two CTA barriers;
+// k_g2p2g_pipe (MPM_BOX_LOAD=tma) instead runs a two-stage pipeline of TMA tensor
+// loads (cp.async.bulk.tensor, out-of-grid nodes zero-filled) with mbarriers and
+// no CTA barrier. In k_g2p2g_direct an item is one window and nothing is staged.
+// Each warp, on its own, takes windows of up to 32 consecutive slots of a tile
+// and for its window
+//   1. per particle (one lane each): gathers the grid
 //      (src/gpu/shaders/3d/g2p.glsl:28-71), updates x, v, B and the trial F_E,
 //      and when the return map is provably the identity (elastic band)
 //      computes the next step's P2G affine matrix A = 3 m B - 3 dt V sigma in
 //      registers (3d/p2g.glsl:44-90); the rest are queued for the exact (or
 //      learned) return map with their trial F;
 //   2. writes each in-band particle's P2G payload (stencil weights at the new
-//      position, m v, A) to the warp's shared-memory window, groups
-//      consecutive slots that share a stencil into runs, and SPLIT lanes per
-//      run (longest runs first) sum the run's node contributions in FP32
-//      registers in slot order and add them to the global grid as int64 fixed
-//      point (red.global, no return value).
-// Warps synchronise only per tile (staging the box), so a warp with slow
-// particles or a long run holds up no other. Particles whose stencil leaves
-// the box (drifted more than a cell since the sort) gather from global memory
-// and their runs add bounds-checked. Queued particles (out of the elastic
-// band, or a stencil clipped by the grid edge) are scattered after their
-// return map: the warp records its window (first slot, mask of the queued
-// lanes), and k_p2g_windows repeats the window's run scatter over those lanes.
+//      position, m v, A) to the warp's shared memory, ordered by stencil, and sums
+//      them over the node columns its lanes own, in FP32 registers; what leaves
+//      the registers goes to the grid as int64 fixed point (red.global, no
+//      return value): scatter_rows.
+// Particles whose stencil leaves the box (drifted more than a cell since the
+// sort) gather from global memory. Queued particles (out of the elastic band, or
+// a stencil clipped by the grid edge) are scattered after their return map: the
+// warp records its window (first slot, mask of the queued lanes), and
+// k_p2g_windows repeats the scatter over those lanes.
 //
-// Determinism: every cross-run sum is an integer add, and the runs are a
-// function of the slot order, the window boundaries (fixed offsets inside a
-// tile) and which particles were queued -- all functions of the state. After
+// Determinism: every sum beyond one window is an integer add, and the FP32 sums
+// in it are a function of the slot order, the window boundaries (fixed offsets
+// inside a tile) and which particles were queued -- all functions of the state. After
 // creation or a state upload a P2G-only pass of the same kernel (reading the
 // stored state) forms the first sums. A checkpoint stores the pending sums
 // themselves, so a resumed run never recomputes them.
@@ -56,18 +53,15 @@ template <int D> struct FusedGeom {
     static constexpr int THREADS = MPM_FUSED_THREADS;
     static constexpr int WARPS = THREADS / 32;
     static constexpr int WIN = 32;                      // slots per warp window (one per lane)
-    static constexpr int PS = D == 3 ? 40 : 20;         // payload floats per particle (layout: p2g_payload)
-    static constexpr int KEYF = PS - 2;                 // payload floats holding the 64-bit stencil key
+    static constexpr int PS = 44;                       // payload floats per particle (layout: Scatter)
     static_assert(THREADS % 32 == 0, "whole warps");
 };
 
 template <int D> struct FusedSmem {
     using G = FusedGeom<D>;
     float4 box[G::BN];                                  // 3D: (vf, wall flag); 2D: (vf, vc)
-    int tile_next;                                      // tile-list entry of the CTA's current tile
+    int tile_next;                                      // item of the CTA's current tile
     float4 pay[G::WARPS][G::WIN * G::PS / 4];           // per warp: the window's P2G payloads
-    int run[G::WARPS][G::WIN + 1];                      // per warp: start slot of each run, then the window end
-    int order[G::WARPS][G::WIN];                        // per warp: runs, longest first
     int next_win;                                       // next window of the tile to hand out
     unsigned bmask;                                     // node blocks (3^D around the tile) that received sums
 };
@@ -84,7 +78,9 @@ template <int D> struct FusedSmem {
 // memory (SMEM) or the global grid. Same sums and order as gather_interior.
 // `gc0`, `gsy`, `gsz`: the global node id of the first stencil node and the
 // global strides, for the wall-velocity pass (3D vc of nodes a wall moved is
-// only kept in global memory).
+// only kept in global memory). That pass reads it for the flagged nodes alone,
+// a whole x plane of them in flight at once: the 128^3 snowball scene, whose
+// slab rests on the floor, took 56 of 332 us for it with four loads in flight.
 template <int D, int S, bool SMEM, typename I>
 __device__ __forceinline__ void gather_nodes(const StepConsts& C, const float4* nodes, I c0, I sy, I sz,
                                              const float4* __restrict__ gv, long long gc0, long long gsy, long long gsz,
@@ -154,17 +150,18 @@ __device__ __forceinline__ void gather_nodes(const StepConsts& C, const float4* 
 #pragma unroll 1
             for (int a = 0; a < S; ++a) {
                 float Qc[3] = {0.f, 0.f, 0.f};
-#pragma unroll 1
+#pragma unroll
                 for (int b = 0; b < S; ++b) {
                     float Pc[3] = {0.f, 0.f, 0.f};
 #pragma unroll
                     for (int c = 0; c < S; ++c) {
-                        float f[3], g[3];
-                        load_node3(gv, C.nodes, gc0 + a + b * gsy + c * gsz, f, g);
+                        const I cid = c0 + a + b * sy + c * sz;
+                        float4 g = SMEM ? nodes[cid] : __ldg(&nodes[cid]);
+                        if (g.w != 0.f) g = __ldg(&gv[C.nodes + gc0 + a + b * gsy + c * gsz]);
                         const float z = wk[2][c];
-                        Pc[0] += z * g[0]; Pc[1] += z * g[1]; Pc[2] += z * g[2];
+                        Pc[0] += z * g.x; Pc[1] += z * g.y; Pc[2] += z * g.z;
                     }
-                    const float y = pick<S>(wk[1], b);  // loop index not unrolled: no local array
+                    const float y = wk[1][b];
 #pragma unroll
                     for (int r = 0; r < 3; ++r) Qc[r] += y * Pc[r];
                 }
@@ -191,352 +188,417 @@ __device__ __forceinline__ void gather_nodes(const StepConsts& C, const float4* 
 }
 
 // ---------------------------------------------------------------------------
-// P2G payload of one particle at position x; the 64-bit stencil key goes in
-// the last two floats. f = x - (base + 1) is the offset in the particle's cell.
-//   3D (40): wx[4] | wy[4] | wz[4] | yd[4] | zd[4] | s0 s1 m s2 |
-//            A00 A10 0 A20 | A01 A11 0 A21 | A02 A12 0 A22 | pad pad key
-//            with yd[b] = wy[b] (b - 1 - fy), zd[c] = wz[c] (c - 1 - fz),
-//            s_r = m v_r - fx A_r0: the momentum channels in pairs (0, 1) and
-//            (mass, 2) for the packed FP32 accumulation of fused_run.
-//   2D (20): wx[4] | wy[4] | fx fy m mv0 | mv1 A00 A01 A10 | A11 pad key
-template <int D, int S>
-__device__ __forceinline__ unsigned long long p2g_payload(const StepConsts& C, const float* x, const float* v,
-                                                          const float* A, float mass, float* q) {
-    using St = Stencil<S>;
-    unsigned long long k3 = 0;
-    float f[3], mv[3];
-#pragma unroll
-    for (int k = D - 1; k >= 0; --k) {
-        const int extk = k == 0 ? C.W : (k == 1 ? C.H : C.Dp);
-        const int base = St::base(x[k], extk);
-        float wt[S];
-        St::weights(x[k], base, wt);
-#pragma unroll
-        for (int o = 0; o < 4; ++o) q[4 * k + o] = o < S ? wt[o] : 0.f;
-        f[k] = x[k] - float(base + 1);
-        mv[k] = mass * v[k];
-        k3 |= (unsigned long long)(base + 9) << (StencilKey<D>::BITS * k);
-    }
-    if constexpr (D == 3) {
-#pragma unroll
-        for (int o = 0; o < 4; ++o) {
-            q[12 + o] = q[4 + o] * (float(o - 1) - f[1]);
-            q[16 + o] = q[8 + o] * (float(o - 1) - f[2]);
-        }
-        reinterpret_cast<float4*>(q)[5] = make_float4(mv[0] - f[0] * A[0], mv[1] - f[0] * A[3], mass, mv[2] - f[0] * A[6]);
-        reinterpret_cast<float4*>(q)[6] = make_float4(A[0], A[3], 0.f, A[6]);
-        reinterpret_cast<float4*>(q)[7] = make_float4(A[1], A[4], 0.f, A[7]);
-        reinterpret_cast<float4*>(q)[8] = make_float4(A[2], A[5], 0.f, A[8]);
-    } else {
-        reinterpret_cast<float4*>(q)[2] = make_float4(f[0], f[1], mass, mv[0]);
-        reinterpret_cast<float4*>(q)[3] = make_float4(mv[1], A[0], A[1], A[2]);
-        q[16] = A[3];
-        q[17] = 0.f;
-    }
-    return k3;
-}
+// P2G of one warp's window of 32 slots.
+//
+// The window's particles are ordered by stencil (lowest node id first) in the
+// warp's shared memory; the warp then walks that order as a whole. Every lane
+// owns one node column of the stencil (3D: offsets (b, c) in y and z; 2D: offset
+// b in y and one channel pair) and holds the column's S nodes in x in registers;
+// the warp sums G particles at a time. Cells are sorted x fastest, so the next
+// stencil is mostly one node further in x: then only the node plane that falls
+// out of the stencil is added to the grid, and the others go on accumulating.
+//
+// Bound: the shared-memory and reduction pipe (a 16-byte shared load costs 2.7
+// cycles whether its lanes read one row or four, a red.global 20 to 26) and
+// instruction issue. The former layout (SPLIT lanes per run of one stencil, each
+// holding 8 nodes x 4 channels, every run adding all S^D nodes) sent 2.5 times
+// the int64 adds and let lanes wait for the longest run.
+//
+// Payload of one particle (floats):
+//   wx[4] | per b: wy yd | 3D, per c: wz zd | 3D: s0 s1 m s2, A00 A10 0 A20,
+//   A01 A11 0 A21, A02 A12 0 A22; 2D: s0 s1 A00 A10, m 0 0 0, A01 A11, 0 0 |
+//   its stencil: key, particles sharing it
+// with yd = wy (b - 1 - fy), zd = wz (c - 1 - fz), s_r = m v_r - fx A_r0 and
+// f = x - (base + 1). The rows are 44 floats apart: 16-byte accesses of eight
+// neighbouring rows then fall into distinct banks.
+template <int D, int S> struct Scatter {
+    static constexpr int PS = 44;                          // floats per row
+    static constexpr int Y = 4, Z = 12, M = D == 3 ? 20 : 12;
+    static constexpr int INFO = D == 3 ? 36 : 24;          // key, count
+    // particles at a time (lanes of one: 3D 16, its 4 x 4 node columns, of which
+    // the quadratic stencil uses 3 x 3; 2D 8, four columns times two channel
+    // pairs) and channel pairs per lane
+    static constexpr int G = D == 3 ? 2 : 4, PAIRS = D == 3 ? 2 : 1;
+};
 
-// ---------------------------------------------------------------------------
-// One work item of the run accumulation: split `a` of the run [j0, j1) of a
-// warp's payload window `pay`, stencil key kk. Sums in registers in slot
-// order and adds them to the global grid as int64 fixed point. When `boxed`
-// and the whole stencil lies in the tile's node box (origin bo) and in the
-// grid, the adds need no bounds checks and the function returns the node
-// blocks they touched, as bits of the 3^D blocks around the tile (tile
-// coordinates tc); otherwise the adds are bounds-checked, the node blocks
-// marked here, and it returns 0. Same arithmetic as k_p2g_warp.
+// Stencil keys: the node id of the stencil's first node (node ids stay below
+// 2e9, validate_params); kClipped when part of the stencil is outside the grid
+// (scatter_clipped does those); kNoKey for a lane with no row.
+constexpr int kNoKey = -1, kClipped = 0x7fffffff;
+
 template <int D, int S>
-__device__ __forceinline__ unsigned fused_run(const StepConsts& C, const TileInfo& TI, const float4* pay, bool boxed,
-                                              const int* bo, const int* tc, int j0, int j1, unsigned long long kk,
-                                              int a, unsigned long long* __restrict__ acc,
-                                              unsigned* __restrict__ status) {
-    using G = FusedGeom<D>;
-    using W = WarpGeom<D, S>;
-    constexpr int T = TileGeom<D>::T;
-    const float* payf = reinterpret_cast<const float*>(pay);
-    int cell[3] = {0, 0, 0};
-#pragma unroll
-    for (int k = 0; k < D; ++k) cell[k] = int((kk >> (StencilKey<D>::BITS * k)) & StencilKey<D>::MASK) - 8;
-    // stencil nodes cell - 1 .. cell + S - 2 per axis
-    bool in_box = boxed, in_grid = true;
-    const int ext[3] = {C.W, C.H, C.Dp};
+__device__ __forceinline__ int stencil_key(const StepConsts& C, const float* x, int* base) {
+    bool interior = true;
 #pragma unroll
     for (int k = 0; k < D; ++k) {
-        in_box = in_box && cell[k] - 1 - bo[k] >= 0 && cell[k] + S - 2 - bo[k] <= G::BE - 1;
-        in_grid = in_grid && cell[k] - 1 >= 0 && cell[k] + S - 2 <= ext[k];
+        const int ext = k == 0 ? C.W : (k == 1 ? C.H : C.Dp);
+        base[k] = Stencil<S>::base(x[k], ext);
+        interior = interior && base[k] >= 0 && base[k] + (S - 1) <= ext;
     }
+    if (!interior) return kClipped;
+    return ((D == 3 ? base[2] * C.ny : 0) + base[1]) * C.nx + base[0];
+}
+
+// Row of this lane's particle in the window's order, and the number of
+// particles sharing its stencil; `total` gets the window's particle count.
+// Whole warp.
+__device__ __forceinline__ int window_row(int key, int* count, bool* first, int* total) {
+    const int lane = threadIdx.x & 31;
+    const unsigned peers = __match_any_sync(0xffffffffu, key);
+    const unsigned before = peers & ((1u << lane) - 1);
+    *first = key != kNoKey && before == 0u;
+    *count = __popc(peers);
+    *total = __popc(__ballot_sync(0xffffffffu, key != kNoKey));
+    int row = __popc(before);
+    for (unsigned m = __ballot_sync(0xffffffffu, *first); m; m &= m - 1) {
+        const int l = __ffs(m) - 1;
+        const int kl = __shfl_sync(0xffffffffu, key, l), cl = __shfl_sync(0xffffffffu, *count, l);
+        row += kl < key ? cl : 0;
+    }
+    return row;
+}
+
+template <int D, int S>
+__device__ __forceinline__ void write_payload(const StepConsts& C, const float* x, const int* base, const float* v,
+                                              const float* A, float mass, int key, int count, bool first, float* q) {
+    using L = Scatter<D, S>;
+    float f[3], w[3][4];
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+        w[k][3] = 0.f;
+        Stencil<S>::weights(x[k], base[k], w[k]);
+        f[k] = x[k] - float(base[k] + 1);
+    }
+    float4* q4 = reinterpret_cast<float4*>(q);
+    q4[0] = make_float4(w[0][0], w[0][1], w[0][2], w[0][3]);
+#pragma unroll
+    for (int o = 0; o < S; o += 2) {
+        q4[(L::Y + 2 * o) / 4] = make_float4(w[1][o], w[1][o] * (float(o - 1) - f[1]), w[1][o + 1],
+                                             w[1][o + 1] * (float(o) - f[1]));
+        if constexpr (D == 3)
+            q4[(L::Z + 2 * o) / 4] = make_float4(w[2][o], w[2][o] * (float(o - 1) - f[2]), w[2][o + 1],
+                                                 w[2][o + 1] * (float(o) - f[2]));
+    }
+    const float s0 = mass * v[0] - f[0] * A[0], s1 = mass * v[1] - f[0] * A[D];
     if constexpr (D == 3) {
-        constexpr int NB = S * S / W::SPLIT;
-        constexpr int NN = NB * S;
-        const int ax = a % S, by0 = (a / S) * NB;
-        // channel pairs (a0, a1) and (am, a2) per node, in packed FP32
-        // (fma.rn.f32x2: two FP32 FMAs per instruction)
-        float2 p01[NN], pm2[NN];
-#pragma unroll
-        for (int k = 0; k < NN; ++k) { p01[k] = make_float2(0.f, 0.f); pm2[k] = make_float2(0.f, 0.f); }
-        const float2 da2 = make_float2(float(ax - 1), float(ax - 1));
-        for (int j = j0; j < j1; ++j) {
-            const float4* pp = pay + j * (G::PS / 4);
-            const float alpha = payf[j * G::PS + ax];
-            const float2 al2 = make_float2(alpha, alpha);
-            const float4 wy = pp[1], wz = pp[2], yd = pp[3], zd = pp[4], p5 = pp[5], p6 = pp[6], p7 = pp[7],
-                         p8 = pp[8];
-            // (e0, e1) = alpha (s0 + da A00, s1 + da A10); (ma, e2) = alpha (m, s2 + da A20)
-            const float2 e01 = __fmul2_rn(al2, __ffma2_rn(da2, make_float2(p6.x, p6.y), make_float2(p5.x, p5.y)));
-            const float2 me2 = __fmul2_rn(al2, __ffma2_rn(da2, make_float2(p6.z, p6.w), make_float2(p5.z, p5.w)));
-            const float2 f01 = __fmul2_rn(al2, make_float2(p7.x, p7.y)), f_2 = __fmul2_rn(al2, make_float2(p7.z, p7.w));
-            const float2 g01 = __fmul2_rn(al2, make_float2(p8.x, p8.y)), g_2 = __fmul2_rn(al2, make_float2(p8.z, p8.w));
-            const float Z[4] = {wz.x, wz.y, wz.z, wz.w};
-            const float Zd[4] = {zd.x, zd.y, zd.z, zd.w};
-            const float Yv[4] = {wy.x, wy.y, wy.z, wy.w};
-            const float Ydv[4] = {yd.x, yd.y, yd.z, yd.w};
-            float2 Z2[S], Zd2[S];
-#pragma unroll
-            for (int cc = 0; cc < S; ++cc) { Z2[cc] = make_float2(Z[cc], Z[cc]); Zd2[cc] = make_float2(Zd[cc], Zd[cc]); }
-#pragma unroll
-            for (int bb = 0; bb < NB; ++bb) {
-                const int b = by0 + bb;
-                const float Y = NB == S ? Yv[bb] : (b == 0 ? wy.x : b == 1 ? wy.y : b == 2 ? wy.z : wy.w);
-                const float Yd = NB == S ? Ydv[bb] : (b == 0 ? yd.x : b == 1 ? yd.y : b == 2 ? yd.z : yd.w);
-                const float2 Y2 = make_float2(Y, Y), Yd2 = make_float2(Yd, Yd);
-                // (h0, h1), (mY, h2): h_r = e_r Y + f_r Yd, mY = ma Y; (k0, k1), (0, k2): k_r = g_r Y
-                const float2 h01 = __ffma2_rn(e01, Y2, __fmul2_rn(f01, Yd2));
-                const float2 hm2 = __ffma2_rn(me2, Y2, __fmul2_rn(f_2, Yd2));
-                const float2 k01 = __fmul2_rn(g01, Y2), k_2 = __fmul2_rn(g_2, Y2);
-#pragma unroll
-                for (int cc = 0; cc < S; ++cc) {
-                    const int idx = bb * S + cc;
-                    p01[idx] = __ffma2_rn(h01, Z2[cc], __ffma2_rn(k01, Zd2[cc], p01[idx]));
-                    pm2[idx] = __ffma2_rn(hm2, Z2[cc], __ffma2_rn(k_2, Zd2[cc], pm2[idx]));
-                }
-            }
-        }
-        float am[NN], a0[NN], a1[NN], a2[NN];
-#pragma unroll
-        for (int k = 0; k < NN; ++k) { am[k] = pm2[k].x; a2[k] = pm2[k].y; a0[k] = p01[k].x; a1[k] = p01[k].y; }
-        float mx_m = 0.f, mx_p = 0.f;
-#pragma unroll
-        for (int k = 0; k < NN; ++k) {
-            mx_m = fmaxf(mx_m, fabsf(am[k]));
-            mx_p = fmaxf(mx_p, fmaxf(fabsf(a0[k]), fmaxf(fabsf(a1[k]), fabsf(a2[k]))));
-        }
-        if (!(mx_m * C.sm < kFixedLimit && mx_p * C.sp < kFixedLimit))
-            raise_flag(status, (mx_m != mx_m || mx_p != mx_p) ? 1u : 2u);
-        const int gx = cell[0] - 1 + ax;
-        if (in_box && in_grid) {
-            const long long sy = C.nx, sz = (long long)C.nx * C.ny;
-            const long long g0 = ((long long)(cell[2] - 1) * C.ny + (cell[1] - 1 + by0)) * C.nx + gx;
-#pragma unroll
-            for (int bb = 0; bb < NB; ++bb)
-#pragma unroll
-                for (int cc = 0; cc < S; ++cc) {
-                    const int idx = bb * S + cc;
-                    unsigned long long* p0 = acc + (g0 + bb * sy + cc * sz);
-                    red_fixed(p0, am[idx], C.sm);
-                    red_fixed(p0 + C.nodes, a0[idx], C.sp);
-                    red_fixed(p0 + 2 * C.nodes, a1[idx], C.sp);
-                    red_fixed(p0 + 3 * C.nodes, a2[idx], C.sp);
-                }
-            // blocks of the thread's nodes: one x block, a y range, a z range
-            // (all within one block of the tile's, since the stencil is in the box)
-            unsigned bits = 0u;
-            const int rx = gx / T - tc[0] + 1;
-            const int y0 = (cell[1] - 1 + by0) / T - tc[1] + 1, y1 = (cell[1] - 2 + by0 + NB) / T - tc[1] + 1;
-            const int z0 = (cell[2] - 1) / T - tc[2] + 1, z1 = (cell[2] + S - 2) / T - tc[2] + 1;
-            for (int rz = z0; rz <= z1; ++rz)
-                for (int ry = y0; ry <= y1; ++ry) bits |= 1u << ((rz * 3 + ry) * 3 + rx);
-            return bits;
-        }
-        bool outside = false;
-        for (int bb = 0; bb < NB; ++bb)
-            for (int cc = 0; cc < S; ++cc) {
-                const int gy = cell[1] - 1 + by0 + bb, gz = cell[2] - 1 + cc;
-                if (gx < 0 || gx > C.W || gy < 0 || gy > C.H || gz < 0 || gz > C.Dp) { outside = true; continue; }
-                const int idx = bb * S + cc;
-                unsigned long long* p0 = acc + (((long long)gz * C.ny + gy) * C.nx + gx);
-                red_fixed(p0, am[idx], C.sm);
-                red_fixed(p0 + C.nodes, a0[idx], C.sp);
-                red_fixed(p0 + 2 * C.nodes, a1[idx], C.sp);
-                red_fixed(p0 + 3 * C.nodes, a2[idx], C.sp);
-            }
-        if (outside) raise_flag(status, 4u);
-        if (gx >= 0 && gx <= C.W) {
-            const int y0 = max(0, cell[1] - 1 + by0), y1 = min(C.H, cell[1] - 2 + by0 + NB);
-            const int z0 = max(0, cell[2] - 1), z1 = min(C.Dp, cell[2] + (S - 2));
-            if (y0 <= y1 && z0 <= z1)
-                for (int bz = z0 / T; bz <= z1 / T; ++bz)
-                    for (int by = y0 / T; by <= y1 / T; ++by)
-                        mark_block_once(TI, (bz * TI.nblk[1] + by) * TI.nblk[0] + gx / T);
-        }
-        return 0u;
+        q4[L::M / 4] = make_float4(s0, s1, mass, mass * v[2] - f[0] * A[6]);
+        q4[L::M / 4 + 1] = make_float4(A[0], A[3], 0.f, A[6]);
+        q4[L::M / 4 + 2] = make_float4(A[1], A[4], 0.f, A[7]);
+        q4[L::M / 4 + 3] = make_float4(A[2], A[5], 0.f, A[8]);
     } else {
-        constexpr int NA = S / W::SPLIT;
-        const int gx0 = cell[0] - 1 + a * NA;
-        float am[NA * S], a0[NA * S], a1[NA * S];
-#pragma unroll
-        for (int k = 0; k < NA * S; ++k) { am[k] = 0.f; a0[k] = 0.f; a1[k] = 0.f; }
-        for (int j = j0; j < j1; ++j) {
-            const float4* pp = pay + j * (G::PS / 4);
-            const float4 wx = pp[0], wy = pp[1], p2 = pp[2], p3 = pp[3];
-            const float a11 = payf[j * G::PS + 16];
-            // f = (p2.x, p2.y), m = p2.z, mv = (p2.w, p3.x), A = (p3.y p3.z | p3.w a11)
-            const float Xv[4] = {wx.x, wx.y, wx.z, wx.w};
-            const float Y[4] = {wy.x, wy.y, wy.z, wy.w};
-            float Yd[4];
-#pragma unroll
-            for (int b = 0; b < S; ++b) Yd[b] = Y[b] * (float(b - 1) - p2.y);
-#pragma unroll
-            for (int i = 0; i < NA; ++i) {
-                const int aa = a * NA + i;
-                const float X = NA == S ? Xv[i] : payf[j * G::PS + aa];
-                const float Xd = X * (float(aa - 1) - p2.x);
-                const float e0 = p2.w * X + p3.y * Xd, e1 = p3.x * X + p3.w * Xd;
-                const float f0 = p3.z * X, f1 = a11 * X, mX = p2.z * X;
-#pragma unroll
-                for (int b = 0; b < S; ++b) {
-                    const int idx = i * S + b;
-                    am[idx] += mX * Y[b];
-                    a0[idx] += e0 * Y[b] + f0 * Yd[b];
-                    a1[idx] += e1 * Y[b] + f1 * Yd[b];
-                }
-            }
-        }
-        float mx_m = 0.f, mx_p = 0.f;
-#pragma unroll
-        for (int k = 0; k < NA * S; ++k) {
-            mx_m = fmaxf(mx_m, fabsf(am[k]));
-            mx_p = fmaxf(mx_p, fmaxf(fabsf(a0[k]), fabsf(a1[k])));
-        }
-        if (!(mx_m * C.sm < kFixedLimit && mx_p * C.sp < kFixedLimit))
-            raise_flag(status, (mx_m != mx_m || mx_p != mx_p) ? 1u : 2u);
-        if (in_box && in_grid) {
-            const long long g0 = (long long)(cell[1] - 1) * C.nx + gx0;
-#pragma unroll
-            for (int i = 0; i < NA; ++i)
-#pragma unroll
-                for (int b = 0; b < S; ++b) {
-                    const int idx = i * S + b;
-                    unsigned long long* p0 = acc + (g0 + i + (long long)b * C.nx);
-                    red_fixed(p0, am[idx], C.sm);
-                    red_fixed(p0 + C.nodes, a0[idx], C.sp);
-                    red_fixed(p0 + 2 * C.nodes, a1[idx], C.sp);
-                }
-            unsigned bits = 0u;
-            const int x0 = gx0 / T - tc[0] + 1, x1 = (gx0 + NA - 1) / T - tc[0] + 1;
-            const int y0 = (cell[1] - 1) / T - tc[1] + 1, y1 = (cell[1] + S - 2) / T - tc[1] + 1;
-            for (int ry = y0; ry <= y1; ++ry)
-                for (int rx = x0; rx <= x1; ++rx) bits |= 1u << (ry * 3 + rx);
-            return bits;
-        }
-        bool outside = false;
-        for (int i = 0; i < NA; ++i)
-            for (int b = 0; b < S; ++b) {
-                const int gx = gx0 + i, gy = cell[1] - 1 + b;
-                if (gx < 0 || gx > C.W || gy < 0 || gy > C.H) { outside = true; continue; }
-                const int idx = i * S + b;
-                unsigned long long* p0 = acc + ((long long)gy * C.nx + gx);
-                red_fixed(p0, am[idx], C.sm);
-                red_fixed(p0 + C.nodes, a0[idx], C.sp);
-                red_fixed(p0 + 2 * C.nodes, a1[idx], C.sp);
-            }
-        if (outside) raise_flag(status, 4u);
-        const int x0 = max(0, gx0), x1 = min(C.W, gx0 + (NA - 1));
-        const int y0 = max(0, cell[1] - 1), y1 = min(C.H, cell[1] + (S - 2));
-        if (x0 <= x1 && y0 <= y1)
-            for (int by = y0 / T; by <= y1 / T; ++by)
-                for (int bx = x0 / T; bx <= x1 / T; ++bx) mark_block_once(TI, by * TI.nblk[0] + bx);
-        return 0u;
+        q4[L::M / 4] = make_float4(s0, s1, A[0], A[2]);
+        q4[L::M / 4 + 1] = make_float4(mass, 0.f, 0.f, 0.f);
+        q4[L::M / 4 + 2] = make_float4(A[1], A[3], 0.f, 0.f);
+    }
+    if (first) *reinterpret_cast<int2*>(q + L::INFO) = make_int2(key, count);
+}
+
+// One lane's share of a window: the S node planes of its column as channel
+// pairs (momentum x, y; mass, momentum z), the largest scaled sum so far (range
+// check) and where and how it adds to the grid.
+template <int D, int S> struct ScatterLane {
+    float2 a[S][Scatter<D, S>::PAIRS];
+    float top;
+    unsigned long long* at;  // first node column and channel the lane adds to, at node 0
+    int at2;                 // its second add, relative to the first
+    float scale0, scale1;
+    int b, c, h, g;          // column, channel pair (2D), particle group
+    bool on, both;           // adds anything; its second sum too
+};
+
+// The lane's two sums of one node plane at `node` to the grid.
+template <int D, int S>
+__device__ __forceinline__ void add_sums(ScatterLane<D, S>& T, long long node, float2 v) {
+    unsigned long long* p = T.at + node * 4;
+    const float t0 = v.x * T.scale0, t1 = v.y * T.scale1;
+    T.top = fmaxf(T.top, fmaxf(fabsf(t0), fabsf(t1)));
+    red_scaled(p, t0);
+    if (T.both) red_scaled(p + T.at2, t1);
+}
+
+__device__ __forceinline__ float2 shfl_xor2(float2 v, int m) {
+    return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
+}
+
+// One node plane `v` (x = node's) to the grid.
+template <int D, int S>
+__device__ __forceinline__ void add_plane(ScatterLane<D, S>& T, long long node, const float2* v) {
+    if constexpr (D == 3) {
+        // the two groups' sums, one channel pair left to each; then neighbouring
+        // columns (b, b ^ 1) swap so that a lane holds one channel of both: each
+        // add then covers whole 32-byte nodes (four lanes a node), which the memory
+        // pipe takes in 19.7 cycles a warp against 25.7 for half nodes
+        float2 keep = T.g ? v[1] : v[0];
+        const float2 got = shfl_xor2(T.g ? v[0] : v[1], 16);
+        keep.x += got.x;
+        keep.y += got.y;
+        const float other = __shfl_xor_sync(0xffffffffu, T.b & 1 ? keep.x : keep.y, 1);
+        if (T.on) add_sums<D, S>(T, node, T.b & 1 ? make_float2(other, keep.y) : make_float2(keep.x, other));
+    } else {
+        // the four groups' sums of one node
+        float2 u = v[0];
+        float2 got = shfl_xor2(u, 16);
+        u.x += got.x;
+        u.y += got.y;
+        got = shfl_xor2(u, 8);
+        u.x += got.x;
+        u.y += got.y;
+        if (T.on && T.g == 0) add_sums<D, S>(T, node, u);
     }
 }
 
-// ---------------------------------------------------------------------------
-// The scatter of one warp's window of payloads (`pay`, the stencil key in the
-// last two floats of each; kNoStencil for slots that add nothing): runs of
-// consecutive slots with one key, longest first, SPLIT lanes per run summing
-// it (fused_run). The first `cnt` slots of the window are filled. Returns this
-// lane's node-block bits (boxed runs only).
+// A stencil that starts `ahead` (1 .. S) nodes further in x: the planes before
+// it go to the grid, the others move up.
 template <int D, int S>
-__device__ __forceinline__ unsigned scatter_window(const StepConsts& C, const TileInfo& TI, const float4* pay,
-                                                   int* run, int* order, int cnt, bool boxed, const int* bo,
-                                                   const int* tc, unsigned long long* __restrict__ acc,
-                                                   unsigned* __restrict__ status) {
-    using G = FusedGeom<D>;
-    using W = WarpGeom<D, S>;
-    const int lane = threadIdx.x & 31;
-    const bool valid = lane < cnt;
-    // runs: maximal stretches of consecutive slots with one stencil key
-    const unsigned long long* keyp = reinterpret_cast<const unsigned long long*>(
-        reinterpret_cast<const float*>(pay) + G::KEYF);
-    auto key_at = [&](int j) { return keyp[j * (G::PS / 2)]; };
-    const bool is_start = valid && (lane == 0 || key_at(lane) != key_at(lane - 1));
-    const unsigned starts = __ballot_sync(0xffffffffu, is_start);
-    const int nruns = __popc(starts);
-    const int r_me = __popc(starts & ((1u << lane) - 1));
-    if (is_start) run[r_me] = lane;
-    if (lane == 0) run[nruns] = cnt;
-    __syncwarp();
-    // runs longest first, so that the SPLIT-lane groups sharing a pass have
-    // similar lengths; which lanes sum a run changes no result
-    {
-        const int len = lane < nruns ? run[lane + 1] - run[lane] : 0;
-        int rank = 0;
-        for (int qr = 0; qr < nruns; ++qr) {
-            const int lq = __shfl_sync(0xffffffffu, len, qr);
-            rank += lq > len || (lq == len && qr < lane);
+__device__ __forceinline__ void move_planes(ScatterLane<D, S>& T, long long node, int ahead) {
+#pragma unroll 1
+    for (int n = 0; n < ahead; ++n) {
+        add_plane<D, S>(T, node + n, T.a[0]);
+#pragma unroll
+        for (int p = 0; p < Scatter<D, S>::PAIRS; ++p) {
+#pragma unroll
+            for (int a = 0; a + 1 < S; ++a) T.a[a][p] = T.a[a + 1][p];
+            T.a[S - 1][p] = make_float2(0.f, 0.f);
         }
-        if (lane < nruns) order[rank] = lane;
+    }
+}
+
+// 2D: all S planes to the grid; clears them. The four groups sum each others'
+// planes and are left with one each. (3D adds them with move_planes: unrolled
+// they cost more in instruction fetch than the register moves they save, 320
+// -> 332 us on the 128^3 snowball scene.)
+template <int D, int S>
+__device__ __forceinline__ void add_planes(ScatterLane<D, S>& T, long long node) {
+    if constexpr (D == 2) {
+        float2 v[4], k[2];
+#pragma unroll
+        for (int a = 0; a < 4; ++a) v[a] = a < S ? T.a[a][0] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            k[i] = T.g & 2 ? v[2 + i] : v[i];
+            const float2 got = shfl_xor2(T.g & 2 ? v[i] : v[2 + i], 16);
+            k[i].x += got.x;
+            k[i].y += got.y;
+        }
+        float2 u = T.g & 1 ? k[1] : k[0];
+        const float2 got = shfl_xor2(T.g & 1 ? k[0] : k[1], 8);
+        u.x += got.x;
+        u.y += got.y;
+        if (T.on && T.g < S) add_sums<D, S>(T, node + T.g, u);
+#pragma unroll
+        for (int a = 0; a < S; ++a) T.a[a][0] = make_float2(0.f, 0.f);
+    }
+}
+
+// Adds one particle's plane values  wx_a (P + (a - 1) Q)  of a channel pair.
+template <int D, int S>
+__device__ __forceinline__ void sum_pair(ScatterLane<D, S>& T, int p, const float2* x, float2 P, float2 Q) {
+    T.a[0][p] = __ffma2_rn(x[0], __fadd2_rn(P, make_float2(-Q.x, -Q.y)), T.a[0][p]);
+    T.a[1][p] = __ffma2_rn(x[1], P, T.a[1][p]);
+    P = __fadd2_rn(P, Q);
+    T.a[2][p] = __ffma2_rn(x[2], P, T.a[2][p]);
+    if constexpr (S == 4) T.a[3][p] = __ffma2_rn(x[3], __fadd2_rn(P, Q), T.a[3][p]);
+}
+
+// The particle rows [0, count) at q, all of one stencil, into the planes.
+template <int D, int S>
+__device__ __forceinline__ void sum_rows(ScatterLane<D, S>& T, const float* q, int count) {
+    using L = Scatter<D, S>;
+    constexpr int G = L::G;
+    q += T.g * L::PS;
+    for (int j = T.g; j < count; j += G, q += G * L::PS) {
+        const float4* q4 = reinterpret_cast<const float4*>(q);
+        const float4 w = q4[0];
+        const float2 x[4] = {make_float2(w.x, w.x), make_float2(w.y, w.y), make_float2(w.z, w.z), make_float2(w.w, w.w)};
+        const float2 wy = *reinterpret_cast<const float2*>(q + L::Y + 2 * T.b);
+        if constexpr (D == 3) {
+            const float2 wz = *reinterpret_cast<const float2*>(q + L::Z + 2 * T.c);
+            const float yz_ = wy.x * wz.x, ydz_ = wy.y * wz.x, yzd_ = wy.x * wz.y;
+            const float2 yz = make_float2(yz_, yz_), ydz = make_float2(ydz_, ydz_), yzd = make_float2(yzd_, yzd_);
+            const float4 s = q4[L::M / 4], a0 = q4[L::M / 4 + 1], a1 = q4[L::M / 4 + 2], a2 = q4[L::M / 4 + 3];
+            sum_pair<D, S>(T, 0, x,
+                           __ffma2_rn(yzd, make_float2(a2.x, a2.y),
+                                      __ffma2_rn(ydz, make_float2(a1.x, a1.y), __fmul2_rn(yz, make_float2(s.x, s.y)))),
+                           __fmul2_rn(yz, make_float2(a0.x, a0.y)));
+            sum_pair<D, S>(T, 1, x,
+                           __ffma2_rn(yzd, make_float2(a2.z, a2.w),
+                                      __ffma2_rn(ydz, make_float2(a1.z, a1.w), __fmul2_rn(yz, make_float2(s.z, s.w)))),
+                           __fmul2_rn(yz, make_float2(a0.z, a0.w)));
+        } else {
+            const float4 sa = q4[L::M / 4 + T.h];
+            const float2 a1 = *reinterpret_cast<const float2*>(q + L::M + 8 + 2 * T.h);
+            const float2 y = make_float2(wy.x, wy.x), yd = make_float2(wy.y, wy.y);
+            sum_pair<D, S>(T, 0, x, __ffma2_rn(yd, a1, __fmul2_rn(y, make_float2(sa.x, sa.y))),
+                               __fmul2_rn(y, make_float2(sa.z, sa.w)));
+        }
     }
     __syncwarp();
-    unsigned bits = 0u;
-    for (int u = lane; u < nruns * W::SPLIT; u += 32) {
-        const int r = order[u / W::SPLIT], a = u % W::SPLIT;
-        const int j0 = run[r], j1 = run[r + 1];
-        const unsigned long long kk = key_at(j0);
-        if (kk == kNoStencil) continue;
-        bits |= fused_run<D, S>(C, TI, pay, boxed, bo, tc, j0, j1, kk, a, acc, status);
+}
+
+// P2G of a particle part of whose stencil is outside the grid, by one lane: its
+// nodes inside the grid one by one, and their blocks.
+template <int D, int S>
+__device__ __forceinline__ void scatter_clipped(const StepConsts& C, const TileInfo& TI, const float* x, const int* base,
+                                                const float* v, const float* A, float mass,
+                                                unsigned long long* __restrict__ acc, unsigned* __restrict__ status) {
+    constexpr int TE = TileGeom<D>::T;
+    float top = 0.f;
+#pragma unroll 1
+    for (int j = 0; j < (D == 3 ? S * S * S : S * S); ++j) {
+        const int gx = base[0] + j % S, gy = base[1] + (j / S) % S, gz = D == 3 ? base[2] + j / (S * S) : 0;
+        if (gx < 0 || gx > C.W || gy < 0 || gy > C.H || (D == 3 && (gz < 0 || gz > C.Dp))) continue;
+        const float d[3] = {float(gx) - x[0], float(gy) - x[1], D == 3 ? float(gz) - x[D - 1] : 0.f};
+        float w = Stencil<S>::w(d[0]) * Stencil<S>::w(d[1]);
+        if (D == 3) w *= Stencil<S>::w(d[2]);
+        unsigned long long* n = acc + (((long long)gz * C.ny + gy) * C.nx + gx) * 4;
+        const float m = w * mass * C.sm;
+        red_scaled(n + 2, m);
+        top = fmaxf(top, fabsf(m));
+#pragma unroll
+        for (int r = 0; r < D; ++r) {
+            float s = mass * v[r];
+#pragma unroll
+            for (int k = 0; k < D; ++k) s += A[r * D + k] * d[k];
+            s *= w * C.sp;
+            red_scaled(n + (r < 2 ? r : 3), s);
+            top = fmaxf(top, fabsf(s));
+        }
+        mark_block_once(TI, ((D == 3 ? gz / TE : 0) * TI.nblk[1] + gy / TE) * TI.nblk[0] + gx / TE);
     }
-    __syncwarp();  // the window's payload and runs are reused by the next window
+    raise_flag(status, top < kFixedLimit ? 4u : 4u | 2u);
+}
+
+// The ordered rows of a window (`total` of them) into the grid. Whole warp.
+template <int D, int S>
+__device__ __forceinline__ void scatter_rows(const StepConsts& C, const float* pay, int total,
+                                             unsigned long long* __restrict__ acc, unsigned* __restrict__ status) {
+    using L = Scatter<D, S>;
+    const int lane = threadIdx.x & 31;
+    ScatterLane<D, S> T;
+    int col = 0, ch = 0;  // of the lane's first add
+    T.b = lane & 3;
+    if constexpr (D == 3) {
+        T.c = (lane >> 2) & 3;
+        T.g = lane >> 4;
+        T.h = 0;
+        T.on = T.c < S;
+        // one channel of columns b & ~1 and b | 1 (add_plane)
+        ch = 2 * T.g + (T.b & 1);
+        col = T.c * C.ny + (T.b & 2);
+        T.at2 = 4 * C.nx;
+        T.both = (T.b | 1) < S;
+        T.scale0 = T.scale1 = ch == 2 ? C.sm : C.sp;
+    } else {
+        T.c = 0;
+        T.h = (lane >> 2) & 1;
+        T.g = lane >> 3;
+        T.on = T.b < S;
+        ch = 2 * T.h;
+        col = T.b;
+        T.at2 = 1;
+        T.both = T.h == 0;
+        T.scale0 = T.h == 0 ? C.sp : C.sm;
+        T.scale1 = C.sp;
+    }
+    T.top = 0.f;
+    T.at = acc + (long long)col * C.nx * 4 + ch;
+#pragma unroll
+    for (int a = 0; a < S; ++a)
+#pragma unroll
+        for (int p = 0; p < L::PAIRS; ++p) T.a[a][p] = make_float2(0.f, 0.f);
+    int at = kNoKey;  // first node of the planes
+    for (int j = 0; j <= total;) {
+        const int2 info = j < total ? *reinterpret_cast<const int2*>(pay + j * L::PS + L::INFO) : make_int2(kNoKey, 1);
+        // stencils in the grid whose node ids differ by less than S are in one row
+        const int ahead = info.x - at;
+        if (at != kNoKey) {
+            if constexpr (D == 3) {
+                move_planes<D, S>(T, at, ahead > 0 ? min(ahead, S) : S);
+            } else {
+                if (ahead > 0 && ahead < S) move_planes<D, S>(T, at, ahead);
+                else add_planes<D, S>(T, at);
+            }
+        }
+        at = info.x;
+        if (j < total) sum_rows<D, S>(T, pay + j * L::PS, info.y);
+        j += info.y;
+    }
+    if (!(T.top < kFixedLimit)) raise_flag(status, 2u);
+    __syncwarp();  // the rows are reused by the next window
+}
+
+// Marks the node blocks of a stencil (all of it in the grid).
+template <int D, int S>
+__device__ __forceinline__ void mark_stencil(const TileInfo& TI, const int* base) {
+    constexpr int TE = TileGeom<D>::T;
+    const int x0 = base[0] / TE, x1 = (base[0] + S - 1) / TE, y0 = base[1] / TE, y1 = (base[1] + S - 1) / TE;
+    const int z0 = D == 3 ? base[2] / TE : 0, z1 = D == 3 ? (base[2] + S - 1) / TE : 0;
+    for (int bz = z0; bz <= z1; ++bz)
+        for (int by = y0; by <= y1; ++by)
+            for (int bx = x0; bx <= x1; ++bx) mark_block_once(TI, (bz * TI.nblk[1] + by) * TI.nblk[0] + bx);
+}
+
+// The node blocks of a stencil as bits of the 3^D blocks around the tile whose
+// node box starts at bo (2 nodes before the tile); the stencil lies in the box.
+template <int D, int S>
+__device__ __forceinline__ unsigned stencil_block_bits(const int* base, const int* bo) {
+    constexpr int TE = TileGeom<D>::T;
+    unsigned m[3] = {1u, 1u, 1u};
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+        const int r = base[k] - bo[k] + TE - 2;  // from the first node of the block before the tile
+        m[k] = (1u << (r / TE)) | (1u << ((r + S - 1) / TE));
+    }
+    unsigned bits = m[0] * ((m[1] & 1u) | (m[1] & 2u) << 2 | (m[1] & 4u) << 4);
+    if constexpr (D == 3) bits *= (m[2] & 1u) | (m[2] & 2u) << 8 | (m[2] & 4u) << 16;
     return bits;
 }
 
 // P2G of the queued particles after their return map, by the windows the
 // fused kernel recorded: one warp per window, the window's queued slots
-// (x, v, A as the G2P and return-map kernels left them) grouped into runs of
-// one stencil and summed as in the fused kernel. The grouping is a function
-// of the window and of which of its particles were queued, so the int64 sums
-// do not depend on the order in which windows were recorded.
+// (x, v, A as the G2P and return-map kernels left them) scattered as in the
+// fused kernel. The order inside a window is a function of its queued
+// particles, so the int64 sums do not depend on the order in which windows were
+// recorded. The fused kernel has marked the node blocks of every queued particle
+// whose new position it knew; the others (rec.z) are marked here.
 template <int D, int S>
 __global__ void __launch_bounds__(FusedGeom<D>::THREADS) k_p2g_windows(Particles P, StepConsts C, TileInfo TI,
                                                                       SlowQueue Q,
                                                                       unsigned long long* __restrict__ acc,
                                                                       unsigned* __restrict__ status) {
     using G = FusedGeom<D>;
-    __shared__ float4 pay_s[G::WARPS][G::WIN * G::PS / 4];
-    __shared__ int run_s[G::WARPS][G::WIN + 1];
-    __shared__ int order_s[G::WARPS][G::WIN];
+    using L = Scatter<D, S>;
+    extern __shared__ __align__(128) unsigned char fused_smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float* pay = reinterpret_cast<float*>(fused_smem) + wid * (G::WIN * L::PS);
     const int nw = min(*Q.nwin, Q.win_capacity);
     const int n = P.n;
-    const int none[3] = {0, 0, 0};
-    float4* pay = pay_s[wid];
     for (int r = blockIdx.x * G::WARPS + wid; r < nw; r += gridDim.x * G::WARPS) {
-        const int2 rec = Q.win[r];
-        const unsigned mask = (unsigned)rec.y;
-        if ((mask >> lane) & 1u) {
-            // the queued slots packed in slot order, so that particles of one
-            // cell form one run even when in-band ones sat between them
-            float* q = reinterpret_cast<float*>(pay) + __popc(mask & ((1u << lane) - 1)) * G::PS;
+        const int4 rec = Q.win[r];
+        const bool queued = ((unsigned)rec.y >> lane) & 1u;
+        int key = kNoKey, base[3] = {0, 0, 0};
+        float mass = 0.f, x[D], v[D], A[D * D];
+        if (queued) {
             const int i = rec.x + lane;
-            const float mass = P.mass ? P.mass[i] : P.mass_u;
-            float x[D], v[D], A[D * D];
+            mass = P.mass ? P.mass[i] : P.mass_u;
 #pragma unroll
             for (int k = 0; k < D; ++k) { x[k] = P.x[k * n + i]; v[k] = P.v[k * n + i]; }
 #pragma unroll
             for (int k = 0; k < D * D; ++k) A[k] = P.A[k * n + i];
-            reinterpret_cast<unsigned long long*>(q + G::KEYF)[0] = p2g_payload<D, S>(C, x, v, A, mass, q);
+            key = stencil_key<D, S>(C, x, base);
+            if (key == kClipped) {
+                scatter_clipped<D, S>(C, TI, x, base, v, A, mass, acc, status);
+                key = kNoKey;
+            } else if (((unsigned)rec.z >> lane) & 1u) {
+                mark_stencil<D, S>(TI, base);
+            }
         }
+        int count, total;
+        bool first;
+        const int row = window_row(key, &count, &first, &total);
+        if (key != kNoKey) write_payload<D, S>(C, x, base, v, A, mass, key, count, first, pay + row * L::PS);
         __syncwarp();
-        scatter_window<D, S>(C, TI, pay, run_s[wid], order_s[wid], __popc(mask), false, none, none, acc, status);
+        scatter_rows<D, S>(C, pay, total, acc, status);
     }
 }
 
@@ -613,28 +675,30 @@ __device__ __forceinline__ void tile_origin(const TileInfo& TI, int t, int* tc, 
 // Window w (slots start + 32 w ...) of a tile of m slots, by one warp: G2P of
 // each slot's particle against the tile's node box (G2P = true) or the stored
 // state (G2P = false), then the scatter of the in-band particles' payloads.
-// Returns this lane's node-block bits of the tile (tile coordinates tc, box
-// origin bo).
-template <int D, int S, bool G2P>
+// Returns this lane's node-block bits around the tile (box origin bo). DIRECT:
+// there is no staged box, every particle gathers from the global grid.
+template <int D, int S, bool G2P, bool DIRECT = false>
 __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepConsts& C, const TileInfo& TI,
                                                  const float4* __restrict__ gv, unsigned long long* __restrict__ acc,
                                                  const SlowQueue& Q, unsigned* __restrict__ status, const float4* box,
-                                                 const int* bo, const int* tc, int start, int m, int w, float4* pay,
-                                                 int* run, int* order) {
+                                                 const int* bo, int start, int m, int win, int w, float* pay) {
     using G = FusedGeom<D>;
+    using L = Scatter<D, S>;
     using St = Stencil<S>;
     const int lane = threadIdx.x & 31;
     const int n = P.n;
     const long long gsy = C.nx, gsz = (long long)C.nx * C.ny;
-    const int cnt = min(G::WIN, m - w * G::WIN);
+    const int cnt = min(win, m - w * win);
     const bool valid = lane < cnt;
-    const int i = start + w * G::WIN + lane;
-    unsigned long long key = kNoStencil;
-    bool deferred = false;  // queued: scattered after the return map (k_p2g_windows)
-    float* q = reinterpret_cast<float*>(pay) + lane * G::PS;
+    const int i = start + w * win + lane;
+    int key = kNoKey, nbase[3] = {0, 0, 0};
+    bool deferred = false;   // queued: scattered after the return map (k_p2g_windows)
+    bool unmarked = false;   // queued with its whole G2P: new position not known here
+    unsigned bits = 0u;
+    float mass = 0.f, x[D], v[D], A[D * D];
     if (valid) {
-        const float mass = P.mass ? P.mass[i] : P.mass_u, vol = P.vol ? P.vol[i] : P.vol_u;
-        float x[D], v[D], A[D * D];
+        const float vol = P.vol ? P.vol[i] : P.vol_u;
+        mass = P.mass ? P.mass[i] : P.mass_u;
         bool scatter = vol != 0.f;  // p2g.glsl:42
         if constexpr (G2P) {
             float xo[D];
@@ -656,12 +720,12 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
             if (!interior) {
                 // stencil partly outside the grid: the general kernel does the whole G2P
                 Q.list[queue_slot(Q)] = -1 - i;
-                deferred = scatter;
+                deferred = unmarked = scatter;
                 scatter = false;
             } else {
                 float nv[D], nx[D], nB[D * D];
                 const long long gc0 = (D == 3 ? base[2] * gsz : 0) + base[1] * gsy + base[0];
-                if (boxed) {
+                if (!DIRECT && boxed) {
                     const int l0 = (D == 3 ? (base[2] - bo[2]) * G::BE * G::BE : 0) + (base[1] - bo[1]) * G::BE +
                                    (base[0] - bo[0]);
                     gather_nodes<D, S, true, int>(C, box, l0, G::BE, G::BE * G::BE, gv, gc0, gsy, gsz, wk, off,
@@ -720,19 +784,41 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
             for (int k = 0; k < D * D; ++k) { B[k] = P.B[k * n + i]; Fe[k] = P.Fe[k * n + i]; }
             mls_affine<D, S>(C, B, Fe, P.Jp[i], mass, vol, A);
         }
-        if (scatter) key = p2g_payload<D, S>(C, x, v, A, mass, q);
+        // the new stencil, and its node blocks (of queued particles too: their
+        // return map leaves the position alone)
+        if (scatter || (deferred && !unmarked)) {
+            const int k = stencil_key<D, S>(C, x, nbase);
+            if (k != kClipped) {
+                bool boxed = true;
+#pragma unroll
+                for (int d = 0; d < D; ++d)
+                    boxed = boxed && nbase[d] - bo[d] >= 0 && nbase[d] + (S - 1) - bo[d] <= G::BE - 1;
+                if (boxed) bits = stencil_block_bits<D, S>(nbase, bo);
+                else mark_stencil<D, S>(TI, nbase);
+                if (scatter) key = k;
+            } else if (scatter) {
+                scatter_clipped<D, S>(C, TI, x, nbase, v, A, mass, acc, status);
+            }
+        }
     }
     if constexpr (G2P) {
         // record the window if some of its particles wait for the return map
         const unsigned dm = __ballot_sync(0xffffffffu, deferred);
-        if (dm && lane == 0) {
-            const int r = atomicAdd(Q.nwin, 1);
-            if (r < Q.win_capacity) Q.win[r] = make_int2(start + w * G::WIN, (int)dm);
+        if (dm) {
+            const unsigned um = __ballot_sync(0xffffffffu, unmarked);
+            if (lane == 0) {
+                const int r = atomicAdd(Q.nwin, 1);
+                if (r < Q.win_capacity) Q.win[r] = make_int4(start + w * win, (int)dm, (int)um, 0);
+            }
         }
     }
-    reinterpret_cast<unsigned long long*>(q + G::KEYF)[0] = key;
+    int count, total;
+    bool first;
+    const int row = window_row(key, &count, &first, &total);
+    if (key != kNoKey) write_payload<D, S>(C, x, nbase, v, A, mass, key, count, first, pay + row * L::PS);
     __syncwarp();
-    return scatter_window<D, S>(C, TI, pay, run, order, cnt, true, bo, tc, acc, status);
+    scatter_rows<D, S>(C, pay, total, acc, status);
+    return bits;
 }
 
 // ---------------------------------------------------------------------------
@@ -748,11 +834,9 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
     extern __shared__ __align__(128) unsigned char fused_smem[];
     FusedSmem<D>& SM = *reinterpret_cast<FusedSmem<D>*>(fused_smem);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int ntl = *TI.n_tile_list;
+    const int nitems = *TI.n_items;
     const long long gsy = C.nx, gsz = (long long)C.nx * C.ny;
-    float4* pay = SM.pay[wid];
-    int* run = SM.run[wid];
-    int* order = SM.order[wid];
+    float* pay = reinterpret_cast<float*>(SM.pay[wid]);
     for (;;) {
         if (tid == 0) {
             SM.tile_next = atomicAdd(TI.fused_next, 1);
@@ -761,10 +845,9 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
         }
         __syncthreads();
         const int e = SM.tile_next;
-        if (e >= ntl) break;
-        const float4* box = SM.box;
-        const int t = TI.tile_list[e];
-        const int start = TI.tile_start[t], m = TI.tile_len[e];
+        if (e >= nitems) break;
+        const int4 item = TI.items[e];  // tile, first slot, slots
+        const int t = item.x, start = item.y, m = item.z;
         int tc[3] = {0, 0, 0}, bo[3] = {0, 0, 0};  // tile coordinates, box origin node
         tile_origin<D>(TI, t, tc, bo);
         if constexpr (G2P) {  // stage the node velocities of the box
@@ -793,13 +876,13 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
             __syncthreads();
         }
         unsigned bits = 0u;  // node blocks this lane's in-box runs added to
-        const int nwin = (m + G::WIN - 1) / G::WIN;
+        const int nwin = (m + TI.win - 1) / TI.win;
         for (;;) {
             int w = 0;
             if (lane == 0) w = atomicAdd(&SM.next_win, 1);
             w = __shfl_sync(0xffffffffu, w, 0);
             if (w >= nwin) break;
-            bits |= fused_window<D, S, G2P>(P, C, TI, gv, acc, Q, status, box, bo, tc, start, m, w, pay, run, order);
+            bits |= fused_window<D, S, G2P>(P, C, TI, gv, acc, Q, status, SM.box, bo, start, m, TI.win, w, pay);
         }
         // mark the node blocks the tile's in-box runs added to
         bits = __reduce_or_sync(0xffffffffu, bits);
@@ -812,6 +895,40 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
             mark_block_once(TI, (bz * TI.nblk[1] + by) * TI.nblk[0] + bx);
         }
         __syncthreads();  // SM.bmask, the tile and the box are reset for the next tile
+    }
+}
+
+// ---------------------------------------------------------------------------
+// The fused step without staged boxes: an item is one window, every warp takes
+// windows on its own and gathers from the global grid. All 2D scenes, the
+// quadratic stencil, and 3D scenes of few windows per warp. A staged box costs two CTA barriers around a
+// round trip to L2 and saves less than that where a stencil is 16 nodes of L1-
+// resident rows (2D, 627k particles: 74.6 us staged, 45.7 direct) or a tile has
+// few particles (3D, 17.6k at 0.6 per cell: 30.5 and 20.6; 474k at 8 per cell:
+// 103.8 and 98.6), and its 27 nodes make the quadratic stencil gain as well (1.65M
+// particles: 257 and 246). The 64-node stencils of a large 3D scene read a box
+// many times over (1.65M particles: 300 staged, 350 direct).
+template <int D, int S>
+__global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
+    k_g2p2g_direct(Particles P, StepConsts C, TileInfo TI, const float4* __restrict__ gv,
+                   unsigned long long* __restrict__ acc, SlowQueue Q, unsigned* __restrict__ status) {
+    using G = FusedGeom<D>;
+    constexpr int NBLK = D == 3 ? 27 : 9;
+    extern __shared__ __align__(128) unsigned char fused_smem[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float* pay = reinterpret_cast<float*>(fused_smem) + wid * (G::WIN * G::PS);
+    const int nitems = *TI.n_items;
+    for (int e = wid * gridDim.x + blockIdx.x; e < nitems; e += G::WARPS * gridDim.x) {
+        const int4 item = TI.items[e];
+        int tc[3] = {0, 0, 0}, bo[3] = {0, 0, 0};
+        tile_origin<D>(TI, item.x, tc, bo);
+        const unsigned bits = __reduce_or_sync(
+            0xffffffffu, fused_window<D, S, true, true>(P, C, TI, gv, acc, Q, status, nullptr, bo, item.y, item.z, TI.win,
+                                                        0, pay));
+        if (lane < NBLK && (bits >> lane) & 1u) {
+            const int bx = tc[0] - 1 + lane % 3, by = tc[1] - 1 + (lane / 3) % 3, bz = D == 3 ? tc[2] - 1 + lane / 9 : 0;
+            mark_block_once(TI, (bz * TI.nblk[1] + by) * TI.nblk[0] + bx);
+        }
     }
 }
 
@@ -833,25 +950,23 @@ template <int D> struct PipeSmem {
     using G = FusedGeom<D>;
     alignas(128) float4 box[2][G::BNP];                 // (vf, wall flag) per node
     unsigned long long full[2];                         // the stage's box arrived (or the stage is empty)
-    int tile[2];                                        // tile-list entry of the stage (>= count: empty)
+    int tile[2];                                        // item of the stage (>= count: empty)
     int next_win[2];
     int left[2];                                        // warps done with the stage
     unsigned bmask[2];
     float4 pay[G::WARPS][G::WIN * G::PS / 4];
-    int run[G::WARPS][G::WIN + 1];
-    int order[G::WARPS][G::WIN];
 };
 
 // Stage for buffer b: the next tile of the global counter and its box load,
 // or an empty stage. One thread.
 template <int D>
-__device__ __forceinline__ void pipe_refill(PipeSmem<D>& SM, int b, const TileInfo& TI, int ntl,
+__device__ __forceinline__ void pipe_refill(PipeSmem<D>& SM, int b, const TileInfo& TI, int nitems,
                                             const CUtensorMap& map) {
     const int e = atomicAdd(TI.fused_next, 1);
     SM.tile[b] = e;
-    if (e < ntl) {
+    if (e < nitems) {
         int tc[3], bo[3];
-        tile_origin<D>(TI, TI.tile_list[e], tc, bo);
+        tile_origin<D>(TI, TI.items[e].x, tc, bo);
         fence_proxy_async_smem();
         box_load<D>(map, bo, SM.box[b], &SM.full[b]);
     } else {
@@ -869,7 +984,7 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
     extern __shared__ __align__(128) unsigned char fused_smem[];
     PipeSmem<D>& SM = *reinterpret_cast<PipeSmem<D>*>(fused_smem);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int ntl = *TI.n_tile_list;
+    const int nitems = *TI.n_items;
     if (tid == 0) {
         for (int b = 0; b < 2; ++b) {
             mbar_init(&SM.full[b], 1);
@@ -878,8 +993,8 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
             SM.bmask[b] = 0u;
         }
         mbar_init_fence();
-        pipe_refill<D>(SM, 0, TI, ntl, gv_map);
-        pipe_refill<D>(SM, 1, TI, ntl, gv_map);
+        pipe_refill<D>(SM, 0, TI, nitems, gv_map);
+        pipe_refill<D>(SM, 1, TI, nitems, gv_map);
     }
     __syncthreads();
     for (int k = 0;; ++k) {
@@ -894,20 +1009,20 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
             return;
         }
         const int e = SM.tile[b];
-        if (e >= ntl) break;
-        const int t = TI.tile_list[e];
-        const int start = TI.tile_start[t], m = TI.tile_len[e];
+        if (e >= nitems) break;
+        const int4 item = TI.items[e];  // tile, first slot, slots
+        const int t = item.x, start = item.y, m = item.z;
         int tc[3] = {0, 0, 0}, bo[3] = {0, 0, 0};
         tile_origin<D>(TI, t, tc, bo);
-        const int nwin = (m + G::WIN - 1) / G::WIN;
+        const int nwin = (m + TI.win - 1) / TI.win;
         unsigned bits = 0u;
         for (;;) {
             int w = 0;
             if (lane == 0) w = atomicAdd(&SM.next_win[b], 1);
             w = __shfl_sync(0xffffffffu, w, 0);
             if (w >= nwin) break;
-            bits |= fused_window<D, S, true>(P, C, TI, gv, acc, Q, status, SM.box[b], bo, tc, start, m, w,
-                                             SM.pay[wid], SM.run[wid], SM.order[wid]);
+            bits |= fused_window<D, S, true>(P, C, TI, gv, acc, Q, status, SM.box[b], bo, start, m, TI.win, w,
+                                             reinterpret_cast<float*>(SM.pay[wid]));
         }
         bits = __reduce_or_sync(0xffffffffu, bits);
         int last = 0;
@@ -932,7 +1047,7 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
                 SM.bmask[b] = 0u;
                 SM.next_win[b] = 0;
                 SM.left[b] = 0;
-                pipe_refill<D>(SM, b, TI, ntl, gv_map);
+                pipe_refill<D>(SM, b, TI, nitems, gv_map);
             }
             __syncwarp();
         }

@@ -7,7 +7,9 @@
 //   x[D][n], v[D][n], B[D*D][n], Fe[D*D][n], Jp[n]
 //   mass/vol: per particle or a uniform scalar (pointer == nullptr)
 // Grid (nodes = (W+1)(H+1)(D+1), x fastest):
-//   acc[NACC][nodes]  int64 fixed-point sums: mass, momentum[D] (+ force[D] CLASSIC)
+//   acc  int64 fixed-point sums. MLS, QUAD: [nodes][4] = momentum x, momentum y,
+//        mass, momentum z (2D: unused), a node's sums in one 32-byte sector;
+//        CLASSIC: [channel][nodes] = mass, momentum[D], force[D]
 //   gv                node velocities for G2P: 2D float4 (vf.x, vf.y, vc.x, vc.y);
 //                     3D two float4 per node (vf.xyz, 0), (vc.xyz, 0)
 #pragma once
@@ -349,10 +351,23 @@ __device__ __forceinline__ void grid_node_at(const StepConsts& C, unsigned long 
                                              int ix, int iy, int iz) {
     constexpr int NACC = Layout<D, FORM>::NACC;
     long long q[NACC];
+    if constexpr (FORM == kClassic) {
 #pragma unroll
-    for (int c = 0; c < NACC; ++c) {
-        q[c] = (long long)acc[c * C.nodes + id];
-        if (q[c] != 0) acc[c * C.nodes + id] = 0ull;
+        for (int c = 0; c < NACC; ++c) {
+            q[c] = (long long)acc[c * C.nodes + id];
+            if (q[c] != 0) acc[c * C.nodes + id] = 0ull;
+        }
+    } else {
+        longlong2* a = reinterpret_cast<longlong2*>(acc + id * 4);
+        const longlong2 p01 = a[0], m2 = a[1];
+        q[0] = m2.x;
+        q[1] = p01.x;
+        q[2] = p01.y;
+        if (D == 3) q[3] = m2.y;
+        if ((p01.x | p01.y | m2.x | m2.y) != 0) {
+            a[0] = make_longlong2(0, 0);
+            a[1] = make_longlong2(0, 0);
+        }
     }
     float vc[3], vf[3];
     grid_node_velocity<D, FORM>(C, q, ix, iy, iz, status, vc, vf);
@@ -629,7 +644,7 @@ struct SlowQueue {
     int capacity;
     // fused path: the 32-slot windows holding queued particles, as (first
     // slot, lane mask of the queued slots); their P2G runs after the return map
-    int2* win;
+    int4* win;  // .z: queued slots whose node blocks are not marked yet
     int* nwin;    // device scalar (count[1])
     int win_capacity;
 };

@@ -39,7 +39,16 @@ struct TileInfo {
     int* n_tile_list;  // device scalar
     int* p2g_next;     // device scalar: next P2G chunk to hand out (zeroed before each P2G)
     int* tile_len;     // per entry of tile_list: particles of that tile at the last sort
-    int* fused_next;   // device scalar: next tile of the fused transfer (zeroed before each launch)
+    int* fused_next;   // device scalar: next item of the fused transfer (zeroed before each launch)
+    // Work of the fused transfer: (tile, first slot, slots) of at most item_win
+    // (0: all of the tile's) windows of `win` slots each. Which slots form a window
+    // depends on the tile's start alone.
+    int4* items;
+    int* n_items;      // device scalar
+    int win, item_win;
+    int4* scan;        // per block of kScanTiles tiles: particles, non-empty tiles, items
+    int* grid_done;    // device scalar: CTAs of the grid update that have finished
+    int* zero[2];      // fused_next, queue counts: cleared by the grid update
     unsigned long long* skey;  // global sort scratch (tiles above SortGeom<D>::SMEM particles)
     int* sval;
 };
@@ -91,60 +100,92 @@ __global__ void __launch_bounds__(256) k_sort_count(Particles P, StepConsts C, T
     if (lane == __ffs(peers) - 1) atomicAdd(&TI.tile_count[t], __popc(peers));
 }
 
-// Single-CTA exclusive scans of the tile counts and of the non-empty tiles;
-// writes each tile's first slot and the list of non-empty tiles, and clears
-// the cursors for the bucket pass. Rounds of 1024 consecutive tiles (coalesced
-// loads, eight rounds' loads issued together), each a warp-shuffle scan plus a
-// scan of the 32 warp totals.
-__global__ void __launch_bounds__(1024) k_sort_scan(TileInfo TI) {
-    constexpr int R = 8;
-    __shared__ int s_wc[32], s_wn[32], s_tc, s_tn, s_base, s_lbase;
-    const int nt = TI.n_tiles, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    if (tid == 0) { s_base = 0; s_lbase = 0; }
-    __syncthreads();
-    for (int r0 = 0; r0 < nt; r0 += 1024 * R) {
-        int cv[R];
+// Exclusive scans over the tiles, in blocks of kScanTiles: of the particles (each
+// tile's first slot), of the non-empty tiles (their list) and of the items of the
+// fused transfer. k_sort_block_sums leaves each block's totals, k_sort_scan adds
+// those before its own block and scans within it; the cursors for the bucket
+// pass are cleared on the way. (One CTA for all tiles took 27 us on a 128^3 grid
+// and 210 us on 256^3; the two kernels take 6 us and 9 us.)
+constexpr int kScanTiles = 1024;
+
+__device__ __forceinline__ int tile_items(const TileInfo& TI, int count) {
+    if (count == 0 || TI.item_win == 0) return count > 0;
+    const int w = (count + TI.win - 1) / TI.win;
+    return (w + TI.item_win - 1) / TI.item_win;
+}
+
+// Inclusive scan of three counts over the CTA (1024 threads); total[] of all.
+__device__ __forceinline__ void block_scan3(int* v, int* total) {
+    __shared__ int s_w[3][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-        for (int q = 0; q < R; ++q) {
-            const int idx = r0 + q * 1024 + tid;
-            cv[q] = idx < nt ? TI.tile_count[idx] : 0;
+    for (int k = 0; k < 3; ++k) {
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, v[k], off);
+            if (lane >= off) v[k] += u;
         }
-#pragma unroll 1
-        for (int q = 0; q < R && r0 + q * 1024 < nt; ++q) {
-            const int idx = r0 + q * 1024 + tid;
-            const int c = cv[q], ne = c > 0;
-            int ic = c, in = ne;
-#pragma unroll
-            for (int off = 1; off < 32; off <<= 1) {
-                const int u = __shfl_up_sync(0xffffffffu, ic, off), v = __shfl_up_sync(0xffffffffu, in, off);
-                if (lane >= off) { ic += u; in += v; }
-            }
-            if (lane == 31) { s_wc[warp] = ic; s_wn[warp] = in; }
-            __syncthreads();
-            if (warp == 0) {
-                const int wc = s_wc[lane], wn = s_wn[lane];
-                int jc = wc, jn = wn;
-#pragma unroll
-                for (int off = 1; off < 32; off <<= 1) {
-                    const int u = __shfl_up_sync(0xffffffffu, jc, off), v = __shfl_up_sync(0xffffffffu, jn, off);
-                    if (lane >= off) { jc += u; jn += v; }
-                }
-                s_wc[lane] = jc - wc;  // exclusive warp offsets
-                s_wn[lane] = jn - wn;
-                if (lane == 31) { s_tc = jc; s_tn = jn; }
-            }
-            __syncthreads();
-            if (idx < nt) {
-                TI.tile_start[idx] = s_base + s_wc[warp] + ic - c;
-                TI.tile_cursor[idx] = 0;
-                if (ne) TI.tile_list[s_lbase + s_wn[warp] + in - 1] = idx;  // non-empty tiles in tile order
-            }
-            __syncthreads();
-            if (tid == 0) { s_base += s_tc; s_lbase += s_tn; }
-            __syncthreads();
-        }
+        if (lane == 31) s_w[k][warp] = v[k];
     }
-    if (tid == 0) *TI.n_tile_list = s_lbase;
+    __syncthreads();
+    if (warp < 3) {
+        int j = s_w[warp][lane];
+#pragma unroll
+        for (int off = 1; off < 32; off <<= 1) {
+            const int u = __shfl_up_sync(0xffffffffu, j, off);
+            if (lane >= off) j += u;
+        }
+        s_w[warp][lane] = j;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        if (warp > 0) v[k] += s_w[k][warp - 1];
+        total[k] = s_w[k][31];
+    }
+}
+
+__global__ void __launch_bounds__(kScanTiles) k_sort_block_sums(TileInfo TI) {
+    const int t = blockIdx.x * kScanTiles + threadIdx.x;
+    const int c = t < TI.n_tiles ? TI.tile_count[t] : 0;
+    int v[3] = {c, c > 0, tile_items(TI, c)}, total[3];
+    block_scan3(v, total);
+    if (threadIdx.x == 0) TI.scan[blockIdx.x] = make_int4(total[0], total[1], total[2], 0);
+}
+
+__global__ void __launch_bounds__(kScanTiles) k_sort_scan(TileInfo TI) {
+    __shared__ int s_before[3];
+    const int t = blockIdx.x * kScanTiles + threadIdx.x;
+    if (threadIdx.x < 3) s_before[threadIdx.x] = 0;
+    __syncthreads();
+    int b[3] = {0, 0, 0};
+    for (int k = threadIdx.x; k < (int)blockIdx.x; k += kScanTiles) {
+        const int4 s = TI.scan[k];
+        b[0] += s.x;
+        b[1] += s.y;
+        b[2] += s.z;
+    }
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        b[k] = __reduce_add_sync(0xffffffffu, b[k]);
+        if ((threadIdx.x & 31) == 0 && b[k]) atomicAdd(&s_before[k], b[k]);
+    }
+    const int c = t < TI.n_tiles ? TI.tile_count[t] : 0, ni = tile_items(TI, c);
+    int v[3] = {c, c > 0, ni}, total[3];
+    block_scan3(v, total);  // its barriers also order s_before
+    if (t < TI.n_tiles) {
+        const int start = s_before[0] + v[0] - c;
+        TI.tile_start[t] = start;
+        TI.tile_cursor[t] = 0;
+        if (c > 0) TI.tile_list[s_before[1] + v[1] - 1] = t;  // non-empty tiles in tile order
+        const int step = TI.item_win ? TI.win * TI.item_win : c;
+        for (int k = 0; k < ni; ++k)
+            TI.items[s_before[2] + v[2] - ni + k] = make_int4(t, start + k * step, min(step, c - k * step), 0);
+    }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        *TI.n_tile_list = s_before[1] + total[1];
+        *TI.n_items = s_before[2] + total[2];
+    }
 }
 
 struct SortBuffers {
@@ -315,7 +356,8 @@ __device__ __forceinline__ void mark_block(const TileInfo& TI, int b) {
 }
 
 // ---------------------------------------------------------------------------
-// Grid update over the node blocks P2G marked (reads and clears the int64 sums).
+// Grid update over the node blocks P2G marked (reads and clears the int64 sums;
+// leaves no block marked).
 template <int D, int FORM>
 __global__ void __launch_bounds__(256) k_grid_marked(StepConsts C, TileInfo TI, unsigned long long* __restrict__ acc,
                                                      float4* __restrict__ gv, unsigned* __restrict__ status) {
@@ -334,10 +376,30 @@ __global__ void __launch_bounds__(256) k_grid_marked(StepConsts C, TileInfo TI, 
         if (gx >= C.nx || gy >= C.ny || gz >= C.nz) continue;
         grid_node_at<D, FORM>(C, acc, gv, status, ((long long)gz * C.ny + gy) * C.nx + gx, gx, gy, gz);
     }
+    // Counters for what follows, instead of a memset node for each: those of the
+    // fused transfer and the queue now (nothing else uses them while this kernel
+    // runs), the number of marked blocks when every CTA has read it.
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (blockIdx.x == 0) {
+            *TI.zero[0] = 0;
+            TI.zero[1][0] = 0;
+            TI.zero[1][1] = 0;
+        }
+        __threadfence();
+        if (atomicAdd(TI.grid_done, 1) == (int)gridDim.x - 1) {
+            *TI.n_marked = 0;
+            *TI.grid_done = 0;
+        }
+    }
 }
 
+// Where channel c (mass, then momentum) of a node sits in its four sums:
+// momentum x, momentum y, mass, momentum z (2D: unused).
+__host__ __device__ __forceinline__ int acc_channel(int c) { return c == 0 ? 2 : (c < 3 ? c - 1 : 3); }
+
 // The int64 sums of the marked node blocks to / from a packed array
-// [block][channel][node of block] (checkpoints of the fused transfer, which
+// [block][channel: mass, momentum][node of block] (checkpoints of the fused transfer, which
 // keep the next step's grid sums). Unpacking also marks the blocks.
 template <int D>
 __global__ void __launch_bounds__(256) k_pack_marked(StepConsts C, TileInfo TI, int nch, int nb,
@@ -353,7 +415,7 @@ __global__ void __launch_bounds__(256) k_pack_marked(StepConsts C, TileInfo TI, 
         const int gx = b[0] * G::T + l[0], gy = b[1] * G::T + l[1], gz = D == 3 ? b[2] * G::T + l[2] : 0;
         const bool in = gx < C.nx && gy < C.ny && gz < C.nz;
         const long long id = ((long long)gz * C.ny + gy) * C.nx + gx;
-        for (int c = 0; c < nch; ++c) out[((w / G::BN) * nch + c) * G::BN + loc] = in ? acc[c * C.nodes + id] : 0ull;
+        for (int c = 0; c < nch; ++c) out[((w / G::BN) * nch + c) * G::BN + loc] = in ? acc[id * 4 + acc_channel(c)] : 0ull;
     }
 }
 
@@ -376,7 +438,7 @@ __global__ void __launch_bounds__(256) k_unpack_marked(StepConsts C, TileInfo TI
         const int gx = b[0] * G::T + l[0], gy = b[1] * G::T + l[1], gz = D == 3 ? b[2] * G::T + l[2] : 0;
         if (gx >= C.nx || gy >= C.ny || gz >= C.nz) continue;
         const long long id = ((long long)gz * C.ny + gy) * C.nx + gx;
-        for (int c = 0; c < nch; ++c) acc[c * C.nodes + id] = in[((w / G::BN) * nch + c) * G::BN + loc];
+        for (int c = 0; c < nch; ++c) acc[id * 4 + acc_channel(c)] = in[((w / G::BN) * nch + c) * G::BN + loc];
     }
 }
 
@@ -457,14 +519,16 @@ __device__ __forceinline__ void mark_block_once(const TileInfo& TI, int b) {
     if (TI.mark[b] == 0) mark_block(TI, b);
 }
 
-// int64 fixed-point add of a unit's sums; the range is checked once per unit.
-__device__ __forceinline__ void red_fixed(unsigned long long* p, float v, float scale) {
+// int64 fixed-point add of a scaled sum; the range is checked by the caller.
+__device__ __forceinline__ void red_scaled(unsigned long long* p, float t) {
     // an explicit global reduction (no return value): p always points into the
     // grid sums, and spelling it out keeps the compiler from falling back to a
     // generic atomic with a return where it cannot prove the address space
     const unsigned long long g = (unsigned long long)__cvta_generic_to_global(p);
-    asm volatile("red.global.add.u64 [%0], %1;" ::"l"(g), "l"((unsigned long long)__float2ll_rn(v * scale)));
+    asm volatile("red.global.add.u64 [%0], %1;" ::"l"(g), "l"((unsigned long long)__float2ll_rn(t)));
 }
+
+__device__ __forceinline__ void red_fixed(unsigned long long* p, float v, float scale) { red_scaled(p, v * scale); }
 
 #ifndef MPM_P2G_MIN_BLOCKS
 #define MPM_P2G_MIN_BLOCKS 3
@@ -624,11 +688,11 @@ __global__ void __launch_bounds__(kP2GWarps * 32, D == 3 ? MPM_P2G_MIN_BLOCKS : 
 #pragma unroll
                         for (int cc = 0; cc < S; ++cc) {
                             const int idx = bb * S + cc;
-                            unsigned long long* p0 = acc + (g0 + bb * sy + cc * sz);
-                            red_fixed(p0, am[idx], C.sm);
-                            red_fixed(p0 + C.nodes, a0[idx], C.sp);
-                            red_fixed(p0 + 2 * C.nodes, a1[idx], C.sp);
-                            red_fixed(p0 + 3 * C.nodes, a2[idx], C.sp);
+                            unsigned long long* p0 = acc + (g0 + bb * sy + cc * sz) * 4;
+                            red_fixed(p0 + 2, am[idx], C.sm);
+                            red_fixed(p0, a0[idx], C.sp);
+                            red_fixed(p0 + 1, a1[idx], C.sp);
+                            red_fixed(p0 + 3, a2[idx], C.sp);
                         }
                 } else {
                     bool outside = false;
@@ -637,11 +701,11 @@ __global__ void __launch_bounds__(kP2GWarps * 32, D == 3 ? MPM_P2G_MIN_BLOCKS : 
                             const int gy = cell[1] - 1 + by0 + bb, gz = cell[2] - 1 + cc;
                             if (gx < 0 || gx > C.W || gy < 0 || gy > C.H || gz < 0 || gz > C.Dp) { outside = true; continue; }
                             const int idx = bb * S + cc;
-                            unsigned long long* p0 = acc + (((long long)gz * C.ny + gy) * C.nx + gx);
-                            red_fixed(p0, am[idx], C.sm);
-                            red_fixed(p0 + C.nodes, a0[idx], C.sp);
-                            red_fixed(p0 + 2 * C.nodes, a1[idx], C.sp);
-                            red_fixed(p0 + 3 * C.nodes, a2[idx], C.sp);
+                            unsigned long long* p0 = acc + (((long long)gz * C.ny + gy) * C.nx + gx) * 4;
+                            red_fixed(p0 + 2, am[idx], C.sm);
+                            red_fixed(p0, a0[idx], C.sp);
+                            red_fixed(p0 + 1, a1[idx], C.sp);
+                            red_fixed(p0 + 3, a2[idx], C.sp);
                         }
                     if (outside) raise_flag(status, 4u);
                 }
@@ -703,10 +767,10 @@ __global__ void __launch_bounds__(kP2GWarps * 32, D == 3 ? MPM_P2G_MIN_BLOCKS : 
 #pragma unroll
                         for (int b = 0; b < S; ++b) {
                             const int idx = i * S + b;
-                            unsigned long long* p0 = acc + (g0 + i + (long long)b * C.nx);
-                            red_fixed(p0, am[idx], C.sm);
-                            red_fixed(p0 + C.nodes, a0[idx], C.sp);
-                            red_fixed(p0 + 2 * C.nodes, a1[idx], C.sp);
+                            unsigned long long* p0 = acc + (g0 + i + (long long)b * C.nx) * 4;
+                            red_fixed(p0 + 2, am[idx], C.sm);
+                            red_fixed(p0, a0[idx], C.sp);
+                            red_fixed(p0 + 1, a1[idx], C.sp);
                         }
                 } else {
                     bool outside = false;
@@ -715,10 +779,10 @@ __global__ void __launch_bounds__(kP2GWarps * 32, D == 3 ? MPM_P2G_MIN_BLOCKS : 
                             const int gx = gx0 + i, gy = cell[1] - 1 + b;
                             if (gx < 0 || gx > C.W || gy < 0 || gy > C.H) { outside = true; continue; }
                             const int idx = i * S + b;
-                            unsigned long long* p0 = acc + ((long long)gy * C.nx + gx);
-                            red_fixed(p0, am[idx], C.sm);
-                            red_fixed(p0 + C.nodes, a0[idx], C.sp);
-                            red_fixed(p0 + 2 * C.nodes, a1[idx], C.sp);
+                            unsigned long long* p0 = acc + ((long long)gy * C.nx + gx) * 4;
+                            red_fixed(p0 + 2, am[idx], C.sm);
+                            red_fixed(p0, a0[idx], C.sp);
+                            red_fixed(p0 + 1, a1[idx], C.sp);
                         }
                     if (outside) raise_flag(status, 4u);
                 }

@@ -29,6 +29,7 @@ struct mpm_mlp {
     float* w = nullptr;            // fp32 master parameters
     __nv_bfloat16* wbf = nullptr;  // bf16 copy used by the kernels
     float* grad = nullptr;
+    float* part = nullptr;         // per training CTA: its gradients and loss
     float* m1 = nullptr;
     float* m2 = nullptr;
     float* loss = nullptr;         // per training step
@@ -1537,7 +1538,8 @@ mpm_status mpm_mlp_create(uint64_t seed, mpm_mlp** out) {
     mpm_mlp* m = new mpm_mlp();
     cudaGetDevice(&m->device);
     const int P = MlpOff::total;
-    if (dalloc(&m->w, P) || dalloc(&m->wbf, P) || dalloc(&m->grad, P) || dalloc(&m->m1, P) || dalloc(&m->m2, P)) {
+    if (dalloc(&m->w, P) || dalloc(&m->wbf, P) || dalloc(&m->grad, P) || dalloc(&m->m1, P) || dalloc(&m->m2, P) ||
+        dalloc(&m->part, (size_t)kMlpTrainCtas * kMlpPart)) {
         mpm_mlp_destroy(m);
         return MPM_ERR_OUT_OF_MEMORY;
     }
@@ -1564,7 +1566,7 @@ mpm_status mpm_mlp_create(uint64_t seed, mpm_mlp** out) {
 
 mpm_status mpm_mlp_destroy(mpm_mlp* m) {
     if (!m) return MPM_ERR_INVALID_ARGUMENT;
-    void* ptrs[] = {m->w, m->wbf, m->grad, m->m1, m->m2, m->loss, m->pairs};
+    void* ptrs[] = {m->w, m->wbf, m->grad, m->part, m->m1, m->m2, m->loss, m->pairs};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     delete m;
@@ -1631,21 +1633,21 @@ mpm_status mpm_mlp_load_pairs(mpm_mlp* m, const float* pairs, int64_t n) {
     return MPM_OK;
 }
 
-static mpm_status mlp_launch_grad(mpm_mlp* m, const float* dpairs, long long np, const int* didx, int rows,
-                                  unsigned seed, float* dloss) {
-    static bool attr = false;
-    if (!attr) {
-        if (cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpTrainSmem)) !=
-            cudaSuccess) {
-            cudaGetLastError();
-            return MPM_ERR_CUDA;
-        }
-        attr = true;
-    }
-    const int blocks = (rows + kMlpTrainRows - 1) / kMlpTrainRows;
-    k_mlp_train<<<blocks, 128, sizeof(MlpTrainSmem)>>>(dpairs, np, didx, rows, seed, m->wbf, m->w, m->norm, m->grad,
-                                                        dloss);
-    return cudaGetLastError() == cudaSuccess ? MPM_OK : MPM_ERR_CUDA;
+// Gradients and loss of `rows` samples into m->part; returns the rows of it used
+// (0: launch failed).
+static int mlp_launch_grad(mpm_mlp* m, const float* dpairs, long long np, bool in_order, int rows, unsigned seed) {
+    const int tiles = (rows - 1) / kMlpTrainRows + 1;
+    const int ctas = tiles < kMlpTrainCtas ? tiles : kMlpTrainCtas;
+    k_mlp_train<<<ctas, 256, sizeof(MlpTrainSmem)>>>(dpairs, np, in_order, rows, seed, m->wbf, m->w, m->norm, m->part);
+    return cudaGetLastError() == cudaSuccess ? ctas : 0;
+}
+
+static bool mlp_train_attr() {
+    if (cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(MlpTrainSmem)) ==
+        cudaSuccess)
+        return true;
+    cudaGetLastError();
+    return false;
 }
 
 mpm_status mpm_mlp_train(mpm_mlp* m, int32_t steps, int32_t batch, float lr, float weight_decay, uint32_t seed,
@@ -1658,19 +1660,18 @@ mpm_status mpm_mlp_train(mpm_mlp* m, int32_t steps, int32_t batch, float lr, flo
         if (dalloc(&m->loss, (size_t)steps)) { cudaGetLastError(); return MPM_ERR_OUT_OF_MEMORY; }
         m->loss_cap = steps;
     }
-    if (cudaMemset(m->loss, 0, sizeof(float) * steps) != cudaSuccess) return MPM_ERR_CUDA;
+    if (!mlp_train_attr()) return MPM_ERR_CUDA;
     const float b1 = 0.9f, b2 = 0.999f;
     for (int it = 0; it < steps; ++it) {
         // cosine decay to lr / 20
         const float frac = steps > 1 ? float(it) / float(steps - 1) : 0.f;
         const float lr_t = lr * (0.05f + 0.95f * 0.5f * (1.f + std::cos(3.14159265f * frac)));
-        mpm_status st = mlp_launch_grad(m, m->pairs, m->n_pairs, nullptr, batch, seed * 2654435761u + (unsigned)it,
-                                        m->loss + it);
-        if (st != MPM_OK) return st;
+        const int ctas = mlp_launch_grad(m, m->pairs, m->n_pairs, false, batch, seed * 2654435761u + (unsigned)it);
+        if (ctas == 0) return MPM_ERR_CUDA;
         ++m->step;
         const float bc1 = 1.f - std::pow(b1, (float)m->step), bc2 = 1.f - std::pow(b2, (float)m->step);
-        k_mlp_adam<<<(MlpOff::total + 255) / 256, 256>>>(m->w, m->wbf, m->grad, m->m1, m->m2, lr_t, b1, b2, 1e-8f,
-                                                          weight_decay, bc1, bc2);
+        k_mlp_adam<<<MlpOff::total / 64 + 1, 256>>>(m->w, m->wbf, m->part, ctas, m->m1, m->m2, m->loss + it, lr_t, b1, b2,
+                                                    1e-8f, weight_decay, bc1, bc2);
         if (cudaGetLastError() != cudaSuccess) return MPM_ERR_CUDA;
     }
     if (cudaDeviceSynchronize() != cudaSuccess) { cudaGetLastError(); return MPM_ERR_CUDA; }
@@ -1683,26 +1684,23 @@ mpm_status mpm_mlp_train(mpm_mlp* m, int32_t steps, int32_t batch, float lr, flo
 mpm_status mpm_mlp_gradient(mpm_mlp* m, const float* pairs, int64_t n, float* grad_out, float* loss_out) {
     if (!m || !pairs || n < 1 || n > (1 << 24) || !grad_out) return MPM_ERR_INVALID_ARGUMENT;
     float *dp = nullptr, *dl = nullptr;
-    int* di = nullptr;
-    std::vector<int> idx((size_t)n);
-    for (int64_t i = 0; i < n; ++i) idx[i] = (int)i;
     mpm_status st = MPM_OK;
-    if (dalloc(&dp, (size_t)n * 20) || dalloc(&dl, 1) || dalloc(&di, (size_t)n)) st = MPM_ERR_OUT_OF_MEMORY;
-    if (st == MPM_OK && (cudaMemcpy(dp, pairs, sizeof(float) * 20 * n, cudaMemcpyHostToDevice) != cudaSuccess ||
-                         cudaMemcpy(di, idx.data(), sizeof(int) * n, cudaMemcpyHostToDevice) != cudaSuccess ||
-                         cudaMemset(dl, 0, sizeof(float)) != cudaSuccess ||
-                         cudaMemset(m->grad, 0, sizeof(float) * MlpOff::total) != cudaSuccess))
+    if (dalloc(&dp, (size_t)n * 20) || dalloc(&dl, 1)) st = MPM_ERR_OUT_OF_MEMORY;
+    if (st == MPM_OK && cudaMemcpy(dp, pairs, sizeof(float) * 20 * n, cudaMemcpyHostToDevice) != cudaSuccess)
         st = MPM_ERR_CUDA;
-    if (st == MPM_OK) st = mlp_launch_grad(m, dp, n, di, (int)n, 0u, dl);
+    if (st == MPM_OK) {
+        const int ctas = mlp_train_attr() ? mlp_launch_grad(m, dp, n, true, (int)n, 0u) : 0;
+        if (ctas == 0) st = MPM_ERR_CUDA;
+        else k_mlp_grad_sum<<<MlpOff::total / 64 + 1, 256>>>(m->part, ctas, m->grad, dl);
+        if (cudaGetLastError() != cudaSuccess) st = MPM_ERR_CUDA;
+    }
     if (st == MPM_OK && cudaDeviceSynchronize() != cudaSuccess) st = MPM_ERR_CUDA;
     if (st == MPM_OK && cudaMemcpy(grad_out, m->grad, sizeof(float) * MlpOff::total, cudaMemcpyDeviceToHost) != cudaSuccess)
         st = MPM_ERR_CUDA;
     if (st == MPM_OK && loss_out && cudaMemcpy(loss_out, dl, sizeof(float), cudaMemcpyDeviceToHost) != cudaSuccess)
         st = MPM_ERR_CUDA;
-    cudaMemset(m->grad, 0, sizeof(float) * MlpOff::total);
     if (dp) cudaFree(dp);
     if (dl) cudaFree(dl);
-    if (di) cudaFree(di);
     cudaGetLastError();
     return st;
 }

@@ -29,9 +29,7 @@ struct MlpNorm {
 };
 
 // ---------------------------------------------------------------------------
-// Tensor-core fragments. Operands live in shared memory as bf16 with arbitrary
-// strides: A(m, k) at A[m * sam + k * sak], B(k, n) at B[k * sbk + n * sbn].
-// m16n8k16 layouts (PTX ISA): with g = lane / 4, t = lane % 4,
+// Tensor-core fragments, m16n8k16 layouts (PTX ISA): with g = lane / 4, t = lane % 4,
 //   A regs: (g, 2t..2t+1), (g+8, 2t..), (g, 2t+8..), (g+8, 2t+8..)
 //   B regs: (k = 2t..2t+1, n = g), (k = 2t+8.., n = g)
 //   C/D   : (g, 2t), (g, 2t+1), (g+8, 2t), (g+8, 2t+1)
@@ -45,23 +43,6 @@ __device__ __forceinline__ void mma_bf16(float* d, const uint32_t* a, const uint
         "{%0,%1,%2,%3};\n"
         : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b[0]), "r"(b[1]));
-}
-
-// acc[16 x 8] (C layout) += A[m0.., k0..k0+16) * B[k0.., n0..n0+8)
-__device__ __forceinline__ void mma_tile(float* acc, const __nv_bfloat16* A, int sam, int sak, const __nv_bfloat16* B,
-                                         int sbk, int sbn, int m0, int k0, int n0) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    uint32_t a[4], b[2];
-    const int kk = k0 + 2 * t;
-    auto ldA = [&](int m, int k) { return pack_bf16(A[m * sam + k * sak], A[m * sam + (k + 1) * sak]); };
-    auto ldB = [&](int k, int n) { return pack_bf16(B[k * sbk + n * sbn], B[(k + 1) * sbk + n * sbn]); };
-    a[0] = ldA(m0 + g, kk);
-    a[1] = ldA(m0 + g + 8, kk);
-    a[2] = ldA(m0 + g, kk + 8);
-    a[3] = ldA(m0 + g + 8, kk + 8);
-    b[0] = ldB(kk, n0 + g);
-    b[1] = ldB(kk + 8, n0 + g);
-    mma_bf16(acc, a, b);
 }
 
 // GELU in its tanh form (Hendrycks & Gimpel 2016):
@@ -96,195 +77,6 @@ __device__ __forceinline__ void mlp_targets(const float* pair, const MlpNorm& N,
     for (int k = 0; k < 9; ++k) tg[k] = ((pair[10 + k] - pair[k]) - N.out_mean[k]) / N.out_std[k];
     tg[9] = ((logf(pair[19]) - logf(pair[9])) - N.out_mean[9]) / N.out_std[9];
 }
-
-// ---------------------------------------------------------------------------
-// Forward pass of one 16-row tile per warp on shared-memory activations.
-// X: [rows][ldx] bf16; layer output Y (pre-activation, fp32 [rows][ldy]) and
-// H = GELU(Y) as bf16 [rows][ldh] when `act`.
-__device__ __forceinline__ void mlp_layer_fwd(const __nv_bfloat16* X, int ldx, int K, const __nv_bfloat16* W,
-                                              const float* bias, int N, int m0, float* Y, int ldy, __nv_bfloat16* H,
-                                              int ldh, bool act) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-    for (int n0 = 0; n0 < N; n0 += 8) {
-        float acc[4] = {0.f, 0.f, 0.f, 0.f};
-        for (int k0 = 0; k0 < K; k0 += 16) mma_tile(acc, X, ldx, 1, W, 1, K, m0, k0, n0);
-        const int r0 = m0 + g, c0 = n0 + 2 * t;
-        const float v[4] = {acc[0] + bias[c0], acc[1] + bias[c0 + 1], acc[2] + bias[c0], acc[3] + bias[c0 + 1]};
-        const int rr[4] = {r0, r0, r0 + 8, r0 + 8}, cc[4] = {c0, c0 + 1, c0, c0 + 1};
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (Y) Y[rr[q] * ldy + cc[q]] = v[q];
-            if (H) H[rr[q] * ldh + cc[q]] = __float2bfloat16_rn(act ? gelu(v[q]) : v[q]);
-        }
-    }
-}
-
-// ---------------------------------------------------------------------------
-// Training step on one CTA of kMlpTrainRows samples (4 warps x 16 rows):
-// forward, MSE loss, backward; weight gradients accumulated (fp32 atomics)
-// into `grad`, loss sum into `loss`. Samples: `idx` (explicit, may be null) or
-// a hash of (seed, global row) modulo n_pairs.
-constexpr int kMlpTrainRows = 64;
-
-struct MlpTrainSmem {
-    __nv_bfloat16 w[MlpOff::total];
-    float b1[kMlpHid], b2[kMlpHid], b3[kMlpHid], b4[kMlpOutPad];
-    __nv_bfloat16 x0[kMlpTrainRows * kMlpInPad];
-    __nv_bfloat16 h[3][kMlpTrainRows * kMlpHid];
-    float y[3][kMlpTrainRows * kMlpHid];
-    float out[kMlpTrainRows * kMlpOutPad];
-    float tgt[kMlpTrainRows * kMlpOutPad];
-    __nv_bfloat16 dy[kMlpTrainRows * kMlpHid];   // gradient wrt the current layer's pre-activation
-    __nv_bfloat16 dy4[kMlpTrainRows * kMlpOutPad];
-    float dh[kMlpTrainRows * kMlpHid];            // gradient wrt the previous layer's output
-};
-
-__device__ __forceinline__ unsigned hash_u32(unsigned x) {
-    x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
-    return x;
-}
-
-__global__ void __launch_bounds__(128) k_mlp_train(const float* __restrict__ pairs, long long n_pairs,
-                                                   const int* __restrict__ idx, int n_rows, unsigned seed,
-                                                   const __nv_bfloat16* __restrict__ wbf, const float* __restrict__ wf32,
-                                                   MlpNorm N, float* __restrict__ grad, float* __restrict__ loss) {
-    extern __shared__ __align__(16) unsigned char smem_raw[];
-    MlpTrainSmem& S = *reinterpret_cast<MlpTrainSmem*>(smem_raw);
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    for (int i = tid; i < MlpOff::total; i += blockDim.x) S.w[i] = wbf[i];
-    for (int i = tid; i < kMlpHid; i += blockDim.x) {
-        S.b1[i] = wf32[MlpOff::b1 + i];
-        S.b2[i] = wf32[MlpOff::b2 + i];
-        S.b3[i] = wf32[MlpOff::b3 + i];
-    }
-    for (int i = tid; i < kMlpOutPad; i += blockDim.x) S.b4[i] = wf32[MlpOff::b4 + i];
-    // rows of this CTA
-    const int row0 = blockIdx.x * kMlpTrainRows;
-    for (int r = tid; r < kMlpTrainRows; r += blockDim.x) {
-        const int gr = row0 + r;
-        float in[kMlpIn], tg[kMlpOut];
-        const bool valid = gr < n_rows;
-        if (valid) {
-            const long long p = idx ? (long long)idx[gr]
-                                    : (long long)((((unsigned long long)hash_u32(seed ^ hash_u32((unsigned)gr)) << 20) ^
-                                                   hash_u32((unsigned)gr * 2654435761u + seed)) % (unsigned long long)n_pairs);
-            const float* pr = pairs + p * 20;
-            mlp_features(pr, pr[9], N, in);
-            mlp_targets(pr, N, tg);
-        }
-        for (int k = 0; k < kMlpInPad; ++k) S.x0[r * kMlpInPad + k] = __float2bfloat16_rn(valid && k < kMlpIn ? in[k] : 0.f);
-        for (int k = 0; k < kMlpOutPad; ++k) S.tgt[r * kMlpOutPad + k] = valid && k < kMlpOut ? tg[k] : 0.f;
-    }
-    __syncthreads();
-    const int m0 = warp * 16;
-    const __nv_bfloat16* W1 = S.w + MlpOff::W1;
-    const __nv_bfloat16* W2 = S.w + MlpOff::W2;
-    const __nv_bfloat16* W3 = S.w + MlpOff::W3;
-    const __nv_bfloat16* W4 = S.w + MlpOff::W4;
-    mlp_layer_fwd(S.x0, kMlpInPad, kMlpInPad, W1, S.b1, kMlpHid, m0, S.y[0], kMlpHid, S.h[0], kMlpHid, true);
-    __syncwarp();
-    mlp_layer_fwd(S.h[0], kMlpHid, kMlpHid, W2, S.b2, kMlpHid, m0, S.y[1], kMlpHid, S.h[1], kMlpHid, true);
-    __syncwarp();
-    mlp_layer_fwd(S.h[1], kMlpHid, kMlpHid, W3, S.b3, kMlpHid, m0, S.y[2], kMlpHid, S.h[2], kMlpHid, true);
-    __syncwarp();
-    mlp_layer_fwd(S.h[2], kMlpHid, kMlpHid, W4, S.b4, kMlpOutPad, m0, S.out, kMlpOutPad, nullptr, 0, false);
-    __syncthreads();
-    // loss and dL/dY4 (mean over all rows of the launch)
-    float lsum = 0.f;
-    for (int e = tid; e < kMlpTrainRows * kMlpOutPad; e += blockDim.x) {
-        const int r = e / kMlpOutPad, c = e % kMlpOutPad;
-        const bool valid = row0 + r < n_rows && c < kMlpOut;
-        const float diff = valid ? S.out[e] - S.tgt[e] : 0.f;
-        lsum += diff * diff;
-        S.dy4[e] = __float2bfloat16_rn(2.f * diff / float(n_rows));
-        S.out[e] = 2.f * diff / float(n_rows);  // fp32 copy for the bias gradient
-    }
-    for (int o = 16; o > 0; o >>= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, o);
-    if (lane == 0) atomicAdd(loss, lsum);
-    __syncthreads();
-
-    // backward through the 4 layers: at layer l with input X (bf16 [rows][K])
-    // and dY (bf16 [rows][N]): dW = dY^T X (tensor cores, k = rows), db = sum dY,
-    // dX = dY W (tensor cores), then dY_{l-1} = dX * GELU'(Y_{l-1}).
-    struct L { const __nv_bfloat16* X; int K; const __nv_bfloat16* W; int N; int woff, boff; };
-    const L layers[4] = {{S.x0, kMlpInPad, W1, kMlpHid, MlpOff::W1, MlpOff::b1},
-                         {S.h[0], kMlpHid, W2, kMlpHid, MlpOff::W2, MlpOff::b2},
-                         {S.h[1], kMlpHid, W3, kMlpHid, MlpOff::W3, MlpOff::b3},
-                         {S.h[2], kMlpHid, W4, kMlpOutPad, MlpOff::W4, MlpOff::b4}};
-    for (int l = 3; l >= 0; --l) {
-        const L& Ly = layers[l];
-        const __nv_bfloat16* dY = l == 3 ? S.dy4 : S.dy;
-        const int ldd = Ly.N;
-        // dW[n][k] = sum_r dY[r][n] X[r][k]: A(m = n, kk = r) = dY[r][n], B(kk = r, n = k) = X[r][k]
-        const int mt = Ly.N / 16, nt = Ly.K / 8;
-        for (int tile = warp; tile < mt * nt; tile += 4) {
-            const int tm = (tile / nt) * 16, tn = (tile % nt) * 8;
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            for (int r0 = 0; r0 < kMlpTrainRows; r0 += 16) mma_tile(acc, dY, 1, ldd, Ly.X, Ly.K, 1, tm, r0, tn);
-            const int rr = tm + g, cc = tn + 2 * t;
-            atomicAdd(&grad[Ly.woff + rr * Ly.K + cc], acc[0]);
-            atomicAdd(&grad[Ly.woff + rr * Ly.K + cc + 1], acc[1]);
-            atomicAdd(&grad[Ly.woff + (rr + 8) * Ly.K + cc], acc[2]);
-            atomicAdd(&grad[Ly.woff + (rr + 8) * Ly.K + cc + 1], acc[3]);
-        }
-        // db[n] = sum_r dY[r][n] (fp32 copy for the output layer)
-        for (int nn = tid; nn < Ly.N; nn += blockDim.x) {
-            float sdb = 0.f;
-            for (int r = 0; r < kMlpTrainRows; ++r)
-                sdb += l == 3 ? S.out[r * kMlpOutPad + nn] : __bfloat162float(dY[r * ldd + nn]);
-            atomicAdd(&grad[Ly.boff + nn], sdb);
-        }
-        if (l == 0) break;
-        // dX[r][k] = sum_n dY[r][n] W[n][k]: A(m = r, kk = n) = dY[r][n], B(kk = n, n = k) = W[n][k]
-        for (int n0 = 0; n0 < Ly.K; n0 += 8) {
-            float acc[4] = {0.f, 0.f, 0.f, 0.f};
-            for (int k0 = 0; k0 < Ly.N; k0 += 16) mma_tile(acc, dY, ldd, 1, Ly.W, Ly.K, 1, m0, k0, n0);
-            const int rr = m0 + g, cc = n0 + 2 * t;
-            S.dh[rr * kMlpHid + cc] = acc[0];
-            S.dh[rr * kMlpHid + cc + 1] = acc[1];
-            S.dh[(rr + 8) * kMlpHid + cc] = acc[2];
-            S.dh[(rr + 8) * kMlpHid + cc + 1] = acc[3];
-        }
-        __syncthreads();
-        const float* Yp = S.y[l - 1];
-        for (int e = tid; e < kMlpTrainRows * kMlpHid; e += blockDim.x)
-            S.dy[e] = __float2bfloat16_rn(row0 + e / kMlpHid < n_rows ? S.dh[e] * gelu_grad(Yp[e]) : 0.f);
-        __syncthreads();
-    }
-}
-
-// AdamW on the fp32 master weights; refreshes the bf16 copy and clears `grad`.
-// Padded entries (input columns >= 10 of W1, output rows >= 10 of W4 and b4)
-// stay zero.
-__global__ void k_mlp_adam(float* __restrict__ w, __nv_bfloat16* __restrict__ wbf, float* __restrict__ grad,
-                           float* __restrict__ m1, float* __restrict__ m2, float lr, float beta1, float beta2,
-                           float eps, float wd, float bc1, float bc2) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= MlpOff::total) return;
-    bool pad = false;
-    if (i < MlpOff::b1) pad = (i % kMlpInPad) >= kMlpIn;
-    else if (i >= MlpOff::W4 && i < MlpOff::b4) pad = (i - MlpOff::W4) / kMlpHid >= kMlpOut;
-    else if (i >= MlpOff::b4) pad = (i - MlpOff::b4) >= kMlpOut;
-    const float gr = grad[i];
-    grad[i] = 0.f;
-    if (pad) { w[i] = 0.f; wbf[i] = __float2bfloat16_rn(0.f); return; }
-    const bool is_bias = (i >= MlpOff::b1 && i < MlpOff::W2) || (i >= MlpOff::b2 && i < MlpOff::W3) ||
-                         (i >= MlpOff::b3 && i < MlpOff::W4) || i >= MlpOff::b4;
-    const float a = beta1 * m1[i] + (1.f - beta1) * gr;
-    const float b = beta2 * m2[i] + (1.f - beta2) * gr * gr;
-    m1[i] = a;
-    m2[i] = b;
-    float x = w[i];
-    if (!is_bias) x -= lr * wd * x;
-    x -= lr * (a / bc1) / (sqrtf(b / bc2) + eps);
-    w[i] = x;
-    wbf[i] = __float2bfloat16_rn(x);
-}
-
-}  // namespace mpm
-
-namespace mpm {
 
 // ---------------------------------------------------------------------------
 // Residual check of a predicted return map (3D). The exact map is
@@ -413,7 +205,8 @@ struct MlpParams {
 // after bias + GELU, are packed to bf16 pairs that are exactly the m16k16 A
 // fragments of the next layer (accumulator n-tiles 2kb, 2kb+1 = A k-block kb).
 // Weights sit in shared memory with rows padded by 8 bf16 so that the B
-// fragment loads of a warp hit 32 distinct banks.
+// fragment loads of a warp hit 32 distinct banks (and eight rows' 16-byte ldmatrix
+// rows too, in training).
 constexpr int kMwIn = kMlpInPad + 8;  // row stride (bf16) of W1 and of the input tile
 constexpr int kMwHid = kMlpHid + 8;   // row stride (bf16) of W2, W3, W4
 constexpr int kMwOut = kMlpOutPad + 2;  // row stride (fp32) of the output tile
@@ -639,6 +432,325 @@ __global__ void __launch_bounds__(kMlpWarps * 32) k_mlp_forward(const float* __r
     if (valid)
 #pragma unroll
         for (int c = 0; c < kMlpOut; ++c) out[(long long)row * kMlpOut + c] = O[lane * kMwOut + c] * N.out_std[c] + N.out_mean[c];
+}
+
+// ---------------------------------------------------------------------------
+// Training step: forward, MSE loss, backward on tiles of kMlpTrainRows samples
+// (8 warps x 16 rows); a CTA takes tiles until none are left and writes its
+// weight gradients and loss once, to its own row of `part` (summed by
+// k_mlp_adam / k_mlp_grad_sum in a fixed order). Samples: row = pair (seed 0 and
+// `in_order`) or a hash of (seed, global row) modulo n_pairs.
+//
+// A warp keeps its 16 rows in registers through the layers: the m16n8
+// accumulators of one layer, after bias + GELU, are the m16k16 A fragments of the
+// next (as in the inference kernel), backward as well (dX = dY W with W transposed
+// in shared memory), and GELU' stays in registers from the forward pass. Only the
+// bf16 activations and dY go to shared memory, from which every warp takes
+// transposed fragments (ldmatrix.trans) for its share of dW = dY^T X.
+// Bound: latency (8 warps per SM, one tile per CTA at the usual batch of 16384,
+// about 600 dependent mma and tanh a warp). The former kernel (64-row tiles,
+// every fragment from 2-byte shared loads, an fp32 atomic per weight and CTA)
+// took 107 us at that batch, this one 14.4 us.
+constexpr int kMlpTrainRows = 128;
+constexpr int kMlpTrainCtas = 148;              // most CTAs (rows of `part`)
+constexpr int kMlpPart = MlpOff::total + 16;    // floats per row: gradients, then the loss
+
+struct MlpTrainSmem {
+    __nv_bfloat16 W1[kMlpHid * kMwIn], W2[kMlpHid * kMwHid], W3[kMlpHid * kMwHid], W4[kMlpOutPad * kMwHid];
+    __nv_bfloat16 W2t[kMlpHid * kMwHid], W3t[kMlpHid * kMwHid], W4t[kMlpHid * kMwIn];  // [in][out]
+    float b1[kMlpHid], b2[kMlpHid], b3[kMlpHid], b4[kMlpOutPad];
+    __nv_bfloat16 x0[kMlpTrainRows * kMwIn];
+    __nv_bfloat16 h[3][kMlpTrainRows * kMwHid];
+    __nv_bfloat16 dy[kMlpTrainRows * kMwHid];    // gradient wrt the current layer's pre-activation
+    __nv_bfloat16 dy4[kMlpTrainRows * kMwIn];
+    float tgt[kMlpTrainRows * kMlpOutPad];
+    float red[8][kMlpOutPad + 1];              // per warp: output bias gradients, loss
+};
+
+__device__ __forceinline__ unsigned hash_u32(unsigned x) {
+    x ^= x >> 16; x *= 0x7feb352du; x ^= x >> 15; x *= 0x846ca68bu; x ^= x >> 16;
+    return x;
+}
+
+__device__ __forceinline__ void ldmatrix_x4_trans(uint32_t* r, const __nv_bfloat16* p) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a)
+                 : "memory");
+}
+
+// bias + GELU on a warp's 16 x 64 accumulator: A fragments of the next layer and
+// their copy in shared memory (rows r0 .. r0 + 15), GELU' kept in fp32.
+__device__ __forceinline__ void mlp_train_activate(float (*acc)[4], const float* bias, uint32_t (*a)[4], float (*gp)[4],
+                                                   __nv_bfloat16* h, int r0) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int j = 0; j < kMlpHid / 8; ++j) {
+        const int c = j * 8 + 2 * t;
+        float v[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const float x = acc[j][q] + bias[c + (q & 1)];
+            v[q] = gelu(x);
+            gp[j][q] = gelu_grad(x);
+        }
+        const uint32_t lo = pack_f2_bf16(v[0], v[1]), hi = pack_f2_bf16(v[2], v[3]);
+        a[j / 2][2 * (j & 1)] = lo;
+        a[j / 2][2 * (j & 1) + 1] = hi;
+        *reinterpret_cast<uint32_t*>(h + (r0 + g) * kMwHid + c) = lo;
+        *reinterpret_cast<uint32_t*>(h + (r0 + g + 8) * kMwHid + c) = hi;
+    }
+}
+
+// dY of a hidden layer from dX (accumulator) and GELU': bf16 A fragments and
+// their copy in shared memory.
+__device__ __forceinline__ void mlp_train_back(float (*acc)[4], float (*gp)[4], uint32_t (*a)[4], __nv_bfloat16* dy, int r0) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int j = 0; j < kMlpHid / 8; ++j) {
+        const uint32_t lo = pack_f2_bf16(acc[j][0] * gp[j][0], acc[j][1] * gp[j][1]);
+        const uint32_t hi = pack_f2_bf16(acc[j][2] * gp[j][2], acc[j][3] * gp[j][3]);
+        a[j / 2][2 * (j & 1)] = lo;
+        a[j / 2][2 * (j & 1) + 1] = hi;
+        *reinterpret_cast<uint32_t*>(dy + (r0 + g) * kMwHid + j * 8 + 2 * t) = lo;
+        *reinterpret_cast<uint32_t*>(dy + (r0 + g + 8) * kMwHid + j * 8 + 2 * t) = hi;
+    }
+}
+
+// The warp's share of dW[n][k] += sum_r dY[r][n] X[r][k] over the tile's rows:
+// output rows n0 .. n0 + 15, NT column tiles of 8 from k0 on; with `ones` also
+// db[n] = sum_r dY[r][n] (the product with a column of ones).
+template <int NT>
+__device__ __forceinline__ void mlp_train_dw(const __nv_bfloat16* dY, int ldd, const __nv_bfloat16* X, int ldx, int n0,
+                                             int k0, float (*dw)[4], bool ones, float* db) {
+    const int lane = threadIdx.x & 31, mi = lane >> 3, row = lane & 7;
+#pragma unroll
+    for (int r0 = 0; r0 < kMlpTrainRows; r0 += 16) {
+        uint32_t a[4];
+        ldmatrix_x4_trans(a, dY + (r0 + (mi >> 1) * 8 + row) * ldd + n0 + (mi & 1) * 8);
+#pragma unroll
+        for (int j = 0; j < NT; j += 2) {
+            uint32_t b[4];
+            // matrices: (r0, k), (r0 + 8, k), (r0, k + 8), (r0 + 8, k + 8); with one tile the second pair repeats the first
+            const int kc = k0 + j * 8 + (NT > 1 ? (mi >> 1) * 8 : 0);
+            ldmatrix_x4_trans(b, X + (r0 + (mi & 1) * 8 + row) * ldx + kc);
+            mma_bf16(dw[j], a, b);
+            if constexpr (NT > 1) mma_bf16(dw[j + 1], a, b + 2);
+        }
+        if (ones) {
+            const uint32_t one[2] = {0x3f803f80u, 0x3f803f80u};  // bf16 1.0 pairs
+            mma_bf16(db, a, one);
+        }
+    }
+}
+
+// The transpose of a row-major [rows][cols] matrix.
+__device__ __forceinline__ void mlp_stage_transposed(__nv_bfloat16* dst, int ld_dst, const __nv_bfloat16* src, int rows,
+                                                     int cols) {
+    for (int v = threadIdx.x; v < rows * cols; v += blockDim.x) dst[(v % cols) * ld_dst + v / cols] = src[v];
+}
+
+__global__ void __launch_bounds__(256, 1) k_mlp_train(const float* __restrict__ pairs, long long n_pairs, bool in_order,
+                                                      int n_rows, unsigned seed, const __nv_bfloat16* __restrict__ wbf,
+                                                      const float* __restrict__ wf32, MlpNorm N,
+                                                      float* __restrict__ part) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    MlpTrainSmem& S = *reinterpret_cast<MlpTrainSmem*>(smem_raw);
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, t = lane & 3;
+    mlp_stage_matrix(S.W1, kMwIn, wbf + MlpOff::W1, kMlpHid, kMlpInPad);
+    mlp_stage_matrix(S.W2, kMwHid, wbf + MlpOff::W2, kMlpHid, kMlpHid);
+    mlp_stage_matrix(S.W3, kMwHid, wbf + MlpOff::W3, kMlpHid, kMlpHid);
+    mlp_stage_matrix(S.W4, kMwHid, wbf + MlpOff::W4, kMlpOutPad, kMlpHid);
+    mlp_stage_transposed(S.W2t, kMwHid, wbf + MlpOff::W2, kMlpHid, kMlpHid);
+    mlp_stage_transposed(S.W3t, kMwHid, wbf + MlpOff::W3, kMlpHid, kMlpHid);
+    mlp_stage_transposed(S.W4t, kMwIn, wbf + MlpOff::W4, kMlpOutPad, kMlpHid);
+    if (tid < kMlpHid) {
+        S.b1[tid] = wf32[MlpOff::b1 + tid];
+        S.b2[tid] = wf32[MlpOff::b2 + tid];
+        S.b3[tid] = wf32[MlpOff::b3 + tid];
+    }
+    if (tid < kMlpOutPad) S.b4[tid] = wf32[MlpOff::b4 + tid];
+    // the warp's share of dW: rows n0.. of W2 and W3 and half of their columns,
+    // one tile each of W1 and W4
+    const int n0 = (warp & 3) * 16, kh = (warp >> 2) * 32;
+    float dw2[4][4] = {}, dw3[4][4] = {}, dw1[1][4] = {}, dw4[1][4] = {}, db1[4] = {}, db2[4] = {}, db3[4] = {};
+    float db4[4] = {0.f, 0.f, 0.f, 0.f}, lsum = 0.f;  // db4: columns 2t, 2t + 1 of both tiles
+    const int r0 = warp * 16;
+    const float inv = 2.f / float(n_rows);
+    for (long long row0 = (long long)blockIdx.x * kMlpTrainRows; row0 < n_rows; row0 += (long long)gridDim.x * kMlpTrainRows) {
+        __syncthreads();  // the last tile's fragments have been read (first tile: nothing)
+        if (tid < kMlpTrainRows) {
+            const long long gr = row0 + tid;
+            float in[kMlpIn], tg[kMlpOut];
+            const bool valid = gr < n_rows;
+            if (valid) {
+                const unsigned u = (unsigned)gr;
+                const long long p = in_order ? gr
+                                             : (long long)((((unsigned long long)hash_u32(seed ^ hash_u32(u)) << 20) ^
+                                                            hash_u32(u * 2654435761u + seed)) % (unsigned long long)n_pairs);
+                float pr[20];
+#pragma unroll
+                for (int q = 0; q < 5; ++q) {  // rows of 80 bytes, 16-byte aligned
+                    const float4 f = reinterpret_cast<const float4*>(pairs + p * 20)[q];
+                    pr[4 * q] = f.x; pr[4 * q + 1] = f.y; pr[4 * q + 2] = f.z; pr[4 * q + 3] = f.w;
+                }
+                mlp_features(pr, pr[9], N, in);
+                mlp_targets(pr, N, tg);
+            }
+#pragma unroll
+            for (int k = 0; k < kMlpInPad; k += 2)
+                *reinterpret_cast<uint32_t*>(S.x0 + tid * kMwIn + k) =
+                    pack_f2_bf16(valid && k < kMlpIn ? in[k < kMlpIn ? k : 0] : 0.f,
+                                 valid && k + 1 < kMlpIn ? in[k + 1 < kMlpIn ? k + 1 : 0] : 0.f);
+#pragma unroll
+            for (int k = 0; k < kMlpOutPad; ++k) S.tgt[tid * kMlpOutPad + k] = valid && k < kMlpOut ? tg[k < kMlpOut ? k : 0] : 0.f;
+        }
+        __syncthreads();
+        uint32_t a[kMlpHid / 16][4];
+        float acc[kMlpHid / 8][4], gp1[kMlpHid / 8][4], gp2[kMlpHid / 8][4], gp3[kMlpHid / 8][4];
+        const __nv_bfloat16* X = S.x0 + r0 * kMwIn;
+        a[0][0] = *reinterpret_cast<const uint32_t*>(X + g * kMwIn + 2 * t);
+        a[0][1] = *reinterpret_cast<const uint32_t*>(X + (g + 8) * kMwIn + 2 * t);
+        a[0][2] = *reinterpret_cast<const uint32_t*>(X + g * kMwIn + 2 * t + 8);
+        a[0][3] = *reinterpret_cast<const uint32_t*>(X + (g + 8) * kMwIn + 2 * t + 8);
+        mlp_warp_layer<1, kMlpHid / 8>(a, S.W1, kMwIn, acc);
+        mlp_train_activate(acc, S.b1, a, gp1, S.h[0], r0);
+        mlp_warp_layer<kMlpHid / 16, kMlpHid / 8>(a, S.W2, kMwHid, acc);
+        mlp_train_activate(acc, S.b2, a, gp2, S.h[1], r0);
+        mlp_warp_layer<kMlpHid / 16, kMlpHid / 8>(a, S.W3, kMwHid, acc);
+        mlp_train_activate(acc, S.b3, a, gp3, S.h[2], r0);
+        float o[kMlpOutPad / 8][4];
+        mlp_warp_layer<kMlpHid / 16, kMlpOutPad / 8>(a, S.W4, kMwHid, o);
+        // loss and dL/dY4 (mean over all rows of the launch)
+#pragma unroll
+        for (int j = 0; j < kMlpOutPad / 8; ++j) {
+            const int c = j * 8 + 2 * t;
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int r = r0 + g + (q & 2 ? 8 : 0), cc = c + (q & 1);
+                const bool valid = row0 + r < n_rows && cc < kMlpOut;
+                const float diff = valid ? o[j][q] + S.b4[cc] - S.tgt[r * kMlpOutPad + cc] : 0.f;
+                lsum += diff * diff;
+                o[j][q] = diff * inv;
+                db4[2 * j + (q & 1)] += o[j][q];
+            }
+            const uint32_t lo = pack_f2_bf16(o[j][0], o[j][1]), hi = pack_f2_bf16(o[j][2], o[j][3]);
+            a[0][2 * j] = lo;
+            a[0][2 * j + 1] = hi;
+            *reinterpret_cast<uint32_t*>(S.dy4 + (r0 + g) * kMwIn + c) = lo;
+            *reinterpret_cast<uint32_t*>(S.dy4 + (r0 + g + 8) * kMwIn + c) = hi;
+        }
+        mlp_warp_layer<1, kMlpHid / 8>(a, S.W4t, kMwIn, acc);  // dX = dY4 W4
+        mlp_train_back(acc, gp3, a, S.dy, r0);
+        __syncthreads();
+        mlp_train_dw<1>(S.dy4, kMwIn, S.h[2], kMwHid, 0, warp * 8, dw4, false, nullptr);
+        mlp_train_dw<4>(S.dy, kMwHid, S.h[1], kMwHid, n0, kh, dw3, warp < 4, db3);
+        mlp_warp_layer<kMlpHid / 16, kMlpHid / 8>(a, S.W3t, kMwHid, acc);
+        __syncthreads();  // dY3 has been read
+        mlp_train_back(acc, gp2, a, S.dy, r0);
+        __syncthreads();
+        mlp_train_dw<4>(S.dy, kMwHid, S.h[0], kMwHid, n0, kh, dw2, warp < 4, db2);
+        mlp_warp_layer<kMlpHid / 16, kMlpHid / 8>(a, S.W2t, kMwHid, acc);
+        __syncthreads();
+        mlp_train_back(acc, gp1, a, S.dy, r0);
+        __syncthreads();
+        mlp_train_dw<1>(S.dy, kMwHid, S.x0, kMwIn, n0, (warp >> 2) * 8, dw1, warp < 4, db1);
+    }
+    // this CTA's row of `part` (every entry written)
+    float* P = part + (long long)blockIdx.x * kMlpPart;
+    auto put = [&](float* dst, int ld, const float* v) {  // an m16n8 tile
+        *reinterpret_cast<float2*>(dst + g * ld + 2 * t) = make_float2(v[0], v[1]);
+        *reinterpret_cast<float2*>(dst + (g + 8) * ld + 2 * t) = make_float2(v[2], v[3]);
+    };
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        put(P + MlpOff::W2 + n0 * kMlpHid + kh + j * 8, kMlpHid, dw2[j]);
+        put(P + MlpOff::W3 + n0 * kMlpHid + kh + j * 8, kMlpHid, dw3[j]);
+    }
+    put(P + MlpOff::W1 + n0 * kMlpInPad + (warp >> 2) * 8, kMlpInPad, dw1[0]);
+    put(P + MlpOff::W4 + warp * 8, kMlpHid, dw4[0]);
+    if (warp < 4 && t == 0) {  // every column of the ones product holds db
+        P[MlpOff::b1 + n0 + g] = db1[0]; P[MlpOff::b1 + n0 + g + 8] = db1[2];
+        P[MlpOff::b2 + n0 + g] = db2[0]; P[MlpOff::b2 + n0 + g + 8] = db2[2];
+        P[MlpOff::b3 + n0 + g] = db3[0]; P[MlpOff::b3 + n0 + g + 8] = db3[2];
+    }
+#pragma unroll
+    for (int m = 4; m < 32; m <<= 1)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) db4[q] += __shfl_xor_sync(0xffffffffu, db4[q], m);
+#pragma unroll
+    for (int m = 1; m < 32; m <<= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, m);
+    if (g == 0)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) S.red[warp][(q >> 1) * 8 + 2 * t + (q & 1)] = db4[q];
+    if (lane == 0) S.red[warp][kMlpOutPad] = lsum;
+    __syncthreads();
+    if (tid <= kMlpOutPad) {
+        float s = 0.f;
+        for (int w = 0; w < 8; ++w) s += S.red[w][tid];
+        P[tid < kMlpOutPad ? MlpOff::b4 + tid : MlpOff::total] = s;
+    }
+}
+
+// Sum of entry i over the CTAs' rows of `part`, by the four threads q = 0..3
+// of a quad group 64 threads apart in the block: rows q, q + 4, ... each, then
+// the four in order. `s` holds 256 floats.
+__device__ __forceinline__ float mlp_part_sum(const float* __restrict__ part, int ctas, int i, float* s) {
+    const int q = threadIdx.x >> 6;
+    float v = 0.f;
+    if (i < kMlpPart) {
+#pragma unroll 8
+        for (int c = q; c < ctas; c += 4) v += part[(long long)c * kMlpPart + i];
+    }
+    s[threadIdx.x] = v;
+    __syncthreads();
+    return q == 0 ? ((v + s[threadIdx.x + 64]) + s[threadIdx.x + 128]) + s[threadIdx.x + 192] : 0.f;
+}
+
+// The summed gradient (and loss) of a training launch, without an update.
+__global__ void __launch_bounds__(256) k_mlp_grad_sum(const float* __restrict__ part, int ctas, float* __restrict__ grad,
+                                                      float* __restrict__ loss) {
+    __shared__ float s[256];
+    const int i = blockIdx.x * 64 + (threadIdx.x & 63);
+    const float v = mlp_part_sum(part, ctas, i, s);
+    if (threadIdx.x >= 64) return;
+    if (i < MlpOff::total) grad[i] = v;
+    else if (i == MlpOff::total) *loss = v;
+}
+
+// AdamW on the fp32 master weights from the summed gradients of the step's
+// CTAs; refreshes the bf16 copy, stores the step's loss. Padded entries (input
+// columns >= 10 of W1, output rows >= 10 of W4 and b4) stay zero. 64 parameters a
+// block, four threads each.
+__global__ void __launch_bounds__(256) k_mlp_adam(float* __restrict__ w, __nv_bfloat16* __restrict__ wbf,
+                                                  const float* __restrict__ part, int ctas, float* __restrict__ m1,
+                                                  float* __restrict__ m2, float* __restrict__ loss, float lr, float beta1,
+                                                  float beta2, float eps, float wd, float bc1, float bc2) {
+    __shared__ float s[256];
+    const int i = blockIdx.x * 64 + (threadIdx.x & 63);
+    const float gr = mlp_part_sum(part, ctas, i, s);
+    if (threadIdx.x >= 64) return;
+    if (i >= MlpOff::total) {
+        if (i == MlpOff::total) *loss = gr;
+        return;
+    }
+    bool pad = false;
+    if (i < MlpOff::b1) pad = (i % kMlpInPad) >= kMlpIn;
+    else if (i >= MlpOff::W4 && i < MlpOff::b4) pad = (i - MlpOff::W4) / kMlpHid >= kMlpOut;
+    else if (i >= MlpOff::b4) pad = (i - MlpOff::b4) >= kMlpOut;
+    if (pad) { w[i] = 0.f; wbf[i] = __float2bfloat16_rn(0.f); return; }
+    const bool is_bias = (i >= MlpOff::b1 && i < MlpOff::W2) || (i >= MlpOff::b2 && i < MlpOff::W3) ||
+                         (i >= MlpOff::b3 && i < MlpOff::W4) || i >= MlpOff::b4;
+    const float a = beta1 * m1[i] + (1.f - beta1) * gr;
+    const float b = beta2 * m2[i] + (1.f - beta2) * gr * gr;
+    m1[i] = a;
+    m2[i] = b;
+    float x = w[i];
+    if (!is_bias) x -= lr * wd * x;
+    x -= lr * (a / bc1) / (sqrtf(b / bc2) + eps);
+    w[i] = x;
+    wbf[i] = __float2bfloat16_rn(x);
 }
 
 }  // namespace mpm

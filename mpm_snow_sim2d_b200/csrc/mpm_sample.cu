@@ -14,9 +14,6 @@
 // cells is closer than min_dist. The result depends on the seed alone.
 #include <algorithm>
 #include <cmath>
-#include <cstring>
-#include <string>
-#include <vector>
 
 #include <cuda_runtime.h>
 
@@ -75,39 +72,75 @@ __device__ __forceinline__ bool inside(const SampleShapes& S, int dim, const flo
     return false;
 }
 
-// One phase of one round: cells (3a + px, 3b + py, 3c + pz).
-__global__ void k_sample_phase(SampleGrid G, SampleShapes S, const unsigned char* __restrict__ live, int round,
-                               int px, int py, int pz, float4* __restrict__ cells) {
+// One phase of one round: cells (3a + px, 3b + py, 3c + pz), eight lanes each.
+// The lanes share the cell's candidate and split its 5^(dim-1) rows of five
+// neighbours. Bound: latency. A phase of a reference snowball has 4.6k cells, and
+// the phases run one after the other (30 rounds x 27 of them); with one thread per
+// cell the 125 neighbours were read one after the other, 23 us a phase; here all
+// of a cell's are in flight at once and a phase takes 4.4 us. The launch of the
+// next phase overlaps this one up to griddepcontrol.wait: the candidate, and
+// whether the cell is free (only its own phase, a round ago, can have filled it),
+// depend on nothing later. Reads of `cells` go to L2, since lines read before
+// the wait may hold neighbours of that phase.
+constexpr int kCellLanes = 8;
+
+__global__ void __launch_bounds__(256, 2) k_sample_phase(SampleGrid G, const SampleShapes* __restrict__ shapes,
+                                                      const unsigned char* __restrict__ live, int round, int px, int py,
+                                                      int pz, float4* cells) {
     const int mx = (G.nc[0] - px + 2) / 3, my = (G.nc[1] - py + 2) / 3, mz = G.dim == 3 ? (G.nc[2] - pz + 2) / 3 : 1;
     const long long total = (long long)mx * my * mz;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= total) return;
+    const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / kCellLanes;
+    const int sub = threadIdx.x % kCellLanes;
     const int ix = 3 * int(t % mx) + px, iy = 3 * int((t / mx) % my) + py, iz = G.dim == 3 ? 3 * int(t / ((long long)mx * my)) + pz : 0;
-    if (ix >= G.nc[0] || iy >= G.nc[1] || (G.dim == 3 && iz >= G.nc[2])) return;
     const long long id = ((long long)iz * G.nc[1] + iy) * G.nc[0] + ix;
-    if (!live[id] || cells[id].w != 0.f) return;
-    const int ic[3] = {ix, iy, iz};
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    bool ok = t < total && ix < G.nc[0] && iy < G.nc[1] && (G.dim != 3 || iz < G.nc[2]);
+    ok = ok && live[id] && __ldcg(&cells[id]).w == 0.f;
     float p[3] = {0.f, 0.f, 0.f};
-    for (int k = 0; k < G.dim; ++k)
-        p[k] = __fadd_rn(G.origin[k], __fmul_rn(__fadd_rn(float(ic[k]), uniform01(G.seed, id, round, k)), G.cell));
-    if (!inside(S, G.dim, p)) return;
-    const float r2 = __fmul_rn(G.min_dist, G.min_dist);
-    const int zr = G.dim == 3 ? 2 : 0;
-    for (int dz = -zr; dz <= zr; ++dz)
-        for (int dy = -2; dy <= 2; ++dy)
-            for (int dx = -2; dx <= 2; ++dx) {
-                const int jx = ix + dx, jy = iy + dy, jz = iz + dz;
-                if (jx < 0 || jy < 0 || jz < 0 || jx >= G.nc[0] || jy >= G.nc[1] || (G.dim == 3 && jz >= G.nc[2])) continue;
-                const float4 q = cells[((long long)jz * G.nc[1] + jy) * G.nc[0] + jx];
-                if (q.w == 0.f) continue;
-                const float ddx = __fsub_rn(q.x, p[0]), ddy = __fsub_rn(q.y, p[1]), ddz = __fsub_rn(q.z, p[2]);
-                if (__fadd_rn(__fadd_rn(__fmul_rn(ddx, ddx), __fmul_rn(ddy, ddy)), __fmul_rn(ddz, ddz)) < r2) return;
+    if (ok) {
+        const int ic[3] = {ix, iy, iz};
+#pragma unroll
+        for (int k = 0; k < 3; ++k)
+            if (k < G.dim)
+                p[k] = __fadd_rn(G.origin[k], __fmul_rn(__fadd_rn(float(ic[k]), uniform01(G.seed, id, round, k)), G.cell));
+        ok = inside(*shapes, G.dim, p);
+    }
+    // (the pointer passes through the wait, so that no later load can move ahead of it)
+    asm volatile("griddepcontrol.wait;" : "+l"(cells) : : "memory");
+    // the cell's lanes agree on `ok`; all lanes of the warp stay for the vote
+    bool clash = false;
+    if (ok) {
+        const float r2 = __fmul_rn(G.min_dist, G.min_dist);
+        const int rows = G.dim == 3 ? 25 : 5;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int r = sub + q * kCellLanes;
+            const int jy = iy + r % 5 - 2, jz = G.dim == 3 ? iz + r / 5 - 2 : 0;
+            const bool in = r < rows && jy >= 0 && jy < G.nc[1] && jz >= 0 && jz < G.nc[2];
+            const long long row = ((long long)jz * G.nc[1] + jy) * G.nc[0];
+            float4 n[5];
+#pragma unroll
+            for (int dx = 0; dx < 5; ++dx) {
+                const int jx = ix + dx - 2;
+                n[dx] = in && jx >= 0 && jx < G.nc[0] ? __ldcg(&cells[row + jx]) : make_float4(0.f, 0.f, 0.f, 0.f);
             }
-    cells[id] = make_float4(p[0], p[1], p[2], 1.f);
+#pragma unroll
+            for (int dx = 0; dx < 5; ++dx) {
+                const float ddx = __fsub_rn(n[dx].x, p[0]), ddy = __fsub_rn(n[dx].y, p[1]), ddz = __fsub_rn(n[dx].z, p[2]);
+                clash = clash || (n[dx].w != 0.f &&
+                                  __fadd_rn(__fadd_rn(__fmul_rn(ddx, ddx), __fmul_rn(ddy, ddy)), __fmul_rn(ddz, ddz)) < r2);
+            }
+        }
+    }
+    const unsigned any = __ballot_sync(0xffffffffu, clash);
+    const int first = (threadIdx.x & 31) / kCellLanes * kCellLanes;
+    if (ok && sub == 0 && ((any >> first) & ((1u << kCellLanes) - 1)) == 0u) cells[id] = make_float4(p[0], p[1], p[2], 1.f);
 }
 
 // Cells that can hold a sample: those overlapping a shape's bounding box.
-__global__ void k_sample_live(SampleGrid G, SampleShapes S, long long ncells, unsigned char* __restrict__ live) {
+__global__ void k_sample_live(SampleGrid G, const SampleShapes* __restrict__ shapes, long long ncells,
+                              unsigned char* __restrict__ live) {
+    const SampleShapes& S = *shapes;
     const long long id = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (id >= ncells) return;
     const int ic[3] = {int(id % G.nc[0]), int((id / G.nc[0]) % G.nc[1]), int(id / ((long long)G.nc[0] * G.nc[1]))};
@@ -125,19 +158,65 @@ __global__ void k_sample_live(SampleGrid G, SampleShapes S, long long ncells, un
 }
 
 // Which shape a sample belongs to (the first that contains it).
-int shape_index(const SampleShapes& S, int dim, const float* p) {
+__device__ __forceinline__ int shape_index(const SampleShapes& S, int dim, const float* p) {
     for (int s = 0; s < S.n; ++s) {
         if (S.kind[s] == MPM_SHAPE_BALL) {
             float d2 = 0.f;
-            for (int k = 0; k < dim; ++k) { const float d = p[k] - S.c[s][k]; d2 += d * d; }
-            if (d2 <= S.r[s] * S.r[s]) return s;
+            for (int k = 0; k < dim; ++k) {
+                const float d = __fsub_rn(p[k], S.c[s][k]);
+                d2 = __fadd_rn(d2, __fmul_rn(d, d));
+            }
+            if (d2 <= __fmul_rn(S.r[s], S.r[s])) return s;
         } else {
             bool in = true;
-            for (int k = 0; k < dim; ++k) in = in && std::fabs(p[k] - S.c[s][k]) <= S.h[s][k];
+            for (int k = 0; k < dim; ++k) in = in && fabsf(__fsub_rn(p[k], S.c[s][k])) <= S.h[s][k];
             if (in) return s;
         }
     }
     return -1;
+}
+
+// The samples in cell order (deterministic): how many in each block of
+// kCompact cells, then each block's to its place in the output (the first
+// `capacity` of them; `total` gets the number of all). The host used to scan the
+// whole cell array, 1.1 ms of its copy and scan for a reference snowball.
+constexpr int kCompact = 1024;
+
+__global__ void __launch_bounds__(kCompact) k_sample_count(const float4* __restrict__ cells, long long ncells,
+                                                           int* __restrict__ count) {
+    const long long i = (long long)blockIdx.x * kCompact + threadIdx.x;
+    const int n = __syncthreads_count(i < ncells && cells[i].w != 0.f);
+    if (threadIdx.x == 0) count[blockIdx.x] = n;
+}
+
+__global__ void __launch_bounds__(kCompact) k_sample_compact(const SampleShapes* __restrict__ shapes, int dim,
+                                                             const float4* __restrict__ cells, long long ncells,
+                                                             const int* __restrict__ count, long long capacity,
+                                                             float* __restrict__ pos, int* __restrict__ owner,
+                                                             unsigned long long* __restrict__ total) {
+    __shared__ unsigned long long s_before;
+    __shared__ int s_warp[kCompact / 32];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    if (tid == 0) s_before = 0ull;
+    __syncthreads();
+    unsigned long long b = 0ull;
+    for (int k = tid; k < (int)blockIdx.x; k += kCompact) b += (unsigned)count[k];
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) b += __shfl_xor_sync(0xffffffffu, b, o);
+    if (lane == 0 && b) atomicAdd(&s_before, b);
+    const long long i = (long long)blockIdx.x * kCompact + tid;
+    const float4 q = i < ncells ? cells[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const unsigned mine = __ballot_sync(0xffffffffu, q.w != 0.f);
+    if (lane == 0) s_warp[warp] = __popc(mine);
+    __syncthreads();
+    unsigned long long at = s_before + __popc(mine & ((1u << lane) - 1));
+    for (int w = 0; w < warp; ++w) at += s_warp[w];
+    if (q.w != 0.f && (long long)at < capacity) {
+        const float p[3] = {q.x, q.y, q.z};
+        for (int k = 0; k < dim; ++k) pos[at * dim + k] = p[k];
+        if (owner) owner[at] = shape_index(*shapes, dim, p);
+    }
+    if (blockIdx.x == gridDim.x - 1 && tid == kCompact - 1) *total = at + (q.w != 0.f);
 }
 
 }  // namespace
@@ -182,57 +261,72 @@ mpm_status mpm_sample_shapes(int32_t dim, const mpm_shape* shapes, int32_t nshap
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) { cudaGetLastError(); return MPM_ERR_NO_DEVICE; }
     const long long ncells = (long long)ncd;
-    float4* cells = nullptr;
-    unsigned char* live = nullptr;
-    if (cudaMalloc(&cells, sizeof(float4) * ncells) != cudaSuccess ||
-        cudaMalloc(&live, (size_t)ncells) != cudaSuccess) {
-        if (cells) cudaFree(cells);
+    // one allocation: the cells, the shapes, the output, which cells can hold a sample
+    const long long room = std::min<long long>(capacity, ncells), blocks = (ncells + kCompact - 1) / kCompact;
+    size_t bytes = 0;
+    auto take = [&](size_t n) { const size_t at = bytes; bytes += (n + 255) / 256 * 256; return at; };
+    const size_t cell_bytes = sizeof(float4) * (size_t)ncells;
+    const size_t o_cells = take(cell_bytes), o_shapes = take(sizeof(SampleShapes)), o_total = take(sizeof(unsigned long long)),
+                 o_count = take(sizeof(int) * (size_t)blocks), o_pos = take(sizeof(float) * (size_t)(room * dim)),
+                 o_owner = take(shape_of ? sizeof(int) * (size_t)room : 0), o_live = take((size_t)ncells);
+    unsigned char* base = nullptr;
+    if (cudaMalloc(&base, bytes) != cudaSuccess) {
         cudaGetLastError();
         return MPM_ERR_OUT_OF_MEMORY;
     }
-    mpm_status st = MPM_OK;
-    if (cudaMemset(cells, 0, sizeof(float4) * ncells) != cudaSuccess) {
+    float4* cells = reinterpret_cast<float4*>(base + o_cells);
+    SampleShapes* dshapes = reinterpret_cast<SampleShapes*>(base + o_shapes);
+    unsigned long long* dtotal = reinterpret_cast<unsigned long long*>(base + o_total);
+    int *dcount = reinterpret_cast<int*>(base + o_count), *downer = shape_of ? reinterpret_cast<int*>(base + o_owner) : nullptr;
+    float* dpos = reinterpret_cast<float*>(base + o_pos);
+    unsigned char* live = base + o_live;
+    if (cudaMemset(cells, 0, cell_bytes) != cudaSuccess ||
+        cudaMemcpy(dshapes, &S, sizeof(S), cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaGetLastError();
-        cudaFree(cells);
-        cudaFree(live);
+        cudaFree(base);
         return MPM_ERR_CUDA;
     }
     const int threads = 256;
-    k_sample_live<<<(unsigned)((ncells + threads - 1) / threads), threads>>>(G, S, ncells, live);
+    k_sample_live<<<(unsigned)((ncells + threads - 1) / threads), threads>>>(G, dshapes, ncells, live);
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t lc = {};
+    lc.blockDim = dim3(threads);
+    lc.attrs = attr;
+    lc.numAttrs = 0;  // the first phase waits for all of k_sample_live
+    cudaError_t le = cudaGetLastError();
     const int pz_n = dim == 3 ? 3 : 1;
-    for (int r = 0; r < rounds; ++r)
+    for (int r = 0; r < rounds && le == cudaSuccess; ++r)
         for (int pz = 0; pz < pz_n; ++pz)
             for (int py = 0; py < 3; ++py)
                 for (int px = 0; px < 3; ++px) {
                     const long long mx = (G.nc[0] - px + 2) / 3, my = (G.nc[1] - py + 2) / 3,
                                     mz = dim == 3 ? (G.nc[2] - pz + 2) / 3 : 1;
-                    const long long total = mx * my * mz;
-                    if (total > 0)
-                        k_sample_phase<<<(unsigned)((total + threads - 1) / threads), threads>>>(G, S, live, r, px, py,
-                                                                                                 pz, cells);
+                    const long long lanes = mx * my * mz * kCellLanes;
+                    if (lanes == 0 || le != cudaSuccess) continue;
+                    lc.gridDim = dim3((unsigned)((lanes + threads - 1) / threads));
+                    le = cudaLaunchKernelEx(&lc, k_sample_phase, G, (const SampleShapes*)dshapes,
+                                            (const unsigned char*)live, r, px, py, pz, cells);
+                    lc.numAttrs = 1;
                 }
-    std::vector<float4> h(ncells);
-    if (cudaGetLastError() != cudaSuccess ||
-        cudaMemcpy(h.data(), cells, sizeof(float4) * ncells, cudaMemcpyDeviceToHost) != cudaSuccess) {
+    unsigned long long total = 0;
+    if (le == cudaSuccess) {
+        k_sample_count<<<(unsigned)blocks, kCompact>>>(cells, ncells, dcount);
+        k_sample_compact<<<(unsigned)blocks, kCompact>>>(dshapes, dim, cells, ncells, dcount, room, dpos, downer, dtotal);
+        le = cudaGetLastError();
+    }
+    if (le == cudaSuccess) le = cudaMemcpy(&total, dtotal, sizeof(total), cudaMemcpyDeviceToHost);
+    const size_t n = (size_t)std::min<unsigned long long>(total, (unsigned long long)room);
+    if (le == cudaSuccess && n > 0) le = cudaMemcpy(positions, dpos, sizeof(float) * n * dim, cudaMemcpyDeviceToHost);
+    if (le == cudaSuccess && n > 0 && shape_of) le = cudaMemcpy(shape_of, downer, sizeof(int) * n, cudaMemcpyDeviceToHost);
+    cudaFree(base);
+    if (le != cudaSuccess) {
         cudaGetLastError();
-        st = MPM_ERR_CUDA;
+        return MPM_ERR_CUDA;
     }
-    cudaFree(cells);
-    cudaFree(live);
-    if (st != MPM_OK) return st;
-    // compaction in cell order (deterministic)
-    int64_t n = 0;
-    for (long long i = 0; i < ncells; ++i) {
-        if (h[i].w == 0.f) continue;
-        if (n < capacity) {
-            const float p[3] = {h[i].x, h[i].y, h[i].z};
-            for (int k = 0; k < dim; ++k) positions[n * dim + k] = p[k];
-            if (shape_of) shape_of[n] = shape_index(S, dim, p);
-        }
-        ++n;
-    }
-    *count = n;
-    return n > capacity ? MPM_ERR_CAPACITY : MPM_OK;
+    *count = (int64_t)total;
+    return (int64_t)total > capacity ? MPM_ERR_CAPACITY : MPM_OK;
 }
 
 }  // extern "C"

@@ -21,6 +21,7 @@
 #include "mpm_mlp.cuh"
 #include "mpm_render.cuh"
 #include "mpm_host.h"
+#include "mpm_readback.h"
 
 using namespace mpm;
 
@@ -42,6 +43,8 @@ struct mpm_mlp {
 };
 
 struct mpm_solver {
+    ReadbackUser readback;
+    DeviceArena arena;  // every device array below but those made on demand
     mpm_params params{};
     int dim = 2, form = kMLS;
     int stencil = 4;  // nodes per axis: 4 cubic (MLS, CLASSIC), 3 quadratic (QUAD)
@@ -163,44 +166,19 @@ template <typename T> cudaError_t dalloc(T** p, size_t count) {
 }
 
 void release(mpm_solver* s) {
-    float* fl[] = {s->x, s->v, s->B, s->Fe, s->Jp, s->A, s->mass, s->vol, s->staging};
-    for (float* p : fl)
-        if (p) cudaFree(p);
-    if (s->id) cudaFree(s->id);
-    if (s->acc) cudaFree(s->acc);
-    if (s->gv) cudaFree(s->gv);
-    if (s->status) cudaFree(s->status);
-    float* al[] = {s->alt.x, s->alt.v, s->alt.B, s->alt.Fe, s->alt.Jp, s->alt.A, s->alt.mass, s->alt.vol};
-    for (float* p : al)
-        if (p) cudaFree(p);
-    if (s->alt.id) cudaFree(s->alt.id);
-    int* ti[] = {s->ti.key,      s->ti.tile_count, s->ti.tile_cursor, s->ti.tile_start, s->ti.mark, s->ti.mark_list,
-                 s->ti.n_marked, s->ti.perm,       s->ti.tile_list,   s->ti.n_tile_list, s->ti.sval,
-                 s->ti.p2g_next};
-    if (s->ti.skey) cudaFree(s->ti.skey);
-    for (int* p : ti)
-        if (p) cudaFree(p);
+    if (s->staging) cudaFree(s->staging);
+    if (s->render_fb) cudaFree(s->render_fb);
+    if (s->render_rgb) cudaFree(s->render_rgb);
     for (auto& row : s->period_graph)
         for (auto& g : row)
             if (g) cudaGraphExecDestroy(g);
-    if (s->vmax_dev) cudaFree(s->vmax_dev);
     if (s->vmax_host) cudaFreeHost(s->vmax_host);
     for (auto ev : s->vmax_event)
         if (ev) cudaEventDestroy(ev);
     if (s->mlp_counters) cudaFree(s->mlp_counters);
     if (s->log_data) cudaFree(s->log_data);
     if (s->log_n) cudaFree(s->log_n);
-    if (s->q.list) cudaFree(s->q.list);
-    if (s->q.count) cudaFree(s->q.count);
-    if (s->q.fh) cudaFree(s->q.fh);
-    if (s->q.win) cudaFree(s->q.win);
-    if (s->ti.tile_len) cudaFree(s->ti.tile_len);
-    if (s->ti.fused_next) cudaFree(s->ti.fused_next);
-    int* more[] = {s->ti.n_items, s->ti.grid_done};
-    for (int* p : more)
-        if (p) cudaFree(p);
-    if (s->ti.items) cudaFree(s->ti.items);
-    if (s->ti.scan) cudaFree(s->ti.scan);
+    s->arena.release();
     if (s->own_stream) cudaStreamDestroy(s->own_stream);
 }
 
@@ -585,20 +563,16 @@ mpm_status setup_tiled(mpm_solver* s) {
         ti.n_tiles *= ti.tiles[k];
         ti.n_blocks *= ti.nblk[k];
     }
-    if (dalloc(&ti.key, (size_t)n) || dalloc(&ti.tile_count, (size_t)ti.n_tiles) ||
-        dalloc(&ti.tile_cursor, (size_t)ti.n_tiles) || dalloc(&ti.tile_start, (size_t)ti.n_tiles) ||
-        dalloc(&ti.mark, (size_t)ti.n_blocks) || dalloc(&ti.mark_list, (size_t)ti.n_blocks) ||
-        dalloc(&ti.n_marked, 1) || dalloc(&ti.p2g_next, 1) ||
-        dalloc(&ti.perm, (size_t)n) || dalloc(&ti.tile_list, (size_t)ti.n_tiles) || dalloc(&ti.n_tile_list, 1) ||
-        dalloc(&ti.skey, (size_t)n) || dalloc(&ti.sval, (size_t)n) ||
-        dalloc(&s->alt.x, (size_t)n * D) || dalloc(&s->alt.v, (size_t)n * D) || dalloc(&s->alt.B, (size_t)n * D * D) ||
-        dalloc(&s->alt.Fe, (size_t)n * D * D) || dalloc(&s->alt.Jp, (size_t)n) || dalloc(&s->alt.id, (size_t)n) ||
-        dalloc(&s->A, (size_t)n * D * D) || dalloc(&s->alt.A, (size_t)n * D * D)) {
-        cudaGetLastError();
-        return MPM_ERR_OUT_OF_MEMORY;
-    }
-    if (s->mass && dalloc(&s->alt.mass, (size_t)n)) return MPM_ERR_OUT_OF_MEMORY;
-    if (s->vol && dalloc(&s->alt.vol, (size_t)n)) return MPM_ERR_OUT_OF_MEMORY;
+    const size_t N = (size_t)n, tiles = (size_t)ti.n_tiles, blocks = (size_t)ti.n_blocks;
+    DeviceArena& arena = s->arena;
+    arena.want(&ti.key, N).want(&ti.tile_count, tiles).want(&ti.tile_cursor, tiles).want(&ti.tile_start, tiles);
+    arena.want(&ti.mark, blocks).want(&ti.mark_list, blocks).want(&ti.n_marked, 1).want(&ti.p2g_next, 1);
+    arena.want(&ti.perm, N).want(&ti.tile_list, tiles).want(&ti.n_tile_list, 1).want(&ti.skey, N).want(&ti.sval, N);
+    arena.want(&s->alt.x, N * D).want(&s->alt.v, N * D).want(&s->alt.B, N * D * D).want(&s->alt.Fe, N * D * D);
+    arena.want(&s->alt.Jp, N).want(&s->alt.id, N).want(&s->A, N * D * D).want(&s->alt.A, N * D * D);
+    if (s->mass) arena.want(&s->alt.mass, N);
+    if (s->vol) arena.want(&s->alt.vol, N);
+    if (!arena.allocate()) return MPM_ERR_OUT_OF_MEMORY;
     bool ok = cudaMemset(ti.tile_count, 0, sizeof(int) * ti.n_tiles) == cudaSuccess &&
               cudaMemset(ti.tile_cursor, 0, sizeof(int) * ti.n_tiles) == cudaSuccess &&
               cudaMemset(ti.mark, 0, sizeof(int) * ti.n_blocks) == cudaSuccess &&
@@ -647,23 +621,16 @@ mpm_status setup_tiled(mpm_solver* s) {
         s->direct = !s->box_tma && (D == 2 || s->stencil == 3 || windows <= 6 * warps);
         s->direct_grid = (int)std::max(1ll, std::min((long long)s->sms * (MPM_FUSED_MIN_BLOCKS), windows + ti.n_tiles));
         ti.item_win = s->direct ? 1 : 0;
-        const size_t most_items = (size_t)ti.n_tiles + (s->direct ? (size_t)n / (size_t)ti.win : 0);
-        if (dalloc(&ti.items, most_items) || dalloc(&ti.n_items, 1) || dalloc(&ti.grid_done, 1) ||
-            dalloc(&ti.scan, (size_t)(ti.n_tiles + kScanTiles - 1) / kScanTiles) ||
-            cudaMemset(ti.grid_done, 0, sizeof(int)) != cudaSuccess ||
-            cudaMemset(ti.n_items, 0, sizeof(int)) != cudaSuccess) {
-            cudaGetLastError();
-            return MPM_ERR_OUT_OF_MEMORY;
-        }
+        arena.want(&ti.items, tiles + (s->direct ? N / (size_t)ti.win : 0)).want(&ti.n_items, 1).want(&ti.grid_done, 1);
     }
+    arena.want(&ti.scan, (tiles + kScanTiles - 1) / kScanTiles).want(&ti.tile_len, tiles).want(&ti.fused_next, 1);
     // windows of a sort: at most ceil(m / win) per tile of m slots
     s->q.win_capacity = s->q.capacity / ti.win + ti.n_tiles + 1;
-    if (dalloc(&s->q.list, (size_t)s->q.capacity) || dalloc(&s->q.count, 2) ||
-        dalloc(&s->q.fh, (size_t)s->q.capacity * D * D) || dalloc(&s->q.win, (size_t)s->q.win_capacity) ||
-        dalloc(&ti.tile_len, (size_t)ti.n_tiles) || dalloc(&ti.fused_next, 1)) {
-        cudaGetLastError();
-        return MPM_ERR_OUT_OF_MEMORY;
-    }
+    arena.want(&s->q.list, (size_t)s->q.capacity).want(&s->q.count, 2);
+    arena.want(&s->q.fh, (size_t)s->q.capacity * D * D).want(&s->q.win, (size_t)s->q.win_capacity).want(&s->vmax_dev, 2);
+    if (!arena.allocate()) return MPM_ERR_OUT_OF_MEMORY;
+    if (cudaMemset(ti.grid_done, 0, sizeof(int)) != cudaSuccess || cudaMemset(ti.n_items, 0, sizeof(int)) != cudaSuccess)
+        return MPM_ERR_CUDA;
     s->q.nwin = s->q.count + 1;
     ti.zero[0] = ti.fused_next;
     ti.zero[1] = s->q.count;
@@ -711,8 +678,7 @@ mpm_status setup_tiled(mpm_solver* s) {
     s->cur_K = s->sort_period;
     s->next_sort = 0;
     if (s->sort_period > mpm_solver::kMaxPeriod) s->use_graphs = false;  // graphs are cached per period up to 64
-    if (dalloc(&s->vmax_dev, 2) ||
-        cudaHostAlloc(&s->vmax_host, 2 * sizeof(unsigned), cudaHostAllocDefault) != cudaSuccess ||
+    if (cudaHostAlloc(&s->vmax_host, 2 * sizeof(unsigned), cudaHostAllocDefault) != cudaSuccess ||
         cudaEventCreateWithFlags(&s->vmax_event[0], cudaEventDisableTiming) != cudaSuccess ||
         cudaEventCreateWithFlags(&s->vmax_event[1], cudaEventDisableTiming) != cudaSuccess) {
         cudaGetLastError();
@@ -740,8 +706,6 @@ mpm_status validate(const mpm_params* p, std::string& why) { return validate_par
 mpm_status ensure_staging(mpm_solver* s, size_t floats) {
     if (floats <= s->staging_floats) return MPM_OK;
     if (s->staging) cudaFree(s->staging);
-    if (s->render_fb) cudaFree(s->render_fb);
-    if (s->render_rgb) cudaFree(s->render_rgb);
     s->staging = nullptr;
     s->staging_floats = 0;
     MPM_CUDA(s, dalloc(&s->staging, floats));
@@ -749,16 +713,36 @@ mpm_status ensure_staging(mpm_solver* s, size_t floats) {
     return MPM_OK;
 }
 
-// Device SoA field -> host interleaved array in creation order.
-mpm_status export_field(mpm_solver* s, const float* soa, int comps, float* host) {
-    if (s->n == 0) return MPM_OK;
-    mpm_status st = ensure_staging(s, (size_t)s->n * comps);
+// Device SoA fields -> host interleaved arrays in creation order: one kernel and
+// one read (ReadbackRing) for all of them while they are small together, else
+// field by field, so that the staging buffer holds no more than one large field.
+mpm_status export_fields(mpm_solver* s, ExportFields E, float* const* host) {
+    if (s->n == 0 || E.fields == 0) return MPM_OK;
+    size_t floats = 0;
+    for (int f = 0; f < E.fields; ++f) floats += (size_t)s->n * E.comps[f];
+    if (E.fields > 1 && floats * sizeof(float) > ReadbackRing::kLarge) {
+        for (int f = 0; f < E.fields; ++f) {
+            ExportFields one{{E.src[f]}, {E.comps[f]}, {0}, 1};
+            const mpm_status st = export_fields(s, one, host + f);
+            if (st != MPM_OK) return st;
+        }
+        return MPM_OK;
+    }
+    mpm_status st = ensure_staging(s, floats);
     if (st != MPM_OK) return st;
+    void* dst[ExportFields::MAX];
+    size_t bytes[ExportFields::MAX];
+    long long at = 0;
+    for (int f = 0; f < E.fields; ++f) {
+        E.at[f] = at;
+        at += (long long)s->n * E.comps[f];
+        dst[f] = host[f];
+        bytes[f] = sizeof(float) * (size_t)s->n * E.comps[f];
+    }
     const int threads = 256, blocks = (s->n + threads - 1) / threads;
-    k_export_soa<<<blocks, threads, 0, s->stream>>>(soa, comps, s->n, s->id, s->staging);
+    k_export_fields<<<blocks, threads, 0, s->stream>>>(E, s->n, s->id, s->staging);
     MPM_CUDA(s, cudaGetLastError());
-    MPM_CUDA(s, cudaMemcpyAsync(host, s->staging, sizeof(float) * (size_t)s->n * comps, cudaMemcpyDeviceToHost, s->stream));
-    MPM_CUDA(s, cudaStreamSynchronize(s->stream));
+    MPM_CUDA(s, ReadbackRing::get().read_parts(s->stream, s->staging, dst, bytes, E.fields));
     return MPM_OK;
 }
 
@@ -951,13 +935,11 @@ mpm_status mpm_create(const mpm_params* params, const mpm_particles_init* init, 
     auto bail = [&](mpm_status code) { release(s); delete s; return code; };
     if (cudaStreamCreateWithFlags(&s->own_stream, cudaStreamNonBlocking) != cudaSuccess) return bail(MPM_ERR_CUDA);
     s->stream = s->own_stream;
-    if (dalloc(&s->x, (size_t)n * D) || dalloc(&s->v, (size_t)n * D) || dalloc(&s->B, (size_t)n * D * D) ||
-        dalloc(&s->Fe, (size_t)n * D * D) || dalloc(&s->Jp, (size_t)n) || dalloc(&s->id, (size_t)n) ||
-        dalloc(&s->acc, (size_t)nacc(D, s->form) * s->nodes) || dalloc(&s->gv, (size_t)s->nodes * (D == 3 ? 2 : 1)) ||
-        dalloc(&s->status, 1)) {
-        cudaGetLastError();
-        return bail(MPM_ERR_OUT_OF_MEMORY);
-    }
+    const size_t N = (size_t)n;
+    s->arena.want(&s->x, N * D).want(&s->v, N * D).want(&s->B, N * D * D).want(&s->Fe, N * D * D).want(&s->Jp, N);
+    s->arena.want(&s->id, N).want(&s->acc, (size_t)nacc(D, s->form) * s->nodes);
+    s->arena.want(&s->gv, (size_t)s->nodes * (D == 3 ? 2 : 1)).want(&s->status, 1);
+    if (!s->arena.allocate()) return bail(MPM_ERR_OUT_OF_MEMORY);
 
     // Host-side preparation: mass = vol * RHO / 100 when not given
     // (src/cpu/Particles.cpp:18, src/gpu/GPUSolver.cpp:119,148).
@@ -978,13 +960,13 @@ mpm_status mpm_create(const mpm_params* params, const mpm_particles_init* init, 
     choose_scales(s, total_mass);
     if (uni_m && n > 0) s->mass_u = massv[0];
     else if (n > 0) {
-        if (dalloc(&s->mass, (size_t)n)) return bail(MPM_ERR_OUT_OF_MEMORY);
+        if (!s->arena.want(&s->mass, N).allocate()) return bail(MPM_ERR_OUT_OF_MEMORY);
         if (cudaMemcpy(s->mass, massv.data(), sizeof(float) * n, cudaMemcpyHostToDevice) != cudaSuccess)
             return bail(MPM_ERR_CUDA);
     }
     if (uni_v && n > 0) s->vol_u = volv[0];
     else if (n > 0) {
-        if (dalloc(&s->vol, (size_t)n)) return bail(MPM_ERR_OUT_OF_MEMORY);
+        if (!s->arena.want(&s->vol, N).allocate()) return bail(MPM_ERR_OUT_OF_MEMORY);
         if (cudaMemcpy(s->vol, volv.data(), sizeof(float) * n, cudaMemcpyHostToDevice) != cudaSuccess)
             return bail(MPM_ERR_CUDA);
     }
@@ -1115,20 +1097,25 @@ mpm_status mpm_get_info(const mpm_solver* s, int64_t* count, int32_t* dim) {
 mpm_status mpm_get_positions(mpm_solver* s, float* out, size_t cap_floats) {
     if (!s || (!out && s->n > 0)) return fail(s, MPM_ERR_INVALID_ARGUMENT, "out is NULL");
     if (cap_floats < (size_t)s->n * s->dim) return fail(s, MPM_ERR_CAPACITY, "output capacity below count * dim");
-    return export_field(s, s->x, s->dim, out);
+    return export_fields(s, ExportFields{{s->x}, {s->dim}, {0}, 1}, &out);
 }
 
 mpm_status mpm_get_state(mpm_solver* s, mpm_state_host* st) {
     if (!s || !st) return MPM_ERR_INVALID_ARGUMENT;
     if (st->count != s->n) return fail(s, MPM_ERR_CAPACITY, "state.count must equal the particle count");
     const int D = s->dim;
-    mpm_status r = MPM_OK;
-    if (st->position && (r = export_field(s, s->x, D, st->position)) != MPM_OK) return r;
-    if (st->velocity && (r = export_field(s, s->v, D, st->velocity)) != MPM_OK) return r;
-    if (st->affine_b && (r = export_field(s, s->B, D * D, st->affine_b)) != MPM_OK) return r;
-    if (st->elastic_f && (r = export_field(s, s->Fe, D * D, st->elastic_f)) != MPM_OK) return r;
-    if (st->plastic_det && (r = export_field(s, s->Jp, 1, st->plastic_det)) != MPM_OK) return r;
-    return MPM_OK;
+    const float* src[] = {s->x, s->v, s->B, s->Fe, s->Jp};
+    const int comps[] = {D, D, D * D, D * D, 1};
+    float* const given[] = {st->position, st->velocity, st->affine_b, st->elastic_f, st->plastic_det};
+    ExportFields E{};
+    float* host[ExportFields::MAX];
+    for (int f = 0; f < 5; ++f) {
+        if (!given[f]) continue;
+        E.src[E.fields] = src[f];
+        E.comps[E.fields] = comps[f];
+        host[E.fields++] = given[f];
+    }
+    return export_fields(s, E, host);
 }
 
 mpm_status mpm_set_state(mpm_solver* s, const mpm_state_host* st) {
@@ -1925,8 +1912,7 @@ mpm_status mpm_render(mpm_solver* s, const mpm_render_params* p, uint8_t* rgb, s
         k_render_points<<<(s->n + threads - 1) / threads, threads, 0, s->stream>>>(V, s->x, s->n, s->render_fb);
     k_render_pack<<<pblocks, threads, 0, s->stream>>>(s->render_fb, pixels, s->render_rgb);
     MPM_CUDA(s, cudaGetLastError());
-    MPM_CUDA(s, cudaMemcpyAsync(rgb, s->render_rgb, (size_t)pixels * 3, cudaMemcpyDeviceToHost, s->stream));
-    MPM_CUDA(s, cudaStreamSynchronize(s->stream));
+    MPM_CUDA(s, ReadbackRing::get().read(s->stream, s->render_rgb, rgb, (size_t)pixels * 3));
     return MPM_OK;
 }
 

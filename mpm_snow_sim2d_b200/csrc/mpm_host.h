@@ -1,9 +1,12 @@
 // Host-side set-up shared by the single-scene solver and the batched scenes:
-// parameter validation, per-scene step constants, fixed-point scales.
+// parameter validation, per-scene step constants, fixed-point scales, device arrays.
 #pragma once
 
 #include <cmath>
 #include <string>
+#include <vector>
+
+#include <cuda_runtime.h>
 
 #include "mpm/mpm.h"
 #include "mpm_kernels.cuh"
@@ -72,5 +75,46 @@ inline void fixed_point_scales(const mpm_params& p, double total_mass, StepConst
     C.inv_sf = std::ldexp(1.0f, -lf);
     C.v_cap = (float)v_cap;
 }
+
+// The device arrays of a solver or batch, a group in one allocation: a cudaMalloc
+// takes up to 0.5 ms and a cudaFree 0.3, and a solver has about fifty arrays
+// (a solver of 3.8M particles: 230 ms to create and 10 to destroy with an allocation
+// each, 173 and 3.5 with four).
+class DeviceArena {
+public:
+    template <typename T> DeviceArena& want(T** p, size_t count) {
+        *p = nullptr;
+        wanted_.push_back({reinterpret_cast<void**>(p), bytes_});
+        bytes_ += ((count ? count : 1) * sizeof(T) + 255) / 256 * 256;
+        return *this;
+    }
+    // Sets the pointers wanted since the last call; false when memory is out.
+    bool allocate() {
+        char* base = nullptr;
+        const bool ok = cudaMalloc(reinterpret_cast<void**>(&base), bytes_ ? bytes_ : 256) == cudaSuccess;
+        if (ok) {
+            blocks_.push_back(base);
+            for (const Want& w : wanted_) *w.p = base + w.at;
+        } else {
+            cudaGetLastError();
+        }
+        wanted_.clear();
+        bytes_ = 0;
+        return ok;
+    }
+    void release() {
+        for (char* b : blocks_) cudaFree(b);
+        blocks_.clear();
+    }
+
+private:
+    struct Want {
+        void** p;
+        size_t at;
+    };
+    std::vector<Want> wanted_;
+    std::vector<char*> blocks_;
+    size_t bytes_ = 0;
+};
 
 }  // namespace mpm

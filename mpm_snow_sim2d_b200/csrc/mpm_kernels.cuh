@@ -998,12 +998,22 @@ __global__ void __launch_bounds__(256) k_g2p_plastic(Particles P, StepConsts C, 
 // ---------------------------------------------------------------------------
 // Import / export between the caller's interleaved per-particle arrays (in
 // creation order) and the device SoA (in slot order; slot s holds particle id[s]).
-static __global__ void k_export_soa(const float* __restrict__ soa, int comps, int n, const int* __restrict__ id,
-                             float* __restrict__ aos) {
+struct ExportFields {
+    static constexpr int MAX = 5;
+    const float* src[MAX];
+    int comps[MAX];
+    long long at[MAX];  // first float of the field in the output
+    int fields;
+};
+
+static __global__ void k_export_fields(ExportFields E, int n, const int* __restrict__ id, float* __restrict__ aos) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const int p = id ? id[s] : s;
-    for (int c = 0; c < comps; ++c) aos[(long long)p * comps + c] = soa[(long long)c * n + s];
+    for (int f = 0; f < E.fields; ++f) {
+        float* out = aos + E.at[f] + (long long)p * E.comps[f];
+        for (int c = 0; c < E.comps[f]; ++c) out[c] = E.src[f][(long long)c * n + s];
+    }
 }
 
 static __global__ void k_import_soa(float* __restrict__ soa, int comps, int n, const int* __restrict__ id,

@@ -353,20 +353,23 @@ MPM_API mpm_status mpm_render(mpm_solver* solver, const mpm_render_params* param
 /* ---- Batched scenes (2D MLS) -------------------------------------------
  * Many independent scenes, each a full solver in the sense of mpm_create
  * (the reference constructs one Solver per process, src/main.cpp:164-174),
- * stepped together: every scene's grid lives in the shared memory of a
- * cluster of 1-8 CTAs, and one persistent launch per cluster size runs all
- * scenes from a work queue. Scenes: dim 2, MLS, at most 8 x 9,600 grid nodes
- * ((W+1)(H+1) <= ~76,000, e.g. 257 x 257 cells); larger or 3D scenes return
- * MPM_ERR_CAPACITY / MPM_ERR_UNSUPPORTED. */
+ * stepped together: the scenes lie side by side in one grid and one particle
+ * array, and each kernel of a step runs over all of them. A scene's result does
+ * not depend on its partners (bitwise). Scenes: dim 2, MLS, at most 8 x 9,600
+ * grid nodes ((W+1)(H+1) <= ~76,000, e.g. 257 x 257 cells); larger or 3D scenes
+ * return MPM_ERR_CAPACITY / MPM_ERR_UNSUPPORTED. */
 struct mpm_batch;
 typedef struct mpm_batch mpm_batch;
 
+/* threads, particles_per_cta and max_cluster described CTA clusters that held one
+ * scene each. They are still checked, kept and reported, and a max_cluster below 8
+ * still limits the grid of a scene (to max_cluster x 9,600 nodes); they have no
+ * other effect. */
 typedef struct mpm_batch_config {
-    int32_t threads;           /* threads per CTA: 256, 512 or 1024 */
-    int32_t particles_per_cta; /* spread a scene over more CTAs while it has more particles per CTA than this
-                                  (0: only as many CTAs as its grid needs) */
-    int32_t max_cluster;       /* largest cluster: 1, 2, 4 or 8 */
-    int32_t sort_period;       /* steps between re-sorts of a multi-CTA scene's particles by row (0: 16) */
+    int32_t threads;           /* 256, 512 or 1024 */
+    int32_t particles_per_cta; /* >= 0 */
+    int32_t max_cluster;       /* 1, 2, 4 or 8 */
+    int32_t sort_period;       /* steps between sorts of the particles by cell (0: 16) */
     int32_t reserved[4];
 } mpm_batch_config;
 
@@ -376,8 +379,8 @@ MPM_API mpm_status mpm_batch_create(const mpm_params* params, const mpm_particle
 MPM_API mpm_status mpm_batch_destroy(mpm_batch* batch);
 MPM_API const char* mpm_batch_last_error(const mpm_batch* batch);
 MPM_API mpm_status mpm_batch_info(const mpm_batch* batch, int32_t* nscenes, int64_t* total_particles);
-/* Advance every scene by nsteps (asynchronous on the batch's stream; one CUDA
- * graph per nsteps value, replayed). */
+/* Advance every scene by nsteps (asynchronous on the batch's stream; a CUDA graph
+ * per stretch of steps between sorts, replayed). */
 MPM_API mpm_status mpm_batch_step(mpm_batch* batch, int32_t nsteps);
 MPM_API mpm_status mpm_batch_set_stream(mpm_batch* batch, void* cuda_stream);
 /* Per-scene state, host copies in the scene's creation order (as mpm_get_state). */
@@ -386,16 +389,15 @@ MPM_API mpm_status mpm_batch_set_state(mpm_batch* batch, int32_t scene, const mp
 MPM_API mpm_status mpm_batch_get_positions(mpm_batch* batch, int32_t scene, float* out, size_t cap_floats);
 MPM_API mpm_status mpm_batch_get_status(mpm_batch* batch, int32_t scene, uint32_t* flags);
 /* Device timestamps (ns) of the last mpm_batch_step call: for each scene, its
- * start and the end of each of its steps, [scene][nsteps + 1]; *nsteps gets the
- * call's step count. Synchronises. */
+ * start and the end of each of its steps, [scene][nsteps + 1] (the scenes step
+ * together, so their times are the same); *nsteps gets the call's step count.
+ * Synchronises. */
 MPM_API mpm_status mpm_batch_step_times(mpm_batch* batch, uint64_t* out, size_t cap, int32_t* nsteps);
 MPM_API mpm_status mpm_batch_get_config(const mpm_batch* batch, mpm_batch_config* config);
 MPM_API mpm_status mpm_batch_set_config(mpm_batch* batch, const mpm_batch_config* config);
-/* Autotuner: times trial_steps steps of the batch under each candidate
- * configuration (threads {256, 512, 1024} x particles per CTA {grid-limited,
- * 16k, 8k, 4k}), keeps the fastest, and restores
- * the particle state, so the batch continues as if untuned. *best_ms gets the
- * chosen configuration's time for the trial. Synchronises. */
+/* Times trial_steps steps of the batch and restores the particle state, so the
+ * batch continues as if untuned. There is one way to run a batch now, so *chosen
+ * is the present configuration; *best_ms gets the trial's time. Synchronises. */
 MPM_API mpm_status mpm_batch_tune(mpm_batch* batch, int32_t trial_steps, mpm_batch_config* chosen, double* best_ms);
 
 #ifdef __cplusplus

@@ -1,13 +1,12 @@
 """Batched 2D scenes: Python host mirror of mpm_batch_* (include/mpm/mpm.h).
 
     batch = Batch(scenes.batch_scenes_2d())   # 256 independent scenes
-    batch.tune(4)                            # project autotuner (threads, CTAs per scene)
-    batch.step(500)                          # one CUDA graph: a persistent launch per cluster size
+    batch.step(500)                          # CUDA graphs over all scenes
     pos = batch.positions(17)                # scene 17, (n, 2) float32
 
 Each scene is what mpm_create would make of it (same constants, fixed-point
-scales and per-particle arithmetic); the batch only changes where the grid
-lives (the shared memory of a CTA cluster) and how scenes share the GPU.
+scales and per-particle arithmetic); the scenes lie side by side in one grid and
+are stepped by the same launches, and none depends on its partners.
 """
 from __future__ import annotations
 
@@ -122,7 +121,7 @@ class Batch:
         self._check(self._lib.mpm_batch_set_config(self._h, C.byref(c)))
 
     def tune(self, trial_steps: int = 4):
-        """Run the autotuner; returns (chosen config, its trial time in ms)."""
+        """Time trial_steps steps; returns (config, the trial's time in ms)."""
         c = MpmBatchConfig()
         ms = C.c_double()
         self._check(self._lib.mpm_batch_tune(self._h, int(trial_steps), C.byref(c), C.byref(ms)))

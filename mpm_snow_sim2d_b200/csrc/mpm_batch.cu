@@ -1,10 +1,11 @@
-// Batched 2D scenes: C ABI (include/mpm/mpm.h, mpm_batch_*), class assignment
-// by cluster size, CUDA-graph capture of the per-class persistent launches,
-// and the autotuner. Kernels: mpm_batch.cuh.
+// Batched 2D scenes: C ABI (include/mpm/mpm.h, mpm_batch_*), the scenes' shared
+// arrays, the step sequence and its CUDA graphs. Kernels: mpm_batch.cuh.
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <map>
 #include <string>
+#include <tuple>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -12,49 +13,52 @@
 #include "mpm/mpm.h"
 #include "mpm_batch.cuh"
 #include "mpm_host.h"
+#include "mpm_readback.h"
 
 using namespace mpm;
 
 namespace {
 
 constexpr int kClusterSizes[4] = {1, 2, 4, 8};
+constexpr int kMaxSegment = 64;    // steps of one graph
+constexpr size_t kMaxGraphs = 64;  // graphs kept
 
-struct BatchClass {
-    int cl = 0;        // CTAs per cluster
-    int cap = 0;       // nodes per accumulator array per CTA
-    int count = 0;     // scenes
-    int first = 0;     // offset into the order array
-    int clusters = 0;  // persistent clusters launched
+struct BatchBuffers {
+    float *x, *v, *B, *Fe, *Jp, *mass, *vol;
+    int* id;  // creation index of the particle within its scene
 };
 
 }  // namespace
 
 struct mpm_batch {
+    ReadbackUser readback;
+    DeviceArena arena;  // every device array below but those made on demand
     int device = 0;
     int nscenes = 0;
+    int sms = 148;
     long long N = 0;
-    std::vector<long long> p0;
     std::vector<int> counts;
-    std::vector<BatchScene> scenes;  // host copy (cl, rows follow the configuration)
+    std::vector<BatchScene> scenes;  // host copy
     BatchBuffers buf[2] = {};
-    BatchScene* d_scenes = nullptr;
-    BatchSceneState* d_state = nullptr;
-    int* d_order = nullptr;
-    int* d_queue = nullptr;
-    int* d_needs_affine = nullptr;
-    unsigned* d_status = nullptr;
-    unsigned long long* d_stamps = nullptr;
+    int parity = 0;                  // which buffer holds the particles
+    float* A = nullptr;              // P2G affine matrix of the queued particles
+    BatchArrays arr{};
+    TileInfo ti{};
+    SlowQueue q{};
+    ManyScenes many{};
+    long long nodes = 0;
     size_t stamps_cap = 0;
     int last_steps = 0;
+    int since_sort = 0;              // steps since the last sort
+    bool needs_sort = true;
+    bool any_fresh = true;           // a scene has no pending grid sums (arr.fresh)
+    float* staging = nullptr;
+    size_t staging_floats = 0;
     cudaStream_t stream = nullptr, own_stream = nullptr;
-    cudaStream_t aux[4] = {nullptr, nullptr, nullptr, nullptr};
-    cudaEvent_t fork = nullptr, join[4] = {nullptr, nullptr, nullptr, nullptr};
     mpm_batch_config cfg{};
-    BatchClass cls[4];
-    int smem_max = 0;  // dynamic shared memory opt-in per CTA, bytes
-    int cap_max = 0;   // nodes per accumulator array that fit in it
-    cudaGraphExec_t graph = nullptr;
-    int graph_steps = -1;
+    int cap_max = 0;                 // nodes per CTA of the largest scene's cluster (limit on a scene's grid)
+    // graphs of [sort +] n steps, by (steps, sort, buffer)
+    std::map<std::tuple<int, int, int>, cudaGraphExec_t> graphs;
     bool use_graphs = true;
     std::string err;
 };
@@ -81,82 +85,136 @@ template <typename T> cudaError_t balloc(T** p, size_t count) {
     return cudaMalloc(reinterpret_cast<void**>(p), (count ? count : 1) * sizeof(T));
 }
 
-void drop_graph(mpm_batch* b) {
-    if (b->graph) {
-        cudaStreamSynchronize(b->stream);
-        cudaGraphExecDestroy(b->graph);
-    }
-    b->graph = nullptr;
-    b->graph_steps = -1;
+void drop_graphs(mpm_batch* b) {
+    if (b->graphs.empty()) return;
+    cudaStreamSynchronize(b->stream);
+    for (auto& g : b->graphs)
+        if (g.second) cudaGraphExecDestroy(g.second);
+    b->graphs.clear();
 }
 
 void release(mpm_batch* b) {
-    drop_graph(b);
-    for (BatchBuffers& f : b->buf) {
-        float* fl[] = {f.x, f.v, f.B, f.Fe, f.Jp, f.A, f.mass, f.vol};
-        for (float* p : fl)
-            if (p) cudaFree(p);
-        if (f.id) cudaFree(f.id);
-    }
-    if (b->d_scenes) cudaFree(b->d_scenes);
-    if (b->d_state) cudaFree(b->d_state);
-    if (b->d_order) cudaFree(b->d_order);
-    if (b->d_queue) cudaFree(b->d_queue);
-    if (b->d_needs_affine) cudaFree(b->d_needs_affine);
-    if (b->d_status) cudaFree(b->d_status);
-    if (b->d_stamps) cudaFree(b->d_stamps);
-    for (int c = 0; c < 4; ++c) {
-        if (b->aux[c]) cudaStreamDestroy(b->aux[c]);
-        if (b->join[c]) cudaEventDestroy(b->join[c]);
-    }
-    if (b->fork) cudaEventDestroy(b->fork);
+    drop_graphs(b);
+    if (b->staging) cudaFree(b->staging);
+    if (b->arr.stamps) cudaFree(b->arr.stamps);
+    b->arena.release();
     if (b->own_stream) cudaStreamDestroy(b->own_stream);
 }
 
-using BatchKernel = void (*)(BatchParticles, BatchRun);
-
-BatchKernel kernel_for(int threads) {
-    return threads == 1024 ? k_batch_run<1024> : threads == 512 ? k_batch_run<512> : k_batch_run<256>;
+Particles particles(const mpm_batch* b) {
+    const BatchBuffers& f = b->buf[b->parity];
+    Particles P{};
+    P.x = f.x; P.v = f.v; P.B = f.B; P.Fe = f.Fe; P.Jp = f.Jp; P.A = b->A;
+    P.mass = f.mass; P.vol = f.vol;
+    P.n = (int)b->N;
+    return P;
 }
 
-BatchParticles particles(const mpm_batch* b) { return BatchParticles{{b->buf[0], b->buf[1]}, b->N}; }
+// ---- the step sequence ----
 
-// Where each scene's particles are now (buffer parity) and their slot order.
-mpm_status scene_states(mpm_batch* b, std::vector<BatchSceneState>& st) {
-    st.resize(b->nscenes);
-    BATCH_CUDA(b, cudaMemcpyAsync(st.data(), b->d_state, sizeof(BatchSceneState) * st.size(), cudaMemcpyDeviceToHost,
-                                  b->stream));
+// All scenes' particles into the other buffer, by (tile, cell, id).
+cudaError_t enqueue_sort(mpm_batch* b) {
+    if (b->N == 0) return cudaSuccess;
+    const Particles P = particles(b);
+    const int threads = 256;
+    const unsigned blocks = (unsigned)((b->N + threads - 1) / threads);
+    k_sort_count<2, 4, ManyScenes><<<blocks, threads, 0, b->stream>>>(P, b->many, b->ti);
+    const int scan_blocks = (b->ti.n_tiles + kScanTiles - 1) / kScanTiles;
+    k_sort_block_sums<<<scan_blocks, kScanTiles, 0, b->stream>>>(b->ti);
+    k_sort_scan<<<scan_blocks, kScanTiles, 0, b->stream>>>(b->ti);
+    k_sort_bucket<<<blocks, threads, 0, b->stream>>>((int)b->N, b->ti);
+    const BatchBuffers& t = b->buf[b->parity ^ 1];
+    const SortBuffers dst{t.x, t.v, t.B, t.Fe, t.Jp, nullptr, t.mass, t.vol, t.id};
+    k_tile_sort<2, 4, ManyScenes><<<b->sms * SortGeom<2>::CTAS_PER_SM, 256, 0, b->stream>>>(
+        P, b->buf[b->parity].id, dst, b->many, b->ti);
+    b->parity ^= 1;
+    return cudaGetLastError();
+}
+
+cudaError_t enqueue_step(mpm_batch* b) {
+    k_batch_grid<<<b->sms * 8, 256, 0, b->stream>>>(b->arr, b->ti);
+    if (b->N > 0) {
+        const Particles P = particles(b);
+        k_batch_step<true><<<b->sms * MPM_FUSED_MIN_BLOCKS, FusedGeom<2>::THREADS, 0, b->stream>>>(P, b->arr, b->ti, b->q);
+        k_batch_plastic<<<b->sms * 4, 256, 0, b->stream>>>(P, b->arr, b->q);
+        k_batch_windows<<<b->sms * 8, FusedGeom<2>::THREADS, 0, b->stream>>>(P, b->arr, b->ti, b->q);
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t enqueue_segment(mpm_batch* b, int steps, bool sort) {
+    cudaError_t e = sort ? enqueue_sort(b) : cudaSuccess;
+    for (int k = 0; k < steps && e == cudaSuccess; ++k) e = enqueue_step(b);
+    return e;
+}
+
+// [sort +] steps, from a graph captured on first use on a stream of its own.
+mpm_status run_segment(mpm_batch* b, int steps, bool sort) {
+    if (!b->use_graphs) {
+        BATCH_CUDA(b, enqueue_segment(b, steps, sort));
+        return MPM_OK;
+    }
+    const auto key = std::make_tuple(steps, (int)sort, b->parity);
+    auto it = b->graphs.find(key);
+    if (it == b->graphs.end()) {
+        if (b->graphs.size() >= kMaxGraphs) drop_graphs(b);
+        cudaStream_t cap = nullptr;
+        cudaGraph_t g = nullptr;
+        cudaGraphExec_t ex = nullptr;
+        const cudaStream_t saved = b->stream;
+        const int parity = b->parity;
+        cudaError_t e = cudaStreamCreateWithFlags(&cap, cudaStreamNonBlocking);
+        if (e == cudaSuccess) e = cudaStreamBeginCapture(cap, cudaStreamCaptureModeThreadLocal);
+        if (e == cudaSuccess) {
+            b->stream = cap;
+            const cudaError_t e1 = enqueue_segment(b, steps, sort);
+            b->stream = saved;
+            const cudaError_t e2 = cudaStreamEndCapture(cap, &g);
+            e = e1 != cudaSuccess ? e1 : e2;
+        }
+        b->parity = parity;  // nothing ran
+        if (e == cudaSuccess) e = cudaGraphInstantiate(&ex, g, 0);
+        if (g) cudaGraphDestroy(g);
+        if (cap) cudaStreamDestroy(cap);
+        if (e != cudaSuccess) {  // direct launches for the life of the batch
+            cudaGetLastError();
+            b->use_graphs = false;
+            BATCH_CUDA(b, enqueue_segment(b, steps, sort));
+            return MPM_OK;
+        }
+        it = b->graphs.emplace(key, ex).first;
+    }
+    BATCH_CUDA(b, cudaGraphLaunch(it->second, b->stream));
+    if (sort && b->N > 0) b->parity ^= 1;
+    return MPM_OK;
+}
+
+int sort_period(const mpm_batch* b) { return b->cfg.sort_period > 0 ? b->cfg.sort_period : 16; }
+
+mpm_status ensure_staging(mpm_batch* b, size_t floats) {
+    if (floats <= b->staging_floats) return MPM_OK;
     BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
+    if (b->staging) cudaFree(b->staging);
+    b->staging = nullptr;
+    b->staging_floats = 0;
+    BATCH_CUDA(b, balloc(&b->staging, floats));
+    b->staging_floats = floats;
     return MPM_OK;
 }
 
-// Forget every scene's bands (they belong to a cluster size): the next step
-// of each multi-CTA scene starts with a sort.
-mpm_status invalidate_bands(mpm_batch* b) {
-    std::vector<BatchSceneState> st;
-    mpm_status r = scene_states(b, st);
-    if (r != MPM_OK) return r;
-    for (auto& x : st) x.sorted = 0;
-    BATCH_CUDA(b, cudaMemcpy(b->d_state, st.data(), sizeof(BatchSceneState) * st.size(), cudaMemcpyHostToDevice));
+// Every scene's pending sums are void: the next step forms them from the state.
+mpm_status forget_sums(mpm_batch* b) {
+    BATCH_CUDA(b, cudaMemsetAsync(b->arr.acc, 0, sizeof(unsigned long long) * 4 * (size_t)b->nodes, b->stream));
+    BATCH_CUDA(b, cudaMemsetAsync(b->ti.mark, 0, sizeof(int) * (size_t)b->ti.n_blocks, b->stream));
+    BATCH_CUDA(b, cudaMemsetAsync(b->ti.n_marked, 0, sizeof(int), b->stream));
+    BATCH_CUDA(b, cudaMemsetAsync(b->arr.fresh, 1, sizeof(int) * (size_t)b->nscenes, b->stream));
+    b->any_fresh = true;
+    b->needs_sort = true;
     return MPM_OK;
 }
 
-cudaLaunchConfig_t launch_config(const mpm_batch* b, const BatchClass& k, cudaLaunchAttribute* attr, int clusters) {
-    cudaLaunchConfig_t lc = {};
-    lc.gridDim = dim3((unsigned)(clusters * k.cl));
-    lc.blockDim = dim3((unsigned)b->cfg.threads);
-    lc.dynamicSmemBytes = (size_t)kBatchAccs * sizeof(unsigned long long) * (size_t)k.cap;
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = (unsigned)k.cl;
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    lc.attrs = attr;
-    lc.numAttrs = 1;
-    return lc;
-}
-
-// Cluster size and node band of every scene under b->cfg; scenes grouped by
-// cluster size, most particles per CTA first; persistent cluster counts.
+// A configuration is valid when its numbers are and every scene's grid fits the
+// largest cluster it allows (the limit on a scene's size that the interface states).
 mpm_status configure(mpm_batch* b, const mpm_batch_config& cfg) {
     if (cfg.threads != 256 && cfg.threads != 512 && cfg.threads != 1024)
         return bfail(b, MPM_ERR_INVALID_ARGUMENT, "threads must be 256, 512 or 1024");
@@ -164,125 +222,55 @@ mpm_status configure(mpm_batch* b, const mpm_batch_config& cfg) {
         return bfail(b, MPM_ERR_INVALID_ARGUMENT, "max_cluster must be 1, 2, 4 or 8");
     if (cfg.particles_per_cta < 0) return bfail(b, MPM_ERR_INVALID_ARGUMENT, "particles_per_cta must be >= 0");
     if (cfg.sort_period < 0) return bfail(b, MPM_ERR_INVALID_ARGUMENT, "sort_period must be >= 0");
-    std::vector<BatchScene> sc = b->scenes;
-    std::vector<std::vector<int>> members(4);
     for (int s = 0; s < b->nscenes; ++s) {
-        const int nx = sc[s].C.nx, ny = sc[s].C.ny;
-        int ci = -1;
-        for (int c = 0; c < 4 && kClusterSizes[c] <= cfg.max_cluster; ++c) {
-            const long long rows = (ny + kClusterSizes[c] - 1) / kClusterSizes[c];
-            if (rows * nx <= b->cap_max) { ci = c; break; }
-        }
-        if (ci < 0)
+        const int nx = b->scenes[s].C.nx, ny = b->scenes[s].C.ny;
+        bool fits = false;
+        for (int c = 0; c < 4 && kClusterSizes[c] <= cfg.max_cluster; ++c)
+            fits = fits || (long long)((ny + kClusterSizes[c] - 1) / kClusterSizes[c]) * nx <= b->cap_max;
+        if (!fits)
             return bfail(b, MPM_ERR_CAPACITY,
                          "scene " + std::to_string(s) + ": its grid of " + std::to_string((long long)nx * ny) +
                              " nodes does not fit in the shared memory of a cluster of " +
                              std::to_string(cfg.max_cluster) + " CTAs");
-        if (cfg.particles_per_cta > 0)
-            while (ci < 3 && kClusterSizes[ci + 1] <= cfg.max_cluster &&
-                   (long long)sc[s].n > (long long)cfg.particles_per_cta * kClusterSizes[ci])
-                ++ci;
-        sc[s].cl = kClusterSizes[ci];
-        // a multi-CTA scene may give any CTA up to its full capacity in rows
-        sc[s].rows = sc[s].cl == 1 ? ny : b->cap_max / nx;
-        if (sc[s].n > 0) members[ci].push_back(s);
     }
-    std::vector<int> order;
-    BatchClass cls[4];
-    for (int c = 0; c < 4; ++c) {
-        std::sort(members[c].begin(), members[c].end(), [&](int a, int d) {
-            const long long wa = (long long)sc[a].n + (long long)sc[a].C.nodes;
-            const long long wd = (long long)sc[d].n + (long long)sc[d].C.nodes;
-            return wa != wd ? wa > wd : a < d;
-        });
-        cls[c].cl = kClusterSizes[c];
-        cls[c].first = (int)order.size();
-        cls[c].count = (int)members[c].size();
-        for (int s : members[c]) {
-            cls[c].cap = std::max(cls[c].cap, sc[s].rows * sc[s].C.nx);
-            order.push_back(s);
-        }
-        if (cls[c].cl > 1 && cls[c].count > 0) cls[c].cap = b->cap_max;
-    }
-    // Shared-memory opt-in and persistent cluster counts.
     b->cfg = cfg;
-    BatchKernel kern = kernel_for(cfg.threads);
-    BATCH_CUDA(b, cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, b->smem_max));
-    BATCH_CUDA(b, cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 0));
-    for (int c = 0; c < 4; ++c) {
-        if (cls[c].count == 0) continue;
-        cudaLaunchAttribute attr[1];
-        cudaLaunchConfig_t lc = launch_config(b, cls[c], attr, 1);
-        int active = 0;
-        BATCH_CUDA(b, cudaOccupancyMaxActiveClusters(&active, kern, &lc));
-        if (active < 1)
-            return bfail(b, MPM_ERR_UNSUPPORTED,
-                         "a cluster of " + std::to_string(cls[c].cl) + " CTAs x " + std::to_string(cfg.threads) +
-                             " threads cannot be resident on this device");
-        cls[c].clusters = std::min(cls[c].count, active);
-    }
-    drop_graph(b);
-    b->scenes = sc;
-    for (int c = 0; c < 4; ++c) b->cls[c] = cls[c];
-    BATCH_CUDA(b, cudaMemcpy(b->d_scenes, sc.data(), sizeof(BatchScene) * sc.size(), cudaMemcpyHostToDevice));
-    if (!order.empty())
-        BATCH_CUDA(b, cudaMemcpy(b->d_order, order.data(), sizeof(int) * order.size(), cudaMemcpyHostToDevice));
-    // bands of the old cluster sizes are void: each scene re-sorts on its next step
-    return invalidate_bands(b);
-}
-
-// Enqueue one call: zero the queues, then every class's persistent launch on
-// its own stream (fork / join around the batch's stream).
-cudaError_t enqueue(mpm_batch* b, int nsteps) {
-    cudaError_t e = cudaMemsetAsync(b->d_queue, 0, sizeof(int) * 4, b->stream);
-    if (e != cudaSuccess) return e;
-    if ((e = cudaEventRecord(b->fork, b->stream)) != cudaSuccess) return e;
-    const BatchParticles P = particles(b);
-    BatchKernel kern = kernel_for(b->cfg.threads);
-    for (int c = 0; c < 4; ++c) {
-        const BatchClass& k = b->cls[c];
-        if (k.count == 0) continue;
-        if ((e = cudaStreamWaitEvent(b->aux[c], b->fork, 0)) != cudaSuccess) return e;
-        BatchRun R{b->d_scenes, b->d_state, b->d_order + k.first, k.count, k.cap, b->d_queue + c,
-                   b->d_needs_affine, b->d_status, b->d_stamps, nsteps,
-                   b->cfg.sort_period > 0 ? b->cfg.sort_period : 16};
-        cudaLaunchAttribute attr[1];
-        cudaLaunchConfig_t lc = launch_config(b, k, attr, k.clusters);
-        lc.stream = b->aux[c];
-        if ((e = cudaLaunchKernelEx(&lc, kern, P, R)) != cudaSuccess) return e;
-        if ((e = cudaEventRecord(b->join[c], b->aux[c])) != cudaSuccess) return e;
-        if ((e = cudaStreamWaitEvent(b->stream, b->join[c], 0)) != cudaSuccess) return e;
-    }
-    return cudaSuccess;
-}
-
-// Scene slice of one field in creation order (slots hold particles id[slot]).
-mpm_status copy_slice_out(mpm_batch* b, int field, int comps, int scene, float* host) {
-    const int n = b->counts[scene];
-    if (n == 0) return MPM_OK;
-    std::vector<BatchSceneState> st;
-    mpm_status r = scene_states(b, st);
-    if (r != MPM_OK) return r;
-    const BatchBuffers& F = b->buf[st[scene].parity & 1];
-    const float* soa[] = {F.x, F.v, F.B, F.Fe, F.Jp};
-    std::vector<float> tmp((size_t)n * comps);
-    std::vector<int> id(n);
-    for (int c = 0; c < comps; ++c)
-        BATCH_CUDA(b, cudaMemcpyAsync(tmp.data() + (size_t)c * n, soa[field] + (size_t)c * b->N + b->p0[scene],
-                                      sizeof(float) * n, cudaMemcpyDeviceToHost, b->stream));
-    BATCH_CUDA(b, cudaMemcpyAsync(id.data(), F.id + b->p0[scene], sizeof(int) * n, cudaMemcpyDeviceToHost, b->stream));
-    BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
-    for (int j = 0; j < n; ++j) {
-        const int i = id[j];
-        if (i < 0 || i >= n) return bfail(b, MPM_ERR_CUDA, "corrupt particle order");
-        for (int c = 0; c < comps; ++c) host[(size_t)i * comps + c] = tmp[(size_t)c * n + j];
-    }
     return MPM_OK;
 }
 
 bool valid_scene(const mpm_batch* b, int32_t s) { return b && s >= 0 && s < b->nscenes; }
 
-enum { kFieldX = 0, kFieldV = 1, kFieldB = 2, kFieldFe = 3, kFieldJp = 4 };
+const int kComps[5] = {2, 2, 4, 4, 1};  // position, velocity, B, F_E, J_p
+
+float* field(const mpm_batch* b, int f) {
+    const BatchBuffers& F = b->buf[b->parity];
+    float* soa[] = {F.x, F.v, F.B, F.Fe, F.Jp};
+    return soa[f];
+}
+
+// Fields of a scene in creation order (null: skipped).
+mpm_status read_scene(mpm_batch* b, int scene, float* const* host) {
+    const int n = b->counts[scene];
+    if (n == 0) return MPM_OK;
+    size_t floats = 0;
+    for (int f = 0; f < 5; ++f) floats += host[f] ? (size_t)n * kComps[f] : 0;
+    if (floats == 0) return MPM_OK;
+    const mpm_status st = ensure_staging(b, floats);
+    if (st != MPM_OK) return st;
+    const long long p0 = b->scenes[scene].p0;
+    void* dst[5];
+    size_t bytes[5], at = 0;
+    for (int f = 0; f < 5; ++f) {
+        dst[f] = host[f];
+        bytes[f] = host[f] ? sizeof(float) * (size_t)n * kComps[f] : 0;
+        if (!host[f]) continue;
+        k_batch_export<<<(n + 255) / 256, 256, 0, b->stream>>>(field(b, f), b->N, kComps[f], p0, n, b->buf[b->parity].id,
+                                                               b->staging + at);
+        at += (size_t)n * kComps[f];
+    }
+    BATCH_CUDA(b, cudaGetLastError());
+    BATCH_CUDA(b, ReadbackRing::get().read_parts(b->stream, b->staging, dst, bytes, 5));
+    return MPM_OK;
+}
 
 }  // namespace
 
@@ -309,24 +297,29 @@ mpm_status mpm_batch_create(const mpm_params* params, const mpm_particles_init* 
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) { cudaGetLastError(); return MPM_ERR_NO_DEVICE; }
     if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return MPM_ERR_NO_DEVICE; }
     cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, k_batch_run<256>) != cudaSuccess) { cudaGetLastError(); return MPM_ERR_NO_DEVICE; }
+    if (cudaFuncGetAttributes(&fa, k_batch_step<true>) != cudaSuccess) { cudaGetLastError(); return MPM_ERR_NO_DEVICE; }
 
     mpm_batch* b = new mpm_batch();
     auto bail = [&](mpm_status code) { release(b); delete b; return code; };
     b->device = dev;
     b->nscenes = nscenes;
     b->N = N;
-    int optin = 0;
-    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess) return bail(MPM_ERR_CUDA);
-    b->smem_max = optin - (int)std::max(fa.sharedSizeBytes, (size_t)0) - 1024;
-    b->smem_max -= b->smem_max % 256;
-    b->cap_max = b->smem_max / (int)(kBatchAccs * sizeof(unsigned long long));
+    int optin = 0, sms = 0;
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+        return bail(MPM_ERR_CUDA);
+    b->sms = sms > 0 ? sms : 148;
+    // nodes of 24 bytes in a CTA's shared memory (less 3.7 KB): the size limit of a scene
+    const int smem = (optin - 3776) / 256 * 256;
+    b->cap_max = smem / 24;
 
-    // Per-scene constants and fixed-point scales, as mpm_create chooses them.
-    b->p0.resize(nscenes);
+    // Per-scene constants and fixed-point scales, as mpm_create chooses them; the
+    // scenes' places in the shared arrays.
+    constexpr int T = TileGeom<2>::T;
     b->counts.resize(nscenes);
     b->scenes.resize(nscenes);
     std::vector<float> massv((size_t)N), volv((size_t)N);
+    std::vector<int> of_slots((size_t)N), of_tiles, of_blocks;
     long long off = 0;
     for (int s = 0; s < nscenes; ++s) {
         const int n = (int)init[s].count;
@@ -337,6 +330,7 @@ mpm_status mpm_batch_create(const mpm_params* params, const mpm_particles_init* 
             if (!std::isfinite(vol) || !std::isfinite(m)) return bail(MPM_ERR_INVALID_ARGUMENT);
             volv[off + i] = vol;
             massv[off + i] = m;
+            of_slots[off + i] = s;
             total_mass += m;
         }
         for (long long i = 0; i < 2LL * n; ++i)
@@ -348,73 +342,94 @@ mpm_status mpm_batch_create(const mpm_params* params, const mpm_particles_init* 
         fixed_point_scales(params[s], total_mass, S.C, l2);
         S.p0 = off;
         S.n = n;
-        b->p0[s] = off;
+        S.node0 = b->nodes;
+        S.view = SceneView{{S.C.W, S.C.H, 0}, {(S.C.W + T - 1) / T, (S.C.H + T - 1) / T, 1}, (int)of_tiles.size()};
+        S.nblk[0] = (S.C.nx + T - 1) / T;
+        S.nblk[1] = (S.C.ny + T - 1) / T;
+        S.blk0 = (int)of_blocks.size();
+        of_tiles.insert(of_tiles.end(), (size_t)S.view.tiles[0] * S.view.tiles[1], s);
+        of_blocks.insert(of_blocks.end(), (size_t)S.nblk[0] * S.nblk[1], s);
+        b->nodes += S.C.nodes;
         b->counts[s] = n;
         off += n;
     }
+    mpm_batch_config cfg{};
+    cfg.threads = 512;
+    cfg.particles_per_cta = 8192;
+    cfg.max_cluster = 8;
+    cfg.sort_period = 16;
+    const mpm_status cs = configure(b, cfg);
+    if (cs != MPM_OK) return bail(cs);
 
     if (cudaStreamCreateWithFlags(&b->own_stream, cudaStreamNonBlocking) != cudaSuccess) return bail(MPM_ERR_CUDA);
     b->stream = b->own_stream;
-    for (int c = 0; c < 4; ++c)
-        if (cudaStreamCreateWithFlags(&b->aux[c], cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&b->join[c], cudaEventDisableTiming) != cudaSuccess)
-            return bail(MPM_ERR_CUDA);
-    if (cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) != cudaSuccess) return bail(MPM_ERR_CUDA);
-    const size_t n = (size_t)N;
-    bool alloc_ok = true;
-    for (BatchBuffers& f : b->buf)
-        alloc_ok = alloc_ok && !balloc(&f.x, n * 2) && !balloc(&f.v, n * 2) && !balloc(&f.B, n * 4) &&
-                   !balloc(&f.Fe, n * 4) && !balloc(&f.Jp, n) && !balloc(&f.A, n * 4) && !balloc(&f.mass, n) &&
-                   !balloc(&f.vol, n) && !balloc(&f.id, n);
-    if (!alloc_ok || balloc(&b->d_scenes, (size_t)nscenes) || balloc(&b->d_state, (size_t)nscenes) ||
-        balloc(&b->d_order, (size_t)nscenes) || balloc(&b->d_queue, 4) ||
-        balloc(&b->d_needs_affine, (size_t)nscenes) || balloc(&b->d_status, (size_t)nscenes)) {
-        cudaGetLastError();
-        return bail(MPM_ERR_OUT_OF_MEMORY);
+    const size_t n = (size_t)N, nt = of_tiles.size(), nb = of_blocks.size();
+    TileInfo& ti = b->ti;
+    ti.n_tiles = (int)nt;
+    ti.n_blocks = (int)nb;
+    ti.win = FusedGeom<2>::WIN;
+    ti.item_win = 1;
+    b->q.capacity = n > 0 ? (int)n : 1;
+    b->q.win_capacity = b->q.capacity / ti.win + (int)nt + 1;
+    DeviceArena& arena = b->arena;
+    for (BatchBuffers& f : b->buf) {
+        arena.want(&f.x, n * 2).want(&f.v, n * 2).want(&f.B, n * 4).want(&f.Fe, n * 4).want(&f.Jp, n);
+        arena.want(&f.mass, n).want(&f.vol, n).want(&f.id, n);
     }
+    BatchScene* d_scenes = nullptr;
+    int *d_of_slots = nullptr, *d_of_tiles = nullptr, *d_of_blocks = nullptr;
+    arena.want(&d_scenes, (size_t)nscenes).want(&d_of_slots, n).want(&d_of_tiles, nt).want(&d_of_blocks, nb);
+    arena.want(&b->A, n * 4).want(&b->arr.acc, (size_t)b->nodes * 4).want(&b->arr.gv, (size_t)b->nodes);
+    arena.want(&b->arr.status, (size_t)nscenes).want(&b->arr.fresh, (size_t)nscenes).want(&b->arr.step, 1);
+    arena.want(&ti.key, n).want(&ti.tile_count, nt).want(&ti.tile_cursor, nt).want(&ti.tile_start, nt);
+    arena.want(&ti.mark, nb).want(&ti.mark_list, nb).want(&ti.n_marked, 1).want(&ti.perm, n).want(&ti.tile_list, nt);
+    arena.want(&ti.n_tile_list, 1).want(&ti.tile_len, nt).want(&ti.fused_next, 1);
+    arena.want(&ti.items, nt + n / (size_t)ti.win).want(&ti.n_items, 1).want(&ti.scan, nt / kScanTiles + 1);
+    arena.want(&ti.grid_done, 1).want(&ti.skey, n).want(&ti.sval, n).want(&b->q.list, (size_t)b->q.capacity);
+    arena.want(&b->q.count, 2).want(&b->q.fh, (size_t)b->q.capacity * 4).want(&b->q.win, (size_t)b->q.win_capacity);
+    if (!arena.allocate()) return bail(MPM_ERR_OUT_OF_MEMORY);
+    b->arr.scenes = d_scenes;
+    b->arr.of_slots = d_of_slots;
+    b->arr.of_blocks = d_of_blocks;
+    ti.tile_scene = d_of_tiles;
+    b->q.nwin = b->q.count + 1;
+    ti.zero[0] = ti.fused_next;
+    ti.zero[1] = b->q.count;
+    b->arr.nscenes = nscenes;
+    b->many = ManyScenes{d_scenes, d_of_slots, d_of_tiles};
     // SoA upload into buffer 0: F_E = I, B = 0, J_p = 1 (Particle ctor,
     // src/cpu/Particles.cpp:7-19); slot order = creation order.
     const BatchBuffers& F = b->buf[0];
     std::vector<float> soa(n * 4, 0.f);
     bool ok = true;
-    auto up = [&](float* dst, size_t count) {
-        return cudaMemcpy(dst, soa.data(), sizeof(float) * count, cudaMemcpyHostToDevice) == cudaSuccess;
+    auto up = [&](void* dst, const void* src, size_t bytes) {
+        return bytes == 0 || cudaMemcpy(dst, src, bytes, cudaMemcpyHostToDevice) == cudaSuccess;
     };
+    auto zero = [&](void* dst, size_t bytes) { return cudaMemset(dst, 0, bytes) == cudaSuccess; };
     for (int s = 0; s < nscenes; ++s)
         for (int i = 0; i < b->counts[s]; ++i)
-            for (int k = 0; k < 2; ++k) soa[(size_t)k * n + b->p0[s] + i] = init[s].position[(size_t)i * 2 + k];
-    ok = ok && up(F.x, n * 2);
+            for (int k = 0; k < 2; ++k) soa[(size_t)k * n + b->scenes[s].p0 + i] = init[s].position[(size_t)i * 2 + k];
+    ok = ok && up(F.x, soa.data(), sizeof(float) * n * 2);
     for (int s = 0; s < nscenes; ++s)
         for (int i = 0; i < b->counts[s]; ++i)
             for (int k = 0; k < 2; ++k)
-                soa[(size_t)k * n + b->p0[s] + i] = init[s].velocity ? init[s].velocity[(size_t)i * 2 + k] : 0.f;
-    ok = ok && up(F.v, n * 2);
-    std::fill(soa.begin(), soa.end(), 0.f);
-    ok = ok && up(F.B, n * 4) && up(F.A, n * 4);
-    for (int k = 0; k < 4; ++k)
-        for (size_t i = 0; i < n; ++i) soa[(size_t)k * n + i] = (k % 3 == 0) ? 1.f : 0.f;
-    ok = ok && up(F.Fe, n * 4);
-    std::fill(soa.begin(), soa.begin() + n, 1.f);
-    ok = ok && up(F.Jp, n);
-    ok = ok && cudaMemcpy(F.mass, massv.data(), sizeof(float) * n, cudaMemcpyHostToDevice) == cudaSuccess;
-    ok = ok && cudaMemcpy(F.vol, volv.data(), sizeof(float) * n, cudaMemcpyHostToDevice) == cudaSuccess;
+                soa[(size_t)k * n + b->scenes[s].p0 + i] = init[s].velocity ? init[s].velocity[(size_t)i * 2 + k] : 0.f;
+    ok = ok && up(F.v, soa.data(), sizeof(float) * n * 2) && zero(F.B, sizeof(float) * n * 4);
+    for (int k = 0; k < 4; ++k) std::fill(soa.begin() + k * n, soa.begin() + (k + 1) * n, (k % 3 == 0) ? 1.f : 0.f);
+    ok = ok && up(F.Fe, soa.data(), sizeof(float) * n * 4) && up(F.Jp, soa.data(), sizeof(float) * n);
+    ok = ok && up(F.mass, massv.data(), sizeof(float) * n) && up(F.vol, volv.data(), sizeof(float) * n);
     std::vector<int> ids(n);
     for (int s = 0; s < nscenes; ++s)
-        for (int i = 0; i < b->counts[s]; ++i) ids[b->p0[s] + i] = i;
-    ok = ok && cudaMemcpy(F.id, ids.data(), sizeof(int) * n, cudaMemcpyHostToDevice) == cudaSuccess;
-    std::vector<BatchSceneState> st0(nscenes);
-    std::memset(st0.data(), 0, sizeof(BatchSceneState) * nscenes);
-    ok = ok && cudaMemcpy(b->d_state, st0.data(), sizeof(BatchSceneState) * nscenes, cudaMemcpyHostToDevice) == cudaSuccess;
-    std::vector<int> ones(nscenes, 1);
-    ok = ok && cudaMemcpy(b->d_needs_affine, ones.data(), sizeof(int) * nscenes, cudaMemcpyHostToDevice) == cudaSuccess;
-    ok = ok && cudaMemset(b->d_status, 0, sizeof(unsigned) * nscenes) == cudaSuccess;
-    if (!ok) { cudaGetLastError(); return bail(MPM_ERR_CUDA); }
-    mpm_batch_config cfg{};
-    cfg.threads = 512;
-    cfg.particles_per_cta = 8192;
-    cfg.max_cluster = kBatchMaxCluster;
-    cfg.sort_period = 16;
-    mpm_status st = configure(b, cfg);
+        for (int i = 0; i < b->counts[s]; ++i) ids[b->scenes[s].p0 + i] = i;
+    ok = ok && up(F.id, ids.data(), sizeof(int) * n) && up(d_of_slots, of_slots.data(), sizeof(int) * n) &&
+         up(d_of_tiles, of_tiles.data(), sizeof(int) * nt) && up(d_of_blocks, of_blocks.data(), sizeof(int) * nb) &&
+         up(d_scenes, b->scenes.data(), sizeof(BatchScene) * (size_t)nscenes);
+    ok = ok && zero(b->arr.status, sizeof(unsigned) * nscenes) && zero(b->arr.step, sizeof(int)) &&
+         zero(b->arr.gv, sizeof(float4) * (size_t)b->nodes) && zero(ti.tile_count, sizeof(int) * nt) &&
+         zero(ti.tile_cursor, sizeof(int) * nt) && zero(ti.grid_done, sizeof(int)) && zero(ti.n_items, sizeof(int)) &&
+         zero(ti.n_tile_list, sizeof(int)) && zero(ti.fused_next, sizeof(int)) && zero(b->q.count, 2 * sizeof(int));
+    if (!ok || cudaDeviceSynchronize() != cudaSuccess) { cudaGetLastError(); return bail(MPM_ERR_CUDA); }
+    const mpm_status st = forget_sums(b);
     if (st != MPM_OK) return bail(st);
     *out = b;
     return MPM_OK;
@@ -440,131 +455,98 @@ mpm_status mpm_batch_info(const mpm_batch* b, int32_t* nscenes, int64_t* total) 
 mpm_status mpm_batch_step(mpm_batch* b, int32_t nsteps) {
     if (!b || nsteps < 0) return MPM_ERR_INVALID_ARGUMENT;
     if (nsteps == 0) return MPM_OK;
-    const size_t need = (size_t)b->nscenes * (size_t)(nsteps + 1);
+    const size_t need = (size_t)b->nscenes * ((size_t)nsteps + 1);
     if (need > b->stamps_cap) {
-        drop_graph(b);
+        drop_graphs(b);
         BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
-        if (b->d_stamps) cudaFree(b->d_stamps);
-        b->d_stamps = nullptr;
+        if (b->arr.stamps) cudaFree(b->arr.stamps);
+        b->arr.stamps = nullptr;
         b->stamps_cap = 0;
-        BATCH_CUDA(b, balloc(&b->d_stamps, need));
+        BATCH_CUDA(b, balloc(&b->arr.stamps, need));
         b->stamps_cap = need;
     }
     b->last_steps = nsteps;
-    if (b->use_graphs && b->graph_steps != nsteps) {
-        drop_graph(b);
-        cudaGraph_t g = nullptr;
-        cudaError_t e = cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal);
-        if (e == cudaSuccess) {
-            cudaError_t e1 = enqueue(b, nsteps);
-            cudaError_t e2 = cudaStreamEndCapture(b->stream, &g);
-            e = e1 != cudaSuccess ? e1 : e2;
-        }
-        if (e == cudaSuccess) e = cudaGraphInstantiate(&b->graph, g, 0);
-        if (g) cudaGraphDestroy(g);
-        if (e != cudaSuccess) {
-            // fall back to direct launches for the life of the batch
-            cudaGetLastError();
-            b->graph = nullptr;
-            b->use_graphs = false;
-        } else {
-            b->graph_steps = nsteps;
-        }
+    if (b->any_fresh) {
+        // sums of the new states: sort, then their P2G
+        BATCH_CUDA(b, enqueue_sort(b));
+        b->needs_sort = false;
+        b->since_sort = 0;
+        if (b->N > 0)
+            k_batch_step<false><<<b->sms * MPM_FUSED_MIN_BLOCKS, FusedGeom<2>::THREADS, 0, b->stream>>>(particles(b), b->arr,
+                                                                                                       b->ti, b->q);
+        BATCH_CUDA(b, cudaGetLastError());
+        BATCH_CUDA(b, cudaMemsetAsync(b->arr.fresh, 0, sizeof(int) * (size_t)b->nscenes, b->stream));
+        b->any_fresh = false;
     }
-    if (b->graph) BATCH_CUDA(b, cudaGraphLaunch(b->graph, b->stream));
-    else BATCH_CUDA(b, enqueue(b, nsteps));
+    for (int left = nsteps; left > 0;) {
+        const int period = sort_period(b);
+        const bool sort = b->needs_sort || b->since_sort >= period;
+        const int len = std::min({left, kMaxSegment, sort ? period : period - b->since_sort});
+        const mpm_status st = run_segment(b, len, sort);
+        if (st != MPM_OK) return st;
+        b->since_sort = (sort ? 0 : b->since_sort) + len;
+        b->needs_sort = false;
+        left -= len;
+    }
+    k_batch_end<<<1, 256, 0, b->stream>>>(b->arr);
+    BATCH_CUDA(b, cudaGetLastError());
     return MPM_OK;
 }
 
 mpm_status mpm_batch_set_stream(mpm_batch* b, void* stream) {
     if (!b) return MPM_ERR_INVALID_ARGUMENT;
     BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
-    drop_graph(b);
     b->stream = stream ? (cudaStream_t)stream : b->own_stream;
     return MPM_OK;
 }
 
 mpm_status mpm_batch_get_state(mpm_batch* b, int32_t scene, mpm_state_host* st) {
     if (!valid_scene(b, scene) || !st || st->count != b->counts[scene]) return MPM_ERR_INVALID_ARGUMENT;
-    mpm_status r = MPM_OK;
-    if (st->position && (r = copy_slice_out(b, kFieldX, 2, scene, st->position)) != MPM_OK) return r;
-    if (st->velocity && (r = copy_slice_out(b, kFieldV, 2, scene, st->velocity)) != MPM_OK) return r;
-    if (st->affine_b && (r = copy_slice_out(b, kFieldB, 4, scene, st->affine_b)) != MPM_OK) return r;
-    if (st->elastic_f && (r = copy_slice_out(b, kFieldFe, 4, scene, st->elastic_f)) != MPM_OK) return r;
-    if (st->plastic_det && (r = copy_slice_out(b, kFieldJp, 1, scene, st->plastic_det)) != MPM_OK) return r;
-    return MPM_OK;
+    float* const host[5] = {st->position, st->velocity, st->affine_b, st->elastic_f, st->plastic_det};
+    return read_scene(b, scene, host);
 }
 
-// Writes the scene back in creation order (ids reset), so it re-sorts on its
-// next step and re-derives its affine matrices. Fields left NULL keep their
-// values.
+// Fields left NULL keep their values. The scene's pending grid sums are void; it is
+// sorted and its sums formed anew at the next step.
 mpm_status mpm_batch_set_state(mpm_batch* b, int32_t scene, const mpm_state_host* st) {
     if (!valid_scene(b, scene) || !st || st->count != b->counts[scene]) return MPM_ERR_INVALID_ARGUMENT;
     const int n = b->counts[scene];
-    auto finite = [&](const float* p, size_t k) {
-        if (!p) return true;
-        for (size_t i = 0; i < k; ++i)
-            if (!std::isfinite(p[i])) return false;
-        return true;
-    };
-    if (!finite(st->position, 2 * (size_t)n) || !finite(st->velocity, 2 * (size_t)n) ||
-        !finite(st->affine_b, 4 * (size_t)n) || !finite(st->elastic_f, 4 * (size_t)n) ||
-        !finite(st->plastic_det, (size_t)n))
-        return bfail(b, MPM_ERR_INVALID_ARGUMENT, "state holds non-finite values");
+    const float* given[5] = {st->position, st->velocity, st->affine_b, st->elastic_f, st->plastic_det};
+    for (int f = 0; f < 5; ++f)
+        for (size_t i = 0; given[f] && i < (size_t)n * kComps[f]; ++i)
+            if (!std::isfinite(given[f][i])) return bfail(b, MPM_ERR_INVALID_ARGUMENT, "state holds non-finite values");
     if (n == 0) return MPM_OK;
-    std::vector<BatchSceneState> ss;
-    mpm_status r = scene_states(b, ss);
+    mpm_status r = ensure_staging(b, (size_t)n * 4);
     if (r != MPM_OK) return r;
-    const BatchBuffers& F = b->buf[ss[scene].parity & 1];
-    // current contents in creation order, overlaid with what the caller gives
-    const int comps[] = {2, 2, 4, 4, 1};
-    const float* given[] = {st->position, st->velocity, st->affine_b, st->elastic_f, st->plastic_det};
-    float* soa[] = {F.x, F.v, F.B, F.Fe, F.Jp};
-    std::vector<int> id(n);
-    BATCH_CUDA(b, cudaMemcpyAsync(id.data(), F.id + b->p0[scene], sizeof(int) * n, cudaMemcpyDeviceToHost, b->stream));
-    std::vector<float> mass(n), vol(n), ms(n), vs(n);
-    BATCH_CUDA(b, cudaMemcpyAsync(ms.data(), F.mass + b->p0[scene], sizeof(float) * n, cudaMemcpyDeviceToHost, b->stream));
-    BATCH_CUDA(b, cudaMemcpyAsync(vs.data(), F.vol + b->p0[scene], sizeof(float) * n, cudaMemcpyDeviceToHost, b->stream));
-    BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
-    for (int j = 0; j < n; ++j) {
-        if (id[j] < 0 || id[j] >= n) return bfail(b, MPM_ERR_CUDA, "corrupt particle order");
-        mass[id[j]] = ms[j];
-        vol[id[j]] = vs[j];
-    }
+    const BatchScene& S = b->scenes[scene];
     for (int f = 0; f < 5; ++f) {
-        std::vector<float> host((size_t)n * comps[f]);
-        if (given[f]) std::memcpy(host.data(), given[f], sizeof(float) * host.size());
-        else if ((r = copy_slice_out(b, f, comps[f], scene, host.data())) != MPM_OK) return r;
-        std::vector<float> tmp(host.size());
-        for (int i = 0; i < n; ++i)
-            for (int c = 0; c < comps[f]; ++c) tmp[(size_t)c * n + i] = host[(size_t)i * comps[f] + c];
-        for (int c = 0; c < comps[f]; ++c)
-            BATCH_CUDA(b, cudaMemcpyAsync(soa[f] + (size_t)c * b->N + b->p0[scene], tmp.data() + (size_t)c * n,
-                                          sizeof(float) * n, cudaMemcpyHostToDevice, b->stream));
+        if (!given[f]) continue;
+        BATCH_CUDA(b, cudaMemcpyAsync(b->staging, given[f], sizeof(float) * (size_t)n * kComps[f], cudaMemcpyHostToDevice,
+                                      b->stream));
+        k_batch_import<<<(n + 255) / 256, 256, 0, b->stream>>>(field(b, f), b->N, kComps[f], S.p0, n, b->buf[b->parity].id,
+                                                               b->staging);
+        BATCH_CUDA(b, cudaGetLastError());
         BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
     }
-    for (int i = 0; i < n; ++i) id[i] = i;
-    BATCH_CUDA(b, cudaMemcpy(F.mass + b->p0[scene], mass.data(), sizeof(float) * n, cudaMemcpyHostToDevice));
-    BATCH_CUDA(b, cudaMemcpy(F.vol + b->p0[scene], vol.data(), sizeof(float) * n, cudaMemcpyHostToDevice));
-    BATCH_CUDA(b, cudaMemcpy(F.id + b->p0[scene], id.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
-    ss[scene].sorted = 0;
-    ss[scene].step = 0;
-    BATCH_CUDA(b, cudaMemcpy(b->d_state + scene, &ss[scene], sizeof(BatchSceneState), cudaMemcpyHostToDevice));
-    const int one = 1;
-    BATCH_CUDA(b, cudaMemcpy(b->d_needs_affine + scene, &one, sizeof(int), cudaMemcpyHostToDevice));
+    BATCH_CUDA(b, cudaMemsetAsync(b->arr.acc + S.node0 * 4, 0, sizeof(unsigned long long) * 4 * (size_t)S.C.nodes, b->stream));
+    BATCH_CUDA(b, cudaMemsetAsync(b->arr.fresh + scene, 1, sizeof(int), b->stream));
+    BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
+    b->any_fresh = true;
+    b->needs_sort = true;
     return MPM_OK;
 }
 
 mpm_status mpm_batch_get_positions(mpm_batch* b, int32_t scene, float* out, size_t cap_floats) {
     if (!valid_scene(b, scene) || (!out && b->counts[scene] > 0)) return MPM_ERR_INVALID_ARGUMENT;
     if (cap_floats < (size_t)b->counts[scene] * 2) return bfail(b, MPM_ERR_CAPACITY, "output buffer too small");
-    return copy_slice_out(b, kFieldX, 2, scene, out);
+    float* const host[5] = {out, nullptr, nullptr, nullptr, nullptr};
+    return read_scene(b, scene, host);
 }
 
 mpm_status mpm_batch_get_status(mpm_batch* b, int32_t scene, uint32_t* flags) {
     if (!valid_scene(b, scene) || !flags) return MPM_ERR_INVALID_ARGUMENT;
     unsigned f = 0;
-    BATCH_CUDA(b, cudaMemcpyAsync(&f, b->d_status + scene, sizeof(f), cudaMemcpyDeviceToHost, b->stream));
+    BATCH_CUDA(b, cudaMemcpyAsync(&f, b->arr.status + scene, sizeof(f), cudaMemcpyDeviceToHost, b->stream));
     BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
     *flags = f;
     return MPM_OK;
@@ -573,11 +555,14 @@ mpm_status mpm_batch_get_status(mpm_batch* b, int32_t scene, uint32_t* flags) {
 mpm_status mpm_batch_step_times(mpm_batch* b, uint64_t* out, size_t cap, int32_t* nsteps) {
     if (!b || !nsteps) return MPM_ERR_INVALID_ARGUMENT;
     *nsteps = b->last_steps;
-    const size_t need = (size_t)b->nscenes * (size_t)(b->last_steps + 1);
+    const size_t steps = (size_t)b->last_steps + 1, k = (size_t)b->nscenes;
     if (b->last_steps == 0) return MPM_OK;
-    if (!out || cap < need) return bfail(b, MPM_ERR_CAPACITY, "output buffer too small");
-    BATCH_CUDA(b, cudaMemcpyAsync(out, b->d_stamps, sizeof(uint64_t) * need, cudaMemcpyDeviceToHost, b->stream));
+    if (!out || cap < steps * k) return bfail(b, MPM_ERR_CAPACITY, "output buffer too small");
+    std::vector<unsigned long long> t(steps * k);  // [step][scene] on the device
+    BATCH_CUDA(b, cudaMemcpyAsync(t.data(), b->arr.stamps, sizeof(uint64_t) * t.size(), cudaMemcpyDeviceToHost, b->stream));
     BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
+    for (size_t s = 0; s < k; ++s)
+        for (size_t j = 0; j < steps; ++j) out[s * steps + j] = t[j * k + s];
     return MPM_OK;
 }
 
@@ -589,108 +574,66 @@ mpm_status mpm_batch_get_config(const mpm_batch* b, mpm_batch_config* cfg) {
 
 mpm_status mpm_batch_set_config(mpm_batch* b, const mpm_batch_config* cfg) {
     if (!b || !cfg) return MPM_ERR_INVALID_ARGUMENT;
-    BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
-    const mpm_batch_config old = b->cfg;
-    mpm_status st = configure(b, *cfg);
-    if (st != MPM_OK) {
-        const std::string why = b->err;
-        configure(b, old);
-        b->err = why;
-    }
-    return st;
+    return configure(b, *cfg);
 }
 
 mpm_status mpm_batch_tune(mpm_batch* b, int32_t trial_steps, mpm_batch_config* chosen, double* best_ms) {
     if (!b || trial_steps < 1) return MPM_ERR_INVALID_ARGUMENT;
     BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
     const size_t n = (size_t)b->N;
-    // Snapshot of everything a step changes: both particle buffers (a sort
-    // moves particles between them), per-scene state, flags.
+    // Snapshot of the particles and flags; the sums are formed anew from them.
+    const BatchBuffers F = b->buf[b->parity];
     struct Span { void* p; size_t bytes; };
-    std::vector<Span> spans;
-    for (BatchBuffers& f : b->buf) {
-        spans.push_back({f.x, sizeof(float) * 2 * n});
-        spans.push_back({f.v, sizeof(float) * 2 * n});
-        spans.push_back({f.B, sizeof(float) * 4 * n});
-        spans.push_back({f.Fe, sizeof(float) * 4 * n});
-        spans.push_back({f.Jp, sizeof(float) * n});
-        spans.push_back({f.A, sizeof(float) * 4 * n});
-        spans.push_back({f.mass, sizeof(float) * n});
-        spans.push_back({f.vol, sizeof(float) * n});
-        spans.push_back({f.id, sizeof(int) * n});
-    }
-    spans.push_back({b->d_state, sizeof(BatchSceneState) * (size_t)b->nscenes});
-    spans.push_back({b->d_needs_affine, sizeof(int) * (size_t)b->nscenes});
-    spans.push_back({b->d_status, sizeof(unsigned) * (size_t)b->nscenes});
+    const Span spans[] = {{F.x, 8 * n}, {F.v, 8 * n}, {F.B, 16 * n}, {F.Fe, 16 * n}, {F.Jp, 4 * n}, {F.mass, 4 * n},
+                          {F.vol, 4 * n}, {F.id, 4 * n}, {b->arr.status, sizeof(unsigned) * (size_t)b->nscenes}};
     size_t total = 0;
     for (const Span& sp : spans) total += (sp.bytes + 255) / 256 * 256;
     unsigned char* snap = nullptr;
     BATCH_CUDA(b, balloc(&snap, total));
+    const int parity = b->parity, last = b->last_steps;
     auto copy_all = [&](bool save) {
         size_t o = 0;
         cudaError_t e = cudaSuccess;
         for (const Span& sp : spans) {
-            if (e != cudaSuccess) break;
-            e = save ? cudaMemcpyAsync(snap + o, sp.p, sp.bytes, cudaMemcpyDeviceToDevice, b->stream)
-                     : cudaMemcpyAsync(sp.p, snap + o, sp.bytes, cudaMemcpyDeviceToDevice, b->stream);
+            if (e == cudaSuccess && sp.bytes)
+                e = cudaMemcpyAsync(save ? snap + o : sp.p, save ? sp.p : snap + o, sp.bytes, cudaMemcpyDeviceToDevice,
+                                    b->stream);
             o += (sp.bytes + 255) / 256 * 256;
         }
         if (e == cudaSuccess) e = cudaStreamSynchronize(b->stream);
         return e;
     };
-    const mpm_batch_config start = b->cfg;
-    mpm_batch_config best = start;
-    double best_t = 1e300;
-    mpm_status st = MPM_OK;
     cudaEvent_t e0 = nullptr, e1 = nullptr;
+    float ms = 0.f;
+    mpm_status st = MPM_OK;
     cudaError_t ce = copy_all(true);
     if (ce == cudaSuccess) ce = cudaEventCreate(&e0);
     if (ce == cudaSuccess) ce = cudaEventCreate(&e1);
-    const int threads_c[3] = {256, 512, 1024};
-    const int ppc_c[4] = {0, 16384, 8192, 4096};
-    for (int ti = 0; ti < 3 && ce == cudaSuccess && st == MPM_OK; ++ti)
-        for (int pi = 0; pi < 4 && ce == cudaSuccess && st == MPM_OK; ++pi) {
-            mpm_batch_config cfg = start;
-            cfg.threads = threads_c[ti];
-            cfg.particles_per_cta = ppc_c[pi];
-            if (configure(b, cfg) != MPM_OK) { b->err.clear(); continue; }  // not resident: skip the candidate
-            // one untimed call (graph capture, first-touch), then the timed one
-            for (int rep = 0; rep < 2 && ce == cudaSuccess && st == MPM_OK; ++rep) {
-                if ((ce = copy_all(false)) != cudaSuccess) break;
-                if ((st = invalidate_bands(b)) != MPM_OK) break;
-                if ((ce = cudaEventRecord(e0, b->stream)) != cudaSuccess) break;
-                st = mpm_batch_step(b, trial_steps);
-                if (st != MPM_OK) break;
-                if ((ce = cudaEventRecord(e1, b->stream)) != cudaSuccess) break;
-                if ((ce = cudaEventSynchronize(e1)) != cudaSuccess) break;
-            }
-            float ms = 0.f;
-            if (ce == cudaSuccess && st == MPM_OK && cudaEventElapsedTime(&ms, e0, e1) == cudaSuccess && ms < best_t) {
-                best_t = ms;
-                best = cfg;
-            }
-        }
+    // one untimed call (graph capture, sort, sums), then the timed one
+    if (ce == cudaSuccess) st = mpm_batch_step(b, trial_steps);
+    if (ce == cudaSuccess && st == MPM_OK) ce = cudaEventRecord(e0, b->stream);
+    if (ce == cudaSuccess && st == MPM_OK) st = mpm_batch_step(b, trial_steps);
+    if (ce == cudaSuccess && st == MPM_OK) ce = cudaEventRecord(e1, b->stream);
+    if (ce == cudaSuccess && st == MPM_OK) ce = cudaEventSynchronize(e1);
+    if (ce == cudaSuccess && st == MPM_OK) ce = cudaEventElapsedTime(&ms, e0, e1);
     // put the batch back as it was, whatever happened above
-    const cudaError_t ce_restore = copy_all(false);
-    if (ce == cudaSuccess) ce = ce_restore;
+    cudaStreamSynchronize(b->stream);
+    b->parity = parity;
+    b->last_steps = last;
+    const cudaError_t cr = copy_all(false);
+    if (ce == cudaSuccess) ce = cr;
+    const mpm_status sf = forget_sums(b);
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
     cudaFree(snap);
     if (ce != cudaSuccess) {
         cudaGetLastError();
-        configure(b, start);
         return bfail(b, MPM_ERR_CUDA, std::string("tuner: ") + cudaGetErrorString(ce));
     }
-    if (st != MPM_OK) {
-        const std::string why = b->err;
-        configure(b, start);
-        b->err = why;
-        return st;
-    }
-    st = configure(b, best);
     if (st != MPM_OK) return st;
-    if (chosen) *chosen = best;
-    if (best_ms) *best_ms = best_t;
+    if (sf != MPM_OK) return sf;
+    if (chosen) *chosen = b->cfg;
+    if (best_ms) *best_ms = ms;
     return MPM_OK;
 }
 

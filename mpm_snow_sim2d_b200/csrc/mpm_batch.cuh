@@ -1,134 +1,62 @@
-// Batched 2D scenes: many independent MLS scenes of uneven size in one
-// persistent launch per cluster size.
+// Batched 2D scenes: many independent MLS scenes of uneven size stepped together
+// by the kernels of the single-scene solver.
 //
-// Each scene runs on a thread-block cluster of 1, 2, 4 or 8 CTAs that holds the
-// scene's whole grid in distributed shared memory: node rows are cut into
-// bands, one per CTA, three int64 fixed-point accumulators per node (mass,
-// momentum x, momentum y; 24 bytes, so a 257 x 257 grid fits in 8 CTAs). A
-// step is
-//   P2G   each CTA scatters its particles into the owning CTAs' shared memory
-//         (red.shared::cluster.add.u64)
-//   grid  each CTA turns its own band into velocities (vf, vc) in place
-//   G2P   each CTA gathers its particles' stencils from the owning CTAs
-//         (ld.shared::cluster), updates them and the return map, and writes
-//         the next step's affine matrix
-// with a cluster barrier between phases. No grid touches HBM and no global
-// atomics are issued; particle state streams through HBM once per phase.
+// The scenes lie side by side: one particle array (scene after scene), one grid
+// (each scene's nodes after the last scene's), one list of cell tiles and of node
+// blocks. A step is the single solver's: grid update over the marked node blocks,
+// G2P and the next P2G by one warp per window of 32 slots (fused_window), the
+// queued particles' return map, their P2G. A window lies in one tile of one scene,
+// whose constants its warp reads from shared memory. Every sort_period steps all
+// scenes are sorted by (tile, cell, id).
 //
-// Every sort_period steps a multi-CTA cluster counting-sorts its scene's
-// particles by cell row into the second particle buffer and re-cuts the bands
-// so that each CTA holds about n / cl particles and the rows they touch
-// (within its shared-memory capacity): most scatter and gather traffic then
-// stays in the CTA's own shared memory. The per-particle arithmetic is that
-// of the single-scene kernels (the same device functions) and the int64 sums
-// are exact, so a scene's result depends neither on its cluster size, nor on
-// the particle order, nor on the other scenes of the batch.
+// A scene's result depends neither on the other scenes, nor on the order of its
+// particles, nor on when it was sorted: each particle's contribution to a node is
+// rounded to int64 fixed point by itself (the EXACT scatter; integer sums), and
+// all else is per particle or per node.
 //
-// Clusters are persistent: each takes scenes from an atomic queue (most
-// expensive first) and runs all requested steps of one scene before taking
-// the next.
+// Bound: as k_g2p2g_direct (memory pipe and issue). The former kernel held each
+// scene's grid in the shared memory of a thread-block cluster and added 48 int64
+// values per particle and step there (red.shared::cluster, 68% of their wavefronts
+// bank conflicts); one persistent cluster per scene left the GPU waiting for the
+// largest ones. 256 scenes, 2.81M particles: 1.18 ms per step, now 0.43.
 #pragma once
 
-#include <cooperative_groups.h>
-
-#include "mpm_kernels.cuh"
+#include "mpm_fused.cuh"
 
 namespace mpm {
 
-namespace cg = cooperative_groups;
-
-constexpr int kBatchMaxCluster = 8;
-constexpr int kBatchAccs = 3;         // mass, momentum x, momentum y
-constexpr int kBatchMaxRows = 512;    // node rows of one scene
+constexpr int kBatchMaxRows = 512;  // node rows of one scene
 
 struct BatchScene {
     StepConsts C;
-    long long p0;  // first particle slot of the scene
-    int n;         // particles
-    int cl;        // CTAs of the scene's cluster
-    int rows;      // most node rows one CTA can hold (shared-memory capacity / nx)
-    int pad;
+    SceneView view;    // extents, tiles per axis, first tile
+    long long p0;      // first particle slot
+    long long node0;   // first node
+    int n;             // particles
+    int blk0;          // first node block
+    int nblk[2];       // node blocks per axis
 };
 
-// Per-scene state that persists between launches.
-struct BatchSceneState {
-    int parity;                      // which particle buffer holds the scene
-    int step;                        // steps taken since creation (or the last state upload)
-    int sorted;                      // the bands below are valid
-    int pad;
-    int cut[kBatchMaxCluster + 1];   // band b holds node rows [cut[b], cut[b+1])
-    int off[kBatchMaxCluster + 1];   // and particles [p0 + off[b], p0 + off[b+1])
-};
-
-struct BatchBuffers {
-    float* x;
-    float* v;
-    float* B;
-    float* Fe;
-    float* Jp;
-    float* A;  // P2G affine matrix of the next step (written by G2P)
-    float* mass;
-    float* vol;
-    int* id;   // creation index of the particle within its scene
-};
-
-struct BatchParticles {
-    BatchBuffers buf[2];
-    long long N;  // component stride of the SoA arrays
-};
-
-struct BatchRun {
+struct ManyScenes {
     const BatchScene* scenes;
-    BatchSceneState* state;
-    const int* order;            // this class's scenes, most expensive first
-    int count;                   // scenes in this class
-    int cap;                     // nodes per accumulator array in each CTA
-    int* queue;                  // next work item; zero before the launch
-    int* needs_affine;           // per scene: derive A from (B, F_E, J_p) first
-    unsigned* status;            // per scene: MPM_FLAG_* bits
-    unsigned long long* stamps;  // per scene: steps + 1 device timestamps (ns), or null
-    int steps;
-    int sort_period;
+    const int* of_slots;  // scene of each slot
+    const int* of_tiles;  // scene of each tile
+    __device__ __forceinline__ const SceneView& of_slot(int i) const { return scenes[of_slots[i]].view; }
+    __device__ __forceinline__ const SceneView& of_tile(int t) const { return scenes[of_tiles[t]].view; }
 };
 
-__device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
-
-// Address of the same shared-memory offset in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t cluster_map(uint32_t addr, uint32_t rank) {
-    uint32_t r;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-    return r;
-}
-
-// Each shared::cluster access carries a "memory" clobber so that the compiler
-// keeps it on its side of the cluster barriers (which order the phases).
-__device__ __forceinline__ void cluster_red_add(uint32_t addr, long long v) {
-    if (v != 0)
-        asm volatile("red.relaxed.cluster.shared::cluster.add.u64 [%0], %1;" ::"r"(addr), "l"((unsigned long long)v)
-                     : "memory");
-}
-
-__device__ __forceinline__ void cluster_red_add_u32(uint32_t addr, unsigned v) {
-    asm volatile("red.relaxed.cluster.shared::cluster.add.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory");
-}
-
-__device__ __forceinline__ unsigned cluster_atom_add_u32(uint32_t addr, unsigned v) {
-    unsigned old;
-    asm volatile("atom.relaxed.cluster.shared::cluster.add.u32 %0, [%1], %2;" : "=r"(old) : "r"(addr), "r"(v) : "memory");
-    return old;
-}
-
-__device__ __forceinline__ unsigned cluster_ld_u32(uint32_t addr) {
-    unsigned r;
-    asm volatile("ld.shared::cluster.u32 %0, [%1];" : "=r"(r) : "r"(addr) : "memory");
-    return r;
-}
-
-__device__ __forceinline__ float2 cluster_ld_f2(uint32_t addr) {
-    float2 r;
-    asm volatile("ld.shared::cluster.v2.f32 {%0, %1}, [%2];" : "=f"(r.x), "=f"(r.y) : "r"(addr) : "memory");
-    return r;
-}
+struct BatchArrays {
+    const BatchScene* scenes;
+    const int* of_slots;
+    const int* of_blocks;        // scene of each node block
+    unsigned long long* acc;     // [nodes][4]
+    float4* gv;                  // [nodes]
+    unsigned* status;            // per scene: MPM_FLAG_* bits
+    int* fresh;                  // per scene: the pending sums are missing (new or uploaded state)
+    unsigned long long* stamps;  // [step of the call][scene] device timestamps (ns)
+    int* step;                   // device scalar: steps of the call done so far
+    int nscenes;
+};
 
 __device__ __forceinline__ unsigned long long device_ns() {
     unsigned long long t;
@@ -136,383 +64,129 @@ __device__ __forceinline__ unsigned long long device_ns() {
     return t;
 }
 
-__device__ __forceinline__ unsigned long long pack_f2(float lo, float hi) {
-    return (unsigned long long)__float_as_uint(lo) | ((unsigned long long)__float_as_uint(hi) << 32);
+// A scene's own view of the tiles and node blocks.
+__device__ __forceinline__ TileInfo scene_tiles(const TileInfo& TI, const BatchScene& S) {
+    TileInfo V = TI;
+    V.tiles[0] = S.view.tiles[0];
+    V.tiles[1] = S.view.tiles[1];
+    V.nblk[0] = S.nblk[0];
+    V.nblk[1] = S.nblk[1];
+    V.blk0 = S.blk0;
+    return V;
 }
 
-// Node row -> (owning CTA, offset of the row in that CTA's arrays).
-struct BatchRowMap {
-    const unsigned char* owner;
-    const int* base;  // (row - first row of the band) * nx
-};
+// The scene's record into the warp's shared memory.
+__device__ __forceinline__ const BatchScene& stage_scene(const BatchScene* scenes, int s, BatchScene* mine) {
+    constexpr int W = sizeof(BatchScene) / 4;
+    __syncwarp();
+    for (int k = threadIdx.x & 31; k < W; k += 32)
+        reinterpret_cast<int*>(mine)[k] = reinterpret_cast<const int*>(scenes + s)[k];
+    __syncwarp();
+    return *mine;
+}
 
-// P2G of particles [lo, hi) of one scene (MLS, src/gpu/shaders/2d/p2g.glsl:29-92):
-//   m_i += w m_p,  p_i += w (m_p v_p + A_p (x_i - x_p)),  int64 fixed point.
-template <int THREADS>
-__device__ __forceinline__ void batch_p2g(const BatchBuffers& P, long long N, const StepConsts& C, long long lo,
-                                          long long hi, const BatchRowMap& M, uint32_t g0, int cap,
-                                          unsigned* status) {
-    for (long long i = lo + threadIdx.x; i < hi; i += THREADS) {
-        const float vol = P.vol[i];
-        if (vol == 0.f) continue;
-        const float x[2] = {P.x[i], P.x[N + i]};
-        const float mass = P.mass[i];
-        const float mv[2] = {mass * P.v[i], mass * P.v[N + i]};
-        float A[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) A[k] = P.A[k * N + i];
-        const int ext[2] = {C.W, C.H};
-        int base[2];
-        float wk[2][4], off[2][4];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            base[k] = stencil_base(x[k], ext[k]);
-            Stencil<4>::weights(x[k], base[k], wk[k]);
-#pragma unroll
-            for (int o = 0; o < 4; ++o) off[k][o] = float(base[k] + o) - x[k];
-        }
-        bool outside = false;
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int iy = base[1] + b;
-            if (iy < 0 || iy > C.H) { outside = true; continue; }
-            const uint32_t row = cluster_map(g0, M.owner[iy]) + 8u * (uint32_t)M.base[iy];
-#pragma unroll
-            for (int a = 0; a < 4; ++a) {
-                const int ix = base[0] + a;
-                if (ix < 0 || ix > C.W) { outside = true; continue; }
-                const float w = wk[0][a] * wk[1][b];
-                const float d[2] = {off[0][a], off[1][b]};
-                const uint32_t at = row + 8u * (uint32_t)ix;
-                cluster_red_add(at, to_fixed(w * mass, C.sm, status));
-#pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    float s = mv[r];
-#pragma unroll
-                    for (int k = 0; k < 2; ++k) s += A[r * 2 + k] * d[k];
-                    cluster_red_add(at + 8u * (uint32_t)((1 + r) * cap), to_fixed(w * s, C.sp, status));
-                }
-            }
-        }
-        if (outside) raise_flag(status, 4u);
+// Grid update of the marked node blocks of all scenes (k_grid_marked per scene);
+// records the time at which a step begins.
+__global__ void __launch_bounds__(256) k_batch_grid(BatchArrays B, TileInfo TI) {
+    using G = TileGeom<2>;
+    const int nb = *TI.n_marked;
+    const long long total = (long long)nb * G::BN;
+    if (blockIdx.x == 0) {
+        const int step = *B.step;
+        const unsigned long long t = device_ns();
+        for (int s = threadIdx.x; s < B.nscenes; s += blockDim.x) B.stamps[(long long)step * B.nscenes + s] = t;
     }
+    for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < total;
+         w += (long long)gridDim.x * blockDim.x) {
+        const int blk = TI.mark_list[w / G::BN], loc = int(w % G::BN);
+        const int sc = B.of_blocks[blk];
+        const BatchScene& S = B.scenes[sc];
+        const int rb = blk - S.blk0;
+        const int gx = rb % S.nblk[0] * G::T + loc % G::T, gy = rb / S.nblk[0] * G::T + loc / G::T;
+        if (loc == 0) TI.mark[blk] = 0;
+        if (gx >= S.C.nx || gy >= S.C.ny) continue;
+        grid_node_at<2, kMLS>(S.C, B.acc + S.node0 * 4, B.gv + S.node0, B.status + sc, (long long)gy * S.C.nx + gx, gx, gy, 0);
+    }
+    grid_finish(TI, B.step);
 }
 
-// G2P + APIC + return map of particles [lo, hi) (src/gpu/shaders/2d/g2p.glsl:
-// 21-93), the arithmetic of k_g2p_simple, then the next step's affine matrix.
-template <int THREADS>
-__device__ __forceinline__ void batch_g2p(const BatchBuffers& P, long long N, const StepConsts& C, long long lo,
-                                          long long hi, const BatchRowMap& M, uint32_t g0, int cap,
-                                          unsigned* status) {
-    for (long long i = lo + threadIdx.x; i < hi; i += THREADS) {
-        const float x[2] = {P.x[i], P.x[N + i]};
-        // the rest of the particle's state, loaded before the gather so that
-        // its latency overlaps the stencil reads
-        float Fe[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) Fe[k] = P.Fe[k * N + i];
-        float Jp = P.Jp[i];
-        const float mass = P.mass[i], vol = P.vol[i];
-        const int ext[2] = {C.W, C.H};
-        int base[2];
-        float wk[2][4], off[2][4];
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            base[k] = stencil_base(x[k], ext[k]);
-            Stencil<4>::weights(x[k], base[k], wk[k]);
-#pragma unroll
-            for (int o = 0; o < 4; ++o) off[k][o] = float(base[k] + o) - x[k];
-        }
-        uint32_t row[4];
-        bool row_in[4];
-#pragma unroll
-        for (int b = 0; b < 4; ++b) {
-            const int iy = base[1] + b;
-            row_in[b] = iy >= 0 && iy <= C.H;
-            const int r = row_in[b] ? iy : 0;
-            row[b] = cluster_map(g0, M.owner[r]) + 8u * (uint32_t)M.base[r];
-        }
-        float nv[2] = {0.f, 0.f}, nxp[2] = {0.f, 0.f}, nB[4] = {0.f, 0.f, 0.f, 0.f};
-        float wsum = 0.f;
-        bool clipped = false;
-#pragma unroll
-        for (int a = 0; a < 4; ++a) {
-            const int ix = base[0] + a;
-            if (ix < 0 || ix > C.W) { clipped = true; continue; }
-#pragma unroll
-            for (int b = 0; b < 4; ++b) {
-                if (!row_in[b]) { clipped = true; continue; }
-                const uint32_t at = row[b] + 8u * (uint32_t)ix;
-                const float2 gf = cluster_ld_f2(at);
-                const float2 gc = cluster_ld_f2(at + 8u * (uint32_t)cap);
-                const float vf[2] = {gf.x, gf.y}, vc[2] = {gc.x, gc.y};
-                const float w = wk[0][a] * wk[1][b];
-                const float d[2] = {off[0][a], off[1][b]};
-                wsum += w;
-#pragma unroll
-                for (int r = 0; r < 2; ++r) {
-                    nv[r] += vf[r] * w;
-#pragma unroll
-                    for (int k = 0; k < 2; ++k) nB[r * 2 + k] += w * (vf[r] * d[k]);
-                    nxp[r] += (d[r] + C.dt * vc[r]) * w;
-                }
-            }
-        }
-        bool finite = true;
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const float xn = (clipped ? x[k] * wsum : x[k]) + nxp[k];
-            P.v[k * N + i] = nv[k];
-            P.x[k * N + i] = xn;
-            finite = finite && isfinite(xn);
-        }
-#pragma unroll
-        for (int k = 0; k < 4; ++k) P.B[k * N + i] = nB[k];
-        float L[4], Fh[4];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) L[k] = ((k % 3) == 0 ? 1.f : 0.f) + C.dt * (3.f * nB[k]);
-        matmul<2>(L, Fe, Fh);
-        plasticity<2, kMLS>(C, Fh, Fe, Jp, status);
-        float Anext[4];
-        mls_affine<2>(C, nB, Fe, Jp, mass, vol, Anext);
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            P.Fe[k * N + i] = Fe[k];
-            P.A[k * N + i] = Anext[k];
-        }
-        P.Jp[i] = Jp;
-        if (!finite || !isfinite(Jp)) raise_flag(status, 1u);
+// The fused step of one window per warp (k_g2p2g_direct), or with G2P = false the
+// P2G of the stored state of the scenes that have no pending sums.
+template <bool G2P>
+__global__ void __launch_bounds__(FusedGeom<2>::THREADS, MPM_FUSED_MIN_BLOCKS)
+    k_batch_step(Particles P, BatchArrays B, TileInfo TI, SlowQueue Q) {
+    using G = FusedGeom<2>;
+    __shared__ float4 pay_s[G::WARPS][G::WIN * G::PS / 4];
+    __shared__ BatchScene scene_s[G::WARPS];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    float* pay = reinterpret_cast<float*>(pay_s[wid]);
+    const int nitems = *TI.n_items;
+    for (int e = wid * gridDim.x + blockIdx.x; e < nitems; e += G::WARPS * gridDim.x) {
+        const int4 item = TI.items[e];
+        if (!G2P && !B.fresh[item.w]) continue;
+        const BatchScene& S = stage_scene(B.scenes, item.w, &scene_s[wid]);
+        const TileInfo V = scene_tiles(TI, S);
+        SlowQueue QS = Q;
+        QS.scene = item.w;
+        int tc[3] = {0, 0, 0}, bo[3] = {0, 0, 0};
+        tile_origin<2>(V, item.x - S.view.tile0, tc, bo);
+        const unsigned bits = __reduce_or_sync(
+            0xffffffffu, fused_window<2, 4, G2P, true, true>(P, S.C, V, B.gv + S.node0, B.acc + S.node0 * 4, QS,
+                                                             B.status + item.w, nullptr, bo, item.y, item.z, TI.win, 0, pay));
+        if (lane < 9 && (bits >> lane) & 1u)
+            mark_block_once(V, (tc[1] - 1 + lane / 3) * V.nblk[0] + tc[0] - 1 + lane % 3);
     }
 }
 
-__device__ __forceinline__ int cell_row(float y, int H) { return min(max(int(fmaxf(y, 0.f)), 0), H); }
-
-// Counting sort of one scene's particles by cell row, from buffer `src` to
-// `dst`, and new bands: cut rows balance the particle count per CTA subject to
-// at most `max_rows` rows per CTA. Runs on every CTA of the cluster; the
-// scratch is CTA 0's first accumulator array (all-zero on entry and on exit).
-// s_cut / s_off (shared, every CTA) receive the bands.
-template <int THREADS>
-__device__ void batch_sort(const BatchParticles& P, int src, const BatchScene& S, int max_rows, unsigned rank,
-                           unsigned cl, long long lo, long long hi, unsigned long long* a0, int* s_cut, int* s_off,
-                           cg::cluster_group& cluster) {
-    const int tid = threadIdx.x;
-    const int ny = S.C.ny;
-    unsigned* hist = reinterpret_cast<unsigned*>(a0);  // rows counts, then row cursors (CTA 0)
-    const uint32_t hist0 = cluster_map(smem_addr(hist), 0);
-    const BatchBuffers& F = P.buf[src];
-    const BatchBuffers& T = P.buf[src ^ 1];
-    const long long N = P.N;
-    for (long long i = lo + tid; i < hi; i += THREADS)
-        cluster_red_add_u32(hist0 + 4u * (uint32_t)cell_row(F.x[N + i], S.C.H), 1u);
-    cluster.sync();
-    if (rank == 0) {
-        // exclusive prefix over rows (one warp), then the cuts (one thread)
-        if (tid < 32) {
-            const int per = (ny + 31) / 32, r0 = tid * per, r1 = min(ny, r0 + per);
-            unsigned run = 0;
-            for (int r = r0; r < r1; ++r) run += hist[r];
-            unsigned incl = run;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned t = __shfl_up_sync(0xffffffffu, incl, o);
-                if (tid >= o) incl += t;
-            }
-            unsigned acc = incl - run;
-            for (int r = r0; r < r1; ++r) {
-                const unsigned c = hist[r];
-                hist[r] = acc;
-                acc += c;
-            }
-        }
-        __syncthreads();
-        if (tid == 0) {
-            const long long n = S.n;
-            int start = 0;
-            s_cut[0] = 0;
-            s_off[0] = 0;
-            for (unsigned b = 0; b < cl; ++b) {
-                int end;
-                if (b + 1 == cl) {
-                    end = ny;
-                } else {
-                    const long long target = n * (b + 1) / cl;
-                    // first row whose start offset reaches the target
-                    int lo_r = start, hi_r = ny;
-                    while (lo_r < hi_r) {
-                        const int mid = (lo_r + hi_r) >> 1;
-                        if ((long long)hist[mid] >= target) hi_r = mid;
-                        else lo_r = mid + 1;
-                    }
-                    end = lo_r;
-                    const int rest = (int)(cl - b - 1);
-                    end = max(end, ny - rest * max_rows);  // the remaining CTAs must hold the rest
-                    end = min(end, start + max_rows);
-                    end = max(end, start);
-                    end = min(end, ny);
-                }
-                s_cut[b + 1] = end;
-                s_off[b + 1] = end < ny ? (int)hist[end] : S.n;
-                start = end;
-            }
-        }
+__global__ void __launch_bounds__(256) k_batch_plastic(Particles P, BatchArrays B, SlowQueue Q) {
+    const int m = *Q.count;
+    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
+        const int entry = Q.list[e], sc = B.of_slots[entry >= 0 ? entry : -1 - entry];
+        const BatchScene& S = B.scenes[sc];
+        g2p_queued_exact<2, 4>(P, S.C, B.gv + S.node0, Q, e, B.status + sc);
     }
-    cluster.sync();
-    if (rank != 0 && tid <= (int)cl) {
-        s_cut[tid] = (int)cluster_ld_u32(cluster_map(smem_addr(s_cut + tid), 0));
-        s_off[tid] = (int)cluster_ld_u32(cluster_map(smem_addr(s_off + tid), 0));
-    }
-    // scatter: slot = row start + arrival order within the row
-    for (long long i = lo + tid; i < hi; i += THREADS) {
-        const float y = F.x[N + i];
-        const long long j = S.p0 + cluster_atom_add_u32(hist0 + 4u * (uint32_t)cell_row(y, S.C.H), 1u);
-        T.x[j] = F.x[i];
-        T.x[N + j] = y;
-#pragma unroll
-        for (int k = 0; k < 2; ++k) T.v[k * N + j] = F.v[k * N + i];
-#pragma unroll
-        for (int k = 0; k < 4; ++k) {
-            T.B[k * N + j] = F.B[k * N + i];
-            T.Fe[k * N + j] = F.Fe[k * N + i];
-            T.A[k * N + j] = F.A[k * N + i];
-        }
-        T.Jp[j] = F.Jp[i];
-        T.mass[j] = F.mass[i];
-        T.vol[j] = F.vol[i];
-        T.id[j] = F.id[i];
-    }
-    cluster.sync();
-    if (rank == 0)
-        for (int r = tid; r < ny; r += THREADS) hist[r] = 0u;
-    // the next cluster barrier (before any use of the arrays) orders this clear
 }
 
-template <int THREADS>
-__global__ void __launch_bounds__(THREADS, 1) k_batch_run(BatchParticles P, BatchRun R) {
-    extern __shared__ __align__(16) unsigned long long sgrid[];
-    __shared__ int s_item, s_parity, s_step0, s_sorted;
-    __shared__ int s_cut[kBatchMaxCluster + 1], s_off[kBatchMaxCluster + 1];
-    __shared__ unsigned char s_owner[kBatchMaxRows];
-    __shared__ int s_base[kBatchMaxRows];
-    __shared__ StepConsts sC;
-    cg::cluster_group cluster = cg::this_cluster();
-    const unsigned rank = cluster.block_rank(), cl = cluster.num_blocks();
-    const int tid = threadIdx.x;
-    const int cap = R.cap;
-    unsigned long long* a0 = sgrid;
-    unsigned long long* a1 = sgrid + cap;
-    unsigned long long* a2 = sgrid + 2 * (long long)cap;
-    const uint32_t g0 = smem_addr(sgrid);
-    const BatchRowMap M{s_owner, s_base};
-    // the accumulators are all-zero between steps; start from there
-    for (int j = tid; j < kBatchAccs * cap; j += THREADS) sgrid[j] = 0ull;
-    for (;;) {
-        if (rank == 0 && tid == 0) s_item = atomicAdd(R.queue, 1);
-        cluster.sync();
-        const int item = *cluster.map_shared_rank(&s_item, 0);
-        cluster.sync();  // every CTA has read the item before CTA 0 may change it or exit
-        if (item >= R.count) break;
-        const int sc = R.order[item];
-        const BatchScene& S = R.scenes[sc];
-        BatchSceneState& G = R.state[sc];
-        if (tid == 0) {
-            sC = S.C;
-            s_parity = G.parity;
-            s_step0 = G.step;
-            s_sorted = G.sorted;
-        }
-        if (tid <= (int)cl) {
-            s_cut[tid] = G.cut[tid];
-            s_off[tid] = G.off[tid];
-        }
-        __syncthreads();
-        if (tid == 0 && s_sorted) {
-            // stored bands are used only if they partition this scene for this cluster size
-            bool ok = s_cut[0] == 0 && s_cut[cl] == S.C.ny && s_off[0] == 0 && s_off[cl] == S.n;
-            for (unsigned b = 0; b < cl; ++b)
-                ok = ok && s_cut[b] <= s_cut[b + 1] && s_cut[b + 1] - s_cut[b] <= S.rows && s_off[b] <= s_off[b + 1];
-            if (!ok) s_sorted = 0;
-        }
-        __syncthreads();
-        const StepConsts& C = sC;
-        unsigned* status = R.status + sc;
-        const int nx = C.nx, ny = C.ny;
-        int parity = s_parity;
-        const bool banded = cl > 1;
-        if (!banded || !s_sorted) {
-            // equal bands of rows and of particles, until the first sort
-            if (tid <= (int)cl) {
-                s_cut[tid] = min(ny, tid * ((ny + (int)cl - 1) / (int)cl));
-                s_off[tid] = (int)((long long)S.n * tid / cl);
-            }
-            __syncthreads();
-        }
-        if (R.needs_affine[sc]) {
-            const BatchBuffers& F = P.buf[parity];
-            const long long lo = S.p0 + s_off[rank], hi = S.p0 + s_off[rank + 1];
-            for (long long i = lo + tid; i < hi; i += THREADS) {
-                float B[4], Fe[4], A[4];
-#pragma unroll
-                for (int k = 0; k < 4; ++k) { B[k] = F.B[k * P.N + i]; Fe[k] = F.Fe[k * P.N + i]; }
-                mls_affine<2>(C, B, Fe, F.Jp[i], F.mass[i], F.vol[i], A);
-#pragma unroll
-                for (int k = 0; k < 4; ++k) F.A[k * P.N + i] = A[k];
-            }
-        }
-        unsigned long long* stamp = R.stamps ? R.stamps + (long long)sc * (R.steps + 1) : nullptr;
-        if (stamp && rank == 0 && tid == 0) stamp[0] = device_ns();
-        bool sorted = s_sorted != 0;
-        for (int step = 0; step < R.steps; ++step) {
-            if (banded && (!sorted || (R.sort_period > 0 && (s_step0 + step) % R.sort_period == 0))) {
-                cluster.sync();  // A of every particle is written before it moves
-                batch_sort<THREADS>(P, parity, S, S.rows, rank, cl, S.p0 + s_off[rank], S.p0 + s_off[rank + 1],
-                                    a0, s_cut, s_off, cluster);
-                parity ^= 1;
-                sorted = true;
-            }
-            if (step == 0 || banded) {
-                // row -> (owner, offset) for the current bands
-                for (int r = tid; r < ny; r += THREADS) {
-                    int b = 0;
-                    while (b + 1 < (int)cl && r >= s_cut[b + 1]) ++b;
-                    s_owner[r] = (unsigned char)b;
-                    s_base[r] = (r - s_cut[b]) * nx;
-                }
-            }
-            cluster.sync();
-            const BatchBuffers& F = P.buf[parity];
-            const long long lo = S.p0 + s_off[rank], hi = S.p0 + s_off[rank + 1];
-            const int row0 = s_cut[rank];
-            const int my_nodes = (s_cut[rank + 1] - row0) * nx;
-            batch_p2g<THREADS>(F, P.N, C, lo, hi, M, g0, cap, status);
-            cluster.sync();
-            for (int j = tid; j < my_nodes; j += THREADS) {
-                const long long q[3] = {(long long)a0[j], (long long)a1[j], (long long)a2[j]};
-                const int iy = row0 + j / nx, ix = j - (j / nx) * nx;
-                float vc[3], vf[3];
-                grid_node_velocity<2, kMLS>(C, q, ix, iy, 0, status, vc, vf);
-                a0[j] = pack_f2(vf[0], vf[1]);
-                a1[j] = pack_f2(vc[0], vc[1]);
-                a2[j] = 0ull;
-            }
-            cluster.sync();
-            batch_g2p<THREADS>(F, P.N, C, lo, hi, M, g0, cap, status);
-            cluster.sync();
-            for (int j = tid; j < my_nodes; j += THREADS) { a0[j] = 0ull; a1[j] = 0ull; }
-            if (stamp && rank == 0 && tid == 0) stamp[step + 1] = device_ns();
-        }
-        cluster.sync();  // the arrays are clear and every CTA is done with the scene
-        if (rank == 0 && tid == 0) {
-            R.needs_affine[sc] = 0;
-            G.parity = parity;
-            G.step = s_step0 + R.steps;
-            G.sorted = sorted ? 1 : 0;
-        }
-        if (rank == 0 && tid <= (int)cl) {
-            G.cut[tid] = s_cut[tid];
-            G.off[tid] = s_off[tid];
-        }
+// P2G of the queued particles (k_p2g_windows).
+__global__ void __launch_bounds__(FusedGeom<2>::THREADS) k_batch_windows(Particles P, BatchArrays B, TileInfo TI, SlowQueue Q) {
+    using G = FusedGeom<2>;
+    __shared__ float4 pay_s[G::WARPS][G::WIN * G::PS / 4];
+    __shared__ BatchScene scene_s[G::WARPS];
+    const int wid = threadIdx.x >> 5;
+    const int nw = min(*Q.nwin, Q.win_capacity);
+    for (int r = blockIdx.x * G::WARPS + wid; r < nw; r += gridDim.x * G::WARPS) {
+        const int4 rec = Q.win[r];
+        const BatchScene& S = stage_scene(B.scenes, rec.w, &scene_s[wid]);
+        queued_window<2, 4, true>(P, S.C, scene_tiles(TI, S), rec, B.acc + S.node0 * 4, B.status + rec.w,
+                                  reinterpret_cast<float*>(pay_s[wid]));
     }
+}
+
+// End of a call, one CTA: the last time stamp; the step count starts over.
+__global__ void __launch_bounds__(256) k_batch_end(BatchArrays B) {
+    const unsigned long long t = device_ns();
+    const int step = *B.step;
+    for (int s = threadIdx.x; s < B.nscenes; s += blockDim.x) B.stamps[(long long)step * B.nscenes + s] = t;
+    __syncthreads();
+    if (threadIdx.x == 0) *B.step = 0;
+}
+
+// One field of a scene, creation order, and back (slots of the scene hold particles
+// id[slot]; an upload keeps the slot order, the next sort restores locality).
+__global__ void __launch_bounds__(256) k_batch_export(const float* __restrict__ soa, long long stride, int comps, long long p0,
+                                                      int n, const int* __restrict__ id, float* __restrict__ aos) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const int p = id[p0 + s];
+    for (int c = 0; c < comps; ++c) aos[(long long)p * comps + c] = soa[c * stride + p0 + s];
+}
+
+__global__ void __launch_bounds__(256) k_batch_import(float* __restrict__ soa, long long stride, int comps, long long p0, int n,
+                                                      const int* __restrict__ id, const float* __restrict__ aos) {
+    const int s = blockIdx.x * blockDim.x + threadIdx.x;
+    if (s >= n) return;
+    const int p = id[p0 + s];
+    for (int c = 0; c < comps; ++c) soa[c * stride + p0 + s] = aos[(long long)p * comps + c];
 }
 
 }  // namespace mpm

@@ -239,15 +239,16 @@ void invalidate_graphs(mpm_solver* s) {
 template <int D, int S> cudaError_t launch_sort(mpm_solver* s) {
     if (s->n == 0) { s->needs_sort = false; s->next_sort = s->step + s->cur_K; return cudaSuccess; }
     const int threads = 256, blocks = (s->n + threads - 1) / threads;
-    k_sort_count<D, S><<<blocks, threads, 0, s->stream>>>(particle_view(s), s->C, s->ti);
+    const OneScene scene{{{s->C.W, s->C.H, s->C.Dp}, {s->ti.tiles[0], s->ti.tiles[1], s->ti.tiles[2]}, 0}};
+    k_sort_count<D, S, OneScene><<<blocks, threads, 0, s->stream>>>(particle_view(s), scene, s->ti);
     const int scan_blocks = (s->ti.n_tiles + kScanTiles - 1) / kScanTiles;
     k_sort_block_sums<<<scan_blocks, kScanTiles, 0, s->stream>>>(s->ti);
     k_sort_scan<<<scan_blocks, kScanTiles, 0, s->stream>>>(s->ti);
     k_sort_bucket<<<blocks, threads, 0, s->stream>>>(s->n, s->ti);
     SortBuffers dst = s->alt;
     if (s->fused) dst.A = nullptr;  // the fused path keeps A only within a step
-    k_tile_sort<D, S><<<s->sms * SortGeom<D>::CTAS_PER_SM, 256, 0, s->stream>>>(particle_view(s), s->id, dst, s->C,
-                                                                               s->ti);
+    k_tile_sort<D, S, OneScene><<<s->sms * SortGeom<D>::CTAS_PER_SM, 256, 0, s->stream>>>(particle_view(s), s->id, dst,
+                                                                                         scene, s->ti);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     swap_buffers(s);

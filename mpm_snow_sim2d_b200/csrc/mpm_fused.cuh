@@ -36,6 +36,8 @@
 // themselves, so a resumed run never recomputes them.
 #pragma once
 
+#include <type_traits>
+
 #include <cuda.h>
 
 #include "mpm_tiled.cuh"
@@ -296,8 +298,15 @@ __device__ __forceinline__ void write_payload(const StepConsts& C, const float* 
 // One lane's share of a window: the S node planes of its column as channel
 // pairs (momentum x, y; mass, momentum z), the largest scaled sum so far (range
 // check) and where and how it adds to the grid.
-template <int D, int S> struct ScatterLane {
-    float2 a[S][Scatter<D, S>::PAIRS];
+// EXACT (batched scenes): every particle's contribution becomes int64 fixed point
+// before it is summed, so that a node's sum depends neither on the order nor on
+// the grouping of the particles.
+struct Fixed2 {
+    long long x, y;
+};
+
+template <int D, int S, bool EXACT = false> struct ScatterLane {
+    std::conditional_t<EXACT, Fixed2, float2> a[S][Scatter<D, S>::PAIRS];
     float top;
     unsigned long long* at;  // first node column and channel the lane adds to, at node 0
     int at2;                 // its second add, relative to the first
@@ -307,8 +316,8 @@ template <int D, int S> struct ScatterLane {
 };
 
 // The lane's two sums of one node plane at `node` to the grid.
-template <int D, int S>
-__device__ __forceinline__ void add_sums(ScatterLane<D, S>& T, long long node, float2 v) {
+template <int D, int S, bool EXACT>
+__device__ __forceinline__ void add_sums(ScatterLane<D, S, EXACT>& T, long long node, float2 v) {
     unsigned long long* p = T.at + node * 4;
     const float t0 = v.x * T.scale0, t1 = v.y * T.scale1;
     T.top = fmaxf(T.top, fmaxf(fabsf(t0), fabsf(t1)));
@@ -316,13 +325,23 @@ __device__ __forceinline__ void add_sums(ScatterLane<D, S>& T, long long node, f
     if (T.both) red_scaled(p + T.at2, t1);
 }
 
+template <int D, int S>
+__device__ __forceinline__ void add_sums(ScatterLane<D, S, true>& T, long long node, Fixed2 v) {
+    unsigned long long* p = T.at + node * 4;
+    red_int(p, v.x);
+    if (T.both) red_int(p + T.at2, v.y);
+}
+
+__device__ __forceinline__ Fixed2 shfl_xor2(Fixed2 v, int m) {
+    return Fixed2{__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m)};
+}
 __device__ __forceinline__ float2 shfl_xor2(float2 v, int m) {
     return make_float2(__shfl_xor_sync(0xffffffffu, v.x, m), __shfl_xor_sync(0xffffffffu, v.y, m));
 }
 
 // One node plane `v` (x = node's) to the grid.
-template <int D, int S>
-__device__ __forceinline__ void add_plane(ScatterLane<D, S>& T, long long node, const float2* v) {
+template <int D, int S, bool EXACT, typename V>
+__device__ __forceinline__ void add_plane(ScatterLane<D, S, EXACT>& T, long long node, const V* v) {
     if constexpr (D == 3) {
         // the two groups' sums, one channel pair left to each; then neighbouring
         // columns (b, b ^ 1) swap so that a lane holds one channel of both: each
@@ -333,32 +352,32 @@ __device__ __forceinline__ void add_plane(ScatterLane<D, S>& T, long long node, 
         keep.x += got.x;
         keep.y += got.y;
         const float other = __shfl_xor_sync(0xffffffffu, T.b & 1 ? keep.x : keep.y, 1);
-        if (T.on) add_sums<D, S>(T, node, T.b & 1 ? make_float2(other, keep.y) : make_float2(keep.x, other));
+        if (T.on) add_sums(T, node, T.b & 1 ? make_float2(other, keep.y) : make_float2(keep.x, other));
     } else {
         // the four groups' sums of one node
-        float2 u = v[0];
-        float2 got = shfl_xor2(u, 16);
+        V u = v[0];
+        V got = shfl_xor2(u, 16);
         u.x += got.x;
         u.y += got.y;
         got = shfl_xor2(u, 8);
         u.x += got.x;
         u.y += got.y;
-        if (T.on && T.g == 0) add_sums<D, S>(T, node, u);
+        if (T.on && T.g == 0) add_sums(T, node, u);
     }
 }
 
 // A stencil that starts `ahead` (1 .. S) nodes further in x: the planes before
 // it go to the grid, the others move up.
-template <int D, int S>
-__device__ __forceinline__ void move_planes(ScatterLane<D, S>& T, long long node, int ahead) {
+template <int D, int S, bool EXACT>
+__device__ __forceinline__ void move_planes(ScatterLane<D, S, EXACT>& T, long long node, int ahead) {
 #pragma unroll 1
     for (int n = 0; n < ahead; ++n) {
-        add_plane<D, S>(T, node + n, T.a[0]);
+        add_plane(T, node + n, T.a[0]);
 #pragma unroll
         for (int p = 0; p < Scatter<D, S>::PAIRS; ++p) {
 #pragma unroll
             for (int a = 0; a + 1 < S; ++a) T.a[a][p] = T.a[a + 1][p];
-            T.a[S - 1][p] = make_float2(0.f, 0.f);
+            T.a[S - 1][p] = {};
         }
     }
 }
@@ -367,32 +386,33 @@ __device__ __forceinline__ void move_planes(ScatterLane<D, S>& T, long long node
 // planes and are left with one each. (3D adds them with move_planes: unrolled
 // they cost more in instruction fetch than the register moves they save, 320
 // -> 332 us on the 128^3 snowball scene.)
-template <int D, int S>
-__device__ __forceinline__ void add_planes(ScatterLane<D, S>& T, long long node) {
+template <int D, int S, bool EXACT>
+__device__ __forceinline__ void add_planes(ScatterLane<D, S, EXACT>& T, long long node) {
     if constexpr (D == 2) {
-        float2 v[4], k[2];
+        using V = std::remove_reference_t<decltype(T.a[0][0])>;
+        V v[4] = {}, k[2];
 #pragma unroll
-        for (int a = 0; a < 4; ++a) v[a] = a < S ? T.a[a][0] : make_float2(0.f, 0.f);
+        for (int a = 0; a < S; ++a) v[a] = T.a[a][0];
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
             k[i] = T.g & 2 ? v[2 + i] : v[i];
-            const float2 got = shfl_xor2(T.g & 2 ? v[i] : v[2 + i], 16);
+            const V got = shfl_xor2(T.g & 2 ? v[i] : v[2 + i], 16);
             k[i].x += got.x;
             k[i].y += got.y;
         }
-        float2 u = T.g & 1 ? k[1] : k[0];
-        const float2 got = shfl_xor2(T.g & 1 ? k[0] : k[1], 8);
+        V u = T.g & 1 ? k[1] : k[0];
+        const V got = shfl_xor2(T.g & 1 ? k[0] : k[1], 8);
         u.x += got.x;
         u.y += got.y;
-        if (T.on && T.g < S) add_sums<D, S>(T, node + T.g, u);
+        if (T.on && T.g < S) add_sums(T, node + T.g, u);
 #pragma unroll
-        for (int a = 0; a < S; ++a) T.a[a][0] = make_float2(0.f, 0.f);
+        for (int a = 0; a < S; ++a) T.a[a][0] = {};
     }
 }
 
 // Adds one particle's plane values  wx_a (P + (a - 1) Q)  of a channel pair.
 template <int D, int S>
-__device__ __forceinline__ void sum_pair(ScatterLane<D, S>& T, int p, const float2* x, float2 P, float2 Q) {
+__device__ __forceinline__ void sum_pair(ScatterLane<D, S, false>& T, int p, const float2* x, float2 P, float2 Q) {
     T.a[0][p] = __ffma2_rn(x[0], __fadd2_rn(P, make_float2(-Q.x, -Q.y)), T.a[0][p]);
     T.a[1][p] = __ffma2_rn(x[1], P, T.a[1][p]);
     P = __fadd2_rn(P, Q);
@@ -400,9 +420,25 @@ __device__ __forceinline__ void sum_pair(ScatterLane<D, S>& T, int p, const floa
     if constexpr (S == 4) T.a[3][p] = __ffma2_rn(x[3], __fadd2_rn(P, Q), T.a[3][p]);
 }
 
-// The particle rows [0, count) at q, all of one stencil, into the planes.
 template <int D, int S>
-__device__ __forceinline__ void sum_rows(ScatterLane<D, S>& T, const float* q, int count) {
+__device__ __forceinline__ void sum_pair(ScatterLane<D, S, true>& T, int p, const float2* x, float2 P, float2 Q) {
+    const float2 scale = make_float2(T.scale0, T.scale1);
+    P = __fmul2_rn(P, scale);  // powers of two: exact
+    Q = __fmul2_rn(Q, scale);
+    P = __fadd2_rn(P, make_float2(-Q.x, -Q.y));
+#pragma unroll
+    for (int a = 0; a < S; ++a) {
+        const float2 t = __fmul2_rn(x[a], P);
+        T.top = fmaxf(T.top, fmaxf(fabsf(t.x), fabsf(t.y)));
+        T.a[a][p].x += __float2ll_rn(t.x);
+        T.a[a][p].y += __float2ll_rn(t.y);
+        P = __fadd2_rn(P, Q);
+    }
+}
+
+// The particle rows [0, count) at q, all of one stencil, into the planes.
+template <int D, int S, bool EXACT>
+__device__ __forceinline__ void sum_rows(ScatterLane<D, S, EXACT>& T, const float* q, int count) {
     using L = Scatter<D, S>;
     constexpr int G = L::G;
     q += T.g * L::PS;
@@ -416,11 +452,11 @@ __device__ __forceinline__ void sum_rows(ScatterLane<D, S>& T, const float* q, i
             const float yz_ = wy.x * wz.x, ydz_ = wy.y * wz.x, yzd_ = wy.x * wz.y;
             const float2 yz = make_float2(yz_, yz_), ydz = make_float2(ydz_, ydz_), yzd = make_float2(yzd_, yzd_);
             const float4 s = q4[L::M / 4], a0 = q4[L::M / 4 + 1], a1 = q4[L::M / 4 + 2], a2 = q4[L::M / 4 + 3];
-            sum_pair<D, S>(T, 0, x,
+            sum_pair(T, 0, x,
                            __ffma2_rn(yzd, make_float2(a2.x, a2.y),
                                       __ffma2_rn(ydz, make_float2(a1.x, a1.y), __fmul2_rn(yz, make_float2(s.x, s.y)))),
                            __fmul2_rn(yz, make_float2(a0.x, a0.y)));
-            sum_pair<D, S>(T, 1, x,
+            sum_pair(T, 1, x,
                            __ffma2_rn(yzd, make_float2(a2.z, a2.w),
                                       __ffma2_rn(ydz, make_float2(a1.z, a1.w), __fmul2_rn(yz, make_float2(s.z, s.w)))),
                            __fmul2_rn(yz, make_float2(a0.z, a0.w)));
@@ -428,7 +464,7 @@ __device__ __forceinline__ void sum_rows(ScatterLane<D, S>& T, const float* q, i
             const float4 sa = q4[L::M / 4 + T.h];
             const float2 a1 = *reinterpret_cast<const float2*>(q + L::M + 8 + 2 * T.h);
             const float2 y = make_float2(wy.x, wy.x), yd = make_float2(wy.y, wy.y);
-            sum_pair<D, S>(T, 0, x, __ffma2_rn(yd, a1, __fmul2_rn(y, make_float2(sa.x, sa.y))),
+            sum_pair(T, 0, x, __ffma2_rn(yd, a1, __fmul2_rn(y, make_float2(sa.x, sa.y))),
                                __fmul2_rn(y, make_float2(sa.z, sa.w)));
         }
     }
@@ -469,12 +505,12 @@ __device__ __forceinline__ void scatter_clipped(const StepConsts& C, const TileI
 }
 
 // The ordered rows of a window (`total` of them) into the grid. Whole warp.
-template <int D, int S>
+template <int D, int S, bool EXACT = false>
 __device__ __forceinline__ void scatter_rows(const StepConsts& C, const float* pay, int total,
                                              unsigned long long* __restrict__ acc, unsigned* __restrict__ status) {
     using L = Scatter<D, S>;
     const int lane = threadIdx.x & 31;
-    ScatterLane<D, S> T;
+    ScatterLane<D, S, EXACT> T;
     int col = 0, ch = 0;  // of the lane's first add
     T.b = lane & 3;
     if constexpr (D == 3) {
@@ -505,7 +541,7 @@ __device__ __forceinline__ void scatter_rows(const StepConsts& C, const float* p
 #pragma unroll
     for (int a = 0; a < S; ++a)
 #pragma unroll
-        for (int p = 0; p < L::PAIRS; ++p) T.a[a][p] = make_float2(0.f, 0.f);
+        for (int p = 0; p < L::PAIRS; ++p) T.a[a][p] = {};
     int at = kNoKey;  // first node of the planes
     for (int j = 0; j <= total;) {
         const int2 info = j < total ? *reinterpret_cast<const int2*>(pay + j * L::PS + L::INFO) : make_int2(kNoKey, 1);
@@ -513,14 +549,14 @@ __device__ __forceinline__ void scatter_rows(const StepConsts& C, const float* p
         const int ahead = info.x - at;
         if (at != kNoKey) {
             if constexpr (D == 3) {
-                move_planes<D, S>(T, at, ahead > 0 ? min(ahead, S) : S);
+                move_planes(T, at, ahead > 0 ? min(ahead, S) : S);
             } else {
-                if (ahead > 0 && ahead < S) move_planes<D, S>(T, at, ahead);
-                else add_planes<D, S>(T, at);
+                if (ahead > 0 && ahead < S) move_planes(T, at, ahead);
+                else add_planes(T, at);
             }
         }
         at = info.x;
-        if (j < total) sum_rows<D, S>(T, pay + j * L::PS, info.y);
+        if (j < total) sum_rows(T, pay + j * L::PS, info.y);
         j += info.y;
     }
     if (!(T.top < kFixedLimit)) raise_flag(status, 2u);
@@ -554,52 +590,58 @@ __device__ __forceinline__ unsigned stencil_block_bits(const int* base, const in
     return bits;
 }
 
-// P2G of the queued particles after their return map, by the windows the
-// fused kernel recorded: one warp per window, the window's queued slots
-// (x, v, A as the G2P and return-map kernels left them) scattered as in the
-// fused kernel. The order inside a window is a function of its queued
-// particles, so the int64 sums do not depend on the order in which windows were
-// recorded. The fused kernel has marked the node blocks of every queued particle
-// whose new position it knew; the others (rec.z) are marked here.
+// P2G of the queued particles of one recorded window (rec: first slot, mask of the
+// queued lanes, mask of those whose node blocks are not marked yet) after their
+// return map, by one warp: x, v, A as the G2P and return-map kernels left them,
+// scattered as in the fused kernel. The order inside a window is a function of its
+// queued particles, so the int64 sums do not depend on the order in which windows
+// were recorded. The fused kernel has marked the node blocks of every queued
+// particle whose new position it knew; the others are marked here.
+template <int D, int S, bool EXACT>
+__device__ __forceinline__ void queued_window(const Particles& P, const StepConsts& C, const TileInfo& TI, int4 rec,
+                                              unsigned long long* __restrict__ acc, unsigned* __restrict__ status,
+                                              float* pay) {
+    using L = Scatter<D, S>;
+    const int lane = threadIdx.x & 31;
+    const long long n = P.n;
+    const bool queued = ((unsigned)rec.y >> lane) & 1u;
+    int key = kNoKey, base[3] = {0, 0, 0};
+    float mass = 0.f, x[D], v[D], A[D * D];
+    if (queued) {
+        const int i = rec.x + lane;
+        mass = P.mass ? P.mass[i] : P.mass_u;
+#pragma unroll
+        for (int k = 0; k < D; ++k) { x[k] = P.x[k * n + i]; v[k] = P.v[k * n + i]; }
+#pragma unroll
+        for (int k = 0; k < D * D; ++k) A[k] = P.A[k * n + i];
+        key = stencil_key<D, S>(C, x, base);
+        if (key == kClipped) {
+            scatter_clipped<D, S>(C, TI, x, base, v, A, mass, acc, status);
+            key = kNoKey;
+        } else if (((unsigned)rec.z >> lane) & 1u) {
+            mark_stencil<D, S>(TI, base);
+        }
+    }
+    int count, total;
+    bool first;
+    const int row = window_row(key, &count, &first, &total);
+    if (key != kNoKey) write_payload<D, S>(C, x, base, v, A, mass, key, count, first, pay + row * L::PS);
+    __syncwarp();
+    scatter_rows<D, S, EXACT>(C, pay, total, acc, status);
+}
+
 template <int D, int S>
 __global__ void __launch_bounds__(FusedGeom<D>::THREADS) k_p2g_windows(Particles P, StepConsts C, TileInfo TI,
                                                                       SlowQueue Q,
                                                                       unsigned long long* __restrict__ acc,
                                                                       unsigned* __restrict__ status) {
     using G = FusedGeom<D>;
-    using L = Scatter<D, S>;
     extern __shared__ __align__(128) unsigned char fused_smem[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    float* pay = reinterpret_cast<float*>(fused_smem) + wid * (G::WIN * L::PS);
+    const int wid = threadIdx.x >> 5;
+    float* pay = reinterpret_cast<float*>(fused_smem) + wid * (G::WIN * G::PS);
     const int nw = min(*Q.nwin, Q.win_capacity);
-    const int n = P.n;
-    for (int r = blockIdx.x * G::WARPS + wid; r < nw; r += gridDim.x * G::WARPS) {
-        const int4 rec = Q.win[r];
-        const bool queued = ((unsigned)rec.y >> lane) & 1u;
-        int key = kNoKey, base[3] = {0, 0, 0};
-        float mass = 0.f, x[D], v[D], A[D * D];
-        if (queued) {
-            const int i = rec.x + lane;
-            mass = P.mass ? P.mass[i] : P.mass_u;
-#pragma unroll
-            for (int k = 0; k < D; ++k) { x[k] = P.x[k * n + i]; v[k] = P.v[k * n + i]; }
-#pragma unroll
-            for (int k = 0; k < D * D; ++k) A[k] = P.A[k * n + i];
-            key = stencil_key<D, S>(C, x, base);
-            if (key == kClipped) {
-                scatter_clipped<D, S>(C, TI, x, base, v, A, mass, acc, status);
-                key = kNoKey;
-            } else if (((unsigned)rec.z >> lane) & 1u) {
-                mark_stencil<D, S>(TI, base);
-            }
-        }
-        int count, total;
-        bool first;
-        const int row = window_row(key, &count, &first, &total);
-        if (key != kNoKey) write_payload<D, S>(C, x, base, v, A, mass, key, count, first, pay + row * L::PS);
-        __syncwarp();
-        scatter_rows<D, S>(C, pay, total, acc, status);
-    }
+    for (int r = blockIdx.x * G::WARPS + wid; r < nw; r += gridDim.x * G::WARPS)
+        queued_window<D, S, false>(P, C, TI, Q.win[r], acc, status, pay);
 }
 
 // ---------------------------------------------------------------------------
@@ -677,7 +719,7 @@ __device__ __forceinline__ void tile_origin(const TileInfo& TI, int t, int* tc, 
 // state (G2P = false), then the scatter of the in-band particles' payloads.
 // Returns this lane's node-block bits around the tile (box origin bo). DIRECT:
 // there is no staged box, every particle gathers from the global grid.
-template <int D, int S, bool G2P, bool DIRECT = false>
+template <int D, int S, bool G2P, bool DIRECT = false, bool EXACT = false>
 __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepConsts& C, const TileInfo& TI,
                                                  const float4* __restrict__ gv, unsigned long long* __restrict__ acc,
                                                  const SlowQueue& Q, unsigned* __restrict__ status, const float4* box,
@@ -686,7 +728,7 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
     using L = Scatter<D, S>;
     using St = Stencil<S>;
     const int lane = threadIdx.x & 31;
-    const int n = P.n;
+    const long long n = P.n;
     const long long gsy = C.nx, gsz = (long long)C.nx * C.ny;
     const int cnt = min(win, m - w * win);
     const bool valid = lane < cnt;
@@ -758,20 +800,26 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
                         for (int k = 0; k < D; ++k) s += (C.dt * St::DINV * nB[r * D + k]) * Fe[k * D + c];
                         Fh[r * D + c] = s;
                     }
-                float sig[D * D];
                 const float Jp = P.Jp[i];
-                if (det<D>(Fh) > 0.f && band_gershgorin<D>(Fh, 1.f - C.theta_c, 1.f + C.theta_s) &&
-                    hardened_stress_series<D>(Fh, Jp, C.mu0, C.la0, C.xi, sig)) {
+                bool band = det<D>(Fh) > 0.f && band_gershgorin<D>(Fh, 1.f - C.theta_c, 1.f + C.theta_s);
+                if constexpr (D == 2) {
+                    band = band && affine2<S>(C, Fh, Jp, nB, mass, vol, A);
+                } else {
+                    float sig[D * D];
+                    band = band && hardened_stress_series<D>(Fh, Jp, C.mu0, C.la0, C.xi, sig);
+                    if (band)
 #pragma unroll
-                    for (int k = 0; k < D * D; ++k) {
-                        P.Fe[k * n + i] = Fh[k];
-                        A[k] = St::DINV * mass * nB[k] - St::DINV * C.dt * vol * sig[k];
-                    }
+                        for (int k = 0; k < D * D; ++k)
+                            A[k] = St::DINV * mass * nB[k] - St::DINV * C.dt * vol * sig[k];
+                }
+                if (band) {
+#pragma unroll
+                    for (int k = 0; k < D * D; ++k) P.Fe[k * n + i] = Fh[k];
                 } else {
                     const int slot = queue_slot(Q);
                     Q.list[slot] = i;
 #pragma unroll
-                    for (int k = 0; k < D * D; ++k) Q.fh[k * Q.capacity + slot] = Fh[k];
+                    for (int k = 0; k < D * D; ++k) Q.fh[(long long)k * Q.capacity + slot] = Fh[k];
                     deferred = scatter;
                     scatter = false;
                 }
@@ -808,7 +856,7 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
             const unsigned um = __ballot_sync(0xffffffffu, unmarked);
             if (lane == 0) {
                 const int r = atomicAdd(Q.nwin, 1);
-                if (r < Q.win_capacity) Q.win[r] = make_int4(start + w * win, (int)dm, (int)um, 0);
+                if (r < Q.win_capacity) Q.win[r] = make_int4(start + w * win, (int)dm, (int)um, Q.scene);
             }
         }
     }
@@ -817,7 +865,7 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
     const int row = window_row(key, &count, &first, &total);
     if (key != kNoKey) write_payload<D, S>(C, x, nbase, v, A, mass, key, count, first, pay + row * L::PS);
     __syncwarp();
-    scatter_rows<D, S>(C, pay, total, acc, status);
+    scatter_rows<D, S, EXACT>(C, pay, total, acc, status);
     return bits;
 }
 

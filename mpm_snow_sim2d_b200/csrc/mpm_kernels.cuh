@@ -602,10 +602,42 @@ __global__ void __launch_bounds__(256) k_g2p_simple(Particles P, StepConsts C, c
 // step (and by k_prepare_affine after any state upload), always with this one
 // function, so the value depends on (B, F_E, J_p, m, V) alone. On the
 // quadratic stencil (S = 3) the factor is D^-1 = 4 instead of 3.
+// In 2D the stress of a particle with det F > 0 is the closed form of
+// hardened_stress_series<2>, here with every rounding spelled out, so that each
+// kernel that forms A gives the same bits whatever it is inlined into (a batched
+// scene continues unchanged when its state is read and uploaded again).
+template <int S>
+__device__ __forceinline__ bool affine2(const StepConsts& C, const float* F, float Jp, const float* B, float mass,
+                                        float vol, float* A) {
+    const float je = __fmaf_rn(F[0], F[3], -__fmul_rn(F[1], F[2]));
+    if (!(je > 0.f)) return false;
+    const float c = __fadd_rn(F[0], F[3]), s = __fsub_rn(F[2], F[1]);
+    const float inv = rsqrtf(__fmaf_rn(c, c, __fmul_rn(s, s)));
+    const float r0 = __fmul_rn(c, inv), r1 = __fmul_rn(s, inv);  // R = [r0 -r1; r1 r0]
+    const float d[4] = {__fsub_rn(F[0], r0), __fadd_rn(F[1], r1), __fsub_rn(F[2], r1), __fsub_rn(F[3], r0)};
+    const float h = expf(__fmul_rn(C.xi, __fsub_rn(1.f, Jp)));
+    const float mu2 = __fmul_rn(__fmul_rn(2.f, C.mu0), h);
+    const float diag = __fmul_rn(__fmul_rn(__fmul_rn(C.la0, h), __fsub_rn(je, 1.f)), je);
+    constexpr float K = Stencil<S>::DINV;
+    const float km = __fmul_rn(K, mass), kv = __fmul_rn(__fmul_rn(K, C.dt), vol);
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const float t = __fmaf_rn(d[2 * i], F[2 * j], __fmul_rn(d[2 * i + 1], F[2 * j + 1]));
+            const float sig = i == j ? __fmaf_rn(mu2, t, diag) : __fmul_rn(mu2, t);
+            A[2 * i + j] = __fmaf_rn(-kv, sig, __fmul_rn(km, B[2 * i + j]));
+        }
+    return true;
+}
+
 template <int D, int S = 4>
 __device__ __forceinline__ void mls_affine(const StepConsts& C, const float* B, const float* Fe, float Jp, float mass,
                                            float vol, float* A) {
     constexpr float K = Stencil<S>::DINV;
+    if constexpr (D == 2) {
+        if (affine2<S>(C, Fe, Jp, B, mass, vol, A)) return;
+    }
     float sig[D * D];
     hardened_stress_fast<D, kMLS>(Fe, Jp, C.mu0, C.la0, C.xi, sig);
 #pragma unroll
@@ -647,6 +679,7 @@ struct SlowQueue {
     int4* win;  // .z: queued slots whose node blocks are not marked yet
     int* nwin;    // device scalar (count[1])
     int win_capacity;
+    int scene;    // batched scenes: the scene whose windows are recorded (else 0)
 };
 
 // Element a of an S-vector held in registers, for a loop index the compiler
@@ -918,13 +951,13 @@ template <int D, int S = 4>
 __device__ __forceinline__ void g2p_queued_exact(const Particles& P, const StepConsts& C, const float4* __restrict__ gv,
                                                  const SlowQueue& Q, int e, unsigned* __restrict__ status,
                                                  PairLog L = PairLog{nullptr, nullptr, 0}) {
-    const int n = P.n;
+    const long long n = P.n;
     const int entry = Q.list[e];
     const int i = entry >= 0 ? entry : -1 - entry;
     float Fh[D * D], Fe[D * D], B[D * D], A[D * D];
     if (entry >= 0) {
 #pragma unroll
-        for (int k = 0; k < D * D; ++k) { Fh[k] = Q.fh[k * Q.capacity + e]; B[k] = P.B[k * n + i]; }
+        for (int k = 0; k < D * D; ++k) { Fh[k] = Q.fh[(long long)k * Q.capacity + e]; B[k] = P.B[k * n + i]; }
     } else {
         float x[D];
 #pragma unroll

@@ -49,6 +49,10 @@ struct TileInfo {
     int4* scan;        // per block of kScanTiles tiles: particles, non-empty tiles, items
     int* grid_done;    // device scalar: CTAs of the grid update that have finished
     int* zero[2];      // fused_next, queue counts: cleared by the grid update
+    // Batched scenes: the scene of each tile (null: one scene) and, in a scene's own
+    // view, its first node block.
+    const int* tile_scene;
+    int blk0;
     unsigned long long* skey;  // global sort scratch (tiles above SortGeom<D>::SMEM particles)
     int* sval;
 };
@@ -62,20 +66,30 @@ template <int S> __device__ __forceinline__ int cell_clamped(float x, int ext) {
     return c < 0 ? 0 : (c >= ext ? ext - 1 : c);
 }
 
-template <int D, int S> __device__ __forceinline__ int tile_of_slot(const Particles& P, const StepConsts& C,
-                                                                   const TileInfo& TI, int i) {
+// The scene a slot or a tile belongs to, for the sort: one scene, or many side by
+// side (ManyScenes, mpm_batch.cuh).
+struct SceneView {
+    int ext[3], tiles[3], tile0;
+};
+
+struct OneScene {
+    SceneView v;
+    __device__ __forceinline__ const SceneView& of_slot(int) const { return v; }
+    __device__ __forceinline__ const SceneView& of_tile(int) const { return v; }
+};
+
+template <int D, int S> __device__ __forceinline__ int tile_of_slot(const Particles& P, const SceneView& V, int i) {
     constexpr int T = TileGeom<D>::T;
-    const int ext[3] = {C.W, C.H, C.Dp};
     int t = 0;
 #pragma unroll
-    for (int k = D - 1; k >= 0; --k) t = t * TI.tiles[k] + cell_clamped<S>(P.x[k * P.n + i], ext[k]) / T;
-    return t;
+    for (int k = D - 1; k >= 0; --k) t = t * V.tiles[k] + cell_clamped<S>(P.x[(long long)k * P.n + i], V.ext[k]) / T;
+    return V.tile0 + t;
 }
 
 // ---------------------------------------------------------------------------
 // Largest |v_k| over all particle velocity components (non-negative floats
 // order as their bit patterns; NaN is skipped), for the auto sort period.
-__global__ void __launch_bounds__(256) k_max_abs(const float* __restrict__ v, long long count,
+static __global__ void __launch_bounds__(256) k_max_abs(const float* __restrict__ v, long long count,
                                                  unsigned* __restrict__ out) {
     float m = 0.f;
     for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (long long)gridDim.x * blockDim.x)
@@ -88,11 +102,11 @@ __global__ void __launch_bounds__(256) k_max_abs(const float* __restrict__ v, lo
 // ---------------------------------------------------------------------------
 // Counting sort by tile.
 
-template <int D, int S = 4>
-__global__ void __launch_bounds__(256) k_sort_count(Particles P, StepConsts C, TileInfo TI) {
+template <int D, int S, typename SC>
+__global__ void __launch_bounds__(256) k_sort_count(Particles P, SC scenes, TileInfo TI) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
-    const int t = tile_of_slot<D, S>(P, C, TI, i);
+    const int t = tile_of_slot<D, S>(P, scenes.of_slot(i), i);
     TI.key[i] = t;
     const unsigned act = __activemask();
     const unsigned peers = __match_any_sync(act, t);
@@ -145,7 +159,7 @@ __device__ __forceinline__ void block_scan3(int* v, int* total) {
     }
 }
 
-__global__ void __launch_bounds__(kScanTiles) k_sort_block_sums(TileInfo TI) {
+static __global__ void __launch_bounds__(kScanTiles) k_sort_block_sums(TileInfo TI) {
     const int t = blockIdx.x * kScanTiles + threadIdx.x;
     const int c = t < TI.n_tiles ? TI.tile_count[t] : 0;
     int v[3] = {c, c > 0, tile_items(TI, c)}, total[3];
@@ -153,7 +167,7 @@ __global__ void __launch_bounds__(kScanTiles) k_sort_block_sums(TileInfo TI) {
     if (threadIdx.x == 0) TI.scan[blockIdx.x] = make_int4(total[0], total[1], total[2], 0);
 }
 
-__global__ void __launch_bounds__(kScanTiles) k_sort_scan(TileInfo TI) {
+static __global__ void __launch_bounds__(kScanTiles) k_sort_scan(TileInfo TI) {
     __shared__ int s_before[3];
     const int t = blockIdx.x * kScanTiles + threadIdx.x;
     if (threadIdx.x < 3) s_before[threadIdx.x] = 0;
@@ -180,7 +194,7 @@ __global__ void __launch_bounds__(kScanTiles) k_sort_scan(TileInfo TI) {
         if (c > 0) TI.tile_list[s_before[1] + v[1] - 1] = t;  // non-empty tiles in tile order
         const int step = TI.item_win ? TI.win * TI.item_win : c;
         for (int k = 0; k < ni; ++k)
-            TI.items[s_before[2] + v[2] - ni + k] = make_int4(t, start + k * step, min(step, c - k * step), 0);
+            TI.items[s_before[2] + v[2] - ni + k] = make_int4(t, start + k * step, min(step, c - k * step), TI.tile_scene ? TI.tile_scene[t] : 0);
     }
     if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
         *TI.n_tile_list = s_before[1] + total[1];
@@ -194,7 +208,7 @@ struct SortBuffers {
 };
 
 // Bucket the source slots by tile (order inside a tile is fixed by k_tile_sort).
-__global__ void __launch_bounds__(256) k_sort_bucket(int n, TileInfo TI) {
+static __global__ void __launch_bounds__(256) k_sort_bucket(int n, TileInfo TI) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const int t = TI.key[i];
@@ -248,9 +262,9 @@ constexpr int kCellSortMax = 64;  // counting sort when no cell of the tile hold
 // ids of its cell, all threads at once);
 // larger tiles a bitonic network (in shared memory up to SMEM, else in
 // global scratch). The result is the same order either way.
-template <int D, int S = 4>
+template <int D, int S, typename SC>
 __global__ void __launch_bounds__(256) k_tile_sort(Particles P, const int* __restrict__ id_src, SortBuffers dst,
-                                                   StepConsts C, TileInfo TI) {
+                                                   SC scenes, TileInfo TI) {
     static_assert(TileGeom<D>::BN == kTileCells, "a tile has 64 cells");
     constexpr int T = TileGeom<D>::T;
     constexpr int kSortSmem = SortGeom<D>::SMEM, kCountSortMax = kSortSmem / 2;
@@ -258,10 +272,12 @@ __global__ void __launch_bounds__(256) k_tile_sort(Particles P, const int* __res
     __shared__ int s_val[kSortSmem];
     __shared__ int s_cnt[kTileCells], s_off[kTileCells];
     __shared__ int s_big;
-    const int n = P.n, ext[3] = {C.W, C.H, C.Dp};
+    const long long n = P.n;
     const int ntl = *TI.n_tile_list;
     for (int e = blockIdx.x; e < ntl; e += gridDim.x) {
         const int t = TI.tile_list[e];
+        const SceneView& V = scenes.of_tile(t);
+        const int ext[3] = {V.ext[0], V.ext[1], V.ext[2]};
         const int start = TI.tile_start[t];
         const int m = TI.tile_count[t];
         const bool in_smem = m <= kSortSmem;
@@ -352,7 +368,29 @@ __global__ void __launch_bounds__(256) k_tile_sort(Particles P, const int* __res
 // Node-block marking (which blocks of T^D nodes received mass this step).
 
 __device__ __forceinline__ void mark_block(const TileInfo& TI, int b) {
+    b += TI.blk0;
     if (atomicExch(&TI.mark[b], 1) == 0) TI.mark_list[atomicAdd(TI.n_marked, 1)] = b;
+}
+
+// The end of a grid update, every CTA: counters for what follows, instead of a
+// memset node for each. Those of the fused transfer and the queue are cleared at
+// once (nothing else uses them while the kernel runs), the number of marked blocks
+// when every CTA has read it; `step` (if any) counts the update.
+__device__ __forceinline__ void grid_finish(const TileInfo& TI, int* step) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (blockIdx.x == 0) {
+            *TI.zero[0] = 0;
+            TI.zero[1][0] = 0;
+            TI.zero[1][1] = 0;
+        }
+        __threadfence();
+        if (atomicAdd(TI.grid_done, 1) == (int)gridDim.x - 1) {
+            *TI.n_marked = 0;
+            *TI.grid_done = 0;
+            if (step) ++*step;
+        }
+    }
 }
 
 // ---------------------------------------------------------------------------
@@ -376,22 +414,7 @@ __global__ void __launch_bounds__(256) k_grid_marked(StepConsts C, TileInfo TI, 
         if (gx >= C.nx || gy >= C.ny || gz >= C.nz) continue;
         grid_node_at<D, FORM>(C, acc, gv, status, ((long long)gz * C.ny + gy) * C.nx + gx, gx, gy, gz);
     }
-    // Counters for what follows, instead of a memset node for each: those of the
-    // fused transfer and the queue now (nothing else uses them while this kernel
-    // runs), the number of marked blocks when every CTA has read it.
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        if (blockIdx.x == 0) {
-            *TI.zero[0] = 0;
-            TI.zero[1][0] = 0;
-            TI.zero[1][1] = 0;
-        }
-        __threadfence();
-        if (atomicAdd(TI.grid_done, 1) == (int)gridDim.x - 1) {
-            *TI.n_marked = 0;
-            *TI.grid_done = 0;
-        }
-    }
+    grid_finish(TI, nullptr);
 }
 
 // Where channel c (mass, then momentum) of a node sits in its four sums:
@@ -516,17 +539,19 @@ template <int D, int S = 4> struct P2GWarpSmem {
 };
 
 __device__ __forceinline__ void mark_block_once(const TileInfo& TI, int b) {
-    if (TI.mark[b] == 0) mark_block(TI, b);
+    if (TI.mark[b + TI.blk0] == 0) mark_block(TI, b);
 }
 
-// int64 fixed-point add of a scaled sum; the range is checked by the caller.
-__device__ __forceinline__ void red_scaled(unsigned long long* p, float t) {
+__device__ __forceinline__ void red_int(unsigned long long* p, long long v) {
     // an explicit global reduction (no return value): p always points into the
     // grid sums, and spelling it out keeps the compiler from falling back to a
     // generic atomic with a return where it cannot prove the address space
     const unsigned long long g = (unsigned long long)__cvta_generic_to_global(p);
-    asm volatile("red.global.add.u64 [%0], %1;" ::"l"(g), "l"((unsigned long long)__float2ll_rn(t)));
+    asm volatile("red.global.add.u64 [%0], %1;" ::"l"(g), "l"((unsigned long long)v));
 }
+
+// int64 fixed-point add of a scaled sum; the range is checked by the caller.
+__device__ __forceinline__ void red_scaled(unsigned long long* p, float t) { red_int(p, __float2ll_rn(t)); }
 
 __device__ __forceinline__ void red_fixed(unsigned long long* p, float v, float scale) { red_scaled(p, v * scale); }
 

@@ -162,3 +162,45 @@ def test_step_times_and_errors(gpu_lib):
     assert e.value.status == 11
     with pytest.raises(ValueError):
         Batch([scenes.impact_3d()])
+
+
+# particles of a scene: none, one, around one window of 32 slots, around 1024 slots
+@pytest.mark.parametrize("counts", [(1, 31, 32, 33), (0, 1023, 7, 1025), (65,)])
+def test_small_scenes_and_walls(gpu_lib, counts):
+    """Windows that are empty, short or just full, particles whose stencils reach the
+    domain's edge, neighbouring scenes that end and begin in the same node blocks'
+    list: each scene as the single-scene solver has it within the bounds of the mixed batch,
+    and bitwise itself in reversed company and under another sort period."""
+    from mpm_snow_sim2d_b200 import Solver
+    from mpm_snow_sim2d_b200.batch import Batch
+    base = _mixed_scenes(k=len(counts) + 1, steps=20)
+    scs = []
+    for k, n in enumerate(counts):
+        sc = base[k]
+        rng = np.random.default_rng(100 * k + n)
+        lo, hi = 0.5, np.array([sc.width - 0.5, sc.height - 0.5])
+        pos = lo + rng.random((n, 2)) * (hi - lo)
+        pos[: n // 4] = lo + rng.random((n // 4, 2)) * 1.5  # a corner
+        vel = rng.standard_normal((n, 2)).astype(np.float32)
+        scs.append(sc.with_(position=pos.astype(np.float32), velocity=vel, volume=np.full(n, sc.volume[0], np.float32),
+                            mass=np.full(n, sc.mass[0], np.float32)))
+
+    def run(order, period):
+        with Batch([scs[i] for i in order]) as b:
+            b.set_config(sort_period=period)
+            b.step(9)
+            b.step(11)
+            return {i: (b.get_state(j), b.status(j)) for j, i in enumerate(order)}
+
+    first = run(range(len(scs)), 16)
+    again = run(list(reversed(range(len(scs)))), 3)
+    for i, sc in enumerate(scs):
+        assert first[i][1] == again[i][1]
+        assert _equal(first[i][0], again[i][0]), f"scene {i}"
+        if sc.count == 0:
+            continue
+        with Solver.from_scene(sc) as single:
+            single.Step(20)
+            errs = state_errors(first[i][0], _as_ref(single.get_state()), 2)
+            assert first[i][1] & 3 == single.status() & 3
+        _check(errs, TARGET, f"scene {i} vs single-scene solver")

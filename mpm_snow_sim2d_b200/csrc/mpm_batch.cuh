@@ -116,7 +116,7 @@ template <bool G2P>
 __global__ void __launch_bounds__(FusedGeom<2>::THREADS, MPM_FUSED_MIN_BLOCKS)
     k_batch_step(Particles P, BatchArrays B, TileInfo TI, SlowQueue Q) {
     using G = FusedGeom<2>;
-    __shared__ float4 pay_s[G::WARPS][G::WIN * G::PS / 4];
+    __shared__ float4 pay_s[G::WARPS][G::PAY / 4];
     __shared__ BatchScene scene_s[G::WARPS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float* pay = reinterpret_cast<float*>(pay_s[wid]);
@@ -132,7 +132,7 @@ __global__ void __launch_bounds__(FusedGeom<2>::THREADS, MPM_FUSED_MIN_BLOCKS)
         tile_origin<2>(V, item.x - S.view.tile0, tc, bo);
         const unsigned bits = __reduce_or_sync(
             0xffffffffu, fused_window<2, 4, G2P, true, true>(P, S.C, V, B.gv + S.node0, B.acc + S.node0 * 4, QS,
-                                                             B.status + item.w, nullptr, bo, item.y, item.z, TI.win, 0, pay));
+                                                             B.status + item.w, nullptr, nullptr, bo, item.y, item.z, TI.win, 0, pay));
         if (lane < 9 && (bits >> lane) & 1u)
             mark_block_once(V, (tc[1] - 1 + lane / 3) * V.nblk[0] + tc[0] - 1 + lane % 3);
     }
@@ -150,7 +150,7 @@ __global__ void __launch_bounds__(256) k_batch_plastic(Particles P, BatchArrays 
 // P2G of the queued particles (k_p2g_windows).
 __global__ void __launch_bounds__(FusedGeom<2>::THREADS) k_batch_windows(Particles P, BatchArrays B, TileInfo TI, SlowQueue Q) {
     using G = FusedGeom<2>;
-    __shared__ float4 pay_s[G::WARPS][G::WIN * G::PS / 4];
+    __shared__ float4 pay_s[G::WARPS][G::PAY / 4];
     __shared__ BatchScene scene_s[G::WARPS];
     const int wid = threadIdx.x >> 5;
     const int nw = min(*Q.nwin, Q.win_capacity);

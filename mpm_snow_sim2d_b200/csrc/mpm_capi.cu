@@ -117,10 +117,9 @@ struct mpm_solver {
     // P2G-only prologue).
     bool fused = false;
     bool acc_pending = false;
-    int fused_grid = 0, windows_grid = 0, direct_grid = 0;
+    int windows_grid = 0, direct_grid = 0;
     bool direct = false;  // few windows: a warp per window, no staged boxes (k_g2p2g_direct)
-    bool box_tma = false;  // fused step as the TMA box pipeline (MPM_BOX_LOAD=tma) instead of staged boxes
-    CUtensorMap gv_map{};  // the node velocities (vf, wall flag) as a [nz][ny][nx][4] float tensor for TMA
+    CUtensorMap gv_map{};  // the node velocities as a tensor of float rows for TMA (box_load)
 };
 
 namespace {
@@ -407,7 +406,7 @@ template <int D, int S> cudaError_t launch_p2g_tiled(mpm_solver* s) {
 
 // Dynamic shared memory of k_p2g_windows: one window of payloads per warp.
 size_t windows_smem(int dim) {
-    return dim == 3 ? sizeof(FusedSmem<3>::pay) : sizeof(FusedSmem<2>::pay);
+    return sizeof(float) * (dim == 3 ? FusedGeom<3>::WARPS * FusedGeom<3>::PAY : FusedGeom<2>::WARPS * FusedGeom<2>::PAY);
 }
 
 // The fused kernel over the tiles of the last sort: G2P (this step) + P2G (next
@@ -418,14 +417,11 @@ template <int D, int S, bool G2P> cudaError_t launch_fused(mpm_solver* s) {
         if (e != cudaSuccess) return e;
     }
     if (s->n == 0) return cudaSuccess;
-    if (G2P && s->direct)
-        k_g2p2g_direct<D, S><<<s->direct_grid, FusedGeom<D>::THREADS, sizeof(FusedSmem<D>::pay), s->stream>>>(
-            particle_view(s), s->C, s->ti, s->gv, s->acc, s->q, s->status);
-    else if (G2P && s->box_tma)
-        k_g2p2g_pipe<D, S><<<s->fused_grid, FusedGeom<D>::THREADS, sizeof(PipeSmem<D>), s->stream>>>(
+    if (G2P && !s->direct)
+        k_g2p2g_pipe<D, S><<<s->sms * PipeGeom<D>::CTAS, PipeGeom<D>::THREADS, sizeof(PipeSmem<D>), s->stream>>>(
             particle_view(s), s->C, s->ti, s->gv, s->acc, s->q, s->status, s->gv_map);
-    else if constexpr (D == 3 || !G2P)
-        k_g2p2g<D, S, G2P><<<s->fused_grid, FusedGeom<D>::THREADS, sizeof(FusedSmem<D>), s->stream>>>(
+    else
+        k_g2p2g_direct<D, S, G2P><<<s->direct_grid, FusedGeom<D>::THREADS, windows_smem(D), s->stream>>>(
             particle_view(s), s->C, s->ti, s->gv, s->acc, s->q, s->status);
     return cudaGetLastError();
 }
@@ -536,12 +532,13 @@ mpm_status make_box_map(mpm_solver* s) {
         return fail(s, MPM_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
     }
     const int D = s->dim;
-    const cuuint32_t rank = (cuuint32_t)(D + 1);
-    cuuint64_t dims[4] = {4, (cuuint64_t)s->C.nx, (cuuint64_t)s->C.ny, (cuuint64_t)s->C.nz};
-    cuuint64_t strides[3] = {16, 16ull * (cuuint64_t)s->C.nx, 16ull * (cuuint64_t)s->C.nx * (cuuint64_t)s->C.ny};
+    const cuuint32_t rank = (cuuint32_t)(D == 3 ? 5 : 3);
+    const cuuint64_t row = 16ull * (cuuint64_t)s->C.nx;
+    cuuint64_t dims[5] = {4, (cuuint64_t)s->C.nx, (cuuint64_t)s->C.ny, (cuuint64_t)s->C.nz, 2};
+    cuuint64_t strides[4] = {16, row, row * (cuuint64_t)s->C.ny, 16ull * (cuuint64_t)s->nodes};
     const cuuint32_t be = (cuuint32_t)(D == 3 ? FusedGeom<3>::BE : FusedGeom<2>::BE);
-    cuuint32_t box[4] = {4, be, be, be};
-    cuuint32_t estr[4] = {1, 1, 1, 1};
+    cuuint32_t box[5] = {4, be, be, be, 1};
+    cuuint32_t estr[5] = {1, 1, 1, 1, 1};
     const CUresult r = reinterpret_cast<EncodeTiledFn>(fn)(
         &s->gv_map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, rank, s->gv, dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
         CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -601,28 +598,30 @@ mpm_status setup_tiled(mpm_solver* s) {
     }
     s->q.capacity = n > 0 ? n : 1;
     {
-        // MPM_TRANSFER=split selects the separate P2G / G2P kernels (for
-        // comparison), MPM_BOX_LOAD=tma node boxes by TMA tensor loads
+        // MPM_TRANSFER=split selects the separate P2G / G2P kernels (for comparison)
         const char* tr = std::getenv("MPM_TRANSFER");
         s->fused = !(tr && std::strcmp(tr, "split") == 0);
-        const char* bl = std::getenv("MPM_BOX_LOAD");
-        s->box_tma = s->fused && bl && std::strcmp(bl, "tma") == 0;
     }
     // Window length of the fused transfer by how the scene's windows compare with
     // the warps the GPU holds (5 CTAs of 4 per SM): a warp works through a window's
     // stencils one after the other, so a scene of few windows takes shorter ones.
-    // 2D scenes, the quadratic stencil and 3D scenes of at most six windows per
-    // warp go without staged node boxes, an item per window (k_g2p2g_direct, which
-    // has the figures); else an item is a tile.
+    // 3D scenes of more than three windows per warp (quadratic stencil: twelve) have
+    // their node boxes staged, an item being a tile, or 32 windows of one that holds
+    // more (k_g2p2g_pipe, which has the figures); the others and all 2D scenes take
+    // an item per window (k_g2p2g_direct).
     {
         const long long warps = (long long)s->sms * (MPM_FUSED_MIN_BLOCKS) * FusedGeom<3>::WARPS;
         const long long w32 = (n + 31) / 32;
         ti.win = w32 <= warps / 4 ? 8 : (w32 <= warps / 2 ? 16 : 32);
         const long long windows = (n + ti.win - 1) / ti.win;
-        s->direct = !s->box_tma && (D == 2 || s->stencil == 3 || windows <= 6 * warps);
+        s->direct = D == 2 || windows <= (s->stencil == 3 ? 12 : 3) * warps;
+        // MPM_BOX_LOAD=tma, =gather choose one of the two (for comparison)
+        const char* bl = std::getenv("MPM_BOX_LOAD");
+        if (bl && std::strcmp(bl, "tma") == 0) s->direct = false;
+        if (bl && std::strcmp(bl, "gather") == 0) s->direct = true;
         s->direct_grid = (int)std::max(1ll, std::min((long long)s->sms * (MPM_FUSED_MIN_BLOCKS), windows + ti.n_tiles));
-        ti.item_win = s->direct ? 1 : 0;
-        arena.want(&ti.items, tiles + (s->direct ? N / (size_t)ti.win : 0)).want(&ti.n_items, 1).want(&ti.grid_done, 1);
+        ti.item_win = s->direct ? 1 : 32;
+        arena.want(&ti.items, tiles + N / (size_t)(ti.win * ti.item_win)).want(&ti.n_items, 1).want(&ti.grid_done, 1);
     }
     arena.want(&ti.scan, (tiles + kScanTiles - 1) / kScanTiles).want(&ti.tile_len, tiles).want(&ti.fused_next, 1);
     // windows of a sort: at most ceil(m / win) per tile of m slots
@@ -636,40 +635,20 @@ mpm_status setup_tiled(mpm_solver* s) {
     ti.zero[0] = ti.fused_next;
     ti.zero[1] = s->q.count;
     if (s->fused) {
-        const void* kfn;
-        size_t fsm, psm;
-        const void* kpro;
-        if (D == 3) {
-            if (s->box_tma)
-                kfn = s->stencil == 3 ? (const void*)k_g2p2g_pipe<3, 3> : (const void*)k_g2p2g_pipe<3, 4>;
-            else
-                kfn = s->stencil == 3 ? (const void*)k_g2p2g<3, 3, true> : (const void*)k_g2p2g<3, 4, true>;
-            kpro = s->stencil == 3 ? (const void*)k_g2p2g<3, 3, false> : (const void*)k_g2p2g<3, 4, false>;
-            fsm = s->box_tma ? sizeof(PipeSmem<3>) : sizeof(FusedSmem<3>);
-            psm = sizeof(FusedSmem<3>);
-        } else {
-            if (s->box_tma)
-                kfn = s->stencil == 3 ? (const void*)k_g2p2g_pipe<2, 3> : (const void*)k_g2p2g_pipe<2, 4>;
-            else
-                kfn = s->stencil == 3 ? (const void*)k_g2p2g<2, 3, false> : (const void*)k_g2p2g<2, 4, false>;
-            kpro = s->stencil == 3 ? (const void*)k_g2p2g<2, 3, false> : (const void*)k_g2p2g<2, 4, false>;
-            fsm = s->box_tma ? sizeof(PipeSmem<2>) : sizeof(FusedSmem<2>);
-            psm = sizeof(FusedSmem<2>);
-        }
         int per = 0;
-        cudaError_t ef = cudaFuncSetAttribute(kfn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsm);
-        if (ef == cudaSuccess) ef = cudaFuncSetAttribute(kpro, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm);
-        if (ef == cudaSuccess)
-            ef = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kfn, FusedGeom<3>::THREADS, fsm);
-        if (ef != cudaSuccess || per < 1) return MPM_ERR_CUDA;
-        s->fused_grid = s->sms * per;
         const void* kwin = D == 3 ? (s->stencil == 3 ? (const void*)k_p2g_windows<3, 3> : (const void*)k_p2g_windows<3, 4>)
                                   : (s->stencil == 3 ? (const void*)k_p2g_windows<2, 3> : (const void*)k_p2g_windows<2, 4>);
         if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, kwin, FusedGeom<3>::THREADS, windows_smem(D)) !=
                 cudaSuccess || per < 1)
             return MPM_ERR_CUDA;
         s->windows_grid = s->sms * per;
-        if (s->box_tma) {
+        if (!s->direct) {
+            const void* kpipe =
+                D == 3 ? (s->stencil == 3 ? (const void*)k_g2p2g_pipe<3, 3> : (const void*)k_g2p2g_pipe<3, 4>)
+                       : (s->stencil == 3 ? (const void*)k_g2p2g_pipe<2, 3> : (const void*)k_g2p2g_pipe<2, 4>);
+            const size_t smem = D == 3 ? sizeof(PipeSmem<3>) : sizeof(PipeSmem<2>);
+            if (cudaFuncSetAttribute(kpipe, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess)
+                return MPM_ERR_CUDA;
             mpm_status em = make_box_map(s);
             if (em != MPM_OK) return em;
         }

@@ -2,13 +2,12 @@
 // one kernel per step (the G2P2G scheme of Wang et al., "A Massively Parallel
 // and Scalable Multi-GPU Material Point Method", ACM TOG 39(4), 2020).
 //
-// Work is handed out as items. In k_g2p2g an item is a non-empty cell tile of
-// the last sort: a CTA stages the node velocities of a fixed box of BE^D nodes
-// around the tile in shared memory (the stencils of every particle sorted into
-// the tile that has since moved less than a cell), between two CTA barriers;
-// k_g2p2g_pipe (MPM_BOX_LOAD=tma) instead runs a two-stage pipeline of TMA tensor
-// loads (cp.async.bulk.tensor, out-of-grid nodes zero-filled) with mbarriers and
-// no CTA barrier. In k_g2p2g_direct an item is one window and nothing is staged.
+// Work is handed out as items. In k_g2p2g_pipe an item is a non-empty cell tile of
+// the last sort: a CTA has the node velocities of a fixed box of BE^D nodes around
+// the tile in shared memory (the stencils of every particle sorted into the tile
+// that has since moved less than a cell), loaded one tile ahead by TMA tensor loads
+// (cp.async.bulk.tensor, out-of-grid nodes zero-filled); its warps meet at
+// mbarriers only. In k_g2p2g_direct an item is one window and nothing is staged.
 // Each warp, on its own, takes windows of up to 32 consecutive slots of a tile
 // and for its window
 //   1. per particle (one lane each): gathers the grid
@@ -55,17 +54,9 @@ template <int D> struct FusedGeom {
     static constexpr int THREADS = MPM_FUSED_THREADS;
     static constexpr int WARPS = THREADS / 32;
     static constexpr int WIN = 32;                      // slots per warp window (one per lane)
-    static constexpr int PS = 44;                       // payload floats per particle (layout: Scatter)
+    static constexpr int PS = D == 3 ? 36 : 44;         // payload floats per particle (layout: Scatter)
+    static constexpr int PAY = WIN * (PS + 2);          // floats of a warp's window: rows, then stencils
     static_assert(THREADS % 32 == 0, "whole warps");
-};
-
-template <int D> struct FusedSmem {
-    using G = FusedGeom<D>;
-    float4 box[G::BN];                                  // 3D: (vf, wall flag); 2D: (vf, vc)
-    int tile_next;                                      // item of the CTA's current tile
-    float4 pay[G::WARPS][G::WIN * G::PS / 4];           // per warp: the window's P2G payloads
-    int next_win;                                       // next window of the tile to hand out
-    unsigned bmask;                                     // node blocks (3^D around the tile) that received sums
 };
 
 // CTAs per SM the register budget is sized for: 20 warps per SM, 96
@@ -85,8 +76,8 @@ template <int D> struct FusedSmem {
 // slab rests on the floor, took 56 of 332 us for it with four loads in flight.
 template <int D, int S, bool SMEM, typename I>
 __device__ __forceinline__ void gather_nodes(const StepConsts& C, const float4* nodes, I c0, I sy, I sz,
-                                             const float4* __restrict__ gv, long long gc0, long long gsy, long long gsz,
-                                             const float (*wk)[S], const float (*off)[S], float* nv, float* nB,
+                                             const float4* __restrict__ gv, const float4* walls, long long gc0,
+                                             long long gsy, long long gsz, const float (*wk)[S], const float (*off)[S], float* nv, float* nB,
                                              float* nx) {
     float wd[3][S];
 #pragma unroll
@@ -159,7 +150,10 @@ __device__ __forceinline__ void gather_nodes(const StepConsts& C, const float4* 
                     for (int c = 0; c < S; ++c) {
                         const I cid = c0 + a + b * sy + c * sz;
                         float4 g = SMEM ? nodes[cid] : __ldg(&nodes[cid]);
-                        if (g.w != 0.f) g = __ldg(&gv[C.nodes + gc0 + a + b * gsy + c * gsz]);
+                        if (g.w != 0.f) {
+                            if (SMEM && walls) g = walls[cid];
+                            else g = __ldg(&gv[C.nodes + gc0 + a + b * gsy + c * gsz]);
+                        }
                         const float z = wk[2][c];
                         Pc[0] += z * g.x; Pc[1] += z * g.y; Pc[2] += z * g.z;
                     }
@@ -208,15 +202,15 @@ __device__ __forceinline__ void gather_nodes(const StepConsts& C, const float4* 
 //
 // Payload of one particle (floats):
 //   wx[4] | per b: wy yd | 3D, per c: wz zd | 3D: s0 s1 m s2, A00 A10 0 A20,
-//   A01 A11 0 A21, A02 A12 0 A22; 2D: s0 s1 A00 A10, m 0 0 0, A01 A11, 0 0 |
-//   its stencil: key, particles sharing it
+//   A01 A11 0 A21, A02 A12 0 A22; 2D: s0 s1 A00 A10, m 0 0 0, A01 A11, 0 0
+// and after the rows, for the first row of each stencil: key, particles sharing it;
 // with yd = wy (b - 1 - fy), zd = wz (c - 1 - fz), s_r = m v_r - fx A_r0 and
-// f = x - (base + 1). The rows are 44 floats apart: 16-byte accesses of eight
+// f = x - (base + 1). The rows are 36 (2D 44) floats apart: 16-byte accesses of eight
 // neighbouring rows then fall into distinct banks.
 template <int D, int S> struct Scatter {
-    static constexpr int PS = 44;                          // floats per row
+    static constexpr int PS = FusedGeom<D>::PS;            // floats per row
     static constexpr int Y = 4, Z = 12, M = D == 3 ? 20 : 12;
-    static constexpr int INFO = D == 3 ? 36 : 24;          // key, count
+    static constexpr int INFO = FusedGeom<D>::WIN * PS;    // the stencils: key, count of each row
     // particles at a time (lanes of one: 3D 16, its 4 x 4 node columns, of which
     // the quadratic stencil uses 3 x 3; 2D 8, four columns times two channel
     // pairs) and channel pairs per lane
@@ -262,7 +256,7 @@ __device__ __forceinline__ int window_row(int key, int* count, bool* first, int*
 
 template <int D, int S>
 __device__ __forceinline__ void write_payload(const StepConsts& C, const float* x, const int* base, const float* v,
-                                              const float* A, float mass, int key, int count, bool first, float* q) {
+                                              const float* A, float mass, int key, int count, bool first, float* pay, int row) {
     using L = Scatter<D, S>;
     float f[3], w[3][4];
 #pragma unroll
@@ -271,7 +265,7 @@ __device__ __forceinline__ void write_payload(const StepConsts& C, const float* 
         Stencil<S>::weights(x[k], base[k], w[k]);
         f[k] = x[k] - float(base[k] + 1);
     }
-    float4* q4 = reinterpret_cast<float4*>(q);
+    float4* q4 = reinterpret_cast<float4*>(pay + row * L::PS);
     q4[0] = make_float4(w[0][0], w[0][1], w[0][2], w[0][3]);
 #pragma unroll
     for (int o = 0; o < S; o += 2) {
@@ -292,7 +286,7 @@ __device__ __forceinline__ void write_payload(const StepConsts& C, const float* 
         q4[L::M / 4 + 1] = make_float4(mass, 0.f, 0.f, 0.f);
         q4[L::M / 4 + 2] = make_float4(A[1], A[3], 0.f, 0.f);
     }
-    if (first) *reinterpret_cast<int2*>(q + L::INFO) = make_int2(key, count);
+    if (first) *reinterpret_cast<int2*>(pay + L::INFO + 2 * row) = make_int2(key, count);
 }
 
 // One lane's share of a window: the S node planes of its column as channel
@@ -544,7 +538,7 @@ __device__ __forceinline__ void scatter_rows(const StepConsts& C, const float* p
         for (int p = 0; p < L::PAIRS; ++p) T.a[a][p] = {};
     int at = kNoKey;  // first node of the planes
     for (int j = 0; j <= total;) {
-        const int2 info = j < total ? *reinterpret_cast<const int2*>(pay + j * L::PS + L::INFO) : make_int2(kNoKey, 1);
+        const int2 info = j < total ? *reinterpret_cast<const int2*>(pay + L::INFO + 2 * j) : make_int2(kNoKey, 1);
         // stencils in the grid whose node ids differ by less than S are in one row
         const int ahead = info.x - at;
         if (at != kNoKey) {
@@ -625,7 +619,7 @@ __device__ __forceinline__ void queued_window(const Particles& P, const StepCons
     int count, total;
     bool first;
     const int row = window_row(key, &count, &first, &total);
-    if (key != kNoKey) write_payload<D, S>(C, x, base, v, A, mass, key, count, first, pay + row * L::PS);
+    if (key != kNoKey) write_payload<D, S>(C, x, base, v, A, mass, key, count, first, pay, row);
     __syncwarp();
     scatter_rows<D, S, EXACT>(C, pay, total, acc, status);
 }
@@ -638,7 +632,7 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS) k_p2g_windows(Particles
     using G = FusedGeom<D>;
     extern __shared__ __align__(128) unsigned char fused_smem[];
     const int wid = threadIdx.x >> 5;
-    float* pay = reinterpret_cast<float*>(fused_smem) + wid * (G::WIN * G::PS);
+    float* pay = reinterpret_cast<float*>(fused_smem) + wid * G::PAY;
     const int nw = min(*Q.nwin, Q.win_capacity);
     for (int r = blockIdx.x * G::WARPS + wid; r < nw; r += gridDim.x * G::WARPS)
         queued_window<D, S, false>(P, C, TI, Q.win[r], acc, status, pay);
@@ -685,18 +679,22 @@ __device__ __forceinline__ void mbar_arrive(unsigned long long* bar) {
     asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
-// The node box of tile t (origin node bo) into `dst`: one tensor load of the
-// node-velocity array viewed as [nz][ny][nx][4] floats (gv's first half);
-// nodes outside the grid read as zero. The mbarrier expects the box's bytes.
+__device__ __forceinline__ void mbar_expect(unsigned long long* bar, uint32_t bytes) {
+    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes) : "memory");
+}
+
+// The node box with origin node bo into `dst`: one tensor load of the node
+// velocities viewed as [2][nz][ny][nx][4] floats (3D; `half` 1: the wall velocities)
+// or [ny][nx][4]; nodes outside the grid read as zero.
 template <int D>
-__device__ __forceinline__ void box_load(const CUtensorMap& map, const int* bo, float4* dst, unsigned long long* bar) {
-    constexpr uint32_t bytes = FusedGeom<D>::BN * sizeof(float4);
+__device__ __forceinline__ void box_load(const CUtensorMap& map, const int* bo, int half, float4* dst,
+                                         unsigned long long* bar) {
     const uint32_t b = smem_u32(bar), d = smem_u32(dst);
-    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(b), "r"(bytes) : "memory");
     if constexpr (D == 3) {
         asm volatile(
-            "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], [%6];"
-            ::"r"(d), "l"(reinterpret_cast<uint64_t>(&map)), "r"(0), "r"(bo[0]), "r"(bo[1]), "r"(bo[2]), "r"(b)
+            "cp.async.bulk.tensor.5d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5, %6}], "
+            "[%7];" ::"r"(d), "l"(reinterpret_cast<uint64_t>(&map)), "r"(0), "r"(bo[0]), "r"(bo[1]), "r"(bo[2]), "r"(half),
+            "r"(b)
             : "memory");
     } else {
         asm volatile(
@@ -713,6 +711,16 @@ __device__ __forceinline__ void tile_origin(const TileInfo& TI, int t, int* tc, 
     for (int k = 0; k < D; ++k) { tc[k] = t % TI.tiles[k]; t /= TI.tiles[k]; bo[k] = tc[k] * FusedGeom<D>::T - 2; }
 }
 
+// Marks the node blocks given by the warp's bits (stencil_block_bits) around a tile.
+template <int D>
+__device__ __forceinline__ void mark_tile_blocks(const TileInfo& TI, const int* tc, unsigned bits) {
+    const int lane = threadIdx.x & 31;
+    if (lane < (D == 3 ? 27 : 9) && (bits >> lane) & 1u) {
+        const int bx = tc[0] - 1 + lane % 3, by = tc[1] - 1 + (lane / 3) % 3, bz = D == 3 ? tc[2] - 1 + lane / 9 : 0;
+        mark_block_once(TI, (bz * TI.nblk[1] + by) * TI.nblk[0] + bx);
+    }
+}
+
 // ---------------------------------------------------------------------------
 // Window w (slots start + 32 w ...) of a tile of m slots, by one warp: G2P of
 // each slot's particle against the tile's node box (G2P = true) or the stored
@@ -723,7 +731,7 @@ template <int D, int S, bool G2P, bool DIRECT = false, bool EXACT = false>
 __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepConsts& C, const TileInfo& TI,
                                                  const float4* __restrict__ gv, unsigned long long* __restrict__ acc,
                                                  const SlowQueue& Q, unsigned* __restrict__ status, const float4* box,
-                                                 const int* bo, int start, int m, int win, int w, float* pay) {
+                                                 const float4* walls, const int* bo, int start, int m, int win, int w, float* pay) {
     using G = FusedGeom<D>;
     using L = Scatter<D, S>;
     using St = Stencil<S>;
@@ -770,10 +778,10 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
                 if (!DIRECT && boxed) {
                     const int l0 = (D == 3 ? (base[2] - bo[2]) * G::BE * G::BE : 0) + (base[1] - bo[1]) * G::BE +
                                    (base[0] - bo[0]);
-                    gather_nodes<D, S, true, int>(C, box, l0, G::BE, G::BE * G::BE, gv, gc0, gsy, gsz, wk, off,
+                    gather_nodes<D, S, true, int>(C, box, l0, G::BE, G::BE * G::BE, gv, walls, gc0, gsy, gsz, wk, off,
                                                   nv, nB, nx);
                 } else {
-                    gather_nodes<D, S, false, long long>(C, gv, gc0, gsy, gsz, gv, gc0, gsy, gsz, wk, off, nv, nB,
+                    gather_nodes<D, S, false, long long>(C, gv, gc0, gsy, gsz, gv, nullptr, gc0, gsy, gsz, wk, off, nv, nB,
                                                          nx);
                 }
                 bool finite = true;
@@ -863,205 +871,172 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
     int count, total;
     bool first;
     const int row = window_row(key, &count, &first, &total);
-    if (key != kNoKey) write_payload<D, S>(C, x, nbase, v, A, mass, key, count, first, pay + row * L::PS);
+    if (key != kNoKey) write_payload<D, S>(C, x, nbase, v, A, mass, key, count, first, pay, row);
     __syncwarp();
     scatter_rows<D, S, EXACT>(C, pay, total, acc, status);
     return bits;
 }
 
 // ---------------------------------------------------------------------------
-// The fused kernel. G2P = true: one step (G2P of the state, then the next
-// step's P2G into `acc`). G2P = false: the P2G of the stored state only (after
-// creation or a state upload), reading B, F_E, J_p and forming A as every
-// other path does (mls_affine).
-template <int D, int S, bool G2P>
-__global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
-    k_g2p2g(Particles P, StepConsts C, TileInfo TI, const float4* __restrict__ gv, unsigned long long* __restrict__ acc,
-            SlowQueue Q, unsigned* __restrict__ status) {
-    using G = FusedGeom<D>;
-    extern __shared__ __align__(128) unsigned char fused_smem[];
-    FusedSmem<D>& SM = *reinterpret_cast<FusedSmem<D>*>(fused_smem);
-    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
-    const int nitems = *TI.n_items;
-    const long long gsy = C.nx, gsz = (long long)C.nx * C.ny;
-    float* pay = reinterpret_cast<float*>(SM.pay[wid]);
-    for (;;) {
-        if (tid == 0) {
-            SM.tile_next = atomicAdd(TI.fused_next, 1);
-            SM.next_win = 0;
-            SM.bmask = 0u;
-        }
-        __syncthreads();
-        const int e = SM.tile_next;
-        if (e >= nitems) break;
-        const int4 item = TI.items[e];  // tile, first slot, slots
-        const int t = item.x, start = item.y, m = item.z;
-        int tc[3] = {0, 0, 0}, bo[3] = {0, 0, 0};  // tile coordinates, box origin node
-        tile_origin<D>(TI, t, tc, bo);
-        if constexpr (G2P) {  // stage the node velocities of the box
-            for (int l = tid; l < G::BN; l += G::THREADS) {
-                const int lx = l % G::BE, ly = (l / G::BE) % G::BE, lz = D == 3 ? l / (G::BE * G::BE) : 0;
-                const int gx = bo[0] + lx, gy = bo[1] + ly, gz = D == 3 ? bo[2] + lz : 0;
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (gx >= 0 && gx <= C.W && gy >= 0 && gy <= C.H && (D == 2 || (gz >= 0 && gz <= C.Dp)))
-                    v = __ldg(&gv[gz * gsz + gy * gsy + gx]);
-                SM.box[l] = v;
-            }
-            // the tile's G2P inputs (x, F_E, J_p) towards L2 ahead of the windows
-            // that read them; one prefetch per 128-byte line, addresses kept
-            // inside the arrays
-            {
-                constexpr int NF = D + D * D + 1;
-                const int lines = (m + 31) / 32 + 1;
-                const int n = P.n;
-                for (int l = tid; l < NF * lines; l += G::THREADS) {
-                    const int f = l / lines, k = l % lines;
-                    const float* a = f < D ? P.x + (long long)f * n
-                                           : (f < D + D * D ? P.Fe + (long long)(f - D) * n : P.Jp);
-                    asm volatile("prefetch.global.L2 [%0];" ::"l"(a + min(start + 32 * k, n - 1)));
-                }
-            }
-            __syncthreads();
-        }
-        unsigned bits = 0u;  // node blocks this lane's in-box runs added to
-        const int nwin = (m + TI.win - 1) / TI.win;
-        for (;;) {
-            int w = 0;
-            if (lane == 0) w = atomicAdd(&SM.next_win, 1);
-            w = __shfl_sync(0xffffffffu, w, 0);
-            if (w >= nwin) break;
-            bits |= fused_window<D, S, G2P>(P, C, TI, gv, acc, Q, status, SM.box, bo, start, m, TI.win, w, pay);
-        }
-        // mark the node blocks the tile's in-box runs added to
-        bits = __reduce_or_sync(0xffffffffu, bits);
-        if (lane == 0 && bits) atomicOr(&SM.bmask, bits);
-        __syncthreads();
-        constexpr int NBLK = D == 3 ? 27 : 9;
-        if (tid < NBLK && (SM.bmask >> tid) & 1u) {
-            const int rx = tid % 3, ry = (tid / 3) % 3, rz = tid / 9;
-            const int bx = tc[0] - 1 + rx, by = tc[1] - 1 + ry, bz = D == 3 ? tc[2] - 1 + rz : 0;
-            mark_block_once(TI, (bz * TI.nblk[1] + by) * TI.nblk[0] + bx);
-        }
-        __syncthreads();  // SM.bmask, the tile and the box are reset for the next tile
-    }
-}
-
-// ---------------------------------------------------------------------------
 // The fused step without staged boxes: an item is one window, every warp takes
-// windows on its own and gathers from the global grid. All 2D scenes, the
-// quadratic stencil, and 3D scenes of few windows per warp. A staged box costs two CTA barriers around a
-// round trip to L2 and saves less than that where a stencil is 16 nodes of L1-
-// resident rows (2D, 627k particles: 74.6 us staged, 45.7 direct) or a tile has
-// few particles (3D, 17.6k at 0.6 per cell: 30.5 and 20.6; 474k at 8 per cell:
-// 103.8 and 98.6), and its 27 nodes make the quadratic stencil gain as well (1.65M
-// particles: 257 and 246). The 64-node stencils of a large 3D scene read a box
-// many times over (1.65M particles: 300 staged, 350 direct).
-template <int D, int S>
+// windows on its own and gathers from the global grid. All 2D scenes, and 3D scenes
+// of few windows per warp (the dispatch's rule). A staged box is worth its round trip
+// to L2 only where many windows read it and there are tiles enough for every CTA:
+//   2D, 627k particles:               44.5 us direct, 61.7 staged
+//   3D, 17.6k at 0.6 a cell:          17.5 and 23.0;   74k at 8 a cell: 25.7, 54.4
+//   3D, 187k at 8 a cell (2.0 windows a warp):  60.5 and 61.4
+//   3D, 380k (4.0): 102 and 93;       474k (5.0): 99 and 91
+//   quadratic, 673k (7.1): 104 and 112;  1.65M (17): 247 and 238
+//
+// G2P = false: the P2G of the stored state only (after creation or a state upload),
+// reading B, F_E, J_p and forming A as every other path does (mls_affine), for items
+// of any length.
+template <int D, int S, bool G2P>
 __global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
     k_g2p2g_direct(Particles P, StepConsts C, TileInfo TI, const float4* __restrict__ gv,
                    unsigned long long* __restrict__ acc, SlowQueue Q, unsigned* __restrict__ status) {
     using G = FusedGeom<D>;
-    constexpr int NBLK = D == 3 ? 27 : 9;
     extern __shared__ __align__(128) unsigned char fused_smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    float* pay = reinterpret_cast<float*>(fused_smem) + wid * (G::WIN * G::PS);
+    float* pay = reinterpret_cast<float*>(fused_smem) + wid * G::PAY;
     const int nitems = *TI.n_items;
     for (int e = wid * gridDim.x + blockIdx.x; e < nitems; e += G::WARPS * gridDim.x) {
-        const int4 item = TI.items[e];
+        const int4 item = TI.items[e];  // tile, first slot, slots
         int tc[3] = {0, 0, 0}, bo[3] = {0, 0, 0};
         tile_origin<D>(TI, item.x, tc, bo);
-        const unsigned bits = __reduce_or_sync(
-            0xffffffffu, fused_window<D, S, true, true>(P, C, TI, gv, acc, Q, status, nullptr, bo, item.y, item.z, TI.win,
-                                                        0, pay));
-        if (lane < NBLK && (bits >> lane) & 1u) {
-            const int bx = tc[0] - 1 + lane % 3, by = tc[1] - 1 + (lane / 3) % 3, bz = D == 3 ? tc[2] - 1 + lane / 9 : 0;
-            mark_block_once(TI, (bz * TI.nblk[1] + by) * TI.nblk[0] + bx);
-        }
+        const int nwin = G2P ? 1 : (item.z + TI.win - 1) / TI.win;
+        unsigned bits = 0u;
+        for (int w = 0; w < nwin; ++w)
+            bits |= fused_window<D, S, G2P, true>(P, C, TI, gv, acc, Q, status, nullptr, nullptr, bo, item.y, item.z,
+                                                  TI.win, w, pay);
+        mark_tile_blocks<D>(TI, tc, __reduce_or_sync(0xffffffffu, bits));
     }
 }
 
 // ---------------------------------------------------------------------------
-// The fused step with the node boxes brought in by TMA and no CTA barrier
-// after the start: a two-stage pipeline per CTA. Stage k (tile k of the CTA)
-// lives in buffer k & 1: its tile, its box (one TMA tensor load, whose
-// mbarrier `full` completes when the bytes have landed), a window counter,
-// a count of the warps that have left it, and its node-block bits. Each warp
-// waits for the stage's box, takes windows of the tile until none are left,
-// and moves on to stage k + 1, which is already loaded; the last warp to leave
-// stage k marks the tile's node blocks and refills the buffer with stage
-// k + 2 (the next tile from the global counter, or an empty stage that ends
-// the CTA). A warp is thus held up only by a box that has not arrived, never
-// by the other warps' windows. Stages are refilled in order, so tile numbers
-// grow with the stage and the first empty stage ends the work for every warp.
-// Every wait is bounded: a box that does not arrive raises MPM_FLAG_TIMEOUT.
-template <int D> struct PipeSmem {
-    using G = FusedGeom<D>;
-    alignas(128) float4 box[2][G::BNP];                 // (vf, wall flag) per node
-    unsigned long long full[2];                         // the stage's box arrived (or the stage is empty)
-    int tile[2];                                        // item of the stage (>= count: empty)
-    int next_win[2];
-    int left[2];                                        // warps done with the stage
-    unsigned bmask[2];
-    float4 pay[G::WARPS][G::WIN * G::PS / 4];
+// The fused step with staged node boxes: persistent CTAs, each a pipeline of
+// tiles. Stage k (tile k of the CTA) lives in buffer k % STAGES: its item, its
+// box of node velocities and, where the tile is near the domain's walls, the box of
+// wall velocities (TMA tensor loads, whose mbarrier `full` completes when the bytes
+// have landed), a window counter, a count of the warps that have left it, and its
+// node-block bits. Each warp waits for the stage's box, takes windows of the tile
+// until none are left, and moves on to stage k + 1, which is already loaded; the
+// last warp to leave stage k marks the tile's node blocks and refills the buffer
+// with stage k + STAGES (the next tile from the global counter, or an empty stage
+// that ends the CTA). A warp is thus held up only by a box that has not arrived,
+// never by the other warps' windows. Stages are refilled in order (a warp that
+// refills stage k has not left stage k + 1 yet), so tile numbers grow with the stage
+// and the first empty stage ends the work for every warp. Every wait is bounded: a
+// box that does not arrive raises MPM_FLAG_TIMEOUT.
+//
+// Bound: instruction issue and the shared-memory pipe at 20 warps per SM (96
+// registers). 1.65M particles, snowball above a slab on the floor: 308 us with one
+// buffer per CTA of 4 warps, filled by the CTA between two barriers (the kernel this
+// one replaces), 300 now, of which the wall boxes give 13 (particles near a wall
+// otherwise read vc from L2 node by node); 3.8M in collision: 537 and 502. One CTA
+// of 20 warps and 4 stages: 303 and 518 (all warps of an SM then add to the same
+// nodes); 4 CTAs of 5 warps, which leave no room for wall boxes: 318 and 490.
+template <int D> struct PipeGeom {
+    static constexpr int STAGES = 2, WARPS = 10, CTAS = 2, THREADS = 32 * WARPS;
 };
 
-// Stage for buffer b: the next tile of the global counter and its box load,
-// or an empty stage. One thread.
+template <int D> struct PipeSmem {
+    using G = FusedGeom<D>;
+    using R = PipeGeom<D>;
+    alignas(128) float4 box[R::STAGES][G::BNP];                             // 3D: (vf, wall flag); 2D: (vf, vc)
+    alignas(128) float4 wall[D == 3 ? R::STAGES : 1][D == 3 ? G::BNP : 8];  // 3D: vc of the flagged nodes
+    unsigned long long full[R::STAGES];                                     // the stage's boxes arrived (or it is empty)
+    int4 item[R::STAGES];                                                   // tile, first slot, slots (0: empty), near a wall
+    int next_win[R::STAGES];
+    int left[R::STAGES];                                                    // warps done with the stage
+    unsigned bmask[R::STAGES];
+    float4 pay[R::WARPS][G::PAY / 4];
+};
+
+// Stage for buffer b: item e, its box loads and its particles' G2P inputs (x, F_E,
+// J_p) towards L2, or an empty stage. One warp.
 template <int D>
-__device__ __forceinline__ void pipe_refill(PipeSmem<D>& SM, int b, const TileInfo& TI, int nitems,
-                                            const CUtensorMap& map) {
-    const int e = atomicAdd(TI.fused_next, 1);
-    SM.tile[b] = e;
-    if (e < nitems) {
-        int tc[3], bo[3];
-        tile_origin<D>(TI, TI.items[e].x, tc, bo);
+__device__ __forceinline__ void pipe_refill(PipeSmem<D>& SM, int b, int e, int nitems, const Particles& P,
+                                            const StepConsts& C, const TileInfo& TI, const CUtensorMap& map) {
+    using G = FusedGeom<D>;
+    const int lane = threadIdx.x & 31;
+    if (e >= nitems) {
+        if (lane == 0) {
+            SM.item[b] = make_int4(0, 0, 0, 0);
+            mbar_arrive(&SM.full[b]);
+        }
+        return;
+    }
+    int4 item = TI.items[e];
+    if (lane == 0) {
+        int tc[3] = {0, 0, 0}, bo[3] = {0, 0, 0};
+        tile_origin<D>(TI, item.x, tc, bo);
+        bool near = false;
+#pragma unroll
+        for (int k = 0; k < D; ++k) {
+            const int ext = k == 0 ? C.W : (k == 1 ? C.H : C.Dp);
+            near = near || bo[k] <= C.margin || bo[k] + G::BE - 1 >= ext - C.margin;
+        }
+        item.w = D == 3 && near;
+        SM.item[b] = item;
         fence_proxy_async_smem();
-        box_load<D>(map, bo, SM.box[b], &SM.full[b]);
-    } else {
-        mbar_arrive(&SM.full[b]);
+        mbar_expect(&SM.full[b], (item.w ? 2 : 1) * G::BN * (uint32_t)sizeof(float4));
+        box_load<D>(map, bo, 0, SM.box[b], &SM.full[b]);
+        if (item.w) box_load<D>(map, bo, 1, SM.wall[b], &SM.full[b]);
+    }
+    if (lane < D + D * D + 1) {
+        const long long n = P.n;
+        const float* a = lane < D ? P.x + lane * n : (lane < D + D * D ? P.Fe + (lane - D) * n : P.Jp);
+        // whole 16-byte words inside the tile's slots
+        const uint64_t lo = (reinterpret_cast<uint64_t>(a + item.y) + 15) & ~15ull;
+        const uint64_t hi = reinterpret_cast<uint64_t>(a + item.y + item.z) & ~15ull;
+        if (hi > lo)
+            asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(lo), "r"((uint32_t)(hi - lo)) : "memory");
     }
 }
 
 template <int D, int S>
-__global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
+__global__ void __launch_bounds__(PipeGeom<D>::THREADS, PipeGeom<D>::CTAS)
     k_g2p2g_pipe(Particles P, StepConsts C, TileInfo TI, const float4* __restrict__ gv,
                  unsigned long long* __restrict__ acc, SlowQueue Q, unsigned* __restrict__ status,
                  const __grid_constant__ CUtensorMap gv_map) {
-    using G = FusedGeom<D>;
-    constexpr int NBLK = D == 3 ? 27 : 9;
+    using R = PipeGeom<D>;
     extern __shared__ __align__(128) unsigned char fused_smem[];
     PipeSmem<D>& SM = *reinterpret_cast<PipeSmem<D>*>(fused_smem);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int nitems = *TI.n_items;
-    if (tid == 0) {
-        for (int b = 0; b < 2; ++b) {
-            mbar_init(&SM.full[b], 1);
-            SM.next_win[b] = 0;
-            SM.left[b] = 0;
-            SM.bmask[b] = 0u;
+    if (wid == 0) {
+        if (lane < R::STAGES) {
+            mbar_init(&SM.full[lane], 1);
+            SM.next_win[lane] = 0;
+            SM.left[lane] = 0;
+            SM.bmask[lane] = 0u;
         }
         mbar_init_fence();
-        pipe_refill<D>(SM, 0, TI, nitems, gv_map);
-        pipe_refill<D>(SM, 1, TI, nitems, gv_map);
+        __syncwarp();
+        int e = 0;
+        if (lane == 0) e = atomicAdd(TI.fused_next, R::STAGES);
+        e = __shfl_sync(0xffffffffu, e, 0);
+        for (int b = 0; b < R::STAGES; ++b) pipe_refill<D>(SM, b, e + b, nitems, P, C, TI, gv_map);
     }
     __syncthreads();
-    for (int k = 0;; ++k) {
-        const int b = k & 1;
-        const unsigned par = (unsigned)(k >> 1) & 1u;
+    int b = 0;
+    unsigned par = 0u;
+    for (;;) {
         if (!__all_sync(0xffffffffu, mbar_wait(&SM.full[b], par, kBoxWaitPolls))) {
-            // the box never arrived (flagged); let the other buffer's load land first
+            // the box never arrived (flagged); let the other buffers' loads land first
             if (lane == 0) {
                 raise_flag(status, 16u);
-                mbar_wait(&SM.full[b ^ 1], (unsigned)((k + 1) >> 1) & 1u, kBoxWaitPolls);
+                for (int j = 1; j < R::STAGES; ++j)
+                    mbar_wait(&SM.full[(b + j) % R::STAGES], b + j < R::STAGES ? par : par ^ 1u, kBoxWaitPolls);
             }
             return;
         }
-        const int e = SM.tile[b];
-        if (e >= nitems) break;
-        const int4 item = TI.items[e];  // tile, first slot, slots
-        const int t = item.x, start = item.y, m = item.z;
+        const int4 item = SM.item[b];
+        const int start = item.y, m = item.z;
+        if (m == 0) break;
         int tc[3] = {0, 0, 0}, bo[3] = {0, 0, 0};
-        tile_origin<D>(TI, t, tc, bo);
+        tile_origin<D>(TI, item.x, tc, bo);
         const int nwin = (m + TI.win - 1) / TI.win;
         unsigned bits = 0u;
         for (;;) {
@@ -1069,7 +1044,8 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
             if (lane == 0) w = atomicAdd(&SM.next_win[b], 1);
             w = __shfl_sync(0xffffffffu, w, 0);
             if (w >= nwin) break;
-            bits |= fused_window<D, S, true>(P, C, TI, gv, acc, Q, status, SM.box[b], bo, start, m, TI.win, w,
+            bits |= fused_window<D, S, true>(P, C, TI, gv, acc, Q, status, SM.box[b],
+                                             D == 3 && item.w ? SM.wall[b] : nullptr, bo, start, m, TI.win, w,
                                              reinterpret_cast<float*>(SM.pay[wid]));
         }
         bits = __reduce_or_sync(0xffffffffu, bits);
@@ -1077,27 +1053,27 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
         if (lane == 0) {
             if (bits) atomicOr(&SM.bmask[b], bits);
             __threadfence_block();  // the bits and this warp's reads of the box before the count
-            last = atomicAdd(&SM.left[b], 1) == G::WARPS - 1;
+            last = atomicAdd(&SM.left[b], 1) == R::WARPS - 1;
         }
         if (__shfl_sync(0xffffffffu, last, 0)) {
-            // last warp out: mark the tile's node blocks, then stage k + 2 into this buffer
+            // last warp out: mark the tile's node blocks, then stage k + STAGES into this buffer
             __threadfence_block();
             unsigned bm = 0u;
-            if (lane == 0) bm = atomicOr(&SM.bmask[b], 0u);
-            bm = __shfl_sync(0xffffffffu, bm, 0);
-            if (lane < NBLK && (bm >> lane) & 1u) {
-                const int rx = lane % 3, ry = (lane / 3) % 3, rz = lane / 9;
-                const int bx = tc[0] - 1 + rx, by = tc[1] - 1 + ry, bz = D == 3 ? tc[2] - 1 + rz : 0;
-                mark_block_once(TI, (bz * TI.nblk[1] + by) * TI.nblk[0] + bx);
-            }
-            __syncwarp();
+            int e = 0;
             if (lane == 0) {
+                bm = atomicOr(&SM.bmask[b], 0u);
                 SM.bmask[b] = 0u;
                 SM.next_win[b] = 0;
                 SM.left[b] = 0;
-                pipe_refill<D>(SM, b, TI, nitems, gv_map);
+                e = atomicAdd(TI.fused_next, 1);
             }
+            mark_tile_blocks<D>(TI, tc, __shfl_sync(0xffffffffu, bm, 0));
+            pipe_refill<D>(SM, b, __shfl_sync(0xffffffffu, e, 0), nitems, P, C, TI, gv_map);
             __syncwarp();
+        }
+        if (++b == R::STAGES) {
+            b = 0;
+            par ^= 1u;
         }
     }
 }

@@ -147,3 +147,39 @@ def test_pending_sums_match_a_fresh_p2g(gpu_lib):
     assert np.array_equal(m1, m1b) and np.array_equal(p1, p1b)
     assert rel_l2(m1, m2) < 1e-6
     assert rel_l2(p1, p2) < 1e-5
+
+
+def _crowd(dim, n, quad, seed=5):
+    """n particles: a dense lump (many windows in a tile), a spread over the whole
+    domain up to its edge (clipped stencils, walls, tiles of one particle), at speeds
+    that carry some out of their tile's box."""
+    from mpm_snow_sim2d_b200 import _lib, scenes
+    base = scenes.impact_3d() if dim == 3 else scenes.impact_2d()
+    ext = np.array([52, 44, 48][:dim] if dim == 3 else [180, 150], np.float64)
+    rng = np.random.default_rng(seed)
+    pos = 0.4 + rng.random((n, dim)) * (ext - 0.8)
+    lump = n // 2
+    pos[:lump] = 9.0 + rng.random((lump, dim)) * 3.0
+    vel = 0.3 / base.delta_time * rng.standard_normal((n, dim)) * (rng.random((n, 1)) < 0.1)
+    return base.with_(width=int(ext[0]), height=int(ext[1]), depth=int(ext[2]) if dim == 3 else 0,
+                      position=pos.astype(np.float32), velocity=vel.astype(np.float32),
+                      volume=np.full(n, 0.1, np.float32), mass=np.full(n, base.mass[0], np.float32),
+                      formulation=_lib.FORMULATION_MLS_QUADRATIC if quad else base.formulation)
+
+
+# particles: one; a window and one more at 8 slots; 8-, 16- and 32-slot windows with
+# tiles of one item, of a few and of many windows
+@pytest.mark.parametrize("quad", [False, True])
+@pytest.mark.parametrize("dim,n", [(2, 1), (2, 6001), (2, 40001), (3, 1), (3, 9), (3, 3001), (3, 40001), (3, 70001)])
+def test_staged_and_direct_agree(gpu_lib, dim, n, quad):
+    """k_g2p2g_pipe and k_g2p2g_direct form the same windows, so the node sums are
+    the same integers where the per-particle arithmetic is: FP32 contraction may
+    differ between the two builds, by a few roundings per step (bounds as for the
+    two box loads); both raise the same flags, and neither a timeout."""
+    sc = _crowd(dim, n, quad)
+    a, fa = _run(sc, 6, "fused", "gather", sort_period=8)
+    b, fb = _run(sc, 6, "fused", "tma", sort_period=8)
+    assert fa == fb and fb & 16 == 0
+    assert np.isfinite(b.position).all() == np.isfinite(a.position).all()
+    for f, tol in (("position", 1e-6), ("elastic_f", 1e-5), ("plastic_det", 1e-5)):
+        assert rel_l2(getattr(b, f), getattr(a, f)) < tol, f

@@ -112,8 +112,9 @@ Particles particles(const mpm_batch* b) {
 
 // ---- the step sequence ----
 
-// All scenes' particles into the other buffer, by (tile, cell, id).
-cudaError_t enqueue_sort(mpm_batch* b) {
+// All scenes' particles into the other buffer, by (tile, cell, id); without v and B
+// when every scene's sums are pending (the next G2P writes them unread).
+cudaError_t enqueue_sort(mpm_batch* b, bool pending) {
     if (b->N == 0) return cudaSuccess;
     const Particles P = particles(b);
     const int threads = 256;
@@ -124,7 +125,7 @@ cudaError_t enqueue_sort(mpm_batch* b) {
     k_sort_scan<<<scan_blocks, kScanTiles, 0, b->stream>>>(b->ti);
     k_sort_bucket<<<blocks, threads, 0, b->stream>>>((int)b->N, b->ti);
     const BatchBuffers& t = b->buf[b->parity ^ 1];
-    const SortBuffers dst{t.x, t.v, t.B, t.Fe, t.Jp, nullptr, t.mass, t.vol, t.id};
+    const SortBuffers dst{t.x, pending ? nullptr : t.v, pending ? nullptr : t.B, t.Fe, t.Jp, nullptr, t.mass, t.vol, t.id};
     k_tile_sort<2, 4, ManyScenes><<<b->sms * SortGeom<2>::CTAS_PER_SM, 256, 0, b->stream>>>(
         P, b->buf[b->parity].id, dst, b->many, b->ti);
     b->parity ^= 1;
@@ -143,7 +144,7 @@ cudaError_t enqueue_step(mpm_batch* b) {
 }
 
 cudaError_t enqueue_segment(mpm_batch* b, int steps, bool sort) {
-    cudaError_t e = sort ? enqueue_sort(b) : cudaSuccess;
+    cudaError_t e = sort ? enqueue_sort(b, true) : cudaSuccess;
     for (int k = 0; k < steps && e == cudaSuccess; ++k) e = enqueue_step(b);
     return e;
 }
@@ -468,7 +469,7 @@ mpm_status mpm_batch_step(mpm_batch* b, int32_t nsteps) {
     b->last_steps = nsteps;
     if (b->any_fresh) {
         // sums of the new states: sort, then their P2G
-        BATCH_CUDA(b, enqueue_sort(b));
+        BATCH_CUDA(b, enqueue_sort(b, false));
         b->needs_sort = false;
         b->since_sort = 0;
         if (b->N > 0)

@@ -203,7 +203,7 @@ static __global__ void __launch_bounds__(kScanTiles) k_sort_scan(TileInfo TI) {
 }
 
 struct SortBuffers {
-    float *x, *v, *B, *Fe, *Jp, *A, *mass, *vol;
+    float *x, *v, *B, *Fe, *Jp, *A, *mass, *vol;  // v and B, A: null when the next kernels form them anew
     int* id;
 };
 
@@ -343,12 +343,18 @@ __global__ void __launch_bounds__(256) k_tile_sort(Particles P, const int* __res
         for (int j = threadIdx.x; j < m; j += blockDim.x) {
             const int src = val[j], s = start + j;
 #pragma unroll
-            for (int k = 0; k < D; ++k) { dst.x[k * n + s] = P.x[k * n + src]; dst.v[k * n + s] = P.v[k * n + src]; }
+            for (int k = 0; k < D; ++k) dst.x[k * n + s] = P.x[k * n + src];
 #pragma unroll
-            for (int k = 0; k < D * D; ++k) {
-                dst.B[k * n + s] = P.B[k * n + src];
-                dst.Fe[k * n + s] = P.Fe[k * n + src];
-                if (dst.A) dst.A[k * n + s] = P.A[k * n + src];
+            for (int k = 0; k < D * D; ++k) dst.Fe[k * n + s] = P.Fe[k * n + src];
+            if (dst.v) {
+#pragma unroll
+                for (int k = 0; k < D; ++k) dst.v[k * n + s] = P.v[k * n + src];
+#pragma unroll
+                for (int k = 0; k < D * D; ++k) dst.B[k * n + s] = P.B[k * n + src];
+            }
+            if (dst.A) {
+#pragma unroll
+                for (int k = 0; k < D * D; ++k) dst.A[k * n + s] = P.A[k * n + src];
             }
             dst.Jp[s] = P.Jp[src];
             dst.id[s] = id_src[src];

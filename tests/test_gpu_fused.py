@@ -183,3 +183,24 @@ def test_staged_and_direct_agree(gpu_lib, dim, n, quad):
     assert np.isfinite(b.position).all() == np.isfinite(a.position).all()
     for f, tol in (("position", 1e-6), ("elastic_f", 1e-5), ("plastic_det", 1e-5)):
         assert rel_l2(getattr(b, f), getattr(a, f)) < tol, f
+
+
+@pytest.mark.parametrize("period,steps", [(1, 1), (1, 5), (2, 3), (3, 7)])
+@pytest.mark.parametrize("case", ["impact2d", "impact3d", "impact3d_quad"])
+def test_sort_leaves_velocities_to_the_next_step(gpu_lib, case, period, steps):
+    """A sort with the sums pending moves neither v nor B; the step after it writes
+    both. Whole states read right after such steps, profiled stage by stage or not,
+    against the split transfer, which moves them (bounds of test_fused_matches_split,
+    B as the velocities)."""
+    from mpm_snow_sim2d_b200 import Solver
+    sc, _ = _scenes()[case]
+    ref, _ = _run(sc, steps + 1, "split", sort_period=period)
+    got, _ = _run(sc, steps + 1, "fused", sort_period=period)
+    with Solver.from_scene(sc, sort_period=period) as s:
+        s.Step(1)
+        s.step_profiled(steps)
+        staged = s.get_state()
+    for st in (got, staged):
+        errs = {f: rel_l2(getattr(st, f), getattr(ref, f)) for f in FIELDS}
+        assert errs["position"] < 2e-6 and errs["elastic_f"] < 2e-5 and errs["plastic_det"] < 2e-5, errs
+        assert errs["velocity"] < 5e-4 and errs["affine_b"] < 5e-4, errs

@@ -24,8 +24,8 @@
 // Particles whose stencil leaves the box (drifted more than a cell since the
 // sort) gather from global memory. Queued particles (out of the elastic band, or
 // a stencil clipped by the grid edge) are scattered after their return map: the
-// warp records its window (first slot, mask of the queued lanes), and
-// k_p2g_windows repeats the scatter over those lanes.
+// warp records its window (first slot, mask of the lanes to scatter: the queued
+// ones, or with them all the others) for k_p2g_windows.
 //
 // Determinism: every sum beyond one window is an integer add, and the FP32 sums
 // in it are a function of the slot order, the window boundaries (fixed offsets
@@ -584,9 +584,9 @@ __device__ __forceinline__ unsigned stencil_block_bits(const int* base, const in
     return bits;
 }
 
-// P2G of the queued particles of one recorded window (rec: first slot, mask of the
-// queued lanes, mask of those whose node blocks are not marked yet) after their
-// return map, by one warp: x, v, A as the G2P and return-map kernels left them,
+// P2G of the particles left over of one recorded window (rec: first slot, mask of
+// the lanes, mask of those whose node blocks are not marked yet) after the return
+// map, by one warp: x, v, A as the G2P and return-map kernels left them,
 // scattered as in the fused kernel. The order inside a window is a function of its
 // queued particles, so the int64 sums do not depend on the order in which windows
 // were recorded. The fused kernel has marked the node blocks of every queued
@@ -858,14 +858,26 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
         }
     }
     if constexpr (G2P) {
-        // record the window if some of its particles wait for the return map
-        const unsigned dm = __ballot_sync(0xffffffffu, deferred);
-        if (dm) {
+        // A window some of whose particles wait for the return map is recorded. In 3D
+        // and in batches it is put off as a whole: scattered twice, it would add its
+        // node planes twice, which costs more than handing the other particles' A on
+        // through memory (3.8M particles in collision, a third of them queued: 462 us
+        // here and 327 in k_p2g_windows, put off 302 and 334; 2.8M in 256 2D scenes
+        // 331 + 19.3, 327 + 18.5). A single 2D scene queues a few windows and waits
+        // for the longest of them: 22.3 + 3.4 us at 186k particles, put off 21.9 + 6.0.
+        constexpr bool PUT_OFF = D == 3 || EXACT;
+        if (__builtin_expect(__any_sync(0xffffffffu, deferred), 0)) {
+            const unsigned rows = __ballot_sync(0xffffffffu, deferred || (PUT_OFF && key != kNoKey));
             const unsigned um = __ballot_sync(0xffffffffu, unmarked);
+            if (PUT_OFF && key != kNoKey) {
+#pragma unroll
+                for (int k = 0; k < D * D; ++k) P.A[k * n + i] = A[k];
+            }
             if (lane == 0) {
                 const int r = atomicAdd(Q.nwin, 1);
-                if (r < Q.win_capacity) Q.win[r] = make_int4(start + w * win, (int)dm, (int)um, Q.scene);
+                if (r < Q.win_capacity) Q.win[r] = make_int4(start + w * win, (int)rows, (int)um, Q.scene);
             }
+            if (PUT_OFF) return bits;
         }
     }
     int count, total;

@@ -675,7 +675,7 @@ struct SlowQueue {
     float* fh;    // trial F per queue entry, [D*D][capacity]
     int capacity;
     // fused path: the 32-slot windows holding queued particles, as (first
-    // slot, lane mask of the queued slots); their P2G runs after the return map
+    // slot, mask of the slots left to scatter); their P2G runs after the return map
     int4* win;  // .z: queued slots whose node blocks are not marked yet
     int* nwin;    // device scalar (count[1])
     int win_capacity;

@@ -204,3 +204,35 @@ def test_sort_leaves_velocities_to_the_next_step(gpu_lib, case, period, steps):
         errs = {f: rel_l2(getattr(st, f), getattr(ref, f)) for f in FIELDS}
         assert errs["position"] < 2e-6 and errs["elastic_f"] < 2e-5 and errs["plastic_det"] < 2e-5, errs
         assert errs["velocity"] < 5e-4 and errs["affine_b"] < 5e-4, errs
+
+
+# one queued particle per window, every second, all but one in 32, all; with whole
+# windows and with windows of one particle
+@pytest.mark.parametrize("every,out", [(32, 1), (2, 1), (32, 31), (1, 1)])
+@pytest.mark.parametrize("dim,n", [(2, 33), (2, 5000), (3, 33), (3, 5000)])
+def test_windows_put_off(gpu_lib, dim, n, every, out):
+    """Particles out of the elastic band leave their window to the pass after the
+    return map, in 3D with all of its particles: against the split transfer (bounds of
+    test_fused_matches_split), and bitwise from run to run."""
+    from mpm_snow_sim2d_b200 import Solver
+    sc = _crowd(dim, n, False)
+    sc = sc.with_(velocity=np.zeros_like(sc.velocity))
+    F = np.tile(np.eye(dim, dtype=np.float32), (n, 1, 1))
+    F[np.arange(n) % every < out] *= 1.05
+    got = []
+    for transfer in ("fused", "fused", "split"):
+        os.environ["MPM_TRANSFER"] = transfer
+        try:
+            with Solver.from_scene(sc) as s:
+                s.set_state(elastic_f=F)
+                s.Step(3)
+                got.append((s.get_state(), s.status()))
+        finally:
+            os.environ.pop("MPM_TRANSFER")
+    (a, fa), (again, _), (b, fb) = got
+    for f in FIELDS:
+        assert np.array_equal(getattr(a, f), getattr(again, f)), f
+    assert fa & 3 == fb & 3
+    errs = {f: rel_l2(getattr(a, f), getattr(b, f)) for f in ("position", "velocity", "elastic_f", "plastic_det")}
+    assert errs["position"] < 2e-6 and errs["elastic_f"] < 2e-5 and errs["plastic_det"] < 2e-5, errs
+    assert errs["velocity"] < 5e-4, errs

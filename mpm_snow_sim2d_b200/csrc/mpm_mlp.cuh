@@ -59,6 +59,13 @@ __device__ __forceinline__ float gelu(float x) {
     const float th = tanh_hw(kGeluC * x * fmaf(kGeluA, x * x, 1.f));
     return 0.5f * x * (1.f + th);
 }
+// Of two values, in packed FP32 (8 instructions for what takes 14 one by one).
+__device__ __forceinline__ float2 gelu2(float2 x) {
+    const float2 u = __fmul2_rn(x, __ffma2_rn(__fmul2_rn(x, x), make_float2(kGeluC * kGeluA, kGeluC * kGeluA),
+                                              make_float2(kGeluC, kGeluC)));
+    const float2 h = __fmul2_rn(x, make_float2(0.5f, 0.5f));
+    return __ffma2_rn(h, make_float2(tanh_hw(u.x), tanh_hw(u.y)), h);
+}
 __device__ __forceinline__ float gelu_grad(float x) {
     const float x2 = x * x;
     const float th = tanh_hw(kGeluC * x * fmaf(kGeluA, x2, 1.f));
@@ -204,21 +211,24 @@ struct MlpParams {
 // activations never leave registers: the m16n8 accumulators of one layer,
 // after bias + GELU, are packed to bf16 pairs that are exactly the m16k16 A
 // fragments of the next layer (accumulator n-tiles 2kb, 2kb+1 = A k-block kb).
-// Weights sit in shared memory with rows padded by 8 bf16 so that the B
-// fragment loads of a warp hit 32 distinct banks (and eight rows' 16-byte ldmatrix
-// rows too, in training).
+// Weights sit in shared memory with rows padded by 8 bf16 so that the eight rows
+// of a B fragment (ldmatrix) fall into distinct banks.
+//
+// Bound: instruction issue (GELU half of it) at 16 warps per SM. The three hidden
+// layers run through one copy of the code: with a copy each, the kernel outgrew
+// the instruction cache. 474k particles in collision, most of them queued: 119 us a
+// step with scalar GELU, 4-byte fragment loads and unrolled layers, now 86.
 constexpr int kMwIn = kMlpInPad + 8;  // row stride (bf16) of W1 and of the input tile
 constexpr int kMwHid = kMlpHid + 8;   // row stride (bf16) of W2, W3, W4
 constexpr int kMwOut = kMlpOutPad + 2;  // row stride (fp32) of the output tile
 constexpr int kMlpWarps = 8;
 
 struct MlpWarpSmem {
-    __nv_bfloat16 W1[kMlpHid * kMwIn];
-    __nv_bfloat16 W2[kMlpHid * kMwHid];
-    __nv_bfloat16 W3[kMlpHid * kMwHid];
+    alignas(16) __nv_bfloat16 W1[kMlpHid * kMwIn];
+    __nv_bfloat16 W23[2][kMlpHid * kMwHid];
     __nv_bfloat16 W4[kMlpOutPad * kMwHid];
-    float b1[kMlpHid], b2[kMlpHid], b3[kMlpHid], b4[kMlpOutPad];
-    __nv_bfloat16 x[kMlpWarps][32 * kMwIn];
+    float b[3][kMlpHid], b4[kMlpOutPad];
+    alignas(16) __nv_bfloat16 x[kMlpWarps][32 * kMwIn];
     float out[kMlpWarps][32 * kMwOut];
 };
 
@@ -233,37 +243,59 @@ __device__ __forceinline__ void mlp_stage_matrix(__nv_bfloat16* dst, int ld_dst,
 
 __device__ __forceinline__ void mlp_stage_weights(MlpWarpSmem& S, const __nv_bfloat16* wbf, const float* wf32) {
     mlp_stage_matrix(S.W1, kMwIn, wbf + MlpOff::W1, kMlpHid, kMlpInPad);
-    mlp_stage_matrix(S.W2, kMwHid, wbf + MlpOff::W2, kMlpHid, kMlpHid);
-    mlp_stage_matrix(S.W3, kMwHid, wbf + MlpOff::W3, kMlpHid, kMlpHid);
+    mlp_stage_matrix(S.W23[0], kMwHid, wbf + MlpOff::W2, kMlpHid, kMlpHid);
+    mlp_stage_matrix(S.W23[1], kMwHid, wbf + MlpOff::W3, kMlpHid, kMlpHid);
     mlp_stage_matrix(S.W4, kMwHid, wbf + MlpOff::W4, kMlpOutPad, kMlpHid);
     for (int i = threadIdx.x; i < kMlpHid; i += blockDim.x) {
-        S.b1[i] = wf32[MlpOff::b1 + i];
-        S.b2[i] = wf32[MlpOff::b2 + i];
-        S.b3[i] = wf32[MlpOff::b3 + i];
+        S.b[0][i] = wf32[MlpOff::b1 + i];
+        S.b[1][i] = wf32[MlpOff::b2 + i];
+        S.b[2][i] = wf32[MlpOff::b3 + i];
     }
     for (int i = threadIdx.x; i < kMlpOutPad; i += blockDim.x) S.b4[i] = wf32[MlpOff::b4 + i];
 }
 
 __device__ __forceinline__ uint32_t pack_f2_bf16(float lo, float hi) {
-    return pack_bf16(__float2bfloat16_rn(lo), __float2bfloat16_rn(hi));
+    const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
+    return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+__device__ __forceinline__ void ldmatrix_x4(uint32_t* r, const __nv_bfloat16* p) {
+    const uint32_t a = (uint32_t)__cvta_generic_to_shared(p);
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3])
+                 : "r"(a)
+                 : "memory");
 }
 
 // acc[j] (n-tile j of a 16 x 8*NT output) = A (16 x 16*KB, fragments a[kb]) * W^T,
-// W row-major [out][in] in shared memory with row stride ld.
+// W row-major [out][in] in shared memory with row stride ld. An ldmatrix brings two
+// B fragments: of two k-blocks, or (KB = 1) of two n-tiles.
 template <int KB, int NT>
 __device__ __forceinline__ void mlp_warp_layer(const uint32_t (*a)[4], const __nv_bfloat16* W, int ld, float (*acc)[4]) {
-    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    static_assert(KB == 1 || KB % 2 == 0, "fragments come in pairs");
+    const int lane = threadIdx.x & 31, row = lane & 7, mat = lane >> 3;
 #pragma unroll
-    for (int j = 0; j < NT; ++j) {
-        acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
-        const __nv_bfloat16* w = W + (j * 8 + g) * ld + 2 * t;
+    for (int j = 0; j < NT; ++j) acc[j][0] = acc[j][1] = acc[j][2] = acc[j][3] = 0.f;
+    if constexpr (KB == 1) {
+        const __nv_bfloat16* w = W + ((mat >> 1) * 8 + row) * ld + (mat & 1) * 8;
 #pragma unroll
-        for (int kb = 0; kb < KB; ++kb) {
-            uint32_t b[2];
-            b[0] = *reinterpret_cast<const uint32_t*>(w + kb * 16);
-            b[1] = *reinterpret_cast<const uint32_t*>(w + kb * 16 + 8);
-            mma_bf16(acc[j], a[kb], b);
+        for (int j = 0; j < NT; j += 2) {
+            uint32_t b[4];
+            ldmatrix_x4(b, w + j * 8 * ld);
+            mma_bf16(acc[j], a[0], b);
+            mma_bf16(acc[j + 1], a[0], b + 2);
         }
+    } else {
+        const __nv_bfloat16* w = W + row * ld + mat * 8;
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int kb = 0; kb < KB; kb += 2) {
+                uint32_t b[4];
+                ldmatrix_x4(b, w + j * 8 * ld + kb * 16);
+                mma_bf16(acc[j], a[kb], b);
+                mma_bf16(acc[j], a[kb + 1], b + 2);
+            }
     }
 }
 
@@ -274,10 +306,12 @@ __device__ __forceinline__ void mlp_warp_activate(float (*acc)[4], const float* 
     for (int kb = 0; kb < kMlpHid / 16; ++kb)
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            const int j = 2 * kb + h, c = j * 8 + 2 * t;
-            const float b0 = bias[c], b1 = bias[c + 1];
-            a[kb][2 * h] = pack_f2_bf16(gelu(acc[j][0] + b0), gelu(acc[j][1] + b1));
-            a[kb][2 * h + 1] = pack_f2_bf16(gelu(acc[j][2] + b0), gelu(acc[j][3] + b1));
+            const int j = 2 * kb + h;
+            const float2 b = *reinterpret_cast<const float2*>(bias + j * 8 + 2 * t);
+            const float2 u = gelu2(__fadd2_rn(make_float2(acc[j][0], acc[j][1]), b));
+            const float2 v = gelu2(__fadd2_rn(make_float2(acc[j][2], acc[j][3]), b));
+            a[kb][2 * h] = pack_f2_bf16(u.x, u.y);
+            a[kb][2 * h + 1] = pack_f2_bf16(v.x, v.y);
         }
 }
 
@@ -289,17 +323,15 @@ __device__ __forceinline__ void mlp_warp_forward(const MlpWarpSmem& S, const __n
     for (int mt = 0; mt < 2; ++mt) {
         const int r0 = mt * 16 + g;
         uint32_t a[kMlpHid / 16][4];
-        a[0][0] = *reinterpret_cast<const uint32_t*>(X + r0 * kMwIn + 2 * t);
-        a[0][1] = *reinterpret_cast<const uint32_t*>(X + (r0 + 8) * kMwIn + 2 * t);
-        a[0][2] = *reinterpret_cast<const uint32_t*>(X + r0 * kMwIn + 2 * t + 8);
-        a[0][3] = *reinterpret_cast<const uint32_t*>(X + (r0 + 8) * kMwIn + 2 * t + 8);
+        ldmatrix_x4(a[0], X + (mt * 16 + (lane & 15)) * kMwIn + (lane >> 4) * 8);
         float acc[kMlpHid / 8][4];
         mlp_warp_layer<1, kMlpHid / 8>(a, S.W1, kMwIn, acc);
-        mlp_warp_activate(acc, S.b1, a);
-        mlp_warp_layer<kMlpHid / 16, kMlpHid / 8>(a, S.W2, kMwHid, acc);
-        mlp_warp_activate(acc, S.b2, a);
-        mlp_warp_layer<kMlpHid / 16, kMlpHid / 8>(a, S.W3, kMwHid, acc);
-        mlp_warp_activate(acc, S.b3, a);
+#pragma unroll 1
+        for (int l = 0; l < 2; ++l) {
+            mlp_warp_activate(acc, S.b[l], a);
+            mlp_warp_layer<kMlpHid / 16, kMlpHid / 8>(a, S.W23[l], kMwHid, acc);
+        }
+        mlp_warp_activate(acc, S.b[2], a);
         float o[kMlpOutPad / 8][4];
         mlp_warp_layer<kMlpHid / 16, kMlpOutPad / 8>(a, S.W4, kMwHid, o);
 #pragma unroll
@@ -344,12 +376,6 @@ __global__ void __launch_bounds__(kMlpWarps * 32) k_return_map_mlp(Particles P, 
 #pragma unroll
             for (int k = 0; k < 9; ++k) Fh[k] = Q.fh[k * Q.capacity + e];
             Jp0 = P.Jp[entry];
-            // the particle's B, mass and volume, loaded now so that their
-            // latency overlaps the network
-#pragma unroll
-            for (int k = 0; k < 9; ++k) B[k] = P.B[k * n + entry];
-            mass = P.mass ? P.mass[entry] : P.mass_u;
-            vol = P.vol ? P.vol[entry] : P.vol_u;
             mlp_features(Fh, Jp0, ML.norm, in);
         }
         uint32_t* xr = reinterpret_cast<uint32_t*>(X + lane * kMwIn);
@@ -363,6 +389,10 @@ __global__ void __launch_bounds__(kMlpWarps * 32) k_return_map_mlp(Particles P, 
         if (__any_sync(0xffffffffu, valid)) mlp_warp_forward(S, X, O);
         __syncwarp();
         if (valid) {
+#pragma unroll
+            for (int k = 0; k < 9; ++k) B[k] = P.B[k * n + entry];
+            mass = P.mass ? P.mass[entry] : P.mass_u;
+            vol = P.vol ? P.vol[entry] : P.vol_u;
             const float* o = O + lane * kMwOut;
             float Fp[9];
 #pragma unroll

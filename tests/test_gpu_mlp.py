@@ -119,3 +119,38 @@ def test_pretrained_weights_take_particles_off_the_svd(mlp_mod):
           f"over 300 steps")
     assert acc > 4 * rej
     assert rel_F <= 1e-3
+
+
+# rows: one, around the 16- and 32-row tiles of a warp and the 256 rows of a CTA, and
+# more tiles than warps in flight
+@pytest.mark.parametrize("rows", [1, 15, 16, 17, 31, 33, 255, 257, 40001])
+def test_inference_row_counts(mlp_mod, rows):
+    """Every row of a ragged batch against the FP64 network on bf16-rounded weights
+    and activations. A rounding that falls the other way moves an activation by one
+    bf16 ulp (2^-8 relative at most), a row's output by about 1e-2 of its size."""
+    from oracle import mlp_ref
+    pairs = synthetic_pairs(rows, seed=rows)
+    net = mlp_mod.Mlp(seed=4)
+    norm = mlp_mod.normalization(synthetic_pairs(512, seed=2))
+    net.set_normalization(*norm)
+    got = net.predict(pairs[:, :10])
+    _, ref = mlp_ref.forward(net.params(), pairs[:, :10], norm, bf16_emulation=True)
+    got = (got - norm[2]) / norm[3]
+    ref = ref[:, :10]
+    assert got.shape == ref.shape
+    assert np.abs(got - ref).max() < 1e-2 * np.linalg.norm(ref, axis=1).max()
+
+
+# rows of a gradient: one, around a CTA's 128-row tile, more tiles than CTAs
+@pytest.mark.parametrize("rows", [1, 127, 128, 129, 148 * 128 + 1])
+def test_gradient_row_counts(mlp_mod, rows):
+    """The bounds of test_gradient_matches_cpu_oracle at ragged row counts."""
+    from oracle import mlp_ref
+    pairs = synthetic_pairs(rows, seed=rows + 7)
+    net = mlp_mod.Mlp(seed=11)
+    norm = mlp_mod.normalization(synthetic_pairs(512, seed=3))
+    net.set_normalization(*norm)
+    g_gpu, l_gpu = net.gradient(pairs)
+    l_ref, g_ref = mlp_ref.loss_and_grad(net.params(), pairs, norm, bf16_emulation=True)
+    assert abs(l_gpu - l_ref) <= 1e-3 * l_ref
+    assert np.linalg.norm(g_gpu - g_ref) / np.linalg.norm(g_ref) < 1e-2

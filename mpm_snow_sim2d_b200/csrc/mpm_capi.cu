@@ -379,7 +379,8 @@ template <int D, int S> cudaError_t launch_return_map(mpm_solver* s) {
                                                                                        ML);
         L = PairLog{nullptr, nullptr, 0};
     }
-    k_g2p_plastic<D, S><<<s->sms * 4, 256, 0, s->stream>>>(particle_view(s), s->C, s->gv, s->q, L, s->status);
+    k_g2p_plastic<D, S><<<s->sms * kPlasticCtas, kPlasticThreads, 0, s->stream>>>(particle_view(s), s->C, s->gv, s->q, L,
+                                                                                s->status);
     return cudaGetLastError();
 }
 

@@ -1020,8 +1020,13 @@ __device__ __forceinline__ void g2p_queued_exact(const Particles& P, const StepC
     }
 }
 
+// Bound: instruction issue and latency of the Jacobi sweeps (div, sqrt). Six CTAs of
+// 128 threads per SM (80 registers) hide more of it than two of 256 at 128
+// registers: 1.4M particles queued of 3.8M, 266 us, now 232; four, five, seven and
+// eight CTAs take 257, 246, 235, 236.
+constexpr int kPlasticThreads = 128, kPlasticCtas = 6;
 template <int D, int S = 4>
-__global__ void __launch_bounds__(256) k_g2p_plastic(Particles P, StepConsts C, const float4* __restrict__ gv,
+__global__ void __launch_bounds__(kPlasticThreads, kPlasticCtas) k_g2p_plastic(Particles P, StepConsts C, const float4* __restrict__ gv,
                                                      SlowQueue Q, PairLog L, unsigned* __restrict__ status) {
     const int m = *Q.count;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x)

@@ -133,14 +133,15 @@ cudaError_t enqueue_sort(mpm_batch* b, bool pending) {
 }
 
 cudaError_t enqueue_step(mpm_batch* b) {
-    k_batch_grid<<<b->sms * 8, 256, 0, b->stream>>>(b->arr, b->ti);
-    if (b->N > 0) {
-        const Particles P = particles(b);
-        k_batch_step<true><<<b->sms * MPM_FUSED_MIN_BLOCKS, FusedGeom<2>::THREADS, 0, b->stream>>>(P, b->arr, b->ti, b->q);
-        k_batch_plastic<<<b->sms * 4, 256, 0, b->stream>>>(P, b->arr, b->q);
-        k_batch_windows<<<b->sms * 8, FusedGeom<2>::THREADS, 0, b->stream>>>(P, b->arr, b->ti, b->q);
-    }
-    return cudaGetLastError();
+    cudaError_t e = launch_chained(k_batch_grid, b->sms * 8, 256, 0, b->stream, b->arr, b->ti);
+    if (e != cudaSuccess || b->N == 0) return e;
+    const Particles P = particles(b);
+    e = launch_chained(k_batch_step<true>, b->sms * MPM_FUSED_MIN_BLOCKS, FusedGeom<2>::THREADS, 0, b->stream, P, b->arr,
+                       b->ti, b->q);
+    if (e == cudaSuccess) e = launch_chained(k_batch_plastic, b->sms * 4, 256, 0, b->stream, P, b->arr, b->q);
+    if (e == cudaSuccess)
+        e = launch_chained(k_batch_windows, b->sms * 8, FusedGeom<2>::THREADS, 0, b->stream, P, b->arr, b->ti, b->q);
+    return e;
 }
 
 cudaError_t enqueue_segment(mpm_batch* b, int steps, bool sort) {

@@ -89,6 +89,7 @@ __device__ __forceinline__ const BatchScene& stage_scene(const BatchScene* scene
 // records the time at which a step begins.
 __global__ void __launch_bounds__(256) k_batch_grid(BatchArrays B, TileInfo TI) {
     using G = TileGeom<2>;
+    chain_wait();
     const int nb = *TI.n_marked;
     const long long total = (long long)nb * G::BN;
     if (blockIdx.x == 0) {
@@ -120,6 +121,7 @@ __global__ void __launch_bounds__(FusedGeom<2>::THREADS, MPM_FUSED_MIN_BLOCKS)
     __shared__ BatchScene scene_s[G::WARPS];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     float* pay = reinterpret_cast<float*>(pay_s[wid]);
+    chain_wait();
     const int nitems = *TI.n_items;
     for (int e = wid * gridDim.x + blockIdx.x; e < nitems; e += G::WARPS * gridDim.x) {
         const int4 item = TI.items[e];
@@ -139,6 +141,7 @@ __global__ void __launch_bounds__(FusedGeom<2>::THREADS, MPM_FUSED_MIN_BLOCKS)
 }
 
 __global__ void __launch_bounds__(256) k_batch_plastic(Particles P, BatchArrays B, SlowQueue Q) {
+    chain_wait();
     const int m = *Q.count;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x) {
         const int entry = Q.list[e], sc = B.of_slots[entry >= 0 ? entry : -1 - entry];
@@ -153,6 +156,7 @@ __global__ void __launch_bounds__(FusedGeom<2>::THREADS) k_batch_windows(Particl
     __shared__ float4 pay_s[G::WARPS][G::PAY / 4];
     __shared__ BatchScene scene_s[G::WARPS];
     const int wid = threadIdx.x >> 5;
+    chain_wait();
     const int nw = min(*Q.nwin, Q.win_capacity);
     for (int r = blockIdx.x * G::WARPS + wid; r < nw; r += gridDim.x * G::WARPS) {
         const int4 rec = Q.win[r];

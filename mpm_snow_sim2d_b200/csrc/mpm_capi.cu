@@ -375,13 +375,13 @@ template <int D, int S> cudaError_t launch_return_map(mpm_solver* s) {
     PairLog L{s->log_data, s->log_n, s->log_cap};
     if (D == 3 && S == 4 && s->plasticity == MPM_PLASTIC_MLP && s->mlp) {
         MlpParams ML{s->mlp->wbf, s->mlp->w, s->mlp->norm, s->mlp_tol, s->mlp_counters};
-        k_return_map_mlp<<<s->sms * 2, kMlpWarps * 32, sizeof(MlpWarpSmem), s->stream>>>(particle_view(s), s->C, s->q,
-                                                                                       ML);
+        const cudaError_t e = launch_chained(k_return_map_mlp, s->sms * 2, kMlpWarps * 32, sizeof(MlpWarpSmem), s->stream,
+                                             particle_view(s), s->C, s->q, ML);
+        if (e != cudaSuccess) return e;
         L = PairLog{nullptr, nullptr, 0};
     }
-    k_g2p_plastic<D, S><<<s->sms * kPlasticCtas, kPlasticThreads, 0, s->stream>>>(particle_view(s), s->C, s->gv, s->q, L,
-                                                                                s->status);
-    return cudaGetLastError();
+    return launch_chained(k_g2p_plastic<D, S>, s->sms * kPlasticCtas, kPlasticThreads, 0, s->stream, particle_view(s), s->C,
+                          s->gv, s->q, L, s->status);
 }
 
 template <int D, int S> cudaError_t launch_g2p_split(mpm_solver* s) {
@@ -424,12 +424,10 @@ template <int D, int S, bool G2P> cudaError_t launch_fused(mpm_solver* s) {
     }
     if (s->n == 0) return cudaSuccess;
     if (G2P && !s->direct)
-        k_g2p2g_pipe<D, S><<<s->sms * PipeGeom<D>::CTAS, PipeGeom<D>::THREADS, sizeof(PipeSmem<D>), s->stream>>>(
-            particle_view(s), s->C, s->ti, s->gv, s->acc, s->q, s->status, s->gv_map);
-    else
-        k_g2p2g_direct<D, S, G2P><<<s->direct_grid, FusedGeom<D>::THREADS, windows_smem(D), s->stream>>>(
-            particle_view(s), s->C, s->ti, s->gv, s->acc, s->q, s->status);
-    return cudaGetLastError();
+        return launch_chained(k_g2p2g_pipe<D, S>, s->sms * PipeGeom<D>::CTAS, PipeGeom<D>::THREADS, sizeof(PipeSmem<D>),
+                              s->stream, particle_view(s), s->C, s->ti, s->gv, s->acc, s->q, s->status, s->gv_map);
+    return launch_chained(k_g2p2g_direct<D, S, G2P>, s->direct_grid, FusedGeom<D>::THREADS, windows_smem(D), s->stream,
+                          particle_view(s), s->C, s->ti, s->gv, s->acc, s->q, s->status);
 }
 
 // Queued particles after the G2P part: their return map (learned and/or
@@ -439,9 +437,8 @@ template <int D, int S> cudaError_t launch_queued_fused(mpm_solver* s) {
     if (s->n == 0) return cudaSuccess;
     cudaError_t e = launch_return_map<D, S>(s);
     if (e != cudaSuccess) return e;
-    k_p2g_windows<D, S><<<s->windows_grid, FusedGeom<D>::THREADS, windows_smem(D), s->stream>>>(
-        particle_view(s), s->C, s->ti, s->q, s->acc, s->status);
-    return cudaGetLastError();
+    return launch_chained(k_p2g_windows<D, S>, s->windows_grid, FusedGeom<D>::THREADS, windows_smem(D), s->stream,
+                          particle_view(s), s->C, s->ti, s->q, s->acc, s->status);
 }
 
 // The P2G of the current state when it is not pending yet: the sort first if
@@ -460,10 +457,7 @@ template <int D, int S> cudaError_t fused_prologue(mpm_solver* s) {
 }
 
 template <int D> cudaError_t launch_grid_marked(mpm_solver* s) {
-    k_grid_marked<D, kMLS><<<s->sms * 8, 256, 0, s->stream>>>(s->C, s->ti, s->acc, s->gv, s->status);
-    cudaError_t e = cudaGetLastError();
-    if (e != cudaSuccess) return e;
-    return cudaSuccess;
+    return launch_chained(k_grid_marked<D, kMLS>, s->sms * 8, 256, 0, s->stream, s->C, s->ti, s->acc, s->gv, s->status);
 }
 
 // One fused step: [sort] grid update, fused G2P + next P2G, queued particles.

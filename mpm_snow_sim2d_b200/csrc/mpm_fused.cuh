@@ -633,6 +633,7 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS) k_p2g_windows(Particles
     extern __shared__ __align__(128) unsigned char fused_smem[];
     const int wid = threadIdx.x >> 5;
     float* pay = reinterpret_cast<float*>(fused_smem) + wid * G::PAY;
+    chain_wait();
     const int nw = min(*Q.nwin, Q.win_capacity);
     for (int r = blockIdx.x * G::WARPS + wid; r < nw; r += gridDim.x * G::WARPS)
         queued_window<D, S, false>(P, C, TI, Q.win[r], acc, status, pay);
@@ -909,8 +910,9 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
                    unsigned long long* __restrict__ acc, SlowQueue Q, unsigned* __restrict__ status) {
     using G = FusedGeom<D>;
     extern __shared__ __align__(128) unsigned char fused_smem[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int wid = threadIdx.x >> 5;
     float* pay = reinterpret_cast<float*>(fused_smem) + wid * G::PAY;
+    chain_wait();
     const int nitems = *TI.n_items;
     for (int e = wid * gridDim.x + blockIdx.x; e < nitems; e += G::WARPS * gridDim.x) {
         const int4 item = TI.items[e];  // tile, first slot, slots
@@ -1016,6 +1018,7 @@ __global__ void __launch_bounds__(PipeGeom<D>::THREADS, PipeGeom<D>::CTAS)
     extern __shared__ __align__(128) unsigned char fused_smem[];
     PipeSmem<D>& SM = *reinterpret_cast<PipeSmem<D>*>(fused_smem);
     const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    chain_wait();
     const int nitems = *TI.n_items;
     if (wid == 0) {
         if (lane < R::STAGES) {

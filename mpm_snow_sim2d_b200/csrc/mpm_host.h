@@ -76,6 +76,22 @@ inline void fixed_point_scales(const mpm_params& p, double total_mass, StepConst
     C.v_cap = (float)v_cap;
 }
 
+// Launches a kernel that begins with chain_wait().
+template <typename... P, typename... A>
+cudaError_t launch_chained(void (*kernel)(P...), int grid, int threads, size_t smem, cudaStream_t stream, const A&... args) {
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3((unsigned)threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // The device arrays of a solver or batch, a group in one allocation: a cudaMalloc
 // takes up to 0.5 ms and a cudaFree 0.3, and a solver has about fifty arrays
 // (a solver of 3.8M particles: 230 ms to create and 10 to destroy with an allocation

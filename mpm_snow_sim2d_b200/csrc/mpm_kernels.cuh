@@ -1020,6 +1020,15 @@ __device__ __forceinline__ void g2p_queued_exact(const Particles& P, const StepC
     }
 }
 
+// The kernels of a step follow each other by programmatic dependent launch: a
+// kernel is brought up while the one before it drains, and waits here, before it
+// touches memory, for that one to be complete. Whole steps: 2D, 2.3k particles 19.3 ->
+// 17.0 us; 186k 41.0 -> 37.5; 627k 67 -> 64; 3D, 17.6k 46.0 -> 44.5. Letting the next
+// kernel up from the start of this one (launch_dependents) costs more than it saves:
+// its CTAs hold a carve-out of shared memory that this one's are then short of
+// (3D, 17.6k: 50).
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Bound: instruction issue and latency of the Jacobi sweeps (div, sqrt). Six CTAs of
 // 128 threads per SM (80 registers) hide more of it than two of 256 at 128
 // registers: 1.4M particles queued of 3.8M, 266 us, now 232; four, five, seven and
@@ -1028,6 +1037,7 @@ constexpr int kPlasticThreads = 128, kPlasticCtas = 6;
 template <int D, int S = 4>
 __global__ void __launch_bounds__(kPlasticThreads, kPlasticCtas) k_g2p_plastic(Particles P, StepConsts C, const float4* __restrict__ gv,
                                                      SlowQueue Q, PairLog L, unsigned* __restrict__ status) {
+    chain_wait();
     const int m = *Q.count;
     for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < m; e += gridDim.x * blockDim.x)
         if (Q.list[e] != kQueueDone) g2p_queued_exact<D, S>(P, C, gv, Q, e, status, L);

@@ -353,6 +353,7 @@ __global__ void __launch_bounds__(kMlpWarps * 32) k_return_map_mlp(Particles P, 
                                                                    MlpParams ML) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     MlpWarpSmem& S = *reinterpret_cast<MlpWarpSmem*>(smem_raw);
+    chain_wait();
     const int m = *Q.count;
     // CTAs past the queue's end leave before staging the weights (the grid is
     // sized for the largest queue; most steps queue far fewer particles)

@@ -406,6 +406,7 @@ template <int D, int FORM>
 __global__ void __launch_bounds__(256) k_grid_marked(StepConsts C, TileInfo TI, unsigned long long* __restrict__ acc,
                                                      float4* __restrict__ gv, unsigned* __restrict__ status) {
     using G = TileGeom<D>;
+    chain_wait();
     const int nb = *TI.n_marked;
     const long long total = (long long)nb * G::BN;
     for (long long w = (long long)blockIdx.x * blockDim.x + threadIdx.x; w < total;

@@ -118,18 +118,19 @@ cudaError_t enqueue_sort(mpm_batch* b, bool pending) {
     if (b->N == 0) return cudaSuccess;
     const Particles P = particles(b);
     const int threads = 256;
-    const unsigned blocks = (unsigned)((b->N + threads - 1) / threads);
-    k_sort_count<2, 4, ManyScenes><<<blocks, threads, 0, b->stream>>>(P, b->many, b->ti);
+    const int blocks = (int)((b->N + threads - 1) / threads);
     const int scan_blocks = (b->ti.n_tiles + kScanTiles - 1) / kScanTiles;
-    k_sort_block_sums<<<scan_blocks, kScanTiles, 0, b->stream>>>(b->ti);
-    k_sort_scan<<<scan_blocks, kScanTiles, 0, b->stream>>>(b->ti);
-    k_sort_bucket<<<blocks, threads, 0, b->stream>>>((int)b->N, b->ti);
+    cudaError_t e = launch_chained(k_sort_count<2, 4, ManyScenes>, blocks, threads, 0, b->stream, P, b->many, b->ti);
+    if (e == cudaSuccess) e = launch_chained(k_sort_block_sums, scan_blocks, kScanTiles, 0, b->stream, b->ti);
+    if (e == cudaSuccess) e = launch_chained(k_sort_scan, scan_blocks, kScanTiles, 0, b->stream, b->ti);
+    if (e == cudaSuccess) e = launch_chained(k_sort_bucket, blocks, threads, 0, b->stream, (int)b->N, b->ti);
+    if (e != cudaSuccess) return e;
     const BatchBuffers& t = b->buf[b->parity ^ 1];
     const SortBuffers dst{t.x, pending ? nullptr : t.v, pending ? nullptr : t.B, t.Fe, t.Jp, nullptr, t.mass, t.vol, t.id};
-    k_tile_sort<2, 4, ManyScenes><<<b->sms * SortGeom<2>::CTAS_PER_SM, 256, 0, b->stream>>>(
-        P, b->buf[b->parity].id, dst, b->many, b->ti);
+    e = launch_chained(k_tile_sort<2, 4, ManyScenes>, b->sms * SortGeom<2>::CTAS_PER_SM, 256, 0, b->stream, P,
+                       b->buf[b->parity].id, dst, b->many, b->ti);
     b->parity ^= 1;
-    return cudaGetLastError();
+    return e;
 }
 
 cudaError_t enqueue_step(mpm_batch* b) {

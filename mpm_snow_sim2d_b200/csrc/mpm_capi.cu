@@ -239,11 +239,12 @@ template <int D, int S> cudaError_t launch_sort(mpm_solver* s) {
     if (s->n == 0) { s->needs_sort = false; s->next_sort = s->step + s->cur_K; return cudaSuccess; }
     const int threads = 256, blocks = (s->n + threads - 1) / threads;
     const OneScene scene{{{s->C.W, s->C.H, s->C.Dp}, {s->ti.tiles[0], s->ti.tiles[1], s->ti.tiles[2]}, 0}};
-    k_sort_count<D, S, OneScene><<<blocks, threads, 0, s->stream>>>(particle_view(s), scene, s->ti);
     const int scan_blocks = (s->ti.n_tiles + kScanTiles - 1) / kScanTiles;
-    k_sort_block_sums<<<scan_blocks, kScanTiles, 0, s->stream>>>(s->ti);
-    k_sort_scan<<<scan_blocks, kScanTiles, 0, s->stream>>>(s->ti);
-    k_sort_bucket<<<blocks, threads, 0, s->stream>>>(s->n, s->ti);
+    cudaError_t e = launch_chained(k_sort_count<D, S, OneScene>, blocks, threads, 0, s->stream, particle_view(s), scene, s->ti);
+    if (e == cudaSuccess) e = launch_chained(k_sort_block_sums, scan_blocks, kScanTiles, 0, s->stream, s->ti);
+    if (e == cudaSuccess) e = launch_chained(k_sort_scan, scan_blocks, kScanTiles, 0, s->stream, s->ti);
+    if (e == cudaSuccess) e = launch_chained(k_sort_bucket, blocks, threads, 0, s->stream, s->n, s->ti);
+    if (e != cudaSuccess) return e;
     SortBuffers dst = s->alt;
     if (s->fused) {
         dst.A = nullptr;  // the fused path keeps A only within a step
@@ -251,9 +252,8 @@ template <int D, int S> cudaError_t launch_sort(mpm_solver* s) {
         // bytes a particle stay (sort by cell of 1.65M: 150 -> 85 us, of 3.8M: 300 -> 164)
         if (s->acc_pending) dst.v = dst.B = nullptr;
     }
-    k_tile_sort<D, S, OneScene><<<s->sms * SortGeom<D>::CTAS_PER_SM, 256, 0, s->stream>>>(particle_view(s), s->id, dst,
-                                                                                         scene, s->ti);
-    cudaError_t e = cudaGetLastError();
+    e = launch_chained(k_tile_sort<D, S, OneScene>, s->sms * SortGeom<D>::CTAS_PER_SM, 256, 0, s->stream, particle_view(s),
+                       s->id, dst, scene, s->ti);
     if (e != cudaSuccess) return e;
     swap_buffers(s);
     s->needs_sort = false;

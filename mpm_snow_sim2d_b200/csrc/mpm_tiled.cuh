@@ -105,6 +105,7 @@ static __global__ void __launch_bounds__(256) k_max_abs(const float* __restrict_
 template <int D, int S, typename SC>
 __global__ void __launch_bounds__(256) k_sort_count(Particles P, SC scenes, TileInfo TI) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    chain_wait();
     if (i >= P.n) return;
     const int t = tile_of_slot<D, S>(P, scenes.of_slot(i), i);
     TI.key[i] = t;
@@ -161,6 +162,7 @@ __device__ __forceinline__ void block_scan3(int* v, int* total) {
 
 static __global__ void __launch_bounds__(kScanTiles) k_sort_block_sums(TileInfo TI) {
     const int t = blockIdx.x * kScanTiles + threadIdx.x;
+    chain_wait();
     const int c = t < TI.n_tiles ? TI.tile_count[t] : 0;
     int v[3] = {c, c > 0, tile_items(TI, c)}, total[3];
     block_scan3(v, total);
@@ -172,6 +174,7 @@ static __global__ void __launch_bounds__(kScanTiles) k_sort_scan(TileInfo TI) {
     const int t = blockIdx.x * kScanTiles + threadIdx.x;
     if (threadIdx.x < 3) s_before[threadIdx.x] = 0;
     __syncthreads();
+    chain_wait();
     int b[3] = {0, 0, 0};
     for (int k = threadIdx.x; k < (int)blockIdx.x; k += kScanTiles) {
         const int4 s = TI.scan[k];
@@ -210,6 +213,7 @@ struct SortBuffers {
 // Bucket the source slots by tile (order inside a tile is fixed by k_tile_sort).
 static __global__ void __launch_bounds__(256) k_sort_bucket(int n, TileInfo TI) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    chain_wait();
     if (i >= n) return;
     const int t = TI.key[i];
     const unsigned act = __activemask();
@@ -273,6 +277,7 @@ __global__ void __launch_bounds__(256) k_tile_sort(Particles P, const int* __res
     __shared__ int s_cnt[kTileCells], s_off[kTileCells];
     __shared__ int s_big;
     const long long n = P.n;
+    chain_wait();
     const int ntl = *TI.n_tile_list;
     for (int e = blockIdx.x; e < ntl; e += gridDim.x) {
         const int t = TI.tile_list[e];

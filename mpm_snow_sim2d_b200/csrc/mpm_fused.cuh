@@ -86,54 +86,75 @@ __device__ __forceinline__ void gather_nodes(const StepConsts& C, const float4* 
         for (int o = 0; o < S; ++o) wd[k][o] = wk[k][o] * off[k][o];
     float vc[D];
     bool wall = false;
-#pragma unroll
-    for (int r = 0; r < D; ++r) { nv[r] = 0.f; vc[r] = 0.f; }
-#pragma unroll
-    for (int k = 0; k < D * D; ++k) nB[k] = 0.f;
+    // x and y components in packed FP32, z in scalar (3D). Whole steps: 1.65M particles
+    // 324 -> 309 us, 3.8M 785 -> 766, quadratic 1.65M 271 -> 265, 2D 627k 62.0 -> 61.3
+    const float2 zero = make_float2(0.f, 0.f);
+    float2 v2 = zero, b2[3] = {zero, zero, zero}, c2 = zero;  // v; B's columns; 2D: vc
+    float v1 = 0.f, b1[3] = {0.f, 0.f, 0.f};
 #pragma unroll 1
     for (int a = 0; a < S; ++a) {
-        float Q[D], Qy[D], Qz[D], Qc[D];
-#pragma unroll
-        for (int r = 0; r < D; ++r) { Q[r] = 0.f; Qy[r] = 0.f; Qz[r] = 0.f; Qc[r] = 0.f; }
+        float2 q2 = zero, qy2 = zero, qz2 = zero, qc2 = zero;
+        float q1 = 0.f, qy1 = 0.f, qz1 = 0.f;
 #pragma unroll
         for (int b = 0; b < S; ++b) {
+            const float y1 = wk[1][b], yd1 = wd[1][b];
+            const float2 y = make_float2(y1, y1), yd = make_float2(yd1, yd1);
             if constexpr (D == 3) {
-                float Pv[3] = {0.f, 0.f, 0.f}, Pd[3] = {0.f, 0.f, 0.f};
+                float2 p2 = zero, d2 = zero;
+                float p1 = 0.f, d1 = 0.f;
 #pragma unroll
                 for (int c = 0; c < S; ++c) {
                     const I cid = c0 + a + b * sy + c * sz;
                     const float4 g = SMEM ? nodes[cid] : __ldg(&nodes[cid]);
                     wall = wall || g.w != 0.f;
                     const float z = wk[2][c], zd = wd[2][c];
-                    Pv[0] += z * g.x; Pv[1] += z * g.y; Pv[2] += z * g.z;
-                    Pd[0] += zd * g.x; Pd[1] += zd * g.y; Pd[2] += zd * g.z;
+                    p2 = __ffma2_rn(make_float2(z, z), make_float2(g.x, g.y), p2);
+                    d2 = __ffma2_rn(make_float2(zd, zd), make_float2(g.x, g.y), d2);
+                    p1 += z * g.z;
+                    d1 += zd * g.z;
                 }
-                const float y = wk[1][b], yd = wd[1][b];
-#pragma unroll
-                for (int r = 0; r < 3; ++r) {
-                    Q[r] += y * Pv[r];
-                    Qy[r] += yd * Pv[r];
-                    Qz[r] += y * Pd[r];
-                }
+                q2 = __ffma2_rn(y, p2, q2);
+                qy2 = __ffma2_rn(yd, p2, qy2);
+                qz2 = __ffma2_rn(y, d2, qz2);
+                q1 += y1 * p1;
+                qy1 += yd1 * p1;
+                qz1 += y1 * d1;
             } else {
                 const I cid = c0 + a + b * sy;
                 const float4 g = SMEM ? nodes[cid] : __ldg(&nodes[cid]);
-                const float y = wk[1][b], yd = wd[1][b];
-                Q[0] += y * g.x; Q[1] += y * g.y;
-                Qy[0] += yd * g.x; Qy[1] += yd * g.y;
-                Qc[0] += y * g.z; Qc[1] += y * g.w;
+                q2 = __ffma2_rn(y, make_float2(g.x, g.y), q2);
+                qy2 = __ffma2_rn(yd, make_float2(g.x, g.y), qy2);
+                qc2 = __ffma2_rn(y, make_float2(g.z, g.w), qc2);
             }
         }
-        const float x = pick<S>(wk[0], a);
-        const float xd = pick<S>(wd[0], a);
-#pragma unroll
-        for (int r = 0; r < D; ++r) {
-            nv[r] += x * Q[r];
-            nB[r * D + 0] += xd * Q[r];
-            nB[r * D + 1] += x * Qy[r];
-            if (D == 3) nB[r * D + 2] += x * Qz[r];
-            else vc[r] += x * Qc[r];
+        const float x1 = pick<S>(wk[0], a), xd1 = pick<S>(wd[0], a);
+        const float2 x = make_float2(x1, x1), xd = make_float2(xd1, xd1);
+        v2 = __ffma2_rn(x, q2, v2);
+        b2[0] = __ffma2_rn(xd, q2, b2[0]);
+        b2[1] = __ffma2_rn(x, qy2, b2[1]);
+        if constexpr (D == 3) {
+            b2[2] = __ffma2_rn(x, qz2, b2[2]);
+            v1 += x1 * q1;
+            b1[0] += xd1 * q1;
+            b1[1] += x1 * qy1;
+            b1[2] += x1 * qz1;
+        } else {
+            c2 = __ffma2_rn(x, qc2, c2);
         }
+    }
+    nv[0] = v2.x;
+    nv[1] = v2.y;
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+        nB[k] = b2[k].x;
+        nB[D + k] = b2[k].y;
+        if (D == 3) nB[2 * D + k] = b1[k];
+    }
+    vc[0] = c2.x;
+    vc[1] = c2.y;
+    if constexpr (D == 3) {
+        nv[2] = v1;
+        vc[2] = 0.f;
     }
     if constexpr (D == 3) {
         if (!wall) {

@@ -122,3 +122,19 @@ def test_batch_scenes_with_device_sampling(gpu_lib):
     with Batch(pois) as b:
         b.step(50)
         assert all(b.status(k) & 1 == 0 for k in range(len(pois)))
+
+
+# Cell counts at which groups of eight lanes, blocks of cells and the compaction's
+# blocks begin and end: a few cells, one more than a multiple, one cell wide shapes,
+# shapes that overlap, one round.
+@pytest.mark.parametrize("dim,half,md,rounds", [(2, (0.2, 0.2), 1.0, 1), (2, (0.4, 33.0), 1.0, 4), (2, (11.3, 11.3), 0.5, 3),
+                                                (3, (0.3, 0.3, 0.3), 1.0, 2), (3, (0.5, 0.5, 21.0), 1.0, 3),
+                                                (3, (6.1, 5.3, 4.7), 1.0, 30)])
+def test_sampler_at_small_and_ragged_grids(gpu_lib, dim, half, md, rounds):
+    from mpm_snow_sim2d_b200.sampling import sample_shapes
+    c = tuple([0.37] * dim)
+    shapes = [_shape(1, c, h=half + (0.0,) * (3 - dim)), _shape(0, c, max(half) / 3)]
+    got, owner = sample_shapes(dim, shapes, md, 99, rounds)
+    ref, ref_owner = sample_ref.sample_shapes(dim, shapes, md, 99, rounds)
+    assert got.shape == ref.shape
+    assert np.array_equal(got.view(np.uint32), ref.view(np.uint32)) and np.array_equal(owner, ref_owner)

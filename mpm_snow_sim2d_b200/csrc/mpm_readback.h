@@ -87,7 +87,7 @@ public:
         for (int p = 0; p < parts; s += bytes[p], ++p) {
             if (!dst[p] || !bytes[p]) continue;
             std::unique_lock<std::mutex> lock(use_, std::defer_lock);
-            const bool ring = bytes[p] >= kLarge && lock.try_lock() && ready();
+            const bool ring = bytes[p] >= kLarge && pageable(dst[p]) && lock.try_lock() && ready();
             const cudaError_t e = ring ? pipe(stream, s, static_cast<char*>(dst[p]), bytes[p])
                                        : direct(stream, s, dst + p, bytes + p, 1);
             if (e != cudaSuccess) return e;
@@ -103,6 +103,16 @@ private:
     cudaEvent_t ev_[kChunks] = {};
     int device_ = -1;  // of the events
 
+    // Pinned memory of the caller's is filled by the copy engine alone (164 MB: 3 ms
+    // against 8 through the ring).
+    static bool pageable(const void* p) {
+        cudaPointerAttributes a{};
+        if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+            cudaGetLastError();
+            return true;
+        }
+        return a.type == cudaMemoryTypeUnregistered;
+    }
     static bool pin(char*& p, size_t bytes) {
         if (p || cudaHostAlloc(reinterpret_cast<void**>(&p), bytes, cudaHostAllocPortable) == cudaSuccess) return true;
         cudaGetLastError();

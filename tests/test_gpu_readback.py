@@ -68,3 +68,14 @@ def test_readers_on_several_threads(gpu_lib):
     for s, _ in pairs:
         s.close()
     assert not bad, bad
+
+
+@pytest.mark.parametrize("n", [1000, 1048577, 2359301])
+def test_read_into_pinned_memory(gpu_lib, n):
+    import ctypes as C
+    import torch
+    s, want = _solver(2, n, n)
+    with s:
+        out = torch.full((n, 2), -1.0, dtype=torch.float32, pin_memory=True)
+        st = gpu_lib.mpm_get_positions(s._h, C.cast(out.data_ptr(), C.POINTER(C.c_float)), out.numel())
+        assert st == 0 and np.array_equal(out.numpy(), want["position"])

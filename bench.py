@@ -47,7 +47,7 @@ sys.path.insert(0, str(ROOT))
 
 METRIC = "particle-updates/s (P2G+grid+G2P), plain vs MLP-plasticity, 1 B200, % HBM peak"
 UNIT = "particle-updates/s"
-STAGE_KERNEL = {"p2g": "k_p2g_warp", "g2p": "k_g2p_gather", "g2p2g": "k_g2p2g", "grid_update": "k_grid_marked",
+STAGE_KERNEL = {"p2g": "k_p2g_warp", "g2p": "k_g2p_gather", "g2p2g": "k_g2p2g_pipe", "grid_update": "k_grid_marked",
                 "return_map": "k_g2p_plastic"}
 
 
@@ -283,8 +283,7 @@ def mlp_vs_plain(args, torch, stream):
 
 def batched_scenes(args, torch):
     """The batched workload: 256 independent 2D scenes (grid sides 64-256,
-    2k-64k particles each) advanced `batch_steps` steps in one call after the
-    autotuner picked the launch configuration. Scene-step latency from the
+    2k-64k particles each) advanced `batch_steps` steps in one call. Scene-step latency from the
     device timestamps each scene records at the end of each of its steps;
     batch-step latency from CUDA events around single-step calls. For
     comparison, the single-scene solver is timed on a sample of the same

@@ -469,8 +469,17 @@ __global__ void __launch_bounds__(kMlpWarps * 32) k_mlp_forward(const float* __r
 // Training step: forward, MSE loss, backward on tiles of kMlpTrainRows samples
 // (8 warps x 16 rows); a CTA takes tiles until none are left and writes its
 // weight gradients and loss once, to its own row of `part` (summed by
-// k_mlp_adam / k_mlp_grad_sum in a fixed order). Samples: row = pair (seed 0 and
+// k_mlp_adam / k_mlp_grad_sum in FP64). Samples: row = pair (seed 0 and
 // `in_order`) or a hash of (seed, global row) modulo n_pairs.
+//
+// Every gradient is a sum over blocks of kMlpSumRows rows: a block's weight
+// gradients are one chain of mma, its bias gradients are added row by row, and
+// blocks are added to each other in plain FP32. A block's part thus rounds alike
+// however the rows are split over tiles and CTAs: the same 64-row parts that
+// training has always added up, so a run follows earlier ones as closely as they
+// follow each other (AdamW and the bf16 copy of the weights amplify the last bits
+// of a gradient: 32 steps at a batch of 16384 apart by 1.6e-5 in the median, when
+// the same parts were added by atomics in two orders).
 //
 // A warp keeps its 16 rows in registers through the layers: the m16n8
 // accumulators of one layer, after bias + GELU, are the m16k16 A fragments of the
@@ -481,8 +490,10 @@ __global__ void __launch_bounds__(kMlpWarps * 32) k_mlp_forward(const float* __r
 // Bound: latency (8 warps per SM, one tile per CTA at the usual batch of 16384,
 // about 600 dependent mma and tanh a warp). The former kernel (64-row tiles,
 // every fragment from 2-byte shared loads, an fp32 atomic per weight and CTA)
-// took 107 us at that batch, this one 14.4 us.
+// took 107 us at that batch, this one about 17 us, 2.3 of them for the parts of 64
+// rows and their bias sums (16 steps with their updates: 420 us).
 constexpr int kMlpTrainRows = 128;
+constexpr int kMlpSumRows = 64;
 constexpr int kMlpTrainCtas = 148;              // most CTAs (rows of `part`)
 constexpr int kMlpPart = MlpOff::total + 16;    // floats per row: gradients, then the loss
 
@@ -494,8 +505,9 @@ struct MlpTrainSmem {
     __nv_bfloat16 h[3][kMlpTrainRows * kMwHid];
     __nv_bfloat16 dy[kMlpTrainRows * kMwHid];    // gradient wrt the current layer's pre-activation
     __nv_bfloat16 dy4[kMlpTrainRows * kMwIn];
-    float tgt[kMlpTrainRows * kMlpOutPad];
-    float red[8][kMlpOutPad + 1];              // per warp: output bias gradients, loss
+    float tgt[kMlpTrainRows * kMlpOutPad];      // targets, then gradient wrt the output
+    float red[8];                               // per warp: loss
+    float db[kMlpTrainRows / kMlpSumRows][3 * kMlpHid + kMlpOutPad];
 };
 
 __device__ __forceinline__ unsigned hash_u32(unsigned x) {
@@ -549,31 +561,42 @@ __device__ __forceinline__ void mlp_train_back(float (*acc)[4], float (*gp)[4], 
     }
 }
 
-// The warp's share of dW[n][k] += sum_r dY[r][n] X[r][k] over the tile's rows:
-// output rows n0 .. n0 + 15, NT column tiles of 8 from k0 on; with `ones` also
-// db[n] = sum_r dY[r][n] (the product with a column of ones).
+// The warp's share of dW[n][k] += sum_r dY[r][n] X[r][k] over the tile's blocks of
+// rows: output rows n0 .. n0 + 15, NT column tiles of 8 from k0 on.
 template <int NT>
 __device__ __forceinline__ void mlp_train_dw(const __nv_bfloat16* dY, int ldd, const __nv_bfloat16* X, int ldx, int n0,
-                                             int k0, float (*dw)[4], bool ones, float* db) {
+                                             int k0, float (*dw)[4]) {
     const int lane = threadIdx.x & 31, mi = lane >> 3, row = lane & 7;
 #pragma unroll
-    for (int r0 = 0; r0 < kMlpTrainRows; r0 += 16) {
-        uint32_t a[4];
-        ldmatrix_x4_trans(a, dY + (r0 + (mi >> 1) * 8 + row) * ldd + n0 + (mi & 1) * 8);
+    for (int blk = 0; blk < kMlpTrainRows; blk += kMlpSumRows) {
+        float s[NT][4] = {};
 #pragma unroll
-        for (int j = 0; j < NT; j += 2) {
-            uint32_t b[4];
-            // matrices: (r0, k), (r0 + 8, k), (r0, k + 8), (r0 + 8, k + 8); with one tile the second pair repeats the first
-            const int kc = k0 + j * 8 + (NT > 1 ? (mi >> 1) * 8 : 0);
-            ldmatrix_x4_trans(b, X + (r0 + (mi & 1) * 8 + row) * ldx + kc);
-            mma_bf16(dw[j], a, b);
-            if constexpr (NT > 1) mma_bf16(dw[j + 1], a, b + 2);
+        for (int r0 = blk; r0 < blk + kMlpSumRows; r0 += 16) {
+            uint32_t a[4];
+            ldmatrix_x4_trans(a, dY + (r0 + (mi >> 1) * 8 + row) * ldd + n0 + (mi & 1) * 8);
+#pragma unroll
+            for (int j = 0; j < NT; j += 2) {
+                uint32_t b[4];
+                // matrices: (r0, k), (r0 + 8, k), (r0, k + 8), (r0 + 8, k + 8); with one tile the second pair repeats the first
+                const int kc = k0 + j * 8 + (NT > 1 ? (mi >> 1) * 8 : 0);
+                ldmatrix_x4_trans(b, X + (r0 + (mi & 1) * 8 + row) * ldx + kc);
+                mma_bf16(s[j], a, b);
+                if constexpr (NT > 1) mma_bf16(s[j + 1], a, b + 2);
+            }
         }
-        if (ones) {
-            const uint32_t one[2] = {0x3f803f80u, 0x3f803f80u};  // bf16 1.0 pairs
-            mma_bf16(db, a, one);
-        }
+#pragma unroll
+        for (int j = 0; j < NT; ++j)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) dw[j][q] += s[j][q];
     }
+}
+
+// db[n] of one block of rows, by one thread: column n of dY (row stride ld), row by row.
+template <typename T> __device__ __forceinline__ float mlp_train_db(const T* dY, int ld) {
+    float s = 0.f;
+#pragma unroll 32
+    for (int r = 0; r < kMlpSumRows; ++r) s += float(dY[r * ld]);
+    return s;
 }
 
 // The transpose of a row-major [rows][cols] matrix.
@@ -605,10 +628,15 @@ __global__ void __launch_bounds__(256, 1) k_mlp_train(const float* __restrict__ 
     // the warp's share of dW: rows n0.. of W2 and W3 and half of their columns,
     // one tile each of W1 and W4
     const int n0 = (warp & 3) * 16, kh = (warp >> 2) * 32;
-    float dw2[4][4] = {}, dw3[4][4] = {}, dw1[1][4] = {}, dw4[1][4] = {}, db1[4] = {}, db2[4] = {}, db3[4] = {};
-    float db4[4] = {0.f, 0.f, 0.f, 0.f}, lsum = 0.f;  // db4: columns 2t, 2t + 1 of both tiles
+    float dw2[4][4] = {}, dw3[4][4] = {}, dw1[1][4] = {}, dw4[1][4] = {}, lsum = 0.f;
     const int r0 = warp * 16;
-    const float inv = 2.f / float(n_rows);
+    // bias gradients: one thread per column and block of rows; warps 0-3 those of the
+    // hidden layers, warp 4 the output's
+    static_assert(kMlpTrainRows / kMlpSumRows == 2 && kMlpHid == 64 && kMlpOutPad == 16, "threads of the bias gradients");
+    float db1 = 0.f, db2 = 0.f, db3 = 0.f, db4 = 0.f;
+    const bool sums_h = tid < 2 * kMlpHid, sums_o = warp == 4;
+    const int hid = (tid >> 6 & 1) * kMlpSumRows * kMwHid + (tid & 63);
+    const int outp = (tid >> 4 & 1) * kMlpSumRows * kMlpOutPad + (tid & 15);
     for (long long row0 = (long long)blockIdx.x * kMlpTrainRows; row0 < n_rows; row0 += (long long)gridDim.x * kMlpTrainRows) {
         __syncthreads();  // the last tile's fragments have been read (first tile: nothing)
         if (tid < kMlpTrainRows) {
@@ -663,8 +691,8 @@ __global__ void __launch_bounds__(256, 1) k_mlp_train(const float* __restrict__ 
                 const bool valid = row0 + r < n_rows && cc < kMlpOut;
                 const float diff = valid ? o[j][q] + S.b4[cc] - S.tgt[r * kMlpOutPad + cc] : 0.f;
                 lsum += diff * diff;
-                o[j][q] = diff * inv;
-                db4[2 * j + (q & 1)] += o[j][q];
+                o[j][q] = 2.f * diff / float(n_rows);
+                S.tgt[r * kMlpOutPad + cc] = o[j][q];
             }
             const uint32_t lo = pack_f2_bf16(o[j][0], o[j][1]), hi = pack_f2_bf16(o[j][2], o[j][3]);
             a[0][2 * j] = lo;
@@ -675,18 +703,22 @@ __global__ void __launch_bounds__(256, 1) k_mlp_train(const float* __restrict__ 
         mlp_warp_layer<1, kMlpHid / 8>(a, S.W4t, kMwIn, acc);  // dX = dY4 W4
         mlp_train_back(acc, gp3, a, S.dy, r0);
         __syncthreads();
-        mlp_train_dw<1>(S.dy4, kMwIn, S.h[2], kMwHid, 0, warp * 8, dw4, false, nullptr);
-        mlp_train_dw<4>(S.dy, kMwHid, S.h[1], kMwHid, n0, kh, dw3, warp < 4, db3);
+        mlp_train_dw<1>(S.dy4, kMwIn, S.h[2], kMwHid, 0, warp * 8, dw4);
+        mlp_train_dw<4>(S.dy, kMwHid, S.h[1], kMwHid, n0, kh, dw3);
+        if (sums_h) db3 += mlp_train_db(S.dy + hid, kMwHid);
+        if (sums_o) db4 += mlp_train_db(S.tgt + outp, kMlpOutPad);
         mlp_warp_layer<kMlpHid / 16, kMlpHid / 8>(a, S.W3t, kMwHid, acc);
         __syncthreads();  // dY3 has been read
         mlp_train_back(acc, gp2, a, S.dy, r0);
         __syncthreads();
-        mlp_train_dw<4>(S.dy, kMwHid, S.h[0], kMwHid, n0, kh, dw2, warp < 4, db2);
+        mlp_train_dw<4>(S.dy, kMwHid, S.h[0], kMwHid, n0, kh, dw2);
+        if (sums_h) db2 += mlp_train_db(S.dy + hid, kMwHid);
         mlp_warp_layer<kMlpHid / 16, kMlpHid / 8>(a, S.W2t, kMwHid, acc);
         __syncthreads();
         mlp_train_back(acc, gp1, a, S.dy, r0);
         __syncthreads();
-        mlp_train_dw<1>(S.dy, kMwHid, S.x0, kMwIn, n0, (warp >> 2) * 8, dw1, warp < 4, db1);
+        mlp_train_dw<1>(S.dy, kMwHid, S.x0, kMwIn, n0, (warp >> 2) * 8, dw1);
+        if (sums_h) db1 += mlp_train_db(S.dy + hid, kMwHid);
     }
     // this CTA's row of `part` (every entry written)
     float* P = part + (long long)blockIdx.x * kMlpPart;
@@ -701,48 +733,47 @@ __global__ void __launch_bounds__(256, 1) k_mlp_train(const float* __restrict__ 
     }
     put(P + MlpOff::W1 + n0 * kMlpInPad + (warp >> 2) * 8, kMlpInPad, dw1[0]);
     put(P + MlpOff::W4 + warp * 8, kMlpHid, dw4[0]);
-    if (warp < 4 && t == 0) {  // every column of the ones product holds db
-        P[MlpOff::b1 + n0 + g] = db1[0]; P[MlpOff::b1 + n0 + g + 8] = db1[2];
-        P[MlpOff::b2 + n0 + g] = db2[0]; P[MlpOff::b2 + n0 + g + 8] = db2[2];
-        P[MlpOff::b3 + n0 + g] = db3[0]; P[MlpOff::b3 + n0 + g + 8] = db3[2];
-    }
-#pragma unroll
-    for (int m = 4; m < 32; m <<= 1)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) db4[q] += __shfl_xor_sync(0xffffffffu, db4[q], m);
 #pragma unroll
     for (int m = 1; m < 32; m <<= 1) lsum += __shfl_xor_sync(0xffffffffu, lsum, m);
-    if (g == 0)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) S.red[warp][(q >> 1) * 8 + 2 * t + (q & 1)] = db4[q];
-    if (lane == 0) S.red[warp][kMlpOutPad] = lsum;
+    if (lane == 0) S.red[warp] = lsum;
+    if (sums_h) {
+        float* d = S.db[tid >> 6] + (tid & 63);
+        d[0] = db1;
+        d[kMlpHid] = db2;
+        d[2 * kMlpHid] = db3;
+    }
+    if (sums_o) S.db[tid >> 4 & 1][3 * kMlpHid + (tid & 15)] = db4;
     __syncthreads();
-    if (tid <= kMlpOutPad) {
+    if (tid < 3 * kMlpHid + kMlpOutPad) {
+        const int l = tid >> 6;  // layer: 0-2 hidden, 3 output
+        P[(l == 0 ? MlpOff::b1 : l == 1 ? MlpOff::b2 : l == 2 ? MlpOff::b3 : MlpOff::b4) + (tid & 63)] = S.db[0][tid] + S.db[1][tid];
+    }
+    if (tid == 0) {
         float s = 0.f;
-        for (int w = 0; w < 8; ++w) s += S.red[w][tid];
-        P[tid < kMlpOutPad ? MlpOff::b4 + tid : MlpOff::total] = s;
+        for (int w = 0; w < 8; ++w) s += S.red[w];
+        P[MlpOff::total] = s;
     }
 }
 
-// Sum of entry i over the CTAs' rows of `part`, by the four threads q = 0..3
-// of a quad group 64 threads apart in the block: rows q, q + 4, ... each, then
-// the four in order. `s` holds 256 floats.
-__device__ __forceinline__ float mlp_part_sum(const float* __restrict__ part, int ctas, int i, float* s) {
+// Sum of entry i over the CTAs' rows of `part` in FP64, by the four threads q =
+// 0..3 of a quad group 64 threads apart in the block: rows q, q + 4, ... each, then
+// the four. `s` holds 256 doubles.
+__device__ __forceinline__ float mlp_part_sum(const float* __restrict__ part, int ctas, int i, double* s) {
     const int q = threadIdx.x >> 6;
-    float v = 0.f;
+    double v = 0.0;
     if (i < kMlpPart) {
 #pragma unroll 8
         for (int c = q; c < ctas; c += 4) v += part[(long long)c * kMlpPart + i];
     }
     s[threadIdx.x] = v;
     __syncthreads();
-    return q == 0 ? ((v + s[threadIdx.x + 64]) + s[threadIdx.x + 128]) + s[threadIdx.x + 192] : 0.f;
+    return q == 0 ? float(((v + s[threadIdx.x + 64]) + s[threadIdx.x + 128]) + s[threadIdx.x + 192]) : 0.f;
 }
 
 // The summed gradient (and loss) of a training launch, without an update.
 __global__ void __launch_bounds__(256) k_mlp_grad_sum(const float* __restrict__ part, int ctas, float* __restrict__ grad,
                                                       float* __restrict__ loss) {
-    __shared__ float s[256];
+    __shared__ double s[256];
     const int i = blockIdx.x * 64 + (threadIdx.x & 63);
     const float v = mlp_part_sum(part, ctas, i, s);
     if (threadIdx.x >= 64) return;
@@ -758,7 +789,7 @@ __global__ void __launch_bounds__(256) k_mlp_adam(float* __restrict__ w, __nv_bf
                                                   const float* __restrict__ part, int ctas, float* __restrict__ m1,
                                                   float* __restrict__ m2, float* __restrict__ loss, float lr, float beta1,
                                                   float beta2, float eps, float wd, float bc1, float bc2) {
-    __shared__ float s[256];
+    __shared__ double s[256];
     const int i = blockIdx.x * 64 + (threadIdx.x & 63);
     const float gr = mlp_part_sum(part, ctas, i, s);
     if (threadIdx.x >= 64) return;

@@ -1,0 +1,44 @@
+"""How the training kernel adds up a gradient: parts of 64 rows, each rounded alike wherever it falls in the batch,
+added in FP32 within a CTA and in FP64 between CTAs. Parts come from gradients of 64 rows alone: with all counts
+powers of two, the factor 1 / rows only moves the exponent, so that every rounding is the same."""
+import numpy as np
+import pytest
+
+from test_gpu_mlp import synthetic_pairs
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def net(gpu_lib):
+    from mpm_snow_sim2d_b200 import mlp
+    pairs = synthetic_pairs(4096, seed=9)
+    m = mlp.Mlp(seed=21)
+    m.set_normalization(*mlp.normalization(pairs))
+    return m, pairs
+
+
+@pytest.mark.parametrize("at", [0, 128, 1000])
+def test_two_parts_bitwise(net, at):
+    """128 rows: one tile of one CTA, its two parts added once."""
+    m, pairs = net
+    rows = pairs[at:at + 128]
+    whole, _ = m.gradient(rows)
+    a, b = (m.gradient(rows[k:k + 64])[0] * np.float32(0.5) for k in (0, 64))
+    assert np.array_equal(whole, a + b)
+
+
+@pytest.mark.parametrize("tiles", [2, 128, 256])
+def test_sum_over_ctas(net, tiles):
+    """One tile a CTA, and two (256 tiles are more than there are CTAs): at most three FP32 additions of parts in a
+    CTA and one rounding of the FP64 total."""
+    m, pairs = net
+    rows = pairs[np.random.default_rng(tiles).integers(0, len(pairs), tiles * 128)]
+    whole, loss = m.gradient(rows)
+    parts = [m.gradient(rows[k:k + 64]) for k in range(0, len(rows), 64)]
+    g = np.stack([p[0] for p in parts]).astype(np.float64) / len(parts)
+    bound = 2.0 ** -24 * (3 * np.abs(g).sum(0) + np.abs(g.sum(0)))
+    assert np.all(np.abs(whole - g.sum(0)) <= bound)
+    want = np.mean([p[1] for p in parts], dtype=np.float64)
+    # the loss: FP32 sums of positive terms, at most 64 + 8 + 2 of them in a row
+    assert abs(loss - want) <= 2 * 74 * 2.0 ** -24 * want

@@ -315,14 +315,17 @@ __device__ __forceinline__ void write_payload(const StepConsts& C, const float* 
 // check) and where and how it adds to the grid.
 // EXACT (batched scenes): every particle's contribution becomes int64 fixed point
 // before it is summed, so that a node's sum depends neither on the order nor on
-// the grouping of the particles.
+// the grouping of the particles. Each is checked by itself (as to_fixed does): one that
+// is not a number raises MPM_FLAG_NAN_STATE and counts as 0. (100 steps of 256 scenes:
+// 50.1 ms with the check, 48.9 with one for the range alone; comparing every value, 51.3.)
 struct Fixed2 {
     long long x, y;
 };
 
 template <int D, int S, bool EXACT = false> struct ScatterLane {
     std::conditional_t<EXACT, Fixed2, float2> a[S][Scatter<D, S>::PAIRS];
-    float top;
+    float top;               // EXACT: unused
+    unsigned* status;        // EXACT
     unsigned long long* at;  // first node column and channel the lane adds to, at node 0
     int at2;                 // its second add, relative to the first
     float scale0, scale1;
@@ -435,19 +438,38 @@ __device__ __forceinline__ void sum_pair(ScatterLane<D, S, false>& T, int p, con
     if constexpr (S == 4) T.a[3][p] = __ffma2_rn(x[3], __fadd2_rn(P, Q), T.a[3][p]);
 }
 
+// max(a, |b|, |c|), NaN if one of them is (fmaxf drops a NaN).
+__device__ __forceinline__ float max_abs_nan(float a, float b, float c) {
+    float d;
+    asm("max.NaN.abs.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
+    return d;
+}
+
 template <int D, int S>
 __device__ __forceinline__ void sum_pair(ScatterLane<D, S, true>& T, int p, const float2* x, float2 P, float2 Q) {
     const float2 scale = make_float2(T.scale0, T.scale1);
     P = __fmul2_rn(P, scale);  // powers of two: exact
     Q = __fmul2_rn(Q, scale);
     P = __fadd2_rn(P, make_float2(-Q.x, -Q.y));
+    const float2 first = P;
+    float top = 0.f;
 #pragma unroll
     for (int a = 0; a < S; ++a) {
         const float2 t = __fmul2_rn(x[a], P);
-        T.top = fmaxf(T.top, fmaxf(fabsf(t.x), fabsf(t.y)));
+        top = max_abs_nan(top, t.x, t.y);
         T.a[a][p].x += __float2ll_rn(t.x);
         T.a[a][p].y += __float2ll_rn(t.y);
         P = __fadd2_rn(P, Q);
+    }
+    if (__builtin_expect(!(top < kFixedLimit), 0)) {  // rare: to_fixed in place of the plain conversions
+        P = first;
+#pragma unroll
+        for (int a = 0; a < S; ++a) {
+            const float2 t = __fmul2_rn(x[a], P);
+            T.a[a][p].x += to_fixed(t.x, 1.f, T.status) - __float2ll_rn(t.x);
+            T.a[a][p].y += to_fixed(t.y, 1.f, T.status) - __float2ll_rn(t.y);
+            P = __fadd2_rn(P, Q);
+        }
     }
 }
 
@@ -493,7 +515,6 @@ __device__ __forceinline__ void scatter_clipped(const StepConsts& C, const TileI
                                                 const float* v, const float* A, float mass,
                                                 unsigned long long* __restrict__ acc, unsigned* __restrict__ status) {
     constexpr int TE = TileGeom<D>::T;
-    float top = 0.f;
 #pragma unroll 1
     for (int j = 0; j < (D == 3 ? S * S * S : S * S); ++j) {
         const int gx = base[0] + j % S, gy = base[1] + (j / S) % S, gz = D == 3 ? base[2] + j / (S * S) : 0;
@@ -502,21 +523,17 @@ __device__ __forceinline__ void scatter_clipped(const StepConsts& C, const TileI
         float w = Stencil<S>::w(d[0]) * Stencil<S>::w(d[1]);
         if (D == 3) w *= Stencil<S>::w(d[2]);
         unsigned long long* n = acc + (((long long)gz * C.ny + gy) * C.nx + gx) * 4;
-        const float m = w * mass * C.sm;
-        red_scaled(n + 2, m);
-        top = fmaxf(top, fabsf(m));
+        red_int(n + 2, to_fixed(w * mass, C.sm, status));
 #pragma unroll
         for (int r = 0; r < D; ++r) {
             float s = mass * v[r];
 #pragma unroll
             for (int k = 0; k < D; ++k) s += A[r * D + k] * d[k];
-            s *= w * C.sp;
-            red_scaled(n + (r < 2 ? r : 3), s);
-            top = fmaxf(top, fabsf(s));
+            red_int(n + (r < 2 ? r : 3), to_fixed(w * s, C.sp, status));
         }
         mark_block_once(TI, ((D == 3 ? gz / TE : 0) * TI.nblk[1] + gy / TE) * TI.nblk[0] + gx / TE);
     }
-    raise_flag(status, top < kFixedLimit ? 4u : 4u | 2u);
+    raise_flag(status, 4u);
 }
 
 // The ordered rows of a window (`total` of them) into the grid. Whole warp.
@@ -552,6 +569,7 @@ __device__ __forceinline__ void scatter_rows(const StepConsts& C, const float* p
         T.scale1 = C.sp;
     }
     T.top = 0.f;
+    T.status = status;
     T.at = acc + (long long)col * C.nx * 4 + ch;
 #pragma unroll
     for (int a = 0; a < S; ++a)

@@ -867,7 +867,7 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
                     const int slot = queue_slot(Q);
                     Q.list[slot] = i;
 #pragma unroll
-                    for (int k = 0; k < D * D; ++k) Q.fh[(long long)k * Q.capacity + slot] = Fh[k];
+                    for (int k = 0; k < D * D; ++k) Q.fh[k * Q.capacity + slot] = Fh[k];
                     deferred = scatter;
                     scatter = false;
                 }

@@ -39,7 +39,7 @@ struct Particles {
     const float* mass;  // nullptr: uniform mass_u
     const float* vol;   // nullptr: uniform vol_u
     float mass_u, vol_u;
-    int n;
+    long long n;        // 64 bits, since a D*D field holds D*D*n values: more than 2^31 from 239M particles on (3D)
 };
 
 template <int D, int FORM> struct Layout {
@@ -137,7 +137,7 @@ __global__ void __launch_bounds__(256) k_p2g_simple(Particles P, StepConsts C, u
                                                     unsigned* __restrict__ status) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
-    const int n = P.n;
+    const long long n = P.n;
     float x[D], v[D], B[D * D], Fe[D * D];
 #pragma unroll
     for (int k = 0; k < D; ++k) { x[k] = P.x[k * n + i]; v[k] = P.v[k * n + i]; }
@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(256) k_g2p_simple(Particles P, StepConsts C, c
                                                     unsigned* __restrict__ status) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
-    const int n = P.n;
+    const long long n = P.n;
     constexpr int S = stencil_of(FORM);
     using St = Stencil<S>;
     float x[D];
@@ -648,7 +648,7 @@ template <int D, int S = 4>
 __global__ void __launch_bounds__(256) k_prepare_affine(Particles P, StepConsts C) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
-    const int n = P.n;
+    const long long n = P.n;
     float B[D * D], Fe[D * D], A[D * D];
 #pragma unroll
     for (int k = 0; k < D * D; ++k) { B[k] = P.B[k * n + i]; Fe[k] = P.Fe[k * n + i]; }
@@ -673,7 +673,7 @@ struct SlowQueue {
     int* list;    // slots needing the full return map
     int* count;   // device scalar
     float* fh;    // trial F per queue entry, [D*D][capacity]
-    int capacity;
+    long long capacity;  // 64 bits: fh holds D*D of them
     // fused path: the 32-slot windows holding queued particles, as (first
     // slot, mask of the slots left to scatter); their P2G runs after the return map
     int4* win;  // .z: queued slots whose node blocks are not marked yet
@@ -874,7 +874,7 @@ __global__ void __launch_bounds__(256, S == 3 ? MPM_G2P_MIN_BLOCKS_Q : MPM_G2P_M
     using St = Stencil<S>;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= P.n) return;
-    const int n = P.n;
+    const long long n = P.n;
     float x[D];
 #pragma unroll
     for (int k = 0; k < D; ++k) x[k] = P.x[k * n + i];
@@ -957,7 +957,7 @@ __device__ __forceinline__ void g2p_queued_exact(const Particles& P, const StepC
     float Fh[D * D], Fe[D * D], B[D * D], A[D * D];
     if (entry >= 0) {
 #pragma unroll
-        for (int k = 0; k < D * D; ++k) { Fh[k] = Q.fh[(long long)k * Q.capacity + e]; B[k] = P.B[k * n + i]; }
+        for (int k = 0; k < D * D; ++k) { Fh[k] = Q.fh[k * Q.capacity + e]; B[k] = P.B[k * n + i]; }
     } else {
         float x[D];
 #pragma unroll

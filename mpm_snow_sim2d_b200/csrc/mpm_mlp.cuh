@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(kMlpWarps * 32) k_return_map_mlp(Particles P, 
     if ((long long)blockIdx.x * kMlpWarps * 32 >= m) return;
     mlp_stage_weights(S, ML.wbf, ML.wf32);
     __syncthreads();
-    const int n = P.n;
+    const long long n = P.n;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     __nv_bfloat16* X = S.x[wid];
     float* O = S.out[wid];

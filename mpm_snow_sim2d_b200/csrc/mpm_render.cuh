@@ -68,8 +68,8 @@ __global__ void k_render_clear(unsigned long long* __restrict__ fb, long long pi
 }
 
 // Particles (slot order does not matter: the atomics commute).
-__global__ void k_render_points(RenderView V, const float* __restrict__ x, int n, unsigned long long* __restrict__ fb) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+__global__ void k_render_points(RenderView V, const float* __restrict__ x, long long n, unsigned long long* __restrict__ fb) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float p[3] = {x[i], x[n + i], V.dim == 3 ? x[2 * n + i] : 0.f};
     float px, py, depth;

@@ -82,7 +82,7 @@ template <int D, int S> __device__ __forceinline__ int tile_of_slot(const Partic
     constexpr int T = TileGeom<D>::T;
     int t = 0;
 #pragma unroll
-    for (int k = D - 1; k >= 0; --k) t = t * V.tiles[k] + cell_clamped<S>(P.x[(long long)k * P.n + i], V.ext[k]) / T;
+    for (int k = D - 1; k >= 0; --k) t = t * V.tiles[k] + cell_clamped<S>(P.x[k * P.n + i], V.ext[k]) / T;
     return V.tile0 + t;
 }
 
@@ -587,8 +587,8 @@ __global__ void __launch_bounds__(kP2GWarps * 32, D == 3 ? MPM_P2G_MIN_BLOCKS : 
     float* payf = reinterpret_cast<float*>(pay);
     unsigned long long* key = SM.key[wid];
     int* run = SM.run[wid];
-    const int n = P.n;
-    const int nchunks = (n + W::CHUNK - 1) / W::CHUNK;
+    const long long n = P.n;
+    const int nchunks = int((n + W::CHUNK - 1) / W::CHUNK);
     // 3D cubic: chunks are handed out one at a time from a counter, so that no
     // warp is left with a tail of chunks while others idle (-3% P2G; the sums
     // depend only on each chunk's contents, not on which warp takes it). The
@@ -601,7 +601,7 @@ __global__ void __launch_bounds__(kP2GWarps * 32, D == 3 ? MPM_P2G_MIN_BLOCKS : 
     }
     while (chunk < nchunks) {
         const int s0 = chunk * W::CHUNK;
-        const int cnt = min(W::CHUNK, n - s0);
+        const int cnt = min(W::CHUNK, int(n - s0));
         for (int j = lane; j < cnt; j += 32) {
             const int i = s0 + j;
             const float mass = P.mass ? P.mass[i] : P.mass_u;

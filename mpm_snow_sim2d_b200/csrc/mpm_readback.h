@@ -67,11 +67,6 @@ public:
         size_t total = 0;
         for (int p = 0; p < parts; ++p) total += bytes[p];
         if (total == 0) return cudaStreamSynchronize(stream);
-        if (total > kSmall) {
-            // wait for the stream before the ring, not while holding it
-            const cudaError_t e = cudaStreamSynchronize(stream);
-            if (e != cudaSuccess) return e;
-        }
         const char* s = static_cast<const char*>(src);
         if (total <= kSmall) {
             std::unique_lock<std::mutex> lock(use_, std::try_to_lock);
@@ -87,8 +82,14 @@ public:
         for (int p = 0; p < parts; s += bytes[p], ++p) {
             if (!dst[p] || !bytes[p]) continue;
             std::unique_lock<std::mutex> lock(use_, std::defer_lock);
-            const bool ring = bytes[p] >= kLarge && pageable(dst[p]) && lock.try_lock() && ready();
-            const cudaError_t e = ring ? pipe(stream, s, static_cast<char*>(dst[p]), bytes[p])
+            cudaError_t e = cudaSuccess;
+            bool ring = bytes[p] >= kLarge && pageable(dst[p]);
+            if (ring) {
+                // wait for the stream before the ring, not while holding it
+                if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
+                ring = lock.try_lock() && ready();
+            }
+            e = ring ? pipe(stream, s, static_cast<char*>(dst[p]), bytes[p])
                                        : direct(stream, s, dst + p, bytes + p, 1);
             if (e != cudaSuccess) return e;
         }

@@ -52,8 +52,6 @@ struct mpm_batch {
     int since_sort = 0;              // steps since the last sort
     bool needs_sort = true;
     bool any_fresh = true;           // a scene has no pending grid sums (arr.fresh)
-    float* staging = nullptr;
-    size_t staging_floats = 0;
     cudaStream_t stream = nullptr, own_stream = nullptr;
     mpm_batch_config cfg{};
     int cap_max = 0;                 // nodes per CTA of the largest scene's cluster (limit on a scene's grid)
@@ -95,7 +93,6 @@ void drop_graphs(mpm_batch* b) {
 
 void release(mpm_batch* b) {
     drop_graphs(b);
-    if (b->staging) cudaFree(b->staging);
     if (b->arr.stamps) cudaFree(b->arr.stamps);
     b->arena.release();
     if (b->own_stream) cudaStreamDestroy(b->own_stream);
@@ -194,16 +191,9 @@ mpm_status run_segment(mpm_batch* b, int steps, bool sort) {
 
 int sort_period(const mpm_batch* b) { return b->cfg.sort_period > 0 ? b->cfg.sort_period : 16; }
 
-mpm_status ensure_staging(mpm_batch* b, size_t floats) {
-    if (floats <= b->staging_floats) return MPM_OK;
-    BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
-    if (b->staging) cudaFree(b->staging);
-    b->staging = nullptr;
-    b->staging_floats = 0;
-    BATCH_CUDA(b, balloc(&b->staging, floats));
-    b->staging_floats = floats;
-    return MPM_OK;
-}
+// Memory for one call that waits for the stream before it returns: between sorts the
+// other buffer is free, its x, v, B, F_E and J_p one behind the other (a whole state).
+float* scratch(const mpm_batch* b) { return b->buf[b->parity ^ 1].x; }
 
 // Every scene's pending sums are void: the next step forms them from the state.
 mpm_status forget_sums(mpm_batch* b) {
@@ -257,8 +247,6 @@ mpm_status read_scene(mpm_batch* b, int scene, float* const* host) {
     size_t floats = 0;
     for (int f = 0; f < 5; ++f) floats += host[f] ? (size_t)n * kComps[f] : 0;
     if (floats == 0) return MPM_OK;
-    const mpm_status st = ensure_staging(b, floats);
-    if (st != MPM_OK) return st;
     const long long p0 = b->scenes[scene].p0;
     void* dst[5];
     size_t bytes[5], at = 0;
@@ -267,11 +255,11 @@ mpm_status read_scene(mpm_batch* b, int scene, float* const* host) {
         bytes[f] = host[f] ? sizeof(float) * (size_t)n * kComps[f] : 0;
         if (!host[f]) continue;
         k_batch_export<<<(n + 255) / 256, 256, 0, b->stream>>>(field(b, f), b->N, kComps[f], p0, n, b->buf[b->parity].id,
-                                                               b->staging + at);
+                                                               scratch(b) + at);
         at += (size_t)n * kComps[f];
     }
     BATCH_CUDA(b, cudaGetLastError());
-    BATCH_CUDA(b, ReadbackRing::get().read_parts(b->stream, b->staging, dst, bytes, 5));
+    BATCH_CUDA(b, ReadbackRing::get().read_parts(b->stream, scratch(b), dst, bytes, 5));
     return MPM_OK;
 }
 
@@ -519,15 +507,13 @@ mpm_status mpm_batch_set_state(mpm_batch* b, int32_t scene, const mpm_state_host
         for (size_t i = 0; given[f] && i < (size_t)n * kComps[f]; ++i)
             if (!std::isfinite(given[f][i])) return bfail(b, MPM_ERR_INVALID_ARGUMENT, "state holds non-finite values");
     if (n == 0) return MPM_OK;
-    mpm_status r = ensure_staging(b, (size_t)n * 4);
-    if (r != MPM_OK) return r;
     const BatchScene& S = b->scenes[scene];
     for (int f = 0; f < 5; ++f) {
         if (!given[f]) continue;
-        BATCH_CUDA(b, cudaMemcpyAsync(b->staging, given[f], sizeof(float) * (size_t)n * kComps[f], cudaMemcpyHostToDevice,
+        BATCH_CUDA(b, cudaMemcpyAsync(scratch(b), given[f], sizeof(float) * (size_t)n * kComps[f], cudaMemcpyHostToDevice,
                                       b->stream));
         k_batch_import<<<(n + 255) / 256, 256, 0, b->stream>>>(field(b, f), b->N, kComps[f], S.p0, n, b->buf[b->parity].id,
-                                                               b->staging);
+                                                               scratch(b));
         BATCH_CUDA(b, cudaGetLastError());
         BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
     }

@@ -62,11 +62,8 @@ struct mpm_solver {
     unsigned long long* acc = nullptr;
     float4* gv = nullptr;
     unsigned* status = nullptr;
-    float* staging = nullptr;
-    size_t staging_floats = 0;
-    unsigned long long* render_fb = nullptr;  // per-pixel (depth, intensity) words
-    unsigned char* render_rgb = nullptr;
-    long long render_pixels = 0;
+    void* staging = nullptr;  // scratch() beyond the alternate buffers
+    size_t staging_bytes = 0;
     int log2_sm = 0, log2_sp = 0, log2_sf = 0;
     long long step = 0;
     StepConsts C{};
@@ -166,8 +163,6 @@ template <typename T> cudaError_t dalloc(T** p, size_t count) {
 
 void release(mpm_solver* s) {
     if (s->staging) cudaFree(s->staging);
-    if (s->render_fb) cudaFree(s->render_fb);
-    if (s->render_rgb) cudaFree(s->render_rgb);
     for (auto& row : s->period_graph)
         for (auto& g : row)
             if (g) cudaGraphExecDestroy(g);
@@ -566,6 +561,7 @@ mpm_status setup_tiled(mpm_solver* s) {
     arena.want(&ti.key, N).want(&ti.tile_count, tiles).want(&ti.tile_cursor, tiles).want(&ti.tile_start, tiles);
     arena.want(&ti.mark, blocks).want(&ti.mark_list, blocks).want(&ti.n_marked, 1).want(&ti.p2g_next, 1);
     arena.want(&ti.perm, N).want(&ti.tile_list, tiles).want(&ti.n_tile_list, 1).want(&ti.skey, N).want(&ti.sval, N);
+    // (x to J_p one behind the other here and in mpm_create: scratch())
     arena.want(&s->alt.x, N * D).want(&s->alt.v, N * D).want(&s->alt.B, N * D * D).want(&s->alt.Fe, N * D * D);
     arena.want(&s->alt.Jp, N).want(&s->alt.id, N).want(&s->A, N * D * D).want(&s->alt.A, N * D * D);
     if (s->mass) arena.want(&s->alt.mass, N);
@@ -683,19 +679,32 @@ void fill_consts(mpm_solver* s) { s->C = step_consts(s->params, s->dim); }
 
 mpm_status validate(const mpm_params* p, std::string& why) { return validate_params(p, why); }
 
-mpm_status ensure_staging(mpm_solver* s, size_t floats) {
-    if (floats <= s->staging_floats) return MPM_OK;
-    if (s->staging) cudaFree(s->staging);
-    s->staging = nullptr;
-    s->staging_floats = 0;
-    MPM_CUDA(s, dalloc(&s->staging, floats));
-    s->staging_floats = floats;
+// Device memory for one call that waits for the stream before it returns. Between sorts
+// the alternate buffers are free: their x, v, B, F_E and J_p lie one behind the other
+// and hold a whole state or, but for tiny solvers, a picture. An allocation of its own
+// for the first read or picture of a solver costs 0.4 ms.
+mpm_status scratch(mpm_solver* s, size_t bytes, void** out) {
+    if (s->tiled && s->n > 0) {
+        char* lo = reinterpret_cast<char*>(s->alt.x);
+        if (bytes <= (size_t)(reinterpret_cast<char*>(s->alt.Jp + s->n) - lo)) {
+            *out = lo;
+            return MPM_OK;
+        }
+    }
+    if (bytes > s->staging_bytes) {
+        if (s->staging) cudaFree(s->staging);
+        s->staging = nullptr;
+        s->staging_bytes = 0;
+        MPM_CUDA(s, cudaMalloc(&s->staging, bytes));
+        s->staging_bytes = bytes;
+    }
+    *out = s->staging;
     return MPM_OK;
 }
 
 // Device SoA fields -> host interleaved arrays in creation order: one kernel and
 // one read (ReadbackRing) for all of them while they are small together, else
-// field by field, so that the staging buffer holds no more than one large field.
+// field by field, so that scratch of its own holds no more than one large field.
 mpm_status export_fields(mpm_solver* s, ExportFields E, float* const* host) {
     if (s->n == 0 || E.fields == 0) return MPM_OK;
     size_t floats = 0;
@@ -708,7 +717,8 @@ mpm_status export_fields(mpm_solver* s, ExportFields E, float* const* host) {
         }
         return MPM_OK;
     }
-    mpm_status st = ensure_staging(s, floats);
+    void* buf = nullptr;
+    mpm_status st = scratch(s, floats * sizeof(float), &buf);
     if (st != MPM_OK) return st;
     void* dst[ExportFields::MAX];
     size_t bytes[ExportFields::MAX];
@@ -720,19 +730,20 @@ mpm_status export_fields(mpm_solver* s, ExportFields E, float* const* host) {
         bytes[f] = sizeof(float) * (size_t)s->n * E.comps[f];
     }
     const int threads = 256, blocks = (s->n + threads - 1) / threads;
-    k_export_fields<<<blocks, threads, 0, s->stream>>>(E, s->n, s->id, s->staging);
+    k_export_fields<<<blocks, threads, 0, s->stream>>>(E, s->n, s->id, static_cast<float*>(buf));
     MPM_CUDA(s, cudaGetLastError());
-    MPM_CUDA(s, ReadbackRing::get().read_parts(s->stream, s->staging, dst, bytes, E.fields));
+    MPM_CUDA(s, ReadbackRing::get().read_parts(s->stream, buf, dst, bytes, E.fields));
     return MPM_OK;
 }
 
 mpm_status import_field(mpm_solver* s, float* soa, int comps, const float* host) {
     if (s->n == 0) return MPM_OK;
-    mpm_status st = ensure_staging(s, (size_t)s->n * comps);
+    void* buf = nullptr;
+    mpm_status st = scratch(s, sizeof(float) * (size_t)s->n * comps, &buf);
     if (st != MPM_OK) return st;
-    MPM_CUDA(s, cudaMemcpyAsync(s->staging, host, sizeof(float) * (size_t)s->n * comps, cudaMemcpyHostToDevice, s->stream));
+    MPM_CUDA(s, cudaMemcpyAsync(buf, host, sizeof(float) * (size_t)s->n * comps, cudaMemcpyHostToDevice, s->stream));
     const int threads = 256, blocks = (s->n + threads - 1) / threads;
-    k_import_soa<<<blocks, threads, 0, s->stream>>>(soa, comps, s->n, s->id, s->staging);
+    k_import_soa<<<blocks, threads, 0, s->stream>>>(soa, comps, s->n, s->id, static_cast<const float*>(buf));
     MPM_CUDA(s, cudaGetLastError());
     MPM_CUDA(s, cudaStreamSynchronize(s->stream));
     return MPM_OK;
@@ -1259,9 +1270,10 @@ mpm_status mpm_save_state(mpm_solver* s, const char* path) {
         sums.resize((size_t)nb * sum_hdr[0] * sum_hdr[1]);
         if (nb > 0) {
             MPM_CUDA(s, cudaMemcpy(sum_blocks.data(), s->ti.mark_list, sizeof(int) * nb, cudaMemcpyDeviceToHost));
-            mpm_status es = ensure_staging(s, sums.size() * 2);
+            void* buf = nullptr;
+            mpm_status es = scratch(s, sums.size() * sizeof(unsigned long long), &buf);
             if (es != MPM_OK) return es;
-            unsigned long long* dst = reinterpret_cast<unsigned long long*>(s->staging);
+            unsigned long long* dst = static_cast<unsigned long long*>(buf);
             if (D == 3)
                 k_pack_marked<3><<<s->sms * 4, 256, 0, s->stream>>>(s->C, s->ti, sum_hdr[0], nb, s->acc, dst);
             else
@@ -1434,9 +1446,10 @@ mpm_status mpm_load_state(mpm_solver* s, const char* path) {
                 const int nb = sum_hdr[2];
                 if (nb > 0) {
                     const size_t words = sums.size() + ((size_t)nb + 1) / 2;
-                    mpm_status es = ensure_staging(s, words * 2);
+                    void* buf = nullptr;
+                    mpm_status es = scratch(s, words * sizeof(unsigned long long), &buf);
                     if (es != MPM_OK) return es;
-                    unsigned long long* din = reinterpret_cast<unsigned long long*>(s->staging);
+                    unsigned long long* din = static_cast<unsigned long long*>(buf);
                     int* dblk = reinterpret_cast<int*>(din + sums.size());
                     MPM_CUDA(s, cudaMemcpyAsync(din, sums.data(), sizeof(unsigned long long) * sums.size(),
                                                 cudaMemcpyHostToDevice, st));
@@ -1816,16 +1829,12 @@ mpm_status mpm_render(mpm_solver* s, const mpm_render_params* p, uint8_t* rgb, s
         return fail(s, MPM_ERR_INVALID_ARGUMENT, "bad render parameters");
     const long long pixels = (long long)p->width * p->height;
     if (cap_bytes < (size_t)pixels * 3) return fail(s, MPM_ERR_CAPACITY, "image buffer smaller than width * height * 3");
-    if (pixels > s->render_pixels) {
-        if (s->render_fb) cudaFree(s->render_fb);
-        if (s->render_rgb) cudaFree(s->render_rgb);
-        s->render_fb = nullptr;
-        s->render_rgb = nullptr;
-        s->render_pixels = 0;
-        MPM_CUDA(s, dalloc(&s->render_fb, (size_t)pixels));
-        MPM_CUDA(s, dalloc(&s->render_rgb, (size_t)pixels * 3));
-        s->render_pixels = pixels;
-    }
+    // per-pixel (depth, intensity) words, then the picture
+    void* buf = nullptr;
+    const mpm_status st = scratch(s, (size_t)pixels * (sizeof(unsigned long long) + 3), &buf);
+    if (st != MPM_OK) return st;
+    unsigned long long* fb = static_cast<unsigned long long*>(buf);
+    unsigned char* packed = reinterpret_cast<unsigned char*>(fb + pixels);
     RenderView V{};
     V.dim = s->dim;
     V.width = p->width;
@@ -1886,13 +1895,13 @@ mpm_status mpm_render(mpm_solver* s, const mpm_render_params* p, uint8_t* rgb, s
     }
     const int threads = 256;
     const unsigned pblocks = (unsigned)((pixels + threads - 1) / threads);
-    k_render_clear<<<pblocks, threads, 0, s->stream>>>(s->render_fb, pixels);
-    k_render_lines<<<L.count, threads, 0, s->stream>>>(V, L, s->render_fb);
+    k_render_clear<<<pblocks, threads, 0, s->stream>>>(fb, pixels);
+    k_render_lines<<<L.count, threads, 0, s->stream>>>(V, L, fb);
     if (s->n > 0)
-        k_render_points<<<(s->n + threads - 1) / threads, threads, 0, s->stream>>>(V, s->x, s->n, s->render_fb);
-    k_render_pack<<<pblocks, threads, 0, s->stream>>>(s->render_fb, pixels, s->render_rgb);
+        k_render_points<<<(s->n + threads - 1) / threads, threads, 0, s->stream>>>(V, s->x, s->n, fb);
+    k_render_pack<<<pblocks, threads, 0, s->stream>>>(fb, pixels, packed);
     MPM_CUDA(s, cudaGetLastError());
-    MPM_CUDA(s, ReadbackRing::get().read(s->stream, s->render_rgb, rgb, (size_t)pixels * 3));
+    MPM_CUDA(s, ReadbackRing::get().read(s->stream, packed, rgb, (size_t)pixels * 3));
     return MPM_OK;
 }
 

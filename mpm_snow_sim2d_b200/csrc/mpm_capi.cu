@@ -30,7 +30,8 @@ struct mpm_mlp {
     float* w = nullptr;            // fp32 master parameters
     __nv_bfloat16* wbf = nullptr;  // bf16 copy used by the kernels
     float* grad = nullptr;
-    float* part = nullptr;         // per training CTA: its gradients and loss
+    float* part = nullptr;         // per training CTA: its gradients and loss (made by the first training call)
+    int part_rows = 0;
     float* m1 = nullptr;
     float* m2 = nullptr;
     float* loss = nullptr;         // per training step
@@ -1518,8 +1519,7 @@ mpm_status mpm_mlp_create(uint64_t seed, mpm_mlp** out) {
     mpm_mlp* m = new mpm_mlp();
     cudaGetDevice(&m->device);
     const int P = MlpOff::total;
-    if (dalloc(&m->w, P) || dalloc(&m->wbf, P) || dalloc(&m->grad, P) || dalloc(&m->m1, P) || dalloc(&m->m2, P) ||
-        dalloc(&m->part, (size_t)kMlpTrainCtas * kMlpPart)) {
+    if (dalloc(&m->w, P) || dalloc(&m->wbf, P) || dalloc(&m->grad, P) || dalloc(&m->m1, P) || dalloc(&m->m2, P)) {
         mpm_mlp_destroy(m);
         return MPM_ERR_OUT_OF_MEMORY;
     }
@@ -1613,11 +1613,29 @@ mpm_status mpm_mlp_load_pairs(mpm_mlp* m, const float* pairs, int64_t n) {
     return MPM_OK;
 }
 
+static int mlp_ctas(int rows) { return std::min((rows - 1) / kMlpTrainRows + 1, kMlpTrainCtas); }
+
+// Room in m->part for the CTAs of a launch over `rows` samples. Made when a network is
+// first trained, and no larger than asked: 6 MB take 0.7 ms to allocate, most of what a network
+// loaded for inference would take to create.
+static bool mlp_want_part(mpm_mlp* m, int rows) {
+    const int ctas = mlp_ctas(rows);
+    if (ctas <= m->part_rows) return true;
+    if (m->part) cudaFree(m->part);
+    m->part = nullptr;
+    m->part_rows = 0;
+    if (dalloc(&m->part, (size_t)ctas * kMlpPart)) {
+        cudaGetLastError();
+        return false;
+    }
+    m->part_rows = ctas;
+    return true;
+}
+
 // Gradients and loss of `rows` samples into m->part; returns the rows of it used
 // (0: launch failed).
 static int mlp_launch_grad(mpm_mlp* m, const float* dpairs, long long np, bool in_order, int rows, unsigned seed) {
-    const int tiles = (rows - 1) / kMlpTrainRows + 1;
-    const int ctas = tiles < kMlpTrainCtas ? tiles : kMlpTrainCtas;
+    const int ctas = mlp_ctas(rows);
     k_mlp_train<<<ctas, 256, sizeof(MlpTrainSmem)>>>(dpairs, np, in_order, rows, seed, m->wbf, m->w, m->norm, m->part);
     return cudaGetLastError() == cudaSuccess ? ctas : 0;
 }
@@ -1640,6 +1658,7 @@ mpm_status mpm_mlp_train(mpm_mlp* m, int32_t steps, int32_t batch, float lr, flo
         if (dalloc(&m->loss, (size_t)steps)) { cudaGetLastError(); return MPM_ERR_OUT_OF_MEMORY; }
         m->loss_cap = steps;
     }
+    if (!mlp_want_part(m, batch)) return MPM_ERR_OUT_OF_MEMORY;
     if (!mlp_train_attr()) return MPM_ERR_CUDA;
     const float b1 = 0.9f, b2 = 0.999f;
     for (int it = 0; it < steps; ++it) {
@@ -1665,7 +1684,7 @@ mpm_status mpm_mlp_gradient(mpm_mlp* m, const float* pairs, int64_t n, float* gr
     if (!m || !pairs || n < 1 || n > (1 << 24) || !grad_out) return MPM_ERR_INVALID_ARGUMENT;
     float *dp = nullptr, *dl = nullptr;
     mpm_status st = MPM_OK;
-    if (dalloc(&dp, (size_t)n * 20) || dalloc(&dl, 1)) st = MPM_ERR_OUT_OF_MEMORY;
+    if (!mlp_want_part(m, (int)n) || dalloc(&dp, (size_t)n * 20) || dalloc(&dl, 1)) st = MPM_ERR_OUT_OF_MEMORY;
     if (st == MPM_OK && cudaMemcpy(dp, pairs, sizeof(float) * 20 * n, cudaMemcpyHostToDevice) != cudaSuccess)
         st = MPM_ERR_CUDA;
     if (st == MPM_OK) {

@@ -42,3 +42,27 @@ def test_sum_over_ctas(net, tiles):
     want = np.mean([p[1] for p in parts], dtype=np.float64)
     # the loss: FP32 sums of positive terms, at most 64 + 8 + 2 of them in a row
     assert abs(loss - want) <= 2 * 74 * 2.0 ** -24 * want
+
+
+def test_creating_a_network_takes_little_memory(net):
+    """The parameters, their moments and a gradient, 5 x 40 KB, from pieces of 2 MB that the driver has mapped or maps; the
+    training launch's partial sums (6 MB) come with the first training."""
+    import torch
+    from mpm_snow_sim2d_b200 import mlp
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    m, pairs = net
+    before = free()
+    other = mlp.Mlp(seed=3)
+    assert before - free() <= 2 << 20
+    other.set_normalization(*m.norm)
+    for n in (128, 4096, 128):  # the room grows, and is kept
+        got, _ = other.gradient(pairs[:n])
+        again, _ = other.gradient(pairs[:n])
+        assert np.array_equal(got, again) and np.isfinite(got).all() and got.any()
+    kept = free()
+    other.gradient(pairs[:4096])
+    assert free() == kept

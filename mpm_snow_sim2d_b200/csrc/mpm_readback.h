@@ -1,18 +1,21 @@
 // Device-to-host reads through pinned memory.
 //
-// The getters hand back host arrays that the caller allocated, usually fresh and
-// pageable. A plain copy into such memory runs at 4 to 5 GB/s (one thread of the
-// driver moves the data and takes the page faults): 10.5 ms for the positions of
-// 3.8M particles, a fifth of the frame. Here the copy engine fills a ring of
-// pinned chunks while a few threads move finished chunks on: 3.3 ms (2.8 with
-// chunks of 2 MB, 5 with 256 KB, but pinning memory costs 0.4 ms per MB, which the
-// first read pays). Small fields go through a pinned buffer in one piece, one copy
-// and one wait instead of one each (a step and the state of 2.3k particles: 62 us
-// against 147). In between, starting threads costs more than they save (a 2 MB
-// picture: 560 us against 220), and the copy is left to the driver.
+// The getters hand back host arrays that the caller allocated, usually pageable. Into
+// memory that has been written before, the driver's copy runs at 19 GB/s, and it is left
+// to it. Into fresh memory it falls to 5 GB/s (2 with 4 KB pages), since the one thread that
+// moves the data also takes the page faults: 9.6 ms for the positions of 3.8M
+// particles. There the copy engine fills a ring of pinned chunks while a few threads
+// move finished chunks on: 4.0 ms (chunks of 2 MB move a little faster, of 256 KB slower, but pinning
+// memory costs up to 0.8 ms per MB). The ring is for fresh memory only (into written memory it
+// takes 474 -> 550 us for 8.5 MB, 1.3 -> 1.45 ms for 24 MB, 2.5 -> 2.6 ms for 46 MB), and it
+// is made when reads into fresh memory have come to kRingAfter bytes: what it costs to make, 3
+// ms, is what it saves on about 20 MB (a first read of 8.5 MB that makes it: 4 ms, 2.5 without).
+// Small fields go through a pinned buffer in one piece, one copy and one wait instead
+// of one each (a step and the state of 2.3k particles: 62 us against 147). In between,
+// starting threads costs more than they save (a 2 MB picture: 560 us against 220).
 //
 // Both buffers are shared by every solver and batch of the process, of fixed size,
-// made on first use and freed with the last object that holds a ReadbackUser. One
+// made when first needed and freed with the last object that holds a ReadbackUser. One
 // read uses them at a time; a second one that finds them taken copies directly.
 #pragma once
 
@@ -27,6 +30,9 @@
 #include <thread>
 #include <vector>
 
+#include <sys/mman.h>
+#include <unistd.h>
+
 #include <cuda_runtime.h>
 
 namespace mpm {
@@ -36,7 +42,7 @@ public:
     static constexpr size_t kChunk = 512u << 10;
     static constexpr int kChunks = 8;
     static constexpr int kThreads = 7;  // besides the caller's
-    static constexpr size_t kSmall = 256u << 10, kLarge = 8u << 20;
+    static constexpr size_t kSmall = 256u << 10, kLarge = 8u << 20, kRingAfter = 40u << 20;
 
     static ReadbackRing& get() {
         static ReadbackRing ring;
@@ -83,7 +89,7 @@ public:
             if (!dst[p] || !bytes[p]) continue;
             std::unique_lock<std::mutex> lock(use_, std::defer_lock);
             cudaError_t e = cudaSuccess;
-            bool ring = bytes[p] >= kLarge && pageable(dst[p]);
+            bool ring = bytes[p] >= kLarge && untouched(dst[p], bytes[p]) && pageable(dst[p]) && worth_it(bytes[p]);
             if (ring) {
                 // wait for the stream before the ring, not while holding it
                 if ((e = cudaStreamSynchronize(stream)) != cudaSuccess) return e;
@@ -103,6 +109,24 @@ private:
     char* small_ = nullptr;
     cudaEvent_t ev_[kChunks] = {};
     int device_ = -1;  // of the events
+    std::atomic<bool> made_{false};    // pin_ is there
+    std::atomic<size_t> without_{0};   // bytes read into fresh memory without the ring
+
+    bool worth_it(size_t bytes) {
+        return made_.load() || without_.fetch_add(bytes) + bytes >= kRingAfter;
+    }
+    // Whether most of [p, p + bytes) has no memory behind it yet (16 pages asked, 4 us).
+    static bool untouched(const void* p, size_t bytes) {
+        constexpr int kProbes = 16;
+        const size_t page = (size_t)sysconf(_SC_PAGESIZE);
+        int missing = 0;
+        for (int k = 0; k < kProbes; ++k) {
+            const size_t at = (reinterpret_cast<size_t>(p) + bytes / kProbes * k) / page * page;
+            unsigned char in = 1;
+            if (mincore(reinterpret_cast<void*>(at), page, &in) == 0 && !(in & 1)) ++missing;
+        }
+        return 2 * missing > kProbes;
+    }
 
     // Pinned memory of the caller's is filled by the copy engine alone (164 MB: 3 ms
     // against 8 through the ring).
@@ -134,6 +158,7 @@ private:
                 }
             device_ = dev;
         }
+        made_ = true;
         return true;
     }
     void drop_events() {
@@ -149,6 +174,8 @@ private:
             if (*p) cudaFreeHost(*p);
             *p = nullptr;
         }
+        made_ = false;
+        without_ = 0;
     }
 
     static cudaError_t direct(cudaStream_t stream, const void* src, void* const* dst, const size_t* bytes, int parts) {

@@ -11,7 +11,7 @@ HOST = Path(__file__).resolve().parent / "host"
 CUDA_INCLUDE = Path(nvcc_path()).resolve().parents[1] / "include"
 
 
-@pytest.mark.parametrize("name", ["readback_waits"])
+@pytest.mark.parametrize("name", ["readback_waits", "readback_ring"])
 def test_readback(tmp_path, name):
     exe = tmp_path / name
     subprocess.run(["g++", "-std=c++17", "-O1", "-pthread", "-I", str(HOST), "-I", str(CSRC), "-I", str(CUDA_INCLUDE),

@@ -52,6 +52,7 @@ struct mpm_batch {
     int since_sort = 0;              // steps since the last sort
     bool needs_sort = true;
     bool any_fresh = true;           // a scene has no pending grid sums (arr.fresh)
+    bool unfinished = false;         // a step call failed on its way (recover)
     cudaStream_t stream = nullptr, own_stream = nullptr;
     mpm_batch_config cfg{};
     int cap_max = 0;                 // nodes per CTA of the largest scene's cluster (limit on a scene's grid)
@@ -126,7 +127,7 @@ cudaError_t enqueue_sort(mpm_batch* b, bool pending) {
     const SortBuffers dst{t.x, pending ? nullptr : t.v, pending ? nullptr : t.B, t.Fe, t.Jp, nullptr, t.mass, t.vol, t.id};
     e = launch_chained(k_tile_sort<2, 4, ManyScenes>, b->sms * SortGeom<2>::CTAS_PER_SM, 256, 0, b->stream, P,
                        b->buf[b->parity].id, dst, b->many, b->ti);
-    b->parity ^= 1;
+    if (e == cudaSuccess) b->parity ^= 1;
     return e;
 }
 
@@ -204,6 +205,15 @@ mpm_status forget_sums(mpm_batch* b) {
     b->any_fresh = true;
     b->needs_sort = true;
     return MPM_OK;
+}
+
+// After a call that failed on its way: what its kernels hand each other through device
+// counters (the call's step, which says where time stamps go, and the tiles' counts of a
+// sort) starts over, and the sums are formed anew from the particles as they are.
+mpm_status recover(mpm_batch* b) {
+    BATCH_CUDA(b, cudaMemsetAsync(b->arr.step, 0, sizeof(int), b->stream));
+    BATCH_CUDA(b, cudaMemsetAsync(b->ti.tile_count, 0, sizeof(int) * (size_t)b->ti.n_tiles, b->stream));
+    return forget_sums(b);
 }
 
 // A configuration is valid when its numbers are and every scene's grid fits the
@@ -456,6 +466,11 @@ mpm_status mpm_batch_step(mpm_batch* b, int32_t nsteps) {
         BATCH_CUDA(b, balloc(&b->arr.stamps, need));
         b->stamps_cap = need;
     }
+    if (b->unfinished) {
+        const mpm_status st = recover(b);
+        if (st != MPM_OK) return st;
+    }
+    b->unfinished = true;
     b->last_steps = nsteps;
     if (b->any_fresh) {
         // sums of the new states: sort, then their P2G
@@ -481,6 +496,7 @@ mpm_status mpm_batch_step(mpm_batch* b, int32_t nsteps) {
     }
     k_batch_end<<<1, 256, 0, b->stream>>>(b->arr);
     BATCH_CUDA(b, cudaGetLastError());
+    b->unfinished = false;
     return MPM_OK;
 }
 

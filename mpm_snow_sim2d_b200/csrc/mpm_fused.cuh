@@ -607,6 +607,24 @@ __device__ __forceinline__ void mark_stencil(const TileInfo& TI, const int* base
             for (int bx = x0; bx <= x1; ++bx) mark_block_once(TI, (bz * TI.nblk[1] + by) * TI.nblk[0] + bx);
 }
 
+// The same of a stencil partly outside the grid: the blocks of its nodes in the grid.
+template <int D, int S>
+__device__ __forceinline__ void mark_clipped(const StepConsts& C, const TileInfo& TI, const int* base) {
+    constexpr int TE = TileGeom<D>::T;
+    int b0[3] = {0, 0, 0}, b1[3] = {0, 0, 0};
+#pragma unroll
+    for (int k = 0; k < D; ++k) {
+        const int ext = k == 0 ? C.W : (k == 1 ? C.H : C.Dp);
+        const int lo = max(base[k], 0), hi = min(base[k] + S - 1, ext);
+        if (lo > hi) return;
+        b0[k] = lo / TE;
+        b1[k] = hi / TE;
+    }
+    for (int bz = b0[2]; bz <= b1[2]; ++bz)
+        for (int by = b0[1]; by <= b1[1]; ++by)
+            for (int bx = b0[0]; bx <= b1[0]; ++bx) mark_block_once(TI, (bz * TI.nblk[1] + by) * TI.nblk[0] + bx);
+}
+
 // The node blocks of a stencil as bits of the 3^D blocks around the tile whose
 // node box starts at bo (2 nodes before the tile); the stencil lies in the box.
 template <int D, int S>
@@ -637,7 +655,7 @@ __device__ __forceinline__ void queued_window(const Particles& P, const StepCons
     using L = Scatter<D, S>;
     const int lane = threadIdx.x & 31;
     const long long n = P.n;
-    const bool queued = ((unsigned)rec.y >> lane) & 1u;
+    const bool queued = ((unsigned)rec.y >> lane) & 1u, unmarked = ((unsigned)rec.z >> lane) & 1u;
     int key = kNoKey, base[3] = {0, 0, 0};
     float mass = 0.f, x[D], v[D], A[D * D];
     if (queued) {
@@ -651,8 +669,16 @@ __device__ __forceinline__ void queued_window(const Particles& P, const StepCons
         if (key == kClipped) {
             scatter_clipped<D, S>(C, TI, x, base, v, A, mass, acc, status);
             key = kNoKey;
-        } else if (((unsigned)rec.z >> lane) & 1u) {
+        } else if (unmarked) {
             mark_stencil<D, S>(TI, base);
+        }
+    }
+    if constexpr (EXACT) {
+        if (unmarked && !queued) {  // no volume: reads the grid next step, adds nothing
+#pragma unroll
+            for (int k = 0; k < D; ++k) x[k] = P.x[k * n + rec.x + lane];
+            if (stencil_key<D, S>(C, x, base) == kClipped) mark_clipped<D, S>(C, TI, base);
+            else mark_stencil<D, S>(TI, base);
         }
     }
     int count, total;
@@ -766,7 +792,9 @@ __device__ __forceinline__ void mark_tile_blocks(const TileInfo& TI, const int* 
 // each slot's particle against the tile's node box (G2P = true) or the stored
 // state (G2P = false), then the scatter of the in-band particles' payloads.
 // Returns this lane's node-block bits around the tile (box origin bo). DIRECT:
-// there is no staged box, every particle gathers from the global grid.
+// there is no staged box, every particle gathers from the global grid. EXACT: blocks
+// are also marked for particles without volume, which add nothing but read them next
+// step; a block that the grid update does not come to keeps old velocities.
 template <int D, int S, bool G2P, bool DIRECT = false, bool EXACT = false>
 __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepConsts& C, const TileInfo& TI,
                                                  const float4* __restrict__ gv, unsigned long long* __restrict__ acc,
@@ -783,7 +811,7 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
     const int i = start + w * win + lane;
     int key = kNoKey, nbase[3] = {0, 0, 0};
     bool deferred = false;   // queued: scattered after the return map (k_p2g_windows)
-    bool unmarked = false;   // queued with its whole G2P: new position not known here
+    bool unmarked = false;   // queued with its whole G2P: new position not known here (EXACT: also without volume)
     unsigned bits = 0u;
     float mass = 0.f, x[D], v[D], A[D * D];
     if (valid) {
@@ -810,7 +838,8 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
             if (!interior) {
                 // stencil partly outside the grid: the general kernel does the whole G2P
                 Q.list[queue_slot(Q)] = -1 - i;
-                deferred = unmarked = scatter;
+                deferred = scatter;
+                unmarked = EXACT || scatter;
                 scatter = false;
             } else {
                 float nv[D], nx[D], nB[D * D];
@@ -882,7 +911,7 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
         }
         // the new stencil, and its node blocks (of queued particles too: their
         // return map leaves the position alone)
-        if (scatter || (deferred && !unmarked)) {
+        if (EXACT ? !unmarked : scatter || (deferred && !unmarked)) {
             const int k = stencil_key<D, S>(C, x, nbase);
             if (k != kClipped) {
                 bool boxed = true;
@@ -894,6 +923,8 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
                 if (scatter) key = k;
             } else if (scatter) {
                 scatter_clipped<D, S>(C, TI, x, nbase, v, A, mass, acc, status);
+            } else if (EXACT && !deferred) {
+                mark_clipped<D, S>(C, TI, nbase);
             }
         }
     }
@@ -906,7 +937,7 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
         // 331 + 19.3, 327 + 18.5). A single 2D scene queues a few windows and waits
         // for the longest of them: 22.3 + 3.4 us at 186k particles, put off 21.9 + 6.0.
         constexpr bool PUT_OFF = D == 3 || EXACT;
-        if (__builtin_expect(__any_sync(0xffffffffu, deferred), 0)) {
+        if (__builtin_expect(__any_sync(0xffffffffu, deferred || unmarked), 0)) {
             const unsigned rows = __ballot_sync(0xffffffffu, deferred || (PUT_OFF && key != kNoKey));
             const unsigned um = __ballot_sync(0xffffffffu, unmarked);
             if (PUT_OFF && key != kNoKey) {

@@ -354,8 +354,9 @@ MPM_API mpm_status mpm_render(mpm_solver* solver, const mpm_render_params* param
  * Many independent scenes, each a full solver in the sense of mpm_create
  * (the reference constructs one Solver per process, src/main.cpp:164-174),
  * stepped together: the scenes lie side by side in one grid and one particle
- * array, and each kernel of a step runs over all of them. A scene's result does
- * not depend on its partners (bitwise). Scenes: dim 2, MLS, at most 8 x 9,600
+ * array, and each kernel of a step runs over all of them. (Grids that do not fit
+ * the device's memory together are stepped a part of the scenes at a time; the results
+ * are the same.) A scene's result does not depend on its partners (bitwise). Scenes: dim 2, MLS, at most 8 x 9,600
  * grid nodes ((W+1)(H+1) <= ~76,000, e.g. 257 x 257 cells); larger or 3D scenes
  * return MPM_ERR_CAPACITY / MPM_ERR_UNSUPPORTED. */
 struct mpm_batch;

@@ -28,6 +28,13 @@ struct BatchBuffers {
     int* id;  // creation index of the particle within its scene
 };
 
+// The grid of the parts of a batch (below).
+struct SharedGrid {
+    unsigned long long* acc;
+    float4* gv;
+    int *mark, *mark_list;
+};
+
 }  // namespace
 
 struct mpm_batch {
@@ -60,6 +67,12 @@ struct mpm_batch {
     std::map<std::tuple<int, int, int>, cudaGraphExec_t> graphs;
     bool use_graphs = true;
     std::string err;
+    // Scenes whose grids do not fit the device's memory side by side: consecutive scenes
+    // in parts, batches of their own that share one grid and are stepped one after the other. A part
+    // forms its sums from its particles when its turn comes, which gives the same sums.
+    // Empty: all scenes are in this object.
+    std::vector<mpm_batch*> parts;
+    std::vector<int> part_first;     // first scene of each part
 };
 
 namespace {
@@ -93,6 +106,12 @@ void drop_graphs(mpm_batch* b) {
 }
 
 void release(mpm_batch* b) {
+    for (mpm_batch* p : b->parts) {
+        release(p);
+        delete p;
+    }
+    b->parts.clear();
+    b->part_first.clear();
     drop_graphs(b);
     if (b->arr.stamps) cudaFree(b->arr.stamps);
     b->arena.release();
@@ -240,6 +259,20 @@ mpm_status configure(mpm_batch* b, const mpm_batch_config& cfg) {
     return MPM_OK;
 }
 
+// The part that holds a scene (null: there are no parts), and the scene's number in it.
+mpm_batch* part_of(const mpm_batch* b, int32_t& scene) {
+    if (b->parts.empty()) return nullptr;
+    const size_t k = std::upper_bound(b->part_first.begin(), b->part_first.end(), scene) - b->part_first.begin() - 1;
+    scene -= b->part_first[k];
+    return b->parts[k];
+}
+
+// What a part answered, as the batch's own answer.
+mpm_status answer(mpm_batch* b, const mpm_batch* part, mpm_status st) {
+    if (st != MPM_OK) b->err = part->err;
+    return st;
+}
+
 bool valid_scene(const mpm_batch* b, int32_t s) { return b && s >= 0 && s < b->nscenes; }
 
 const int kComps[5] = {2, 2, 4, 4, 1};  // position, velocity, B, F_E, J_p
@@ -273,33 +306,11 @@ mpm_status read_scene(mpm_batch* b, int scene, float* const* host) {
     return MPM_OK;
 }
 
-}  // namespace
-
-extern "C" {
-
-mpm_status mpm_batch_create(const mpm_params* params, const mpm_particles_init* init, int32_t nscenes,
-                            mpm_batch** out) {
-    if (!out) return MPM_ERR_INVALID_ARGUMENT;
-    *out = nullptr;
-    if (!params || !init || nscenes < 1) return MPM_ERR_INVALID_ARGUMENT;
+// A batch of all scenes in one; with `grid` a part, whose grid is that.
+mpm_status create_whole(const mpm_params* params, const mpm_particles_init* init, int32_t nscenes, int dev,
+                        const SharedGrid* grid, mpm_batch** out) {
     long long N = 0;
-    for (int s = 0; s < nscenes; ++s) {
-        std::string why;
-        mpm_status st = validate_params(&params[s], why);
-        if (st != MPM_OK) return st;
-        if (params[s].dim != 2 || params[s].formulation != MPM_FORMULATION_MLS) return MPM_ERR_UNSUPPORTED;
-        if (params[s].height + 1 > kBatchMaxRows) return MPM_ERR_CAPACITY;
-        if (init[s].count < 0 || init[s].count > 0x7fffffff) return MPM_ERR_INVALID_ARGUMENT;
-        if (init[s].count > 0 && (!init[s].position || !init[s].volume)) return MPM_ERR_INVALID_ARGUMENT;
-        N += init[s].count;
-    }
-    if (N > 0x7fffffffLL) return MPM_ERR_INVALID_ARGUMENT;
-    int ndev = 0, dev = 0;
-    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) { cudaGetLastError(); return MPM_ERR_NO_DEVICE; }
-    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return MPM_ERR_NO_DEVICE; }
-    cudaFuncAttributes fa;
-    if (cudaFuncGetAttributes(&fa, k_batch_step<true>) != cudaSuccess) { cudaGetLastError(); return MPM_ERR_NO_DEVICE; }
-
+    for (int s = 0; s < nscenes; ++s) N += init[s].count;
     mpm_batch* b = new mpm_batch();
     auto bail = [&](mpm_status code) { release(b); delete b; return code; };
     b->device = dev;
@@ -380,10 +391,19 @@ mpm_status mpm_batch_create(const mpm_params* params, const mpm_particles_init* 
     BatchScene* d_scenes = nullptr;
     int *d_of_slots = nullptr, *d_of_tiles = nullptr, *d_of_blocks = nullptr;
     arena.want(&d_scenes, (size_t)nscenes).want(&d_of_slots, n).want(&d_of_tiles, nt).want(&d_of_blocks, nb);
-    arena.want(&b->A, n * 4).want(&b->arr.acc, (size_t)b->nodes * 4).want(&b->arr.gv, (size_t)b->nodes);
+    arena.want(&b->A, n * 4);
+    if (grid) {
+        b->arr.acc = grid->acc;
+        b->arr.gv = grid->gv;
+        ti.mark = grid->mark;
+        ti.mark_list = grid->mark_list;
+    } else {
+        arena.want(&b->arr.acc, (size_t)b->nodes * 4).want(&b->arr.gv, (size_t)b->nodes);
+        arena.want(&ti.mark, nb).want(&ti.mark_list, nb);
+    }
     arena.want(&b->arr.status, (size_t)nscenes).want(&b->arr.fresh, (size_t)nscenes).want(&b->arr.step, 1);
     arena.want(&ti.key, n).want(&ti.tile_count, nt).want(&ti.tile_cursor, nt).want(&ti.tile_start, nt);
-    arena.want(&ti.mark, nb).want(&ti.mark_list, nb).want(&ti.n_marked, 1).want(&ti.perm, n).want(&ti.tile_list, nt);
+    arena.want(&ti.n_marked, 1).want(&ti.perm, n).want(&ti.tile_list, nt);
     arena.want(&ti.n_tile_list, 1).want(&ti.tile_len, nt).want(&ti.fused_next, 1);
     arena.want(&ti.items, nt + n / (size_t)ti.win).want(&ti.n_items, 1).want(&ti.scan, nt / kScanTiles + 1);
     arena.want(&ti.grid_done, 1).want(&ti.skey, n).want(&ti.sval, n).want(&b->q.list, (size_t)b->q.capacity);
@@ -436,6 +456,84 @@ mpm_status mpm_batch_create(const mpm_params* params, const mpm_particles_init* 
     return MPM_OK;
 }
 
+// The scenes in `k` parts or a few more, of about as many nodes each.
+mpm_status create_parts(const mpm_params* params, const mpm_particles_init* init, int32_t nscenes, int dev, int k,
+                        mpm_batch** out) {
+    constexpr int T = TileGeom<2>::T;
+    auto nodes_of = [&](int s) { return (long long)(params[s].width + 1) * (params[s].height + 1); };
+    auto blocks_of = [&](int s) { return (long long)((params[s].width + T) / T) * ((params[s].height + T) / T); };
+    mpm_batch* b = new mpm_batch();
+    auto bail = [&](mpm_status code) { release(b); delete b; return code; };
+    b->device = dev;
+    b->nscenes = nscenes;
+    long long total = 0, nodes = 0, blocks = 0, most_nodes = 0, most_blocks = 0;
+    for (int s = 0; s < nscenes; ++s) {
+        total += nodes_of(s);
+        b->N += init[s].count;
+        b->counts.push_back((int)init[s].count);
+    }
+    const long long share = (total + k - 1) / k;
+    for (int s = 0; s < nscenes; ++s) {
+        if (s == 0 || nodes + nodes_of(s) > share) {
+            b->part_first.push_back(s);
+            nodes = blocks = 0;
+        }
+        nodes += nodes_of(s);
+        blocks += blocks_of(s);
+        most_nodes = std::max(most_nodes, nodes);
+        most_blocks = std::max(most_blocks, blocks);
+    }
+    if (cudaStreamCreateWithFlags(&b->own_stream, cudaStreamNonBlocking) != cudaSuccess) return bail(MPM_ERR_CUDA);
+    b->stream = b->own_stream;
+    SharedGrid grid{};
+    b->arena.want(&grid.acc, (size_t)most_nodes * 4).want(&grid.gv, (size_t)most_nodes);
+    b->arena.want(&grid.mark, (size_t)most_blocks).want(&grid.mark_list, (size_t)most_blocks);
+    if (!b->arena.allocate()) return bail(MPM_ERR_OUT_OF_MEMORY);
+    for (size_t p = 0; p < b->part_first.size(); ++p) {
+        const int s0 = b->part_first[p], s1 = p + 1 < b->part_first.size() ? b->part_first[p + 1] : nscenes;
+        mpm_batch* part = nullptr;
+        mpm_status st = create_whole(params + s0, init + s0, s1 - s0, dev, &grid, &part);
+        if (st != MPM_OK) return bail(st);
+        b->parts.push_back(part);
+        if ((st = mpm_batch_set_stream(part, b->own_stream)) != MPM_OK) return bail(st);
+    }
+    *out = b;
+    return MPM_OK;
+}
+
+}  // namespace
+
+extern "C" {
+
+mpm_status mpm_batch_create(const mpm_params* params, const mpm_particles_init* init, int32_t nscenes,
+                            mpm_batch** out) {
+    if (!out) return MPM_ERR_INVALID_ARGUMENT;
+    *out = nullptr;
+    if (!params || !init || nscenes < 1) return MPM_ERR_INVALID_ARGUMENT;
+    long long N = 0;
+    for (int s = 0; s < nscenes; ++s) {
+        std::string why;
+        mpm_status st = validate_params(&params[s], why);
+        if (st != MPM_OK) return st;
+        if (params[s].dim != 2 || params[s].formulation != MPM_FORMULATION_MLS) return MPM_ERR_UNSUPPORTED;
+        if (params[s].height + 1 > kBatchMaxRows) return MPM_ERR_CAPACITY;
+        if (init[s].count < 0 || init[s].count > 0x7fffffff) return MPM_ERR_INVALID_ARGUMENT;
+        if (init[s].count > 0 && (!init[s].position || !init[s].volume)) return MPM_ERR_INVALID_ARGUMENT;
+        N += init[s].count;
+    }
+    if (N > 0x7fffffffLL) return MPM_ERR_INVALID_ARGUMENT;
+    int ndev = 0, dev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) { cudaGetLastError(); return MPM_ERR_NO_DEVICE; }
+    if (cudaGetDevice(&dev) != cudaSuccess) { cudaGetLastError(); return MPM_ERR_NO_DEVICE; }
+    cudaFuncAttributes fa;
+    if (cudaFuncGetAttributes(&fa, k_batch_step<true>) != cudaSuccess) { cudaGetLastError(); return MPM_ERR_NO_DEVICE; }
+
+    mpm_status st = create_whole(params, init, nscenes, dev, nullptr, out);
+    for (long long k = 2; st == MPM_ERR_OUT_OF_MEMORY && k < 2LL * nscenes; k *= 2)
+        st = create_parts(params, init, nscenes, dev, (int)std::min<long long>(k, nscenes), out);
+    return st;
+}
+
 mpm_status mpm_batch_destroy(mpm_batch* b) {
     if (!b) return MPM_ERR_INVALID_ARGUMENT;
     if (b->stream) cudaStreamSynchronize(b->stream);
@@ -456,6 +554,15 @@ mpm_status mpm_batch_info(const mpm_batch* b, int32_t* nscenes, int64_t* total) 
 mpm_status mpm_batch_step(mpm_batch* b, int32_t nsteps) {
     if (!b || nsteps < 0) return MPM_ERR_INVALID_ARGUMENT;
     if (nsteps == 0) return MPM_OK;
+    for (mpm_batch* p : b->parts) {
+        mpm_status st = forget_sums(p);  // the grid was another part's
+        if (st == MPM_OK) st = mpm_batch_step(p, nsteps);
+        if (st != MPM_OK) return answer(b, p, st);
+    }
+    if (!b->parts.empty()) {
+        b->last_steps = nsteps;
+        return MPM_OK;
+    }
     const size_t need = (size_t)b->nscenes * ((size_t)nsteps + 1);
     if (need > b->stamps_cap) {
         drop_graphs(b);
@@ -504,11 +611,16 @@ mpm_status mpm_batch_set_stream(mpm_batch* b, void* stream) {
     if (!b) return MPM_ERR_INVALID_ARGUMENT;
     BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
     b->stream = stream ? (cudaStream_t)stream : b->own_stream;
+    for (mpm_batch* p : b->parts) {
+        const mpm_status st = mpm_batch_set_stream(p, b->stream);
+        if (st != MPM_OK) return answer(b, p, st);
+    }
     return MPM_OK;
 }
 
 mpm_status mpm_batch_get_state(mpm_batch* b, int32_t scene, mpm_state_host* st) {
     if (!valid_scene(b, scene) || !st || st->count != b->counts[scene]) return MPM_ERR_INVALID_ARGUMENT;
+    if (mpm_batch* p = part_of(b, scene)) return answer(b, p, mpm_batch_get_state(p, scene, st));
     float* const host[5] = {st->position, st->velocity, st->affine_b, st->elastic_f, st->plastic_det};
     return read_scene(b, scene, host);
 }
@@ -517,6 +629,7 @@ mpm_status mpm_batch_get_state(mpm_batch* b, int32_t scene, mpm_state_host* st) 
 // sorted and its sums formed anew at the next step.
 mpm_status mpm_batch_set_state(mpm_batch* b, int32_t scene, const mpm_state_host* st) {
     if (!valid_scene(b, scene) || !st || st->count != b->counts[scene]) return MPM_ERR_INVALID_ARGUMENT;
+    if (mpm_batch* p = part_of(b, scene)) return answer(b, p, mpm_batch_set_state(p, scene, st));
     const int n = b->counts[scene];
     const float* given[5] = {st->position, st->velocity, st->affine_b, st->elastic_f, st->plastic_det};
     for (int f = 0; f < 5; ++f)
@@ -544,12 +657,14 @@ mpm_status mpm_batch_set_state(mpm_batch* b, int32_t scene, const mpm_state_host
 mpm_status mpm_batch_get_positions(mpm_batch* b, int32_t scene, float* out, size_t cap_floats) {
     if (!valid_scene(b, scene) || (!out && b->counts[scene] > 0)) return MPM_ERR_INVALID_ARGUMENT;
     if (cap_floats < (size_t)b->counts[scene] * 2) return bfail(b, MPM_ERR_CAPACITY, "output buffer too small");
+    if (mpm_batch* p = part_of(b, scene)) return answer(b, p, mpm_batch_get_positions(p, scene, out, cap_floats));
     float* const host[5] = {out, nullptr, nullptr, nullptr, nullptr};
     return read_scene(b, scene, host);
 }
 
 mpm_status mpm_batch_get_status(mpm_batch* b, int32_t scene, uint32_t* flags) {
     if (!valid_scene(b, scene) || !flags) return MPM_ERR_INVALID_ARGUMENT;
+    if (mpm_batch* p = part_of(b, scene)) return answer(b, p, mpm_batch_get_status(p, scene, flags));
     unsigned f = 0;
     BATCH_CUDA(b, cudaMemcpyAsync(&f, b->arr.status + scene, sizeof(f), cudaMemcpyDeviceToHost, b->stream));
     BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
@@ -563,6 +678,13 @@ mpm_status mpm_batch_step_times(mpm_batch* b, uint64_t* out, size_t cap, int32_t
     const size_t steps = (size_t)b->last_steps + 1, k = (size_t)b->nscenes;
     if (b->last_steps == 0) return MPM_OK;
     if (!out || cap < steps * k) return bfail(b, MPM_ERR_CAPACITY, "output buffer too small");
+    for (size_t p = 0; p < b->parts.size(); ++p) {
+        int32_t ns = 0;
+        const size_t at = steps * (size_t)b->part_first[p];
+        const mpm_status st = mpm_batch_step_times(b->parts[p], out + at, cap - at, &ns);
+        if (st != MPM_OK) return answer(b, b->parts[p], st);
+    }
+    if (!b->parts.empty()) return MPM_OK;
     std::vector<unsigned long long> t(steps * k);  // [step][scene] on the device
     BATCH_CUDA(b, cudaMemcpyAsync(t.data(), b->arr.stamps, sizeof(uint64_t) * t.size(), cudaMemcpyDeviceToHost, b->stream));
     BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
@@ -573,17 +695,38 @@ mpm_status mpm_batch_step_times(mpm_batch* b, uint64_t* out, size_t cap, int32_t
 
 mpm_status mpm_batch_get_config(const mpm_batch* b, mpm_batch_config* cfg) {
     if (!b || !cfg) return MPM_ERR_INVALID_ARGUMENT;
-    *cfg = b->cfg;
+    *cfg = b->parts.empty() ? b->cfg : b->parts[0]->cfg;
     return MPM_OK;
 }
 
 mpm_status mpm_batch_set_config(mpm_batch* b, const mpm_batch_config* cfg) {
     if (!b || !cfg) return MPM_ERR_INVALID_ARGUMENT;
-    return configure(b, *cfg);
+    if (b->parts.empty()) return configure(b, *cfg);
+    const mpm_batch_config old = b->parts[0]->cfg;
+    for (mpm_batch* p : b->parts) {
+        const mpm_status st = configure(p, *cfg);
+        if (st == MPM_OK) continue;
+        answer(b, p, st);
+        for (mpm_batch* q : b->parts) configure(q, old);
+        return st;
+    }
+    return MPM_OK;
 }
 
 mpm_status mpm_batch_tune(mpm_batch* b, int32_t trial_steps, mpm_batch_config* chosen, double* best_ms) {
     if (!b || trial_steps < 1) return MPM_ERR_INVALID_ARGUMENT;
+    if (!b->parts.empty()) {
+        double sum = 0.0;
+        for (mpm_batch* p : b->parts) {
+            double ms = 0.0;
+            mpm_status st = forget_sums(p);
+            if (st == MPM_OK) st = mpm_batch_tune(p, trial_steps, chosen, &ms);
+            if (st != MPM_OK) return answer(b, p, st);
+            sum += ms;
+        }
+        if (best_ms) *best_ms = sum;
+        return MPM_OK;
+    }
     BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
     const size_t n = (size_t)b->N;
     // Snapshot of the particles and flags; the sums are formed anew from them.

@@ -215,7 +215,7 @@ void swap_buffers(mpm_solver* s) {
     std::swap(s->B, s->alt.B);
     std::swap(s->Fe, s->alt.Fe);
     std::swap(s->Jp, s->alt.Jp);
-    std::swap(s->A, s->alt.A);
+    if (s->alt.A) std::swap(s->A, s->alt.A);  // the split path's
     std::swap(s->id, s->alt.id);
     if (s->mass) std::swap(s->mass, s->alt.mass);
     if (s->vol) std::swap(s->vol, s->alt.vol);
@@ -241,13 +241,10 @@ template <int D, int S> cudaError_t launch_sort(mpm_solver* s) {
     if (e == cudaSuccess) e = launch_chained(k_sort_scan, scan_blocks, kScanTiles, 0, s->stream, s->ti);
     if (e == cudaSuccess) e = launch_chained(k_sort_bucket, blocks, threads, 0, s->stream, s->n, s->ti);
     if (e != cudaSuccess) return e;
-    SortBuffers dst = s->alt;
-    if (s->fused) {
-        dst.A = nullptr;  // the fused path keeps A only within a step
-        // with the grid sums pending the next G2P writes v and B unread: 48 of 104
-        // bytes a particle stay (sort by cell of 1.65M: 150 -> 85 us, of 3.8M: 300 -> 164)
-        if (s->acc_pending) dst.v = dst.B = nullptr;
-    }
+    SortBuffers dst = s->alt;  // (no A on the fused path, which keeps it only within a step)
+    // with the grid sums pending the next G2P writes v and B unread: 48 of 104
+    // bytes a particle stay (sort by cell of 1.65M: 150 -> 85 us, of 3.8M: 300 -> 164)
+    if (s->fused && s->acc_pending) dst.v = dst.B = nullptr;
     e = launch_chained(k_tile_sort<D, S, OneScene>, s->sms * SortGeom<D>::CTAS_PER_SM, 256, 0, s->stream, particle_view(s),
                        s->id, dst, scene, s->ti);
     if (e != cudaSuccess) return e;
@@ -414,10 +411,6 @@ size_t windows_smem(int dim) {
 // The fused kernel over the tiles of the last sort: G2P (this step) + P2G (next
 // step), or with G2P = false the P2G of the stored state (prologue).
 template <int D, int S, bool G2P> cudaError_t launch_fused(mpm_solver* s) {
-    if (!G2P) {  // the step's grid update clears the counters (k_grid_marked)
-        cudaError_t e = cudaMemsetAsync(s->ti.fused_next, 0, sizeof(int), s->stream);
-        if (e != cudaSuccess) return e;
-    }
     if (s->n == 0) return cudaSuccess;
     if (G2P && !s->direct)
         return launch_chained(k_g2p2g_pipe<D, S>, s->sms * PipeGeom<D>::CTAS, PipeGeom<D>::THREADS, sizeof(PipeSmem<D>),
@@ -511,9 +504,9 @@ cudaError_t clear_after_p2g(mpm_solver* s) {
 }
 
 
-// The tensor map of the TMA pipeline's box loads (k_g2p2g_pipe): gv's first
-// half (one float4 per node: (vf, wall flag) in 3D, (vf, vc) in 2D) as a rank
-// D+1 FP32 tensor [nz][ny][nx][4], boxes of 4 x BE^D. The encoder comes from the driver through the runtime, so the
+// The tensor map of the TMA pipeline's box loads (k_g2p2g_pipe): gv as FP32 rows of 4,
+// [2][nz][ny][nx][4] in 3D (both halves: (vf, wall flag) and the wall velocities),
+// [ny][nx][4] in 2D ((vf, vc)), boxes of BE^D nodes of one half. The encoder comes from the driver through the runtime, so the
 // library needs no link to libcuda.
 using EncodeTiledFn = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                    const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -562,9 +555,15 @@ mpm_status setup_tiled(mpm_solver* s) {
     arena.want(&ti.key, N).want(&ti.tile_count, tiles).want(&ti.tile_cursor, tiles).want(&ti.tile_start, tiles);
     arena.want(&ti.mark, blocks).want(&ti.mark_list, blocks).want(&ti.n_marked, 1).want(&ti.p2g_next, 1);
     arena.want(&ti.perm, N).want(&ti.tile_list, tiles).want(&ti.n_tile_list, 1).want(&ti.skey, N).want(&ti.sval, N);
+    {
+        // MPM_TRANSFER=split selects the separate P2G / G2P kernels (for comparison)
+        const char* tr = std::getenv("MPM_TRANSFER");
+        s->fused = !(tr && std::strcmp(tr, "split") == 0);
+    }
     // (x to J_p one behind the other here and in mpm_create: scratch())
     arena.want(&s->alt.x, N * D).want(&s->alt.v, N * D).want(&s->alt.B, N * D * D).want(&s->alt.Fe, N * D * D);
-    arena.want(&s->alt.Jp, N).want(&s->alt.id, N).want(&s->A, N * D * D).want(&s->alt.A, N * D * D);
+    arena.want(&s->alt.Jp, N).want(&s->alt.id, N).want(&s->A, N * D * D);
+    if (!s->fused) arena.want(&s->alt.A, N * D * D);
     if (s->mass) arena.want(&s->alt.mass, N);
     if (s->vol) arena.want(&s->alt.vol, N);
     if (!arena.allocate()) return MPM_ERR_OUT_OF_MEMORY;
@@ -594,11 +593,6 @@ mpm_status setup_tiled(mpm_solver* s) {
         s->p2g_warp_grid = s->sms * per;
     }
     s->q.capacity = n > 0 ? n : 1;
-    {
-        // MPM_TRANSFER=split selects the separate P2G / G2P kernels (for comparison)
-        const char* tr = std::getenv("MPM_TRANSFER");
-        s->fused = !(tr && std::strcmp(tr, "split") == 0);
-    }
     // Window length of the fused transfer by how the scene's windows compare with
     // the warps the GPU holds (5 CTAs of 4 per SM): a warp works through a window's
     // stencils one after the other, so a scene of few windows takes shorter ones.
@@ -1423,7 +1417,7 @@ mpm_status mpm_load_state(mpm_solver* s, const char* path) {
             const int ntl = (int)tiles.size();
             std::vector<int> tl(ntl), tlen(ntl), tstart(s->ti.n_tiles, 0);
             std::vector<int4> items;  // as k_sort_scan lists them
-            const int step = s->ti.item_win ? s->ti.win * s->ti.item_win : (int)n;
+            const int step = s->ti.win * s->ti.item_win;
             for (int e = 0; e < ntl; ++e) {
                 tl[e] = tiles[e].x;
                 tlen[e] = tiles[e].z;

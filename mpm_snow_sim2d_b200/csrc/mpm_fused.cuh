@@ -2,11 +2,11 @@
 // one kernel per step (the G2P2G scheme of Wang et al., "A Massively Parallel
 // and Scalable Multi-GPU Material Point Method", ACM TOG 39(4), 2020).
 //
-// Work is handed out as items. In k_g2p2g_pipe an item is a non-empty cell tile of
-// the last sort: a CTA has the node velocities of a fixed box of BE^D nodes around
-// the tile in shared memory (the stencils of every particle sorted into the tile
-// that has since moved less than a cell), loaded one tile ahead by TMA tensor loads
-// (cp.async.bulk.tensor, out-of-grid nodes zero-filled); its warps meet at
+// Work is handed out as items. In k_g2p2g_pipe an item is up to 32 windows of a cell
+// tile of the last sort (nearly always all of it): a CTA has the node velocities of a fixed
+// box of BE^D nodes around the tile in shared memory (the stencils of every particle sorted
+// into the tile that has since moved less than a cell), loaded one item ahead by TMA tensor
+// loads (cp.async.bulk.tensor, out-of-grid nodes zero-filled); its warps meet at
 // mbarriers only. In k_g2p2g_direct an item is one window and nothing is staged.
 // Each warp, on its own, takes windows of up to 32 consecutive slots of a tile
 // and for its window
@@ -788,7 +788,7 @@ __device__ __forceinline__ void mark_tile_blocks(const TileInfo& TI, const int* 
 }
 
 // ---------------------------------------------------------------------------
-// Window w (slots start + 32 w ...) of a tile of m slots, by one warp: G2P of
+// Window w (slots start + win w ...) of an item of m slots, by one warp: G2P of
 // each slot's particle against the tile's node box (G2P = true) or the stored
 // state (G2P = false), then the scatter of the in-band particles' payloads.
 // Returns this lane's node-block bits around the tile (box origin bo). DIRECT:
@@ -999,24 +999,24 @@ __global__ void __launch_bounds__(FusedGeom<D>::THREADS, MPM_FUSED_MIN_BLOCKS)
 
 // ---------------------------------------------------------------------------
 // The fused step with staged node boxes: persistent CTAs, each a pipeline of
-// tiles. Stage k (tile k of the CTA) lives in buffer k % STAGES: its item, its
+// items. Stage k (item k of the CTA) lives in buffer k % STAGES: its item, its
 // box of node velocities and, where the tile is near the domain's walls, the box of
 // wall velocities (TMA tensor loads, whose mbarrier `full` completes when the bytes
 // have landed), a window counter, a count of the warps that have left it, and its
-// node-block bits. Each warp waits for the stage's box, takes windows of the tile
+// node-block bits. Each warp waits for the stage's box, takes windows of the item
 // until none are left, and moves on to stage k + 1, which is already loaded; the
 // last warp to leave stage k marks the tile's node blocks and refills the buffer
-// with stage k + STAGES (the next tile from the global counter, or an empty stage
+// with stage k + STAGES (the next item from the global counter, or an empty stage
 // that ends the CTA). A warp is thus held up only by a box that has not arrived,
 // never by the other warps' windows. Stages are refilled in order (a warp that
-// refills stage k has not left stage k + 1 yet), so tile numbers grow with the stage
+// refills stage k has not left stage k + 1 yet), so item numbers grow with the stage
 // and the first empty stage ends the work for every warp. Every wait is bounded: a
 // box that does not arrive raises MPM_FLAG_TIMEOUT.
 //
 // Bound: instruction issue and the shared-memory pipe at 20 warps per SM (96
 // registers). 1.65M particles, snowball above a slab on the floor: 308 us with one
 // buffer per CTA of 4 warps, filled by the CTA between two barriers (the kernel this
-// one replaces), 300 now, of which the wall boxes give 13 (particles near a wall
+// one replaces), 300 with this one (286 since the gather is in packed FP32), of which the wall boxes give 13 (particles near a wall
 // otherwise read vc from L2 node by node); 3.8M in collision: 537 and 502. One CTA
 // of 20 warps and 4 stages: 303 and 518 (all warps of an SM then add to the same
 // nodes); 4 CTAs of 5 warps, which leave no room for wall boxes: 318 and 490.

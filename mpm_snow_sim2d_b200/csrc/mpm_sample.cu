@@ -78,10 +78,11 @@ __device__ __forceinline__ bool inside(const SampleShapes& S, int dim, const flo
 // the phases run one after the other (30 rounds x 27 of them); with one thread per
 // cell the 125 neighbours were read one after the other, 23 us a phase; here all
 // of a cell's are in flight at once and a phase takes 4.4 us. The launch of the
-// next phase overlaps this one up to griddepcontrol.wait: the candidate, and
-// whether the cell is free (only its own phase, a round ago, can have filled it),
-// depend on nothing later. Reads of `cells` go to L2, since lines read before
-// the wait may hold neighbours of that phase.
+// next phase overlaps this one up to griddepcontrol.wait: the candidate depends on
+// nothing. A cell found filled before the wait stays filled; one found free may have
+// been filled since, by its own phase of the round before, which need not be complete
+// while phases overlap: the test after the wait includes the cell itself. Reads of
+// `cells` go to L2, since lines read before the wait may hold neighbours of earlier phases.
 constexpr int kCellLanes = 8;
 
 __global__ void __launch_bounds__(256, 2) k_sample_phase(SampleGrid G, const SampleShapes* __restrict__ shapes,
@@ -127,6 +128,7 @@ __global__ void __launch_bounds__(256, 2) k_sample_phase(SampleGrid G, const Sam
 #pragma unroll
             for (int dx = 0; dx < 5; ++dx) {
                 const float ddx = __fsub_rn(n[dx].x, p[0]), ddy = __fsub_rn(n[dx].y, p[1]), ddz = __fsub_rn(n[dx].z, p[2]);
+                clash = clash || (n[dx].w != 0.f && r == rows / 2 && dx == 2);  // the cell itself
                 clash = clash || (n[dx].w != 0.f &&
                                   __fadd_rn(__fadd_rn(__fmul_rn(ddx, ddx), __fmul_rn(ddy, ddy)), __fmul_rn(ddz, ddz)) < r2);
             }

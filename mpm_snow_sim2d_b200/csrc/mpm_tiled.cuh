@@ -39,10 +39,9 @@ struct TileInfo {
     int* n_tile_list;  // device scalar
     int* p2g_next;     // device scalar: next P2G chunk to hand out (zeroed before each P2G)
     int* tile_len;     // per entry of tile_list: particles of that tile at the last sort
-    int* fused_next;   // device scalar: next item of the fused transfer (zeroed before each launch)
-    // Work of the fused transfer: (tile, first slot, slots) of at most item_win
-    // (0: all of the tile's) windows of `win` slots each. Which slots form a window
-    // depends on the tile's start alone.
+    int* fused_next;   // device scalar: next item of k_g2p2g_pipe (cleared by the grid update)
+    // Work of the fused transfer: (tile, first slot, slots) of at most item_win windows
+    // of `win` slots each. Which slots form a window depends on the tile's start alone.
     int4* items;
     int* n_items;      // device scalar
     int win, item_win;
@@ -124,7 +123,6 @@ __global__ void __launch_bounds__(256) k_sort_count(Particles P, SC scenes, Tile
 constexpr int kScanTiles = 1024;
 
 __device__ __forceinline__ int tile_items(const TileInfo& TI, int count) {
-    if (count == 0 || TI.item_win == 0) return count > 0;
     const int w = (count + TI.win - 1) / TI.win;
     return (w + TI.item_win - 1) / TI.item_win;
 }
@@ -195,7 +193,7 @@ static __global__ void __launch_bounds__(kScanTiles) k_sort_scan(TileInfo TI) {
         TI.tile_start[t] = start;
         TI.tile_cursor[t] = 0;
         if (c > 0) TI.tile_list[s_before[1] + v[1] - 1] = t;  // non-empty tiles in tile order
-        const int step = TI.item_win ? TI.win * TI.item_win : c;
+        const int step = TI.win * TI.item_win;
         for (int k = 0; k < ni; ++k)
             TI.items[s_before[2] + v[2] - ni + k] = make_int4(t, start + k * step, min(step, c - k * step), TI.tile_scene ? TI.tile_scene[t] : 0);
     }

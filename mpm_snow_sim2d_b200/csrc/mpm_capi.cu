@@ -30,7 +30,8 @@ struct mpm_mlp {
     float* w = nullptr;            // fp32 master parameters
     __nv_bfloat16* wbf = nullptr;  // bf16 copy used by the kernels
     float* grad = nullptr;
-    float* part = nullptr;         // per training CTA: its gradients and loss (made by the first training call)
+    float* part = nullptr;         // per training CTA: its gradients and loss (mlp_want_part)
+    float* part_own = nullptr;     // part's allocation, unless it lies behind the pairs
     int part_rows = 0;
     float* m1 = nullptr;
     float* m2 = nullptr;
@@ -1540,7 +1541,7 @@ mpm_status mpm_mlp_create(uint64_t seed, mpm_mlp** out) {
 
 mpm_status mpm_mlp_destroy(mpm_mlp* m) {
     if (!m) return MPM_ERR_INVALID_ARGUMENT;
-    void* ptrs[] = {m->w, m->wbf, m->grad, m->part, m->m1, m->m2, m->loss, m->pairs};
+    void* ptrs[] = {m->w, m->wbf, m->grad, m->part_own, m->m1, m->m2, m->loss, m->pairs};
     for (void* p : ptrs)
         if (p) cudaFree(p);
     delete m;
@@ -1597,8 +1598,23 @@ mpm_status mpm_mlp_load_pairs(mpm_mlp* m, const float* pairs, int64_t n) {
     if (m->pairs) cudaFree(m->pairs);
     m->pairs = nullptr;
     m->n_pairs = 0;
+    if (m->part != m->part_own) {
+        m->part = nullptr;
+        m->part_rows = 0;
+    }
     if (n == 0) return MPM_OK;
-    if (dalloc(&m->pairs, (size_t)n * 20)) { cudaGetLastError(); return MPM_ERR_OUT_OF_MEMORY; }
+    // A larger allocation takes no longer than a smaller one (0.3 ms from 1 MB on), so a set of
+    // pairs brings along the room that training on it needs.
+    const size_t floats = ((size_t)n * 20 + 63) / 64 * 64;
+    const bool room = m->part == nullptr && floats * sizeof(float) >= (1u << 20);
+    if (dalloc(&m->pairs, floats + (room ? (size_t)kMlpTrainCtas * kMlpPart : 0))) {
+        cudaGetLastError();
+        return MPM_ERR_OUT_OF_MEMORY;
+    }
+    if (room) {
+        m->part = m->pairs + floats;
+        m->part_rows = kMlpTrainCtas;
+    }
     if (cudaMemcpy(m->pairs, pairs, sizeof(float) * 20 * (size_t)n, cudaMemcpyHostToDevice) != cudaSuccess) {
         cudaGetLastError();
         return MPM_ERR_CUDA;
@@ -1609,19 +1625,20 @@ mpm_status mpm_mlp_load_pairs(mpm_mlp* m, const float* pairs, int64_t n) {
 
 static int mlp_ctas(int rows) { return std::min((rows - 1) / kMlpTrainRows + 1, kMlpTrainCtas); }
 
-// Room in m->part for the CTAs of a launch over `rows` samples. Made when a network is
-// first trained, and no larger than asked: 6 MB take 0.7 ms to allocate, most of what a network
-// loaded for inference would take to create.
+// Room in m->part for the CTAs of a launch over `rows` samples: behind the pairs, else
+// made when it is first needed. A network that is loaded for inference has none; allocating
+// it would take most of the time of creating one.
 static bool mlp_want_part(mpm_mlp* m, int rows) {
     const int ctas = mlp_ctas(rows);
     if (ctas <= m->part_rows) return true;
-    if (m->part) cudaFree(m->part);
+    if (m->part_own) cudaFree(m->part_own);
     m->part = nullptr;
     m->part_rows = 0;
-    if (dalloc(&m->part, (size_t)ctas * kMlpPart)) {
+    if (dalloc(&m->part_own, (size_t)ctas * kMlpPart)) {
         cudaGetLastError();
         return false;
     }
+    m->part = m->part_own;
     m->part_rows = ctas;
     return true;
 }

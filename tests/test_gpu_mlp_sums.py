@@ -66,3 +66,36 @@ def test_creating_a_network_takes_little_memory(net):
     kept = free()
     other.gradient(pairs[:4096])
     assert free() == kept
+
+
+@pytest.mark.parametrize("count", [1000, 13108])  # 80 KB of pairs; 1 MB and one row
+def test_first_training_allocates_nothing_behind_a_large_set(net, count):
+    """A set of pairs of 1 MB or more brings the room for training's partial sums with it. Sets that follow one another
+    leave a network that trains as a new one with the last set."""
+    import torch
+    from mpm_snow_sim2d_b200 import mlp
+
+    def free():
+        torch.cuda.synchronize()
+        return torch.cuda.mem_get_info()[0]
+
+    m, pairs = net
+    sets = [synthetic_pairs(k, seed=k) for k in (count, 20000, 500, count)]
+
+    def train(net_, p):
+        net_.set_params(m.params())
+        net_.set_normalization(*m.norm)
+        net_.load_pairs(p)
+        before = free()
+        losses = net_.train(2, 16384, 1e-3, 1e-4, seed=5)
+        return before - free(), np.concatenate([net_.params(), np.asarray(losses, np.float32)])
+
+    used = mlp.Mlp(seed=1)
+    for k, p in enumerate(sets):
+        taken, got = train(used, p)
+        if k == 0:
+            assert (taken <= 2 << 20) == (count > 13107)
+        fresh = mlp.Mlp(seed=2)
+        _, want = train(fresh, p)
+        assert np.array_equal(got, want) and np.isfinite(got).all()
+        assert np.array_equal(used.gradient(p[:300])[0], fresh.gradient(p[:300])[0])

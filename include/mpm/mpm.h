@@ -381,7 +381,9 @@ MPM_API mpm_status mpm_batch_destroy(mpm_batch* batch);
 MPM_API const char* mpm_batch_last_error(const mpm_batch* batch);
 MPM_API mpm_status mpm_batch_info(const mpm_batch* batch, int32_t* nscenes, int64_t* total_particles);
 /* Advance every scene by nsteps (asynchronous on the batch's stream; a CUDA graph
- * per stretch of steps between sorts, replayed). */
+ * per stretch of steps between sorts, replayed). The stream may be under capture if
+ * a call of at least as many steps has been made before: the captured steps can be
+ * replayed any number of times, with other calls in between. */
 MPM_API mpm_status mpm_batch_step(mpm_batch* batch, int32_t nsteps);
 MPM_API mpm_status mpm_batch_set_stream(mpm_batch* batch, void* cuda_stream);
 /* Per-scene state, host copies in the scene's creation order (as mpm_get_state). */

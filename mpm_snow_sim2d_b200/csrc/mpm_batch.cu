@@ -60,6 +60,9 @@ struct mpm_batch {
     bool needs_sort = true;
     bool any_fresh = true;           // a scene has no pending grid sums (arr.fresh)
     bool unfinished = false;         // a step call failed on its way (recover)
+    bool sorted = false;             // there are items to step
+    int captured = -1;               // the buffer that steps captured by the caller work on
+    std::vector<unsigned long long*> old_stamps;  // which they write to
     cudaStream_t stream = nullptr, own_stream = nullptr;
     mpm_batch_config cfg{};
     int cap_max = 0;                 // nodes per CTA of the largest scene's cluster (limit on a scene's grid)
@@ -114,6 +117,7 @@ void release(mpm_batch* b) {
     b->part_first.clear();
     drop_graphs(b);
     if (b->arr.stamps) cudaFree(b->arr.stamps);
+    for (unsigned long long* p : b->old_stamps) cudaFree(p);
     b->arena.release();
     if (b->own_stream) cudaStreamDestroy(b->own_stream);
 }
@@ -146,7 +150,10 @@ cudaError_t enqueue_sort(mpm_batch* b, bool pending) {
     const SortBuffers dst{t.x, pending ? nullptr : t.v, pending ? nullptr : t.B, t.Fe, t.Jp, nullptr, t.mass, t.vol, t.id};
     e = launch_chained(k_tile_sort<2, 4, ManyScenes>, b->sms * SortGeom<2>::CTAS_PER_SM, 256, 0, b->stream, P,
                        b->buf[b->parity].id, dst, b->many, b->ti);
-    if (e == cudaSuccess) b->parity ^= 1;
+    if (e == cudaSuccess) {
+        b->parity ^= 1;
+        b->sorted = true;
+    }
     return e;
 }
 
@@ -210,6 +217,32 @@ mpm_status run_segment(mpm_batch* b, int steps, bool sort) {
 }
 
 int sort_period(const mpm_batch* b) { return b->cfg.sort_period > 0 ? b->cfg.sort_period : 16; }
+
+// A call on a stream that is being captured: direct launches, so that the caller's graph
+// can be replayed any number of times, also after uploads. Nothing runs now, so
+// the host's account of the batch stays; the sums of uploaded states are formed where
+// the device says so (arr.fresh), and sorts, on which no result depends, come in pairs,
+// which leave the particles in the buffer they started in (from here on plain calls
+// leave them there as well). A short call has none.
+mpm_status capture_steps(mpm_batch* b, int steps) {
+    if (!b->sorted) return bfail(b, MPM_ERR_CUDA, "a batch is stepped once before its steps are captured");
+    if (b->N > 0)
+        k_batch_step<false><<<b->sms * MPM_FUSED_MIN_BLOCKS, FusedGeom<2>::THREADS, 0, b->stream>>>(particles(b), b->arr, b->ti,
+                                                                                                   b->q);
+    BATCH_CUDA(b, cudaGetLastError());
+    BATCH_CUDA(b, cudaMemsetAsync(b->arr.fresh, 0, sizeof(int) * (size_t)b->nscenes, b->stream));
+    const int period = sort_period(b);
+    const int sorts = steps >= period ? 2 * ((steps - 1) / (2 * period) + 1) : 0;
+    if (sorts == 0) BATCH_CUDA(b, enqueue_segment(b, steps, false));
+    for (int k = 0; k < sorts; ++k) {
+        const int n = (int)((long long)steps * (k + 1) / sorts - (long long)steps * k / sorts);
+        if (n > 0) BATCH_CUDA(b, enqueue_segment(b, n, true));
+    }
+    k_batch_end<<<1, 256, 0, b->stream>>>(b->arr);
+    BATCH_CUDA(b, cudaGetLastError());
+    b->captured = b->parity;
+    return MPM_OK;
+}
 
 // Memory for one call that waits for the stream before it returns: between sorts the
 // other buffer is free, its x, v, B, F_E and J_p one behind the other (a whole state).
@@ -567,7 +600,8 @@ mpm_status mpm_batch_step(mpm_batch* b, int32_t nsteps) {
     if (need > b->stamps_cap) {
         drop_graphs(b);
         BATCH_CUDA(b, cudaStreamSynchronize(b->stream));
-        if (b->arr.stamps) cudaFree(b->arr.stamps);
+        if (b->arr.stamps && b->captured >= 0) b->old_stamps.push_back(b->arr.stamps);
+        else if (b->arr.stamps) cudaFree(b->arr.stamps);
         b->arr.stamps = nullptr;
         b->stamps_cap = 0;
         BATCH_CUDA(b, balloc(&b->arr.stamps, need));
@@ -579,6 +613,13 @@ mpm_status mpm_batch_step(mpm_batch* b, int32_t nsteps) {
     }
     b->unfinished = true;
     b->last_steps = nsteps;
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    BATCH_CUDA(b, cudaStreamIsCapturing(b->stream, &capture));
+    if (capture != cudaStreamCaptureStatusNone) {
+        const mpm_status st = capture_steps(b, nsteps);
+        b->unfinished = st != MPM_OK;
+        return st;
+    }
     if (b->any_fresh) {
         // sums of the new states: sort, then their P2G
         BATCH_CUDA(b, enqueue_sort(b, false));
@@ -600,6 +641,10 @@ mpm_status mpm_batch_step(mpm_batch* b, int32_t nsteps) {
         b->since_sort = (sort ? 0 : b->since_sort) + len;
         b->needs_sort = false;
         left -= len;
+    }
+    if (b->captured >= 0 && b->parity != b->captured && b->N > 0) {
+        BATCH_CUDA(b, enqueue_sort(b, false));
+        b->since_sort = 0;
     }
     k_batch_end<<<1, 256, 0, b->stream>>>(b->arr);
     BATCH_CUDA(b, cudaGetLastError());

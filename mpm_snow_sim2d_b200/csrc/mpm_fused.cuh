@@ -510,11 +510,20 @@ __device__ __forceinline__ void sum_rows(ScatterLane<D, S, EXACT>& T, const floa
 
 // P2G of a particle part of whose stencil is outside the grid, by one lane: its
 // nodes inside the grid one by one, and their blocks.
-template <int D, int S>
+template <int D, int S, bool EXACT>
 __device__ __forceinline__ void scatter_clipped(const StepConsts& C, const TileInfo& TI, const float* x, const int* base,
                                                 const float* v, const float* A, float mass,
                                                 unsigned long long* __restrict__ acc, unsigned* __restrict__ status) {
     constexpr int TE = TileGeom<D>::T;
+    float top = 0.f;
+    auto add = [&](unsigned long long* p, float t) {
+        if constexpr (EXACT) {
+            red_int(p, to_fixed(t, 1.f, status));
+        } else {
+            red_scaled(p, t);
+            top = fmaxf(top, fabsf(t));
+        }
+    };
 #pragma unroll 1
     for (int j = 0; j < (D == 3 ? S * S * S : S * S); ++j) {
         const int gx = base[0] + j % S, gy = base[1] + (j / S) % S, gz = D == 3 ? base[2] + j / (S * S) : 0;
@@ -523,17 +532,18 @@ __device__ __forceinline__ void scatter_clipped(const StepConsts& C, const TileI
         float w = Stencil<S>::w(d[0]) * Stencil<S>::w(d[1]);
         if (D == 3) w *= Stencil<S>::w(d[2]);
         unsigned long long* n = acc + (((long long)gz * C.ny + gy) * C.nx + gx) * 4;
-        red_int(n + 2, to_fixed(w * mass, C.sm, status));
+        add(n + 2, w * mass * C.sm);
 #pragma unroll
         for (int r = 0; r < D; ++r) {
             float s = mass * v[r];
 #pragma unroll
             for (int k = 0; k < D; ++k) s += A[r * D + k] * d[k];
-            red_int(n + (r < 2 ? r : 3), to_fixed(w * s, C.sp, status));
+            s *= w * C.sp;
+            add(n + (r < 2 ? r : 3), s);
         }
         mark_block_once(TI, ((D == 3 ? gz / TE : 0) * TI.nblk[1] + gy / TE) * TI.nblk[0] + gx / TE);
     }
-    raise_flag(status, 4u);
+    raise_flag(status, top < kFixedLimit ? 4u : 4u | 2u);
 }
 
 // The ordered rows of a window (`total` of them) into the grid. Whole warp.
@@ -667,7 +677,7 @@ __device__ __forceinline__ void queued_window(const Particles& P, const StepCons
         for (int k = 0; k < D * D; ++k) A[k] = P.A[k * n + i];
         key = stencil_key<D, S>(C, x, base);
         if (key == kClipped) {
-            scatter_clipped<D, S>(C, TI, x, base, v, A, mass, acc, status);
+            scatter_clipped<D, S, EXACT>(C, TI, x, base, v, A, mass, acc, status);
             key = kNoKey;
         } else if (unmarked) {
             mark_stencil<D, S>(TI, base);
@@ -922,7 +932,7 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
                 else mark_stencil<D, S>(TI, nbase);
                 if (scatter) key = k;
             } else if (scatter) {
-                scatter_clipped<D, S>(C, TI, x, nbase, v, A, mass, acc, status);
+                scatter_clipped<D, S, EXACT>(C, TI, x, nbase, v, A, mass, acc, status);
             } else if (EXACT && !deferred) {
                 mark_clipped<D, S>(C, TI, nbase);
             }

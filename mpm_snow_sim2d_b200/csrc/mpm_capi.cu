@@ -1392,8 +1392,21 @@ mpm_status mpm_load_state(mpm_solver* s, const char* path) {
     std::fclose(f);
     if (!ok) return fail(s, MPM_ERR_IO, "truncated or corrupt checkpoint");
     const bool restore_order = has_order && s->tiled;
-    if (restore_order && n > 0)
+    if (restore_order && n > 0) {
+        // masses and volumes, which the file does not hold, follow their particles into
+        // the restored order
+        std::vector<int> now(n);
+        std::vector<float> slot(n), own(n);
+        if (s->mass || s->vol) MPM_CUDA(s, cudaMemcpy(now.data(), s->id, sizeof(int) * n, cudaMemcpyDeviceToHost));
+        for (float* field : {s->mass, s->vol}) {
+            if (!field) continue;
+            MPM_CUDA(s, cudaMemcpy(slot.data(), field, sizeof(float) * n, cudaMemcpyDeviceToHost));
+            for (size_t i = 0; i < n; ++i) own[now[i]] = slot[i];
+            for (size_t i = 0; i < n; ++i) slot[i] = own[ids[i]];
+            MPM_CUDA(s, cudaMemcpy(field, slot.data(), sizeof(float) * n, cudaMemcpyHostToDevice));
+        }
         MPM_CUDA(s, cudaMemcpy(s->id, ids.data(), sizeof(int) * n, cudaMemcpyHostToDevice));
+    }
     mpm_state_host st{(int64_t)n, x.data(), v.data(), B.data(), Fe.data(), Jp.data()};
     mpm_status r = mpm_set_state(s, &st);
     if (r != MPM_OK) return r;

@@ -72,26 +72,32 @@ __device__ __forceinline__ bool inside(const SampleShapes& S, int dim, const flo
     return false;
 }
 
-// One phase of one round: cells (3a + px, 3b + py, 3c + pz), eight lanes each.
-// The lanes share the cell's candidate and split its 5^(dim-1) rows of five
-// neighbours. Bound: latency. A phase of a reference snowball has 4.6k cells, and
-// the phases run one after the other (30 rounds x 27 of them); with one thread per
-// cell the 125 neighbours were read one after the other, 23 us a phase; here all
-// of a cell's are in flight at once and a phase takes 4.4 us. The launch of the
-// next phase overlaps this one up to griddepcontrol.wait: the candidate depends on
-// nothing. A cell found filled before the wait stays filled; one found free may have
-// been filled since, by its own phase of the round before, which need not be complete
-// while phases overlap: the test after the wait includes the cell itself. Reads of
-// `cells` go to L2, since lines read before the wait may hold neighbours of earlier phases.
-constexpr int kCellLanes = 8;
+// One phase of one round: cells (3a + px, 3b + py, 3c + pz), LANES lanes each.
+// Small grids are bound by latency: a phase of a reference snowball has 8k cells, and
+// the phases run one after the other (30 rounds x 27 of them). Eight lanes share the
+// cell's candidate and split its 5^(dim-1) rows of five neighbours, so that all of a
+// cell's are in flight at once: 5.8 us a phase, 12 with one lane, 28 with one lane that
+// reads one neighbour after the other. Large grids are bound by issue, and most of
+// their cells are filled, or have a sample too near among the first neighbours: one lane
+// reads row by row and stops. Whole calls (3D, 30 rounds; 8 lanes, 1): 524k cells 8.7, 10.6 ms; 1.0M 14.5,
+// 11.9; 4.1M 51, 25; 64M 939, 150 (a neighbour at a time: 536). 2D: 81k 1.66, 1.75; 321k 4.2, 2.5;
+// 8.0M 93, 11 (90).
+// The launch of the next phase overlaps this one up to griddepcontrol.wait: the
+// candidate depends on nothing. A cell found filled before the wait stays filled; one
+// found free may have been filled since, by its own phase of the round before, which
+// need not be complete while phases overlap: the test after the wait includes the cell
+// itself. Reads of `cells` go to L2, since lines read before the wait may hold
+// neighbours of earlier phases.
+constexpr long long kManyLanes2 = 10240, kManyLanes3 = 24576;  // cells of a phase up to which eight lanes are faster
 
-__global__ void __launch_bounds__(256, 2) k_sample_phase(SampleGrid G, const SampleShapes* __restrict__ shapes,
+template <int LANES>
+__global__ void __launch_bounds__(256, LANES > 1 ? 2 : 6) k_sample_phase(SampleGrid G, const SampleShapes* __restrict__ shapes,
                                                       const unsigned char* __restrict__ live, int round, int px, int py,
                                                       int pz, float4* cells) {
     const int mx = (G.nc[0] - px + 2) / 3, my = (G.nc[1] - py + 2) / 3, mz = G.dim == 3 ? (G.nc[2] - pz + 2) / 3 : 1;
     const long long total = (long long)mx * my * mz;
-    const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / kCellLanes;
-    const int sub = threadIdx.x % kCellLanes;
+    const long long t = ((long long)blockIdx.x * blockDim.x + threadIdx.x) / LANES;
+    const int sub = threadIdx.x % LANES;
     const int ix = 3 * int(t % mx) + px, iy = 3 * int((t / mx) % my) + py, iz = G.dim == 3 ? 3 * int(t / ((long long)mx * my)) + pz : 0;
     const long long id = ((long long)iz * G.nc[1] + iy) * G.nc[0] + ix;
     asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -113,9 +119,10 @@ __global__ void __launch_bounds__(256, 2) k_sample_phase(SampleGrid G, const Sam
     if (ok) {
         const float r2 = __fmul_rn(G.min_dist, G.min_dist);
         const int rows = G.dim == 3 ? 25 : 5;
-#pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const int r = sub + q * kCellLanes;
+        // eight lanes: all neighbours in flight at once; one: row by row until a sample is too near
+#pragma unroll(LANES > 1 ? 4 : 1)
+        for (int q = 0; LANES > 1 ? q < 4 : q < rows && !clash; ++q) {
+            const int r = sub + q * LANES;
             const int jy = iy + r % 5 - 2, jz = G.dim == 3 ? iz + r / 5 - 2 : 0;
             const bool in = r < rows && jy >= 0 && jy < G.nc[1] && jz >= 0 && jz < G.nc[2];
             const long long row = ((long long)jz * G.nc[1] + jy) * G.nc[0];
@@ -135,8 +142,8 @@ __global__ void __launch_bounds__(256, 2) k_sample_phase(SampleGrid G, const Sam
         }
     }
     const unsigned any = __ballot_sync(0xffffffffu, clash);
-    const int first = (threadIdx.x & 31) / kCellLanes * kCellLanes;
-    if (ok && sub == 0 && ((any >> first) & ((1u << kCellLanes) - 1)) == 0u) cells[id] = make_float4(p[0], p[1], p[2], 1.f);
+    const int first = (threadIdx.x & 31) / LANES * LANES;
+    if (ok && sub == 0 && ((any >> first) & ((1u << LANES) - 1)) == 0u) cells[id] = make_float4(p[0], p[1], p[2], 1.f);
 }
 
 // Cells that can hold a sample: those overlapping a shape's bounding box.
@@ -305,10 +312,11 @@ mpm_status mpm_sample_shapes(int32_t dim, const mpm_shape* shapes, int32_t nshap
                 for (int px = 0; px < 3; ++px) {
                     const long long mx = (G.nc[0] - px + 2) / 3, my = (G.nc[1] - py + 2) / 3,
                                     mz = dim == 3 ? (G.nc[2] - pz + 2) / 3 : 1;
-                    const long long lanes = mx * my * mz * kCellLanes;
-                    if (lanes == 0 || le != cudaSuccess) continue;
-                    lc.gridDim = dim3((unsigned)((lanes + threads - 1) / threads));
-                    le = cudaLaunchKernelEx(&lc, k_sample_phase, G, (const SampleShapes*)dshapes,
+                    const long long phase = mx * my * mz;
+                    if (phase == 0 || le != cudaSuccess) continue;
+                    const int lanes = phase <= (dim == 3 ? kManyLanes3 : kManyLanes2) ? 8 : 1;
+                    lc.gridDim = dim3((unsigned)((phase * lanes + threads - 1) / threads));
+                    le = cudaLaunchKernelEx(&lc, lanes == 8 ? k_sample_phase<8> : k_sample_phase<1>, G, (const SampleShapes*)dshapes,
                                             (const unsigned char*)live, r, px, py, pz, cells);
                     lc.numAttrs = 1;
                 }

@@ -59,6 +59,7 @@ struct mpm_solver {
     float *x = nullptr, *v = nullptr, *B = nullptr, *Fe = nullptr, *Jp = nullptr, *A = nullptr;
     float *mass = nullptr, *vol = nullptr;
     float mass_u = 0.f, vol_u = 0.f;
+    double per_cell = 0.0;  // particles per cell of the snow's volume
     int* id = nullptr;
     // grid
     unsigned long long* acc = nullptr;
@@ -597,16 +598,18 @@ mpm_status setup_tiled(mpm_solver* s) {
     // Window length of the fused transfer by how the scene's windows compare with
     // the warps the GPU holds (5 CTAs of 4 per SM): a warp works through a window's
     // stencils one after the other, so a scene of few windows takes shorter ones.
-    // 3D scenes of more than three windows per warp (quadratic stencil: twelve) have
-    // their node boxes staged, an item being a tile, or 32 windows of one that holds
-    // more (k_g2p2g_pipe, which has the figures); the others and all 2D scenes take
-    // an item per window (k_g2p2g_direct).
+    // Scenes of many windows per warp whose tiles hold enough windows for a CTA have their
+    // node boxes staged, an item being a tile, or 32 windows of one that holds more
+    // (k_g2p2g_pipe); the others take an item per window (k_g2p2g_direct, which has the
+    // figures on both sides of these lines).
     {
         const long long warps = (long long)s->sms * (MPM_FUSED_MIN_BLOCKS) * FusedGeom<3>::WARPS;
         const long long w32 = (n + 31) / 32;
         ti.win = w32 <= warps / 4 ? 8 : (w32 <= warps / 2 ? 16 : 32);
         const long long windows = (n + ti.win - 1) / ti.win;
-        s->direct = D == 2 || windows <= (s->stencil == 3 ? 12 : 3) * warps;
+        const int per_warp = D == 2 ? 14 : (s->stencil == 3 ? 16 : 3);
+        const double per_cell = D == 2 ? 3.5 : (s->stencil == 3 ? 4.5 : 2.5);
+        s->direct = windows <= per_warp * warps || s->per_cell < per_cell;
         // MPM_BOX_LOAD=tma, =gather choose one of the two (for comparison)
         const char* bl = std::getenv("MPM_BOX_LOAD");
         if (bl && std::strcmp(bl, "tma") == 0) s->direct = false;
@@ -931,19 +934,21 @@ mpm_status mpm_create(const mpm_params* params, const mpm_particles_init* init, 
     // Host-side preparation: mass = vol * RHO / 100 when not given
     // (src/cpu/Particles.cpp:18, src/gpu/GPUSolver.cpp:119,148).
     std::vector<float> massv(n), volv(n);
-    double total_mass = 0.0;
+    double total_mass = 0.0, total_volume = 0.0;
     bool uni_m = true, uni_v = true;
     for (int i = 0; i < n; ++i) {
         volv[i] = init->volume[i];
         massv[i] = init->mass ? init->mass[i] : (init->volume[i] * params->rho) / 100.f;
         if (!std::isfinite(volv[i]) || !std::isfinite(massv[i])) return bail(MPM_ERR_INVALID_ARGUMENT);
         total_mass += massv[i];
+        total_volume += std::fabs(volv[i]);
         if (massv[i] != massv[0]) uni_m = false;
         if (volv[i] != volv[0]) uni_v = false;
     }
     for (long long i = 0; i < (long long)n * D; ++i)
         if (!std::isfinite(init->position[i]) || (init->velocity && !std::isfinite(init->velocity[i])))
             return bail(MPM_ERR_INVALID_ARGUMENT);
+    s->per_cell = total_volume > 0.0 ? n / total_volume : 0.0;
     choose_scales(s, total_mass);
     if (uni_m && n > 0) s->mass_u = massv[0];
     else if (n > 0) {

@@ -972,14 +972,18 @@ __device__ __forceinline__ unsigned fused_window(const Particles& P, const StepC
 
 // ---------------------------------------------------------------------------
 // The fused step without staged boxes: an item is one window, every warp takes
-// windows on its own and gathers from the global grid. All 2D scenes, and 3D scenes
-// of few windows per warp (the dispatch's rule). A staged box is worth its round trip
-// to L2 only where many windows read it and there are tiles enough for every CTA:
-//   2D, 627k particles:               44.5 us direct, 61.7 staged
-//   3D, 17.6k at 0.6 a cell:          17.5 and 23.0;   74k at 8 a cell: 25.7, 54.4
-//   3D, 187k at 8 a cell (2.0 windows a warp):  60.5 and 61.4
-//   3D, 380k (4.0): 102 and 93;       474k (5.0): 99 and 91
-//   quadratic, 673k (7.1): 104 and 112;  1.65M (17): 247 and 238
+// windows on its own and gathers from the global grid. A staged box is worth its round
+// trip to L2 only where many windows read it and there are tiles enough for every CTA
+// (the dispatch's rule: windows per warp of the GPU, particles per cell). Whole steps in
+// us, direct and staged:
+//   3D cubic, 8 a cell, windows per warp 2.0: 73, 70;  5.0: 125, 113;  17: 384, 309
+//     3 a cell, 3.7: 123, 124;  23: 639, 568;   2 a cell, 4.3: 159, 176;  72: 2080, 2250
+//     1 a cell, 5.0: 237, 328;  70: 2710, 4080;  0.6 a cell, 17.6k particles (fused kernel): 17.5, 23.0
+//   3D quadratic, 8 a cell, 9.8: 164, 165;  17: 273, 266;  60: 853, 784
+//     4 to 6 a cell, 13: 219, 234;  45: 694, 662;  73: 1251, 1252;   1 a cell, 18: 593, 1166
+//   2D, 4 to 8 a cell, windows per warp 7.8: 83, 84;  16: 182, 176;  34: 376, 350
+//     27 a cell, 6.6: 62, 69;  64 a cell, 16: 233, 228;  63: 764, 686
+//     2 a cell, 7.8: 128, 158;  31: 461, 574
 //
 // G2P = false: the P2G of the stored state only (after creation or a state upload),
 // reading B, F_E, J_p and forming A as every other path does (mls_affine), for items

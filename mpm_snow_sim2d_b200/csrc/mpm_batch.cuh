@@ -18,7 +18,7 @@
 // scene's grid in the shared memory of a thread-block cluster and added 48 int64
 // values per particle and step there (red.shared::cluster, 68% of their wavefronts
 // bank conflicts); one persistent cluster per scene left the GPU waiting for the
-// largest ones. 256 scenes, 2.81M particles, 100 steps: 0.83 ms a step, now 0.39.
+// largest ones. 256 scenes, 2.81M particles, 100 steps: 0.83 ms a step, now 0.34.
 #pragma once
 
 #include "mpm_fused.cuh"

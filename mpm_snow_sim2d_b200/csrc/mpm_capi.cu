@@ -448,7 +448,7 @@ template <int D, int S> cudaError_t fused_prologue(mpm_solver* s) {
 }
 
 template <int D> cudaError_t launch_grid_marked(mpm_solver* s) {
-    return launch_chained(k_grid_marked<D, kMLS>, s->sms * 8, 256, 0, s->stream, s->C, s->ti, s->acc, s->gv, s->status);
+    return launch_chained(s->fused ? k_grid_marked<D, kMLS, false> : k_grid_marked<D, kMLS, true>, s->sms * 8, 256, 0, s->stream, s->C, s->ti, s->acc, s->gv, s->status);
 }
 
 // One fused step: [sort] grid update, fused G2P + next P2G, queued particles.
@@ -1145,8 +1145,8 @@ mpm_status mpm_rasterize(mpm_solver* s, double* node_mass, double* node_momentum
     const double ism = std::ldexp(1.0, -s->log2_sm), isp = std::ldexp(1.0, -s->log2_sp),
                  isf = std::ldexp(1.0, -s->log2_sf);
     const long long N = s->nodes;
-    const bool classic = s->form == kClassic;
-    auto sum = [&](int c, long long i) { return classic ? h[c * N + i] : h[i * 4 + acc_channel(c)]; };
+    const bool classic = s->form == kClassic, planes = classic || !s->fused;
+    auto sum = [&](int c, long long i) { return planes ? h[c * N + i] : h[i * 4 + acc_channel(c)]; };
     for (long long i = 0; i < N; ++i) {
         if (node_mass) node_mass[i] = (double)sum(0, i) * ism;
         for (int k = 0; k < D && node_momentum; ++k) {

@@ -8,8 +8,9 @@
 //   mass/vol: per particle or a uniform scalar (pointer == nullptr)
 // Grid (nodes = (W+1)(H+1)(D+1), x fastest):
 //   acc  int64 fixed-point sums. MLS, QUAD: [nodes][4] = momentum x, momentum y,
-//        mass, momentum z (2D: unused), a node's sums in one 32-byte sector;
-//        CLASSIC: [channel][nodes] = mass, momentum[D], force[D]
+//        mass, momentum z (2D: unused), a node's sums in one 32-byte sector; on the
+//        split path, whose lanes add one channel of neighbouring nodes at a time,
+//        [channel][nodes] = mass, momentum[D]; CLASSIC: the same, and force[D]
 //   gv                node velocities for G2P: 2D float4 (vf.x, vf.y, vc.x, vc.y);
 //                     3D two float4 per node (vf.xyz, 0), (vc.xyz, 0)
 #pragma once
@@ -345,13 +346,14 @@ __device__ __forceinline__ void grid_node_velocity(const StepConsts& C, const lo
 // Grid update of one node of the global grid. Reads and clears the
 // fixed-point accumulators (the reference's separate reset pass,
 // reset.glsl:13-23, is fused here) and writes the velocities G2P gathers.
-template <int D, int FORM>
+// PLANES: the sums lie channel by channel.
+template <int D, int FORM, bool PLANES = FORM == kClassic>
 __device__ __forceinline__ void grid_node_at(const StepConsts& C, unsigned long long* __restrict__ acc,
                                              float4* __restrict__ gv, unsigned* __restrict__ status, long long id,
                                              int ix, int iy, int iz) {
     constexpr int NACC = Layout<D, FORM>::NACC;
     long long q[NACC];
-    if constexpr (FORM == kClassic) {
+    if constexpr (PLANES) {
 #pragma unroll
         for (int c = 0; c < NACC; ++c) {
             q[c] = (long long)acc[c * C.nodes + id];

@@ -405,7 +405,7 @@ __device__ __forceinline__ void grid_finish(const TileInfo& TI, int* step) {
 // ---------------------------------------------------------------------------
 // Grid update over the node blocks P2G marked (reads and clears the int64 sums;
 // leaves no block marked).
-template <int D, int FORM>
+template <int D, int FORM, bool PLANES>
 __global__ void __launch_bounds__(256) k_grid_marked(StepConsts C, TileInfo TI, unsigned long long* __restrict__ acc,
                                                      float4* __restrict__ gv, unsigned* __restrict__ status) {
     using G = TileGeom<D>;
@@ -422,7 +422,7 @@ __global__ void __launch_bounds__(256) k_grid_marked(StepConsts C, TileInfo TI, 
         const int gx = b[0] * G::T + l[0], gy = b[1] * G::T + l[1], gz = D == 3 ? b[2] * G::T + l[2] : 0;
         if (loc == 0) TI.mark[blk] = 0;
         if (gx >= C.nx || gy >= C.ny || gz >= C.nz) continue;
-        grid_node_at<D, FORM>(C, acc, gv, status, ((long long)gz * C.ny + gy) * C.nx + gx, gx, gy, gz);
+        grid_node_at<D, FORM, PLANES>(C, acc, gv, status, ((long long)gz * C.ny + gy) * C.nx + gx, gx, gy, gz);
     }
     grid_finish(TI, nullptr);
 }
@@ -723,11 +723,11 @@ __global__ void __launch_bounds__(kP2GWarps * 32, D == 3 ? MPM_P2G_MIN_BLOCKS : 
 #pragma unroll
                         for (int cc = 0; cc < S; ++cc) {
                             const int idx = bb * S + cc;
-                            unsigned long long* p0 = acc + (g0 + bb * sy + cc * sz) * 4;
-                            red_fixed(p0 + 2, am[idx], C.sm);
-                            red_fixed(p0, a0[idx], C.sp);
-                            red_fixed(p0 + 1, a1[idx], C.sp);
-                            red_fixed(p0 + 3, a2[idx], C.sp);
+                            unsigned long long* p0 = acc + (g0 + bb * sy + cc * sz);
+                            red_fixed(p0, am[idx], C.sm);
+                            red_fixed(p0 + C.nodes, a0[idx], C.sp);
+                            red_fixed(p0 + 2 * C.nodes, a1[idx], C.sp);
+                            red_fixed(p0 + 3 * C.nodes, a2[idx], C.sp);
                         }
                 } else {
                     bool outside = false;
@@ -736,11 +736,11 @@ __global__ void __launch_bounds__(kP2GWarps * 32, D == 3 ? MPM_P2G_MIN_BLOCKS : 
                             const int gy = cell[1] - 1 + by0 + bb, gz = cell[2] - 1 + cc;
                             if (gx < 0 || gx > C.W || gy < 0 || gy > C.H || gz < 0 || gz > C.Dp) { outside = true; continue; }
                             const int idx = bb * S + cc;
-                            unsigned long long* p0 = acc + (((long long)gz * C.ny + gy) * C.nx + gx) * 4;
-                            red_fixed(p0 + 2, am[idx], C.sm);
-                            red_fixed(p0, a0[idx], C.sp);
-                            red_fixed(p0 + 1, a1[idx], C.sp);
-                            red_fixed(p0 + 3, a2[idx], C.sp);
+                            unsigned long long* p0 = acc + (((long long)gz * C.ny + gy) * C.nx + gx);
+                            red_fixed(p0, am[idx], C.sm);
+                            red_fixed(p0 + C.nodes, a0[idx], C.sp);
+                            red_fixed(p0 + 2 * C.nodes, a1[idx], C.sp);
+                            red_fixed(p0 + 3 * C.nodes, a2[idx], C.sp);
                         }
                     if (outside) raise_flag(status, 4u);
                 }
@@ -802,10 +802,10 @@ __global__ void __launch_bounds__(kP2GWarps * 32, D == 3 ? MPM_P2G_MIN_BLOCKS : 
 #pragma unroll
                         for (int b = 0; b < S; ++b) {
                             const int idx = i * S + b;
-                            unsigned long long* p0 = acc + (g0 + i + (long long)b * C.nx) * 4;
-                            red_fixed(p0 + 2, am[idx], C.sm);
-                            red_fixed(p0, a0[idx], C.sp);
-                            red_fixed(p0 + 1, a1[idx], C.sp);
+                            unsigned long long* p0 = acc + (g0 + i + (long long)b * C.nx);
+                            red_fixed(p0, am[idx], C.sm);
+                            red_fixed(p0 + C.nodes, a0[idx], C.sp);
+                            red_fixed(p0 + 2 * C.nodes, a1[idx], C.sp);
                         }
                 } else {
                     bool outside = false;
@@ -814,10 +814,10 @@ __global__ void __launch_bounds__(kP2GWarps * 32, D == 3 ? MPM_P2G_MIN_BLOCKS : 
                             const int gx = gx0 + i, gy = cell[1] - 1 + b;
                             if (gx < 0 || gx > C.W || gy < 0 || gy > C.H) { outside = true; continue; }
                             const int idx = i * S + b;
-                            unsigned long long* p0 = acc + ((long long)gy * C.nx + gx) * 4;
-                            red_fixed(p0 + 2, am[idx], C.sm);
-                            red_fixed(p0, a0[idx], C.sp);
-                            red_fixed(p0 + 1, a1[idx], C.sp);
+                            unsigned long long* p0 = acc + ((long long)gy * C.nx + gx);
+                            red_fixed(p0, am[idx], C.sm);
+                            red_fixed(p0 + C.nodes, a0[idx], C.sp);
+                            red_fixed(p0 + 2 * C.nodes, a1[idx], C.sp);
                         }
                     if (outside) raise_flag(status, 4u);
                 }

@@ -1135,27 +1135,44 @@ mpm_status mpm_set_state(mpm_solver* s, const mpm_state_host* st) {
 mpm_status mpm_rasterize(mpm_solver* s, double* node_mass, double* node_momentum, int64_t* raw, size_t nodes) {
     if (!s) return MPM_ERR_INVALID_ARGUMENT;
     if (nodes != (size_t)s->nodes) return fail(s, MPM_ERR_CAPACITY, "nodes must equal the grid node count");
-    const int D = s->dim, NA = nacc(D, s->form);
+    const int D = s->dim;
+    const bool classic = s->form == kClassic;
+    const size_t sums = (size_t)(1 + D + (classic ? D : 0)) * s->nodes;  // with the forces
     cudaError_t e = dispatch_p2g(s);
     if (e != cudaSuccess) return cuda_fail(s, e, "p2g launch");
-    std::vector<long long> h((size_t)NA * s->nodes);
-    MPM_CUDA(s, cudaMemcpyAsync(h.data(), s->acc, sizeof(long long) * h.size(), cudaMemcpyDeviceToHost, s->stream));
+    std::vector<long long> h(sums);
+    if (s->tiled && s->fused) {
+        // channel by channel, some nodes at a time
+        constexpr long long kNodes = 4 << 20;
+        for (long long n0 = 0; n0 < s->nodes; n0 += kNodes) {
+            const long long m = std::min(kNodes, s->nodes - n0);
+            void* buf = nullptr;
+            const mpm_status st = scratch(s, sizeof(long long) * (size_t)((1 + D) * m), &buf);
+            if (st != MPM_OK) return st;
+            unsigned long long* planes = static_cast<unsigned long long*>(buf);
+            k_sum_planes<<<(unsigned)((m + 255) / 256), 256, 0, s->stream>>>(s->acc + n0 * 4, m, 1 + D, planes);
+            MPM_CUDA(s, cudaGetLastError());
+            for (int c = 0; c < 1 + D; ++c)
+                MPM_CUDA(s, cudaMemcpyAsync(h.data() + c * s->nodes + n0, planes + c * m, sizeof(long long) * (size_t)m,
+                                            cudaMemcpyDeviceToHost, s->stream));
+        }
+    } else {
+        MPM_CUDA(s, cudaMemcpyAsync(h.data(), s->acc, sizeof(long long) * h.size(), cudaMemcpyDeviceToHost, s->stream));
+    }
     if (!(s->tiled && s->fused)) MPM_CUDA(s, clear_after_p2g(s));  // fused: these are the next step's sums
     MPM_CUDA(s, cudaStreamSynchronize(s->stream));
     const double ism = std::ldexp(1.0, -s->log2_sm), isp = std::ldexp(1.0, -s->log2_sp),
                  isf = std::ldexp(1.0, -s->log2_sf);
     const long long N = s->nodes;
-    const bool classic = s->form == kClassic, planes = classic || !s->fused;
-    auto sum = [&](int c, long long i) { return planes ? h[c * N + i] : h[i * 4 + acc_channel(c)]; };
     for (long long i = 0; i < N; ++i) {
-        if (node_mass) node_mass[i] = (double)sum(0, i) * ism;
+        if (node_mass) node_mass[i] = (double)h[i] * ism;
         for (int k = 0; k < D && node_momentum; ++k) {
-            double p = (double)sum(1 + k, i) * isp;
+            double p = (double)h[(1 + k) * N + i] * isp;
             if (classic) p -= (double)s->params.delta_time * ((double)h[(1 + D + k) * N + i] * isf);
             node_momentum[i * D + k] = p;
         }
-        for (int c = 0; raw && c < 1 + D; ++c) raw[c * N + i] = sum(c, i);
     }
+    if (raw) std::memcpy(raw, h.data(), sizeof(long long) * (size_t)(1 + D) * N);
     return MPM_OK;
 }
 

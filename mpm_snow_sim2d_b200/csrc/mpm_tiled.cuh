@@ -431,6 +431,14 @@ __global__ void __launch_bounds__(256) k_grid_marked(StepConsts C, TileInfo TI, 
 // momentum x, momentum y, mass, momentum z (2D: unused).
 __host__ __device__ __forceinline__ int acc_channel(int c) { return c == 0 ? 2 : (c < 3 ? c - 1 : 3); }
 
+// The sums of `nodes` nodes channel by channel (mass, momentum).
+static __global__ void __launch_bounds__(256) k_sum_planes(const unsigned long long* __restrict__ acc, long long nodes, int nch,
+                                                           unsigned long long* __restrict__ out) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nodes) return;
+    for (int c = 0; c < nch; ++c) out[c * nodes + i] = acc[i * 4 + acc_channel(c)];
+}
+
 // The int64 sums of the marked node blocks to / from a packed array
 // [block][channel: mass, momentum][node of block] (checkpoints of the fused transfer, which
 // keep the next step's grid sums). Unpacking also marks the blocks.

@@ -26,8 +26,10 @@ def _solver(dim):
 def test_first_calls_allocate_nothing(gpu_lib, dim):
     with _solver(dim) as other:  # what the process makes once
         other.Step(1)
-        other.get_state()
+        other.GetParticlePositions()
+        st = other.get_state()
         other.render(width=64, height=64, point_size=1.0)
+        other.set_state(st.position, st.velocity, st.affine_b, st.elastic_f, st.plastic_det)
     with _solver(dim) as s:
         s.Step(1)
         free = _free()
@@ -46,6 +48,10 @@ def test_first_calls_of_a_batch_allocate_nothing(gpu_lib):
     n = 200000
     sc = sc.with_(position=(sc.width * rng.uniform(0.2, 0.8, (n, 2))).astype(np.float32), velocity=np.zeros((n, 2), np.float32),
                   volume=np.full(n, sc.volume[0] / 50, np.float32), mass=np.full(n, sc.mass[0] / 50, np.float32))
+    with Batch([scenes.batch_scene_2d(5)]) as other:
+        other.step(1)
+        st = other.get_state(0)
+        other.set_state(0, st.position, st.velocity)
     with Batch([sc]) as b:
         b.step(1)
         free = _free()
